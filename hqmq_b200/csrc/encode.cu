@@ -1946,9 +1946,10 @@ static MainGrid main_grid(int T_new, int B, int H) {
 // the sampled norms per head (a 1/32 sample of B * T_new tokens, 32 norms each), so the bracket's half-width is
 // 3 / sqrt(norms) (about six standard errors of a median), at least 0.2 % and at most 1.2 %; calls too small for that,
 // and quantiles out in the tails (few norms nearby: a much larger error), take the multi-pass path as before.
-// d_head 64 as pairs of tokens (see EncGeom::pair16): the call's geometry must allow it.
+// d_head 64 as pairs of tokens (see EncGeom::pair16): the call's geometry must allow it, and a token's row must be whole
+// words without padding (16-bit fields; rows of 13- and 19-bit fields are padded, so two of them are not one longer row).
 static bool pair16_of(const hqmq_encode_args& a) {
-  return a.dst.n_chunks == 16 && is_half_dtype(a.x_dtype) && a.x_stride[2] == 64 && a.T_new >= 2 && a.T_new % 2 == 0 &&
+  return a.dst.n_chunks == 16 && (16 * (idx_bits_for(a.dst.S) + a.dst.radius_bits)) % 32 == 0 && is_half_dtype(a.x_dtype) && a.x_stride[2] == 64 && a.T_new >= 2 && a.T_new % 2 == 0 &&
          a.t_start % 2 == 0;
 }
 constexpr int64_t kBracketMinTokens = 65536;     // B * T_new per head (of 32 chunks each)

@@ -482,3 +482,16 @@ def test_head_dim_64_single_read_pass(kind):
         x = make_kv(kind, (16, 2, 8192, 64), seed=52, dtype=torch.bfloat16).float()
     _threshold_compare(x.bfloat16().float(), 96, 4, 3.0)
     _threshold_compare(x.bfloat16().float()[:, :, :8190], 24, 3, 1.0, quantile=0.5)
+
+
+@pytest.mark.parametrize("S,br", [(24, 3), (192, 6)])
+@pytest.mark.parametrize("C", [None, 3.0])
+def test_d64_rows_with_padding_bits(S, br, C):
+    """d_head 64 with 13- or 19-bit fields: a row is padded to whole words, so the kernels that take two tokens of 64 as
+    one of 128 must not run (even token count, contiguous tokens, more than a small call)."""
+    x = make_kv("spiky", (2, 2, 336, 64), seed=71, dtype=torch.bfloat16)
+    q = hqmq.HQMQ(1, 2, S, br, device="cuda")
+    a = q.encode(x.cuda(), 0, 0, median_mult=C, scale_dtype=torch.float32).to_reference()
+    b = q.encode(x.float().cuda(), 0, 0, median_mult=C, scale_dtype=torch.float32).to_reference()
+    for got, want in zip(a, b):
+        assert got is None and want is None or torch.equal(got, want)
