@@ -5,6 +5,7 @@
 #include <mutex>
 
 #include "attn_kernel.cuh"
+#include "attn_prefill.cuh"
 
 namespace hqmq {
 namespace attn {
@@ -178,6 +179,26 @@ static int resident_ctas(const void* kernel, size_t smem, int threads) {
   return val;
 }
 
+cudaError_t raise_smem_limit(const void* kernel, size_t smem) {
+  struct Entry { const void* k; int dev; };
+  static Entry done[64];
+  static int n_done = 0;
+  static std::mutex mu;
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  for (int i = 0; i < n_done; ++i)
+    if (done[i].k == kernel && done[i].dev == dev) return cudaSuccess;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaFuncAttributes fa;
+  cudaError_t rc = cudaFuncGetAttributes(&fa, kernel);
+  if (rc != cudaSuccess) return rc;
+  const int most = optin - (int)fa.sharedSizeBytes;
+  rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most > (int)smem ? most : (int)smem);
+  if (rc == cudaSuccess && n_done < 64) done[n_done++] = {kernel, dev};
+  return rc;
+}
+
 // Units of at most this many tiles run the staged kernels in warp mode (every warp has at most two tiles of a unit)
 constexpr int kWarpModeMaxTiles = 32;
 
@@ -336,6 +357,8 @@ using namespace hqmq::attn;
 
 extern "C" size_t hqmq_attn_workspace_bytes(const hqmq_attn_args* a) {
   if (validate_attn(a) != HQMQ_OK) return 0;
+  PrefillPlan pp;
+  if (prefill_plan(a, pp)) return pp.ws_bytes;
   Plan pl;
   if (make_plan(a, pl, true) != HQMQ_OK) return 0;
   return pl.ws_bytes;
@@ -354,9 +377,19 @@ extern "C" int hqmq_combine_partials(const float* parts, int n_parts, int64_t ro
   return HQMQ_OK;
 }
 
+static std::atomic<uint32_t> epoch_counter{0x5eed0000u};
+
 extern "C" int hqmq_attn_decode(const hqmq_attn_args* a, void* workspace, size_t workspace_bytes, void* stream) {
   int rc = validate_attn(a);
   if (rc) return rc;
+  // many query positions: tensor cores over a cache decoded once (a scratch too small for that takes the path below)
+  PrefillPlan pp;
+  if (prefill_plan(a, pp) && workspace && workspace_bytes >= pp.ws_bytes) {
+    if ((uintptr_t)workspace & 15) return HQMQ_ERR_ALIGN;
+    const float scale = a->softmax_scale > 0.f ? a->softmax_scale : 1.0f / sqrtf((float)a->d);
+    return prefill_launch(a, pp, workspace, scale * 1.4426950408889634f,
+                          epoch_counter.fetch_add(1u, std::memory_order_relaxed) + 1u, (cudaStream_t)stream);
+  }
   Plan pl;
   rc = make_plan(a, pl, true);
   if (rc) return rc;
@@ -384,7 +417,6 @@ extern "C" int hqmq_attn_decode(const hqmq_attn_args* a, void* workspace, size_t
   p.qmaxf = (float)a->r_qmax;
   p.units = pl.units; p.tpu_v = pl.tpu_v; p.L = pl.L; p.P = pl.P;
   p.Q = a->Q; p.q_dtype = a->q_dtype; p.qs_b = a->q_stride[0]; p.qs_h = a->q_stride[1]; p.qs_t = a->q_stride[2];
-  static std::atomic<uint32_t> epoch_counter{0x5eed0000u};
   p.status = reinterpret_cast<uint32_t*>(workspace);
   p.epoch = epoch_counter.fetch_add(1u, std::memory_order_relaxed) + 1u;
   p.tickets = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(workspace) + 16);

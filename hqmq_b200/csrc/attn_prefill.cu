@@ -1,0 +1,764 @@
+// Attention of many query positions over one compressed cache (a prompt, or a chunk of one): tensor cores, tcgen05.
+//
+// The decode kernels make every query position a unit of its own and decode K and V once per unit: right for one
+// token, 2048 times the decoding for a 2048-token prompt chunk.  Here the cache is decoded ONCE per call into operand
+// tiles, and the attention runs on the tensor cores over those:
+//
+//   expand   (prefill_expand_kernel) per (b, KV head) and 128-token tile: K as a K-major and V^T as a K-major fp16 operand
+//            image in the 128-byte swizzle that tcgen05.mma reads, so that a tile is one contiguous bulk copy later.
+//            A value is codeword * (rq * rs / qmax * 2^(10-e)), e the exponent of the largest scale of the (b, head), outliers
+//            are x * 2^(10-e): everything lies below 2^10 and keeps its 11 bits down to 2^-24 of the largest token.
+//   attend   (prefill_attn_kernel) persistent, one CTA per SM.  A unit is (b, KV head, up to 2 x 128 rows), a row one
+//            (query position, head of the group): all heads of a group share the decoded tile.  Two row blocks ("streams")
+//            alternate on the tensor cores: while the softmax warps of one stream work on S = Q K^T, the other stream's
+//            P V and its next Q K^T run.  Warps 0-3 / 4-7: softmax of stream 0 / 1 (a thread owns a row: S comes out of
+//            TMEM, P goes back as fp16 into the same columns, the accumulator is rescaled only when a row's maximum rises by
+//            more than 2^8); warp 8 issues the MMAs; warp 9 streams the tiles in through two-deep (four at d_head 64) rings.
+//            The tiles of all units form one flat sequence cut into equal pieces, one per CTA, whatever the mask leaves of
+//            each unit; a unit that is cut leaves partials, merged by prefill_merge_kernel.
+//
+// Bound: per 256 rows x 128 keys, 2048 tensor clocks and as many of the exponential unit; the rest has to hide behind them.
+#include "attn_prefill.cuh"
+#include "attn_ring.cuh"
+
+namespace hqmq {
+namespace attn {
+namespace {
+
+constexpr int kPfThreads = 384;             // 2 x 4 softmax warps; MMA warp, loader warp and two idle ones (register shares are per 4 warps)
+// registers per thread: the launch gives 384 x 168; the third warpgroup hands its share to the softmax warps (128 values of
+// a row each): 256 x 208 + 128 x 80 <= 384 x 168
+constexpr int kPfSoftmaxRegs = 208, kPfOtherRegs = 80;
+static_assert(256 * kPfSoftmaxRegs + 128 * kPfOtherRegs <= kPfThreads * 168, "register split beyond the launch's share");
+constexpr float kPfSlack = 8.f;             // log2 units a row's maximum may rise before its accumulator is rescaled
+constexpr uint32_t kPfTmemCols = 512;
+
+__host__ __device__ constexpr int pf_stages(int d) { return d == 128 ? 2 : 4; }
+__host__ __device__ constexpr size_t pf_tile_bytes(int d) { return (size_t)d * 256; }
+__host__ __device__ constexpr size_t pf_smem_bytes(int d) { return (size_t)(2 + 2 * pf_stages(d)) * pf_tile_bytes(d) + 1024 + 256; }
+
+// ---- work decomposition -------------------------------------------------------------------------------------------
+// KV tiles [lo, lo + n) that the rows of unit m see (at least one, so that a fully masked unit still writes its zeros).
+__host__ __device__ inline void pf_unit_tiles(const PrefillParams& p, int m, int& lo, int& n) {
+  const int pos0 = m * p.streams * p.P;
+  int pos1 = pos0 + p.streams * p.P - 1;
+  if (pos1 >= p.Tq) pos1 = p.Tq - 1;
+  int beg, end, beg1, end1;
+  key_range(p.Tkv, p.Tq, p.causal, p.window, pos0, beg, end);
+  key_range(p.Tkv, p.Tq, p.causal, p.window, pos1, beg1, end1);
+  lo = beg / kPfTok;
+  const int hi = (end1 + kPfTok - 1) / kPfTok, last = (p.Tkv - 1) / kPfTok;
+  if (lo > last) lo = last;
+  n = hi > lo ? hi - lo : 1;
+}
+
+struct PfPiece { int bh, m, tile0, n; bool head, tail; };
+// The pieces of one CTA: its stretch [c * L, (c + 1) * L) of the flat tile sequence, unit by unit.
+struct PfIter {
+  int left;
+  int bh, m, off, lo, n;
+  __device__ __forceinline__ void init(const PrefillParams& p, int64_t pos) {
+    left = (int)(p.total - pos < p.L ? p.total - pos : p.L);
+    bh = (int)(pos / p.Wh);
+    int rem = (int)(pos - (int64_t)bh * p.Wh);
+    m = 0;
+    pf_unit_tiles(p, m, lo, n);
+    while (rem >= n) { rem -= n; ++m; pf_unit_tiles(p, m, lo, n); }
+    off = rem;
+  }
+  __device__ __forceinline__ bool next(const PrefillParams& p, PfPiece& q) {
+    if (left <= 0) return false;
+    if (off >= n) {
+      off = 0;
+      if (++m == p.units_m) { m = 0; ++bh; }
+      pf_unit_tiles(p, m, lo, n);
+    }
+    q.bh = bh; q.m = m; q.tile0 = lo + off;
+    q.n = n - off < left ? n - off : left;
+    q.head = off == 0; q.tail = off + q.n == n;
+    left -= q.n; off += q.n;
+    return true;
+  }
+};
+
+// ---- tcgen05 ---------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tc_mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool acc) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+               ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)acc) : "memory");
+}
+__device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool acc) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"((uint32_t)acc) : "memory");
+}
+#define PF_R8(r, o) "=r"((r)[o]), "=r"((r)[o + 1]), "=r"((r)[o + 2]), "=r"((r)[o + 3]), "=r"((r)[o + 4]), "=r"((r)[o + 5]), \
+                    "=r"((r)[o + 6]), "=r"((r)[o + 7])
+#define PF_I8(r, o) "r"((r)[o]), "r"((r)[o + 1]), "r"((r)[o + 2]), "r"((r)[o + 3]), "r"((r)[o + 4]), "r"((r)[o + 5]), \
+                    "r"((r)[o + 6]), "r"((r)[o + 7])
+__device__ __forceinline__ void tc_ld32(uint32_t* r, uint32_t addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,"
+      "%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : PF_R8(r, 0), PF_R8(r, 8), PF_R8(r, 16), PF_R8(r, 24) : "r"(addr));
+}
+__device__ __forceinline__ void tc_st32(uint32_t addr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,"
+      "%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(addr), PF_I8(r, 0), PF_I8(r, 8), PF_I8(r, 16), PF_I8(r, 24) : "memory");
+}
+__device__ __forceinline__ void tc_st16(uint32_t addr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(addr), PF_I8(r, 0), PF_I8(r, 8) : "memory");
+}
+__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// K-major operand in the 128-byte swizzle: rows of 128 bytes, groups of eight rows 1024 bytes apart.
+__device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
+  return (uint64_t)((addr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
+         ((uint64_t)2 << 61);
+}
+// kind::f16, fp16 operands (both K-major), fp32 accumulators
+__device__ __forceinline__ uint32_t f16_idesc(int M, int N) { return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24); }
+
+// ---- attend ----------------------------------------------------------------------------------------------------------------
+template <int D>
+__global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const PrefillParams p) {
+  constexpr int NS = pf_stages(D);
+  constexpr uint32_t TB = (uint32_t)pf_tile_bytes(D);
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t s_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  unsigned char* base = smem_raw + (s_base - smem_u32(smem_raw));
+  const uint32_t sQ = s_base, sK = sQ + 2 * TB, sV = sK + NS * TB, bars = sV + NS * TB;
+  const uint32_t kfull = bars, kempty = kfull + 8 * NS, vfull = kempty + 8 * NS, vempty = vfull + 8 * NS;
+  const uint32_t qfull = vempty + 8 * NS, sfull = qfull + 16, pfull = sfull + 16, odone = pfull + 16;
+  volatile uint32_t* abort_word = reinterpret_cast<volatile uint32_t*>(base + (odone + 16 - s_base));
+  volatile uint32_t* tmem_word = abort_word + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < NS; ++i) {
+      mbar_init(kfull + 8 * i, 1); mbar_init(kempty + 8 * i, 1); mbar_init(vfull + 8 * i, 1); mbar_init(vempty + 8 * i, 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(qfull + 8 * s, 4); mbar_init(sfull + 8 * s, 1); mbar_init(pfull + 8 * s, 4); mbar_init(odone + 8 * s, 1);
+    }
+    *abort_word = 0u;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 8) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(odone + 20), "n"(kPfTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_word;
+  // (a wait that runs out raises the abort word: every role then stops at its next wait)
+  auto wait = [&](uint32_t bar, uint32_t parity) {
+    if (ring_wait(bar, parity, abort_word)) return true;
+    *abort_word = 1u;
+    return false;
+  };
+  if (warp >= 8) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPfOtherRegs));
+  if (warp == 9) {
+    // ================================ loader =====================================================================
+    if (lane == 0) {
+      PfIter it;
+      PfPiece q;
+      it.init(p, (int64_t)blockIdx.x * p.L);
+      uint32_t g = 0;          // tiles issued
+      bool ok = true;
+      while (ok && it.next(p, q)) {
+        const unsigned char* kp = p.kimg + ((int64_t)q.bh * p.nt + (q.tile0 - p.kt0)) * TB;
+        const unsigned char* vp = p.vimg + ((int64_t)q.bh * p.nt + (q.tile0 - p.kt0)) * TB;
+        for (int i = 0; i < q.n; ++i, ++g) {
+          const uint32_t st = g % NS, ph = (g / NS) & 1u;
+          if (g >= NS && !wait(kempty + 8 * st, ph ^ 1u)) { ok = false; break; }
+          mbar_expect_tx(kfull + 8 * st, TB);
+          bulk_g2s(sK + st * TB, kp + (int64_t)i * TB, TB, kfull + 8 * st);
+          if (g >= NS && !wait(vempty + 8 * st, ph ^ 1u)) {
+            ok = false;
+            uint32_t spins = 0;      // the K copy just issued must have landed before the CTA leaves
+            while (!mbar_try_wait(kfull + 8 * st, ph) && ++spins < kWaitLimit) {}
+            break;
+          }
+          mbar_expect_tx(vfull + 8 * st, TB);
+          bulk_g2s(sV + st * TB, vp + (int64_t)i * TB, TB, vfull + 8 * st);
+        }
+      }
+      // no copy may be in flight when the CTA exits (bounded)
+      for (uint32_t k = 1; k <= (g < NS ? g : NS); ++k) {
+        const uint32_t st = (g - k) % NS, ph = ((g - k) / NS) & 1u;
+        uint32_t spins = 0;
+        while (!mbar_try_wait(kfull + 8 * st, ph) && ++spins < kWaitLimit) {}
+        while (!mbar_try_wait(vfull + 8 * st, ph) && ++spins < kWaitLimit) {}
+      }
+    }
+  } else if (warp == 8) {
+    // ================================ MMA issuer =================================================================
+    if (lane == 0) {
+      PfIter it;
+      PfPiece q;
+      it.init(p, (int64_t)blockIdx.x * p.L);
+      const uint32_t id_qk = f16_idesc(128, 128), id_pv = f16_idesc(128, D);
+      auto qk = [&](int s, uint32_t st) {
+        const uint64_t a0 = sw128_desc(sQ + s * TB), b0 = sw128_desc(sK + st * TB);
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+          const uint32_t o = ((k >> 2) * 16384 + (k & 3) * 32) >> 4;
+          tc_mma_ss(tmem + 128 * s, a0 + o, b0 + o, id_qk, k > 0);
+        }
+      };
+      auto pv = [&](int s, uint32_t st, bool acc) {
+        const uint64_t b0 = sw128_desc(sV + st * TB);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          tc_mma_ts(tmem + 256 + D * s, tmem + 128 * s + 8 * k, b0 + (((k >> 2) * D * 128 + (k & 3) * 32) >> 4), id_pv, acc || k > 0);
+      };
+      uint32_t g = 0, u = 0;     // tiles whose P V is issued, units whose queries arrived
+      bool have = it.next(p, q), ok = true;
+      if (have) {
+        for (int s = 0; s < p.streams && ok; ++s) {
+          if (s == 0) ok = wait(kfull, 0);
+          if (ok) ok = wait(qfull + 8 * s, 0);
+          if (!ok) break;
+          tc_fence_after();
+          qk(s, 0);
+          tc_commit(sfull + 8 * s);
+        }
+        if (ok) tc_commit(kempty);
+      }
+      while (ok && have) {
+        PfPiece nq;
+        const bool more = it.next(p, nq);
+        for (int i = 0; i < q.n && ok; ++i, ++g) {
+          const bool last = i + 1 == q.n;
+          const bool nxt = !last || more;
+          const uint32_t st = g % NS, ph = (g / NS) & 1u, st1 = (g + 1) % NS, ph1 = ((g + 1) / NS) & 1u;
+          for (int s = 0; s < p.streams; ++s) {
+            if (s == 0 && !(ok = wait(vfull + 8 * st, ph))) break;
+            if (!(ok = wait(pfull + 8 * s, g & 1u))) break;
+            tc_fence_after();
+            pv(s, st, i > 0);
+            if (last) tc_commit(odone + 8 * s);
+            if (s == p.streams - 1) tc_commit(vempty + 8 * st);
+            if (nxt) {
+              if (s == 0 && !(ok = wait(kfull + 8 * st1, ph1))) break;
+              if (last && !(ok = wait(qfull + 8 * s, (u + 1) & 1u))) break;
+              tc_fence_after();
+              qk(s, st1);
+              tc_commit(sfull + 8 * s);
+              if (s == p.streams - 1) tc_commit(kempty + 8 * st1);
+            }
+          }
+        }
+        q = nq; have = more; ++u;
+      }
+      // the last commits must have arrived before the CTA's shared memory goes away
+      if (ok && g > 0) {
+        const uint32_t st = (g - 1) % NS, ph = ((g - 1) / NS) & 1u;
+        if (wait(vempty + 8 * st, ph)) wait(kempty + 8 * st, ph);
+      }
+    }
+  }
+  } else {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPfSoftmaxRegs));
+  if ((warp >> 2) < p.streams) {
+    // ================================ softmax: one thread per row ===================================================
+    const int s = warp >> 2, row = threadIdx.x & 127;
+    const int pl = row / p.G, gh = row - pl * p.G;
+    const uint32_t lane_sel = (uint32_t)(warp & 3) << 21;               // TMEM lane 32 * (warp & 3), bits 31:16 of an address
+    const uint32_t tS = tmem + 128 * s + lane_sel, tO = tmem + 256 + D * s + lane_sel;
+    const uint32_t q_row = sQ + s * TB + row * 128;
+    auto load_q = [&](const PfPiece& w) {
+      const int bh = p.bh0 + w.bh, b = bh / p.Hkv, h = bh - b * p.Hkv;
+      const int tq = (w.m * p.streams + s) * p.P + pl;
+      const bool live = pl < p.P && tq < p.Tq;
+      const int64_t o = (int64_t)b * p.qs_b + (int64_t)(h * p.G + gh) * p.qs_h + (int64_t)tq * p.qs_t;
+#pragma unroll
+      for (int c = 0; c < D / 8; ++c) {        // 16-byte pieces of the row in fp16
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (live) {
+          if (p.q_vec) {
+            v = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.Q) + o + 8 * c);
+            if (p.q_dtype == HQMQ_BF16) {
+              uint32_t* w4 = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) w4[e] = pack_half2(__uint_as_float(w4[e] << 16), __uint_as_float(w4[e] & 0xffff0000u));
+            }
+          } else {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = load_float(p.Q, o + 8 * c + e, p.q_dtype);
+            v = make_uint4(pack_half2(f[0], f[1]), pack_half2(f[2], f[3]), pack_half2(f[4], f[5]), pack_half2(f[6], f[7]));
+          }
+        }
+        const uint32_t dst = q_row + (c >> 3) * 16384 + (((c & 7) ^ (row & 7)) << 4);
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // the MMA reads it through the async proxy
+      __syncwarp();
+      if (lane == 0) mbar_arrive(qfull + 8 * s);
+    };
+    PfIter it;
+    PfPiece q;
+    it.init(p, (int64_t)blockIdx.x * p.L);
+    uint32_t g = 0, u = 0;
+    bool have = it.next(p, q), ok = true;
+    if (have) load_q(q);
+    while (ok && have) {
+      PfPiece nq;
+      const bool more = it.next(p, nq);
+      const int bh = p.bh0 + q.bh;
+      const int tq = (q.m * p.streams + s) * p.P + pl;
+      const bool live = pl < p.P && tq < p.Tq;
+      // this row's keys; a row without a query is computed unmasked (its queries are zero) and not written
+      int beg = 0, end = 0x7fffffff;
+      if (live) key_range(p.Tkv, p.Tq, p.causal, p.window, tq, beg, end);
+      const int w_beg = __reduce_max_sync(0xffffffffu, beg), w_end = __reduce_min_sync(0xffffffffu, end);
+      const bool w_live = __any_sync(0xffffffffu, live);
+      const float kmul = p.kmul[bh];
+      float m_run = -INFINITY, l0 = 0.f, l1 = 0.f;
+      for (int i = 0; i < q.n; ++i, ++g) {
+        ok = wait(sfull + 8 * s, g & 1u);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        if (w_live) {
+          uint32_t r[128];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tc_ld32(r + 32 * c, tS + 32 * c);
+          tc_wait_ld();
+          const int t0 = (q.tile0 + i) * kPfTok;
+          if (t0 < w_beg || t0 + kPfTok > w_end) {
+            const int lo = beg - t0, hi = end - t0;
+#pragma unroll
+            for (int c = 0; c < 128; ++c)
+              if (c < lo || c >= hi) r[c] = 0xff800000u;
+          }
+          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+          for (int c = 0; c < 128; c += 8)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(r[c + 2 * e]), __uint_as_float(r[c + 2 * e + 1])));
+          const float mc = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * kmul;
+          if (__any_sync(0xffffffffu, mc > m_run + kPfSlack)) {
+            const float m_new = fmaxf(m_run, mc);
+            const float alpha = m_new == -INFINITY ? 1.f : fast_exp2(m_run - m_new);
+            m_run = m_new;
+            l0 *= alpha; l1 *= alpha;
+            if (i > 0) {
+              // (S of this tile was issued behind the previous tile's P V: the accumulator is complete)
+#pragma unroll 1
+              for (int c = 0; c < D; c += 32) {
+                uint32_t o[32];
+                tc_ld32(o, tO + c);
+                tc_wait_ld();
+#pragma unroll
+                for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+                tc_st32(tO + c, o);
+              }
+            }
+          }
+          const float nb = m_run == -INFINITY ? 0.f : -m_run;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              const float a = fast_exp2(fmaf(__uint_as_float(r[32 * c + 2 * e]), kmul, nb));
+              const float b = fast_exp2(fmaf(__uint_as_float(r[32 * c + 2 * e + 1]), kmul, nb));
+              const __half2 h = __floats2half2_rn(a, b);
+              // (the weights that are summed are the rounded ones the tensor cores see: the rounding cancels)
+              const float2 f = __half22float2(h);
+              l0 += f.x; l1 += f.y;
+              pk[e] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            tc_st16(tS + 16 * c, pk);
+          }
+          tc_wait_st();
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(pfull + 8 * s);
+      }
+      if (!ok) break;
+      // the last Q K^T of the unit is complete: the next unit's queries may take the place of this one's
+      if (more) load_q(nq);
+      ok = wait(odone + 8 * s, u & 1u);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      if (w_live) {
+        const int b = bh / p.Hkv, h = bh - b * p.Hkv;
+        const float l = l0 + l1, vmul = p.vmul[bh];
+        const bool whole = q.head && q.tail;
+        const float mul = whole ? (l > 0.f ? vmul / l : 0.f) : vmul;
+        float* part = p.part + (((int64_t)blockIdx.x * 2 + (q.head ? 1 : 0)) * 256 + s * 128 + row) * (D + 2);
+        const int64_t oo = (int64_t)b * p.os_b + (int64_t)(h * p.G + gh) * p.os_h + (int64_t)tq * p.os_t;
+#pragma unroll 1
+        for (int c = 0; c < D; c += 32) {
+          uint32_t o[32];
+          __syncwarp();
+          tc_ld32(o, tO + c);
+          tc_wait_ld();
+          if (!live) continue;
+          if (!whole) {
+#pragma unroll
+            for (int e = 0; e < 32; e += 2)
+              *reinterpret_cast<float2*>(part + c + e) = make_float2(__uint_as_float(o[e]) * mul, __uint_as_float(o[e + 1]) * mul);
+          } else if (p.o_vec) {
+            uint16_t* op = reinterpret_cast<uint16_t*>(p.O) + oo + c;
+#pragma unroll
+            for (int e = 0; e < 32; e += 8) {
+              uint32_t w[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float f0 = __uint_as_float(o[e + 2 * k]) * mul, f1 = __uint_as_float(o[e + 2 * k + 1]) * mul;
+                w[k] = (uint32_t)float_to_bits16(f0, p.o_dtype) | ((uint32_t)float_to_bits16(f1, p.o_dtype) << 16);
+              }
+              *reinterpret_cast<uint4*>(op + e) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) store_float(p.O, oo + c + e, __uint_as_float(o[e]) * mul, p.o_dtype);
+          }
+        }
+        if (!whole && live) *reinterpret_cast<float2*>(part + D) = make_float2(m_run, l);
+        __syncwarp();
+        tc_fence_before();
+      }
+      q = nq; have = more; ++u;
+    }
+  }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_word) *p.status = p.epoch;
+  if (warp == 8) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kPfTmemCols) : "memory");
+  }
+}
+
+// ---- merge of the units that were cut between CTAs: blockIdx.x + 1 = a CTA whose piece starts inside a unit ----------------
+template <int D>
+__global__ void __launch_bounds__(256) prefill_merge_kernel(const PrefillParams p) {
+  const int c = blockIdx.x + 1;
+  const int64_t pos = (int64_t)c * p.L;
+  PfIter it;
+  it.init(p, pos);
+  if (it.off == 0) return;                                  // the unit starts with the CTA
+  const int64_t s_u = pos - it.off;
+  if ((int64_t)(c - 1) * p.L > s_u) return;                 // the unit's first boundary does the merge
+  const int c0 = c - 1, n_parts = (int)((s_u + it.n - 1) / p.L) - c0 + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int bh = p.bh0 + it.bh, b = bh / p.Hkv, h = bh - b * p.Hkv;
+  const bool failed = *p.status == p.epoch;                 // the attention kernel gave up on a wait
+  constexpr int E = D / 32;
+  for (int row = blockIdx.y * 32 + warp; row < (blockIdx.y + 1) * 32; row += 8) {
+    const int s = row >> 7, rl = row & 127, pl = rl / p.G, gh = rl - pl * p.G;
+    const int tq = (it.m * p.streams + s) * p.P + pl;
+    if (s >= p.streams || pl >= p.P || tq >= p.Tq) continue;
+    // the CTA that holds the unit's first tile wrote its second slot, the others their first
+    const float* part = p.part + ((int64_t)c0 * 2 * 256 + row) * (D + 2);
+    constexpr int64_t kCta = (int64_t)2 * 256 * (D + 2);
+    float m = -INFINITY;
+    for (int k = lane; k < n_parts; k += 32) m = fmaxf(m, part[k * kCta + (k == 0 ? 256 * (D + 2) : 0) + D]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float mu = m == -INFINITY ? 0.f : m;
+    float l = 0.f, acc[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) acc[e] = 0.f;
+    for (int k = 0; k < n_parts; ++k) {
+      const float* pp = part + k * kCta + (k == 0 ? 256 * (D + 2) : 0);
+      const float w = fast_exp2(pp[D] - mu);
+      l = fmaf(pp[D + 1], w, l);
+#pragma unroll
+      for (int e = 0; e < E; e += 2) {
+        const float2 v = *reinterpret_cast<const float2*>(pp + lane * E + e);
+        acc[e] = fmaf(v.x, w, acc[e]); acc[e + 1] = fmaf(v.y, w, acc[e + 1]);
+      }
+    }
+    const float inv = failed ? NAN : l > 0.f ? 1.f / l : 0.f;
+    const int64_t oo = (int64_t)b * p.os_b + (int64_t)(h * p.G + gh) * p.os_h + (int64_t)tq * p.os_t + lane * E;
+#pragma unroll
+    for (int e = 0; e < E; ++e) store_float(p.O, oo + e, acc[e] * inv, p.o_dtype);
+  }
+}
+
+// ---- expand -------------------------------------------------------------------------------------------------------------------
+// 2^(10 - e) and 2^(e - 10) for the largest scale of a (b, head), e its exponent (largest < 2^e)
+__device__ __forceinline__ void pf_scale_of(float big, float& mul, float& inv) {
+  int e = big > 0.f ? (int)((__float_as_uint(big) >> 23) & 255u) - 126 : 10;
+  e = min(120, max(-110, e));
+  mul = __uint_as_float((uint32_t)(10 - e + 127) << 23);
+  inv = __uint_as_float((uint32_t)(e - 10 + 127) << 23);
+}
+
+// grid (tile chunks, (b, head) of the group, 2): blockIdx.z = 0 K, 1 V.  Eight warps; a warp takes the 16 tokens of one
+// outlier block of the tile with a lane per chunk (rows and flag words are read in order, so a flagged chunk's payload entry
+// is a running count).  K goes straight to its image (the lanes of a token fill whole 128-byte rows); V is unpacked to
+// shared memory first and decoded with a lane per token, so that the transposed image is written 64 bytes at a time.
+template <int N, int LAYOUT>
+__global__ void __launch_bounds__(256) prefill_expand_kernel(const ExpandParams e) {
+  constexpr int D = 4 * N;
+  constexpr uint32_t TB = (uint32_t)pf_tile_bytes(D);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint4* img = reinterpret_cast<uint4*>(smem_raw);                                       // V only: the tile's image
+  uint32_t* fields = reinterpret_cast<uint32_t*>(smem_raw + (blockIdx.z ? TB : 0));         // V only: [128][N + 1]
+  uint2* tbl = reinterpret_cast<uint2*>(smem_raw + (blockIdx.z ? TB + 128 * (N + 1) * 4 : 0));
+  __shared__ float s_big[8], s_fac[kPfTok];
+  const bool is_v = blockIdx.z != 0;
+  const hqmq_packed& pk = is_v ? e.V : e.K;
+  const hqmq_ref_packed& rf = is_v ? e.Vr : e.Kr;
+  const int bh = e.bh0 + blockIdx.y, b = bh / e.Hkv, h = bh - b * e.Hkv;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  // ---- the head's table, the largest scale of the keys in range ------------------------------------------------------
+  if (LAYOUT == 0) {
+    const uint2* src = reinterpret_cast<const uint2*>(is_v ? e.tblV : e.tblK) + (int64_t)h * e.table_rows;
+    for (int i = threadIdx.x; i < e.table_rows; i += 256) tbl[i] = src[i];
+  } else {
+    const void* j = is_v ? e.jV : e.jK;
+    for (int i = threadIdx.x; i < e.table_rows; i += 256) {
+      const int64_t o = ((int64_t)h * e.table_rows + i) * 4;
+      tbl[i] = make_uint2(pack_half2(load_float(j, o, e.j_dtype), load_float(j, o + 1, e.j_dtype)),
+                          pack_half2(load_float(j, o + 2, e.j_dtype), load_float(j, o + 3, e.j_dtype)));
+    }
+  }
+  const int t_first = e.kt0 * kPfTok, t_end = min(e.Tkv, (e.kt0 + e.nt) * kPfTok);
+  auto scale_of = [&](int t) {
+    return LAYOUT == 0 ? load_scale(pk, (int64_t)bh * pk.T_cap + t)
+                       : load_float(rf.rs, b * rf.rs_stride[0] + h * rf.rs_stride[1] + t, rf.rs_dtype);
+  };
+  float big = 0.f;
+  if (LAYOUT == 0 && pk.scale_dtype != HQMQ_F32) {
+    // eight 16-bit scales per load (they are positive: their bits order like their values)
+    const uint16_t* rs = reinterpret_cast<const uint16_t*>(pk.rs) + (int64_t)bh * pk.T_cap;
+    uint32_t mx = 0u;
+    for (int t = t_first + threadIdx.x * 8; t + 8 <= t_end; t += 256 * 8) {
+      const uint4 v = *reinterpret_cast<const uint4*>(rs + t);
+      mx = __vmaxu2(mx, __vmaxu2(__vmaxu2(v.x, v.y), __vmaxu2(v.z, v.w)));
+    }
+    big = fmaxf(bits16_to_float(mx & 0xffff, pk.scale_dtype), bits16_to_float(mx >> 16, pk.scale_dtype));
+    const int t = (t_end & ~7) + (int)threadIdx.x;
+    if (t < t_end) big = fmaxf(big, scale_of(t));
+  } else {
+    for (int t = t_first + threadIdx.x; t < t_end; t += 256) big = fmaxf(big, fabsf(scale_of(t)));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+  if (lane == 0) s_big[warp] = big;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) big = fmaxf(big, s_big[w]);
+  float mul, inv;
+  pf_scale_of(big, mul, inv);
+  if (blockIdx.x == 0 && threadIdx.x == 0) (is_v ? e.vmul : e.kmul)[bh] = is_v ? inv : inv * e.qscale;
+
+  const bool outl = LAYOUT == 0 && pk.flags != nullptr;
+  const int cb = e.ib + pk.radius_bits;
+  const unsigned char* vals = reinterpret_cast<const unsigned char*>(pk.out_vals) + (int64_t)bh * pk.out_cap * 4 * (pk.out_dtype == HQMQ_F32 ? 4 : 2);
+  // four fp16 values of a chunk: an outlier's payload entry (bit 31 set), or codeword and radius code
+  auto value_of = [&](uint32_t f, float fac) {
+    float x0, x1, x2, x3;
+    if (outl && (f >> 31)) {
+      const uint32_t slot = f & 0x7fffffffu;
+      x0 = x1 = x2 = x3 = 0.f;
+      if (slot < (uint32_t)pk.out_cap) {          // (an entry the encoder dropped reads as 0)
+        if (pk.out_dtype == HQMQ_F32) {
+          const float4 v = *reinterpret_cast<const float4*>(vals + (int64_t)slot * 16);
+          x0 = v.x; x1 = v.y; x2 = v.z; x3 = v.w;
+        } else {
+          const uint2 v = *reinterpret_cast<const uint2*>(vals + (int64_t)slot * 8);
+          const float2 a = pair16_to_float2(v.x, pk.out_dtype), c = pair16_to_float2(v.y, pk.out_dtype);
+          x0 = a.x; x1 = a.y; x2 = c.x; x3 = c.y;
+        }
+      }
+      fac = mul;
+    } else {
+      const uint2 cw = tbl[f & 0xffffu];
+      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&cw.x)), c = __half22float2(*reinterpret_cast<const __half2*>(&cw.y));
+      fac *= (float)(f >> 16);
+      x0 = a.x; x1 = a.y; x2 = c.x; x3 = c.y;
+    }
+    return make_uint2(pack_half2(x0 * fac, x1 * fac), pack_half2(x2 * fac, x3 * fac));
+  };
+
+  constexpr int TPW = 32 / N;                 // tokens a warp takes at a time
+  const int half = N == 32 ? 0 : lane >> 4, c = N == 32 ? lane : lane & 15;
+  const int tile_hi = min(e.nt, (int)(blockIdx.x + 1) * e.per);
+  for (int tile = blockIdx.x * e.per; tile < tile_hi; ++tile) {
+    const int t0 = (e.kt0 + tile) * kPfTok;
+    unsigned char* dst = (is_v ? e.vimg : e.kimg) + ((int64_t)blockIdx.y * e.nt + tile) * TB;
+    {
+      const int tb = t0 + warp * 16;
+      uint32_t run = outl && tb < e.Tkv ? pk.out_off[(int64_t)bh * (pk.T_cap / HQMQ_OUT_BLOCK + 1) + tb / HQMQ_OUT_BLOCK] : 0u;
+      float myfac = 0.f;                     // lanes 0..15: the factor of the block's tokens
+      uint32_t myflag = 0u;
+      if (lane < 16 && tb + lane < e.Tkv) {
+        myfac = scale_of(tb + lane) * e.vscale * mul;
+        if (outl) myflag = pk.flags[(int64_t)bh * pk.T_cap + tb + lane];
+      }
+      if (is_v && lane < 16) s_fac[warp * 16 + lane] = myfac;
+#pragma unroll 4
+      for (int k = 0; k < 16; k += TPW) {
+        const int tl = warp * 16 + k + half, t = t0 + tl;
+        uint32_t f = 0u;
+        if (t < e.Tkv) {
+          if constexpr (LAYOUT == 0) {
+            const uint32_t raw = row_field(reinterpret_cast<const uint32_t*>(pk.codes + ((int64_t)bh * pk.T_cap + t) * pk.row_bytes), c, cb);
+            f = (raw & ((1u << e.ib) - 1u)) | ((raw >> e.ib) << 16);
+          } else {
+            long long i = load_int(rf.idx, b * rf.idx_stride[0] + h * rf.idx_stride[1] + t * rf.idx_stride[2] + c, rf.idx_dtype);
+            i = i < 0 ? 0 : (i >= e.table_rows ? e.table_rows - 1 : i);
+            long long r = load_int(rf.rq, b * rf.rq_stride[0] + h * rf.rq_stride[1] + t * rf.rq_stride[2] + c, rf.rq_dtype);
+            r = r < 0 ? 0 : (r > 1023 ? 1023 : r);
+            f = (uint32_t)i | ((uint32_t)r << 16);
+          }
+        }
+        if (outl) {
+          const uint32_t w0 = __shfl_sync(0xffffffffu, myflag, k), w1 = N == 32 ? 0u : __shfl_sync(0xffffffffu, myflag, (k + 1) & 31);
+          const uint32_t w = half ? w1 : w0;
+          if ((w >> c) & 1u) f = 0x80000000u | (run + (half ? __popc(w0) : 0u) + __popc(w & ((1u << c) - 1u)));
+          run += __popc(w0) + (N == 32 ? 0 : __popc(w1));
+        }
+        if (is_v) {
+          fields[tl * (N + 1) + c] = f;
+        } else {
+          const float fac = __shfl_sync(0xffffffffu, myfac, k + half);
+          const uint2 v = value_of(f, fac);
+          *reinterpret_cast<uint2*>(dst + (c >> 4) * 16384 + tl * 128 + ((((c & 15) >> 1) ^ (tl & 7)) << 4) + (c & 1) * 8) = v;
+        }
+      }
+    }
+    if (is_v) {
+      __syncthreads();
+      const int tl = (warp & 3) * 32 + lane;
+      const float fac = s_fac[tl];
+      unsigned char* im = reinterpret_cast<unsigned char*>(img) + (tl >> 6) * (D * 128) + (tl & 7) * 2;
+      const int oct = (tl & 63) >> 3;
+#pragma unroll 4
+      for (int k = 0; k < N / 2; ++k) {
+        const int cc = (warp >> 2) * (N / 2) + k;
+        const uint2 v = value_of(fields[tl * (N + 1) + cc], fac);
+        const uint32_t w[2] = {v.x, v.y};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int d = 4 * cc + x;
+          *reinterpret_cast<uint16_t*>(im + d * 128 + ((oct ^ (d & 7)) << 4)) = (uint16_t)(w[x >> 1] >> (16 * (x & 1)));
+        }
+      }
+      __syncthreads();
+      for (int i = threadIdx.x; i < (int)(TB / 16); i += 256) reinterpret_cast<uint4*>(dst)[i] = img[i];
+      // (a warp ahead writes the next tile's `fields` and `s_fac` meanwhile; `img` only behind the next barrier)
+    }
+  }
+}
+
+}  // namespace
+
+// ---- host --------------------------------------------------------------------------------------------------------------------
+// Workspace: status word (16 bytes) | kmul, vmul [B * H_kv] | K images, V images of a group of (b, head) | partials
+bool prefill_plan(const hqmq_attn_args* a, PrefillPlan& pl) {
+  const int G = a->H_q / a->H_kv;
+  const int rows = a->layout == 0 ? 24 * a->K.S : a->K_size;
+  if ((a->d != 64 && a->d != 128) || a->T_q < kPrefillMinQueries || a->T_kv < 1 || a->partials_only || a->kv_splits > 0) return false;
+  if (rows > kPrefillMaxTable) return false;
+  PrefillParams& p = pl.p;
+  memset(&p, 0, sizeof(p));
+  p.Hkv = a->H_kv; p.G = G; p.Tq = a->T_q; p.Tkv = a->T_kv; p.causal = a->causal; p.window = a->window;
+  p.P = 128 / G;
+  p.streams = a->T_q > p.P ? 2 : 1;
+  p.units_m = (a->T_q + p.streams * p.P - 1) / (p.streams * p.P);
+  int kt1 = 0;
+  for (int m = 0; m < p.units_m; ++m) {
+    int lo, n;
+    pf_unit_tiles(p, m, lo, n);
+    if (m == 0) p.kt0 = lo;
+    p.kt0 = lo < p.kt0 ? lo : p.kt0;
+    kt1 = lo + n > kt1 ? lo + n : kt1;
+    p.Wh += n;
+  }
+  p.nt = kt1 - p.kt0;
+  const int bh_all = a->B * a->H_kv;
+  const size_t tile = 2 * pf_tile_bytes(a->d);
+  // the operand images of as many (b, head) at a time as kPrefillImageBytes hold
+  int64_t gb = (int64_t)(kPrefillImageBytes / ((size_t)p.nt * tile));
+  pl.group = gb < 1 ? 1 : gb > bh_all ? bh_all : (int)gb;
+  p.total = (int64_t)pl.group * p.Wh;
+  int64_t L = (p.total + 147) / 148;
+  p.L = L < 1 ? 1 : L;
+  pl.grid = (int)((p.total + p.L - 1) / p.L);
+  pl.off_mul = 16;
+  pl.off_img = (16 + (size_t)bh_all * 8 + 255) & ~(size_t)255;
+  pl.off_part = pl.off_img + (size_t)pl.group * p.nt * tile;
+  pl.ws_bytes = pl.off_part + (size_t)pl.grid * 2 * 256 * (a->d + 2) * sizeof(float);
+  return true;
+}
+
+int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspace, float qscale, uint32_t epoch, cudaStream_t st) {
+  PrefillParams p = pl.p;
+  unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
+  const int bh_all = a->B * a->H_kv, d = a->d;
+  p.Q = a->Q; p.q_dtype = a->q_dtype; p.qs_b = a->q_stride[0]; p.qs_h = a->q_stride[1]; p.qs_t = a->q_stride[2];
+  p.O = a->O; p.o_dtype = a->o_dtype; p.os_b = a->o_stride[0]; p.os_h = a->o_stride[1]; p.os_t = a->o_stride[2];
+  auto vec = [](const void* ptr, const int64_t* s, int dt) {
+    return dt != HQMQ_F32 && ((uintptr_t)ptr & 15) == 0 && s[0] % 8 == 0 && s[1] % 8 == 0 && s[2] % 8 == 0;
+  };
+  p.q_vec = vec(a->Q, a->q_stride, a->q_dtype); p.o_vec = vec(a->O, a->o_stride, a->o_dtype);
+  p.status = reinterpret_cast<uint32_t*>(ws); p.epoch = epoch;
+  float* mul = reinterpret_cast<float*>(ws + pl.off_mul);
+  p.kmul = mul; p.vmul = mul + bh_all;
+  ExpandParams e;
+  memset(&e, 0, sizeof(e));
+  e.Hkv = a->H_kv; e.Tkv = a->T_kv; e.kt0 = p.kt0; e.nt = p.nt;
+  e.qscale = qscale; e.vscale = 1.0f / (float)a->r_qmax;
+  e.kmul = mul; e.vmul = mul + bh_all;
+  if (a->layout == 0) {
+    e.K = a->K; e.V = a->V; e.tblK = a->table_K; e.tblV = a->table_V;
+    e.ib = idx_bits_for(a->K.S); e.table_rows = 24 * a->K.S;
+  } else {
+    e.Kr = a->K_ref; e.Vr = a->V_ref; e.jK = a->joint_K; e.jV = a->joint_V; e.j_dtype = a->joint_dtype;
+    e.ib = 16; e.table_rows = a->K_size;
+  }
+  const size_t img_bytes = (size_t)pl.group * p.nt * pf_tile_bytes(d);
+  e.kimg = ws + pl.off_img; e.vimg = e.kimg + img_bytes;
+  p.kimg = e.kimg; p.vimg = e.vimg;
+  p.part = reinterpret_cast<float*>(ws + pl.off_part);
+  const int N = d / 4;
+  const size_t esmem = pf_tile_bytes(d) + (size_t)128 * (N + 1) * 4 + (size_t)e.table_rows * 8;
+  const void* ek = N == 32 ? (a->layout == 0 ? (const void*)&prefill_expand_kernel<32, 0> : (const void*)&prefill_expand_kernel<32, 1>)
+                           : (a->layout == 0 ? (const void*)&prefill_expand_kernel<16, 0> : (const void*)&prefill_expand_kernel<16, 1>);
+  const void* ak = d == 128 ? (const void*)&prefill_attn_kernel<128> : (const void*)&prefill_attn_kernel<64>;
+  const void* mk = d == 128 ? (const void*)&prefill_merge_kernel<128> : (const void*)&prefill_merge_kernel<64>;
+  HQMQ_CHECK_CUDA(raise_smem_limit(ek, esmem));
+  HQMQ_CHECK_CUDA(raise_smem_limit(ak, pf_smem_bytes(d)));
+  for (int bh0 = 0; bh0 < bh_all; bh0 += pl.group) {
+    const int n_bh = bh_all - bh0 < pl.group ? bh_all - bh0 : pl.group;
+    e.bh0 = p.bh0 = bh0;
+    p.total = (int64_t)n_bh * p.Wh;
+    p.L = (p.total + pl.grid - 1) / pl.grid;
+    const int grid = (int)((p.total + p.L - 1) / p.L);
+    // tiles per expand CTA: about four CTAs per SM in all, so that a CTA's table and scale scan serve several tiles
+    int64_t per = ((int64_t)p.nt * n_bh * 2 + 4 * 148 - 1) / (4 * 148);
+    e.per = per < 1 ? 1 : per > p.nt ? p.nt : (int)per;
+    void* ea[] = {&e};
+    HQMQ_CHECK_CUDA(cudaLaunchKernel(ek, dim3((p.nt + e.per - 1) / e.per, n_bh, 2), dim3(256), ea, esmem, st));
+    void* pa[] = {&p};
+    HQMQ_CHECK_CUDA(cudaLaunchKernel(ak, dim3(grid), dim3(kPfThreads), pa, pf_smem_bytes(d), st));
+    if (grid > 1) HQMQ_CHECK_CUDA(cudaLaunchKernel(mk, dim3(grid - 1, 4 * p.streams), dim3(256), pa, 0, st));
+  }
+  return HQMQ_OK;
+}
+
+}  // namespace attn
+}  // namespace hqmq

@@ -1,0 +1,52 @@
+// Attention of many query positions over one compressed cache: parameters and the host entry points (attn_prefill.cu).
+#pragma once
+#include "attn_kernel.cuh"
+
+namespace hqmq {
+namespace attn {
+
+constexpr int kPfTok = 128;                       // tokens per operand tile
+constexpr int kPrefillMinQueries = 16;
+constexpr int kPrefillMaxTable = 8192;            // codewords per head that fit the expand kernel's shared memory
+constexpr size_t kPrefillImageBytes = (size_t)512 << 20;   // operand images held at a time; larger caches go by groups of (b, head)
+
+struct PrefillParams {
+  const void* Q; int q_dtype; int64_t qs_b, qs_h, qs_t;
+  void* O; int o_dtype; int64_t os_b, os_h, os_t;
+  int q_vec, o_vec;                               // 16-byte accesses to Q / O rows are aligned (16-bit types)
+  int Hkv, G, Tq, Tkv, causal, window;
+  int P, streams, units_m;                        // query positions per stream, row blocks per unit, units per (b, head)
+  int kt0, nt;                                    // first KV tile that any query sees, tiles in the images
+  int bh0;                                        // first (b, head) of the group
+  int64_t Wh, total, L;                           // tiles per (b, head), in all, per CTA
+  const unsigned char* kimg; const unsigned char* vimg;
+  const float* kmul; const float* vmul;           // [B * H_kv] what a score / an output is multiplied by
+  float* part;                                    // [CTA][2][256 rows][d + 2]
+  uint32_t* status; uint32_t epoch;
+};
+
+struct ExpandParams {
+  hqmq_packed K, V;
+  hqmq_ref_packed Kr, Vr;
+  const uint16_t* tblK; const uint16_t* tblV;
+  const void* jK; const void* jV; int j_dtype;
+  int ib, table_rows, Hkv, Tkv, kt0, nt, per, bh0;
+  float qscale, vscale;                           // softmax scale * log2(e), 1 / qmax
+  unsigned char* kimg; unsigned char* vimg;
+  float* kmul; float* vmul;
+};
+
+struct PrefillPlan {
+  PrefillParams p;
+  int group, grid;
+  size_t off_mul, off_img, off_part, ws_bytes;
+};
+
+// The plan of a call that takes this path, or false.
+bool prefill_plan(const hqmq_attn_args* a, PrefillPlan& pl);
+int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspace, float qscale, uint32_t epoch, cudaStream_t st);
+// Raises a kernel's dynamic shared-memory limit to the device's maximum, once per kernel and device (attn.cu).
+cudaError_t raise_smem_limit(const void* kernel, size_t smem);
+
+}  // namespace attn
+}  // namespace hqmq

@@ -1,0 +1,76 @@
+"""Attention of many query positions (tensor-core path) against a plain fp32 evaluation of the same operation on the
+dense reconstruction: edges of the 128-token tiles and of the row blocks, ragged groups, every mask, units cut between CTAs."""
+import math
+
+import pytest
+import torch
+
+import hqmq_b200 as hqmq
+from hqmq_b200 import kernels
+from tests.util import make_kv, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _dense_attention(Q, K, V, causal, window):
+    """fp32 softmax(scale Q K^T + mask) V; causal as fused_attention_packed takes it; rows that see no key are zero."""
+    B, Hq, Tq, d = Q.shape
+    T, G = K.shape[2], Hq // K.shape[1]
+    K, V = K.float().repeat_interleave(G, 1), V.float().repeat_interleave(G, 1)
+    i, t = torch.arange(Tq, device=Q.device)[:, None], torch.arange(T, device=Q.device)[None, :]
+    end = (i + 1).clamp(max=T) if causal is True else (T - Tq + i + 1).clamp(min=0) if causal == "bottom_right" else torch.full_like(i, T)
+    ok = (t < end) & (t >= (end - window if window else torch.zeros_like(end)))
+    s = (Q.half().float() @ K.transpose(-1, -2)) / math.sqrt(d)
+    p = torch.softmax(s.masked_fill(~ok, float("-inf")), -1).nan_to_num(0.0)
+    return p @ V
+
+
+def _check(got, want):
+    # (rows that see a few keys return values of a spike's size, to 11 bits)
+    assert ((got - want).abs() / want.abs().clamp(min=1.0)).max().item() < 2e-3 and rel_l2(got, want) < 1e-3
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,d,T,Tq,causal,window", [
+    (1, 32, 8, 128, 1024, 16, "bottom_right", None),     # one stream, units over many CTAs
+    (2, 8, 2, 128, 700, 33, "bottom_right", None),       # the second stream holds one position
+    (1, 14, 2, 128, 519, 37, "bottom_right", None),      # seven heads per group: 18 positions in 126 rows
+    (2, 16, 2, 64, 129, 129, "bottom_right", None),      # a prompt from empty, one key in the last tile
+    (1, 8, 1, 64, 128, 100, False, None),                # no mask, exactly one tile
+    (1, 32, 8, 128, 3000, 200, "bottom_right", 128),     # window: early tiles untouched
+    (3, 8, 2, 64, 640, 40, False, 77),
+    (1, 16, 1, 128, 300, 20, True, None),                # sixteen heads per group, top-left mask
+    (1, 4, 2, 128, 40, 64, "bottom_right", None),        # more queries than keys: the first rows see nothing
+])
+@pytest.mark.parametrize("outliers", [True, False])
+def test_packed_prompt_attention(B, Hq, Hkv, d, T, Tq, causal, window, outliers):
+    S, br = (96, 4) if d == 64 or outliers else (192, 6)
+    q = hqmq.HQMQ(1, Hkv, S, br, device="cuda")
+    K = make_kv("hot" if d == 128 and outliers else "spiky", (B, Hkv, T, d), seed=81, dtype=torch.bfloat16).cuda()
+    V = make_kv("spiky", (B, Hkv, T, d), seed=82, dtype=torch.bfloat16).cuda()
+    mult = 3.0 if outliers else None
+    Kp, Vp = q.encode(K, 0, 0, median_mult=mult), q.encode(V, 0, 1, median_mult=mult)
+    tk, tv = q.tables(0, 0, "cuda"), q.tables(0, 1, "cuda")
+    Q = (torch.randn(B, Hq, Tq, d, generator=torch.Generator().manual_seed(83)) / math.sqrt(d)).bfloat16().cuda()
+    want = _dense_attention(Q, q.decode(Kp, 0, 0), q.decode(Vp, 0, 1), causal, window)
+    O = torch.empty(Q.shape, dtype=torch.float32, device="cuda")
+    hqmq.fused_attention_packed(Q, Kp, Vp, tk["table16"], tv["table16"], causal=causal, window=window, out=O)
+    _check(O, want)
+    # the 16-bit output of a strided query tensor is that result rounded once
+    Qs = Q.transpose(1, 2).contiguous().transpose(1, 2)
+    O16 = hqmq.fused_attention_packed(Qs, Kp, Vp, tk["table16"], tv["table16"], causal=causal, window=window)
+    assert torch.equal(O16, O.bfloat16())
+
+
+@pytest.mark.parametrize("Hq,Hkv,d,T,Tq,causal", [(32, 8, 128, 257, 257, True), (7, 1, 64, 127, 127, True), (8, 2, 128, 390, 50, False)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_tuple_prompt_attention(Hq, Hkv, d, T, Tq, causal, dtype):
+    q = hqmq.HQMQ(1, Hkv, 192, 6, device="cuda")
+    args, dense = [], []
+    for kv in (0, 1):
+        idx, rq, rs, _ = q.encode(make_kv("randn", (1, Hkv, T, d), seed=84 + kv, dtype=torch.bfloat16).cuda(), 0, kv).to_reference()
+        args += [idx, rq, rs.to(dtype), q.tables(0, kv, "cuda")["joint"].to(dtype)]
+        dense.append(kernels.decode_dequant(idx, rq, args[-2].float(), args[-1].float(), 63))
+    Q = (torch.randn(1, Hq, Tq, d, generator=torch.Generator().manual_seed(86)) / math.sqrt(d)).to(dtype).cuda()
+    O = torch.empty(Q.shape, dtype=torch.float32, device="cuda")
+    hqmq.fused_attention(Q, *args, 63, causal=causal, out=O)
+    _check(O, _dense_attention(Q, *dense, causal, None))
