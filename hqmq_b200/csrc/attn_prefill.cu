@@ -13,7 +13,8 @@
 //            alternate on the tensor cores: while the softmax warps of one stream work on S = Q K^T, the other stream's
 //            P V and its next Q K^T run.  Warps 0-3 / 4-7: softmax of stream 0 / 1 (a thread owns a row: S comes out of
 //            TMEM, P goes back as fp16 into the same columns, the accumulator is rescaled only when a row's maximum rises by
-//            more than 2^8); warp 8 issues the MMAs; warp 9 streams the tiles in through two-deep (four at d_head 64) rings.
+//            more than 2^8); warps 8 / 10 issue the MMAs of stream 0 / 1; warp 9 streams the tiles in through two-deep (four at
+//            d_head 64) rings.
 //            The tiles of all units form one flat sequence cut into equal pieces, one per CTA, whatever the mask leaves of
 //            each unit; a unit that is cut leaves partials, merged by prefill_merge_kernel.
 //
@@ -25,7 +26,7 @@ namespace hqmq {
 namespace attn {
 namespace {
 
-constexpr int kPfThreads = 384;             // 2 x 4 softmax warps; MMA warp, loader warp and two idle ones (register shares are per 4 warps)
+constexpr int kPfThreads = 384;             // 2 x 4 softmax warps; two MMA warps, a loader warp and an idle one (register shares are per 4 warps)
 // registers per thread: the launch gives 384 x 168; the third warpgroup hands its share to the softmax warps (128 values of
 // a row each): 256 x 208 + 128 x 80 <= 384 x 168
 constexpr int kPfSoftmaxRegs = 208, kPfOtherRegs = 80;
@@ -35,7 +36,8 @@ constexpr uint32_t kPfTmemCols = 512;
 
 __host__ __device__ constexpr int pf_stages(int d) { return d == 128 ? 2 : 4; }
 __host__ __device__ constexpr size_t pf_tile_bytes(int d) { return (size_t)d * 256; }
-__host__ __device__ constexpr size_t pf_smem_bytes(int d) { return (size_t)(2 + 2 * pf_stages(d)) * pf_tile_bytes(d) + 1024 + 256; }
+constexpr int kPfOutRow = 80;                // bytes of a row in a warp's output staging area: 64 + padding
+__host__ __device__ constexpr size_t pf_smem_bytes(int d) { return (size_t)(2 + 2 * pf_stages(d)) * pf_tile_bytes(d) + 8 * 32 * kPfOutRow + 1024 + 256; }
 
 // ---- work decomposition -------------------------------------------------------------------------------------------
 // KV tiles [lo, lo + n) that the rows of unit m see (at least one, so that a fully masked unit still writes its zeros).
@@ -57,14 +59,12 @@ struct PfPiece { int bh, m, tile0, n; bool head, tail; };
 struct PfIter {
   int left;
   int bh, m, off, lo, n;
-  __device__ __forceinline__ void init(const PrefillParams& p, int64_t pos) {
+  __device__ __forceinline__ void init(const PrefillParams& p, int cta) {
+    const int64_t pos = (int64_t)cta * p.L;
     left = (int)(p.total - pos < p.L ? p.total - pos : p.L);
     bh = (int)(pos / p.Wh);
-    int rem = (int)(pos - (int64_t)bh * p.Wh);
-    m = 0;
+    m = p.start_m[cta]; off = p.start_off[cta];
     pf_unit_tiles(p, m, lo, n);
-    while (rem >= n) { rem -= n; ++m; pf_unit_tiles(p, m, lo, n); }
-    off = rem;
   }
   __device__ __forceinline__ bool next(const PrefillParams& p, PfPiece& q) {
     if (left <= 0) return false;
@@ -84,16 +84,24 @@ struct PfIter {
 // ---- tcgen05 ---------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Issued inside `if (elect_one())` by a converged warp: the compiler then knows that one lane is active and that descriptors
+// and addresses are uniform.  (Measured, 128 x 128 x 16: 64 clocks per MMA -- the tensor cores' own rate -- against 75 to 90
+// from a branch on the lane number or with the instruction predicated.)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+  return r != 0u;
+}
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tc_mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool acc) {
+__device__ __forceinline__ void tc_mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-               ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)acc) : "memory");
+               ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
 }
-__device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool acc) {
+__device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"((uint32_t)acc) : "memory");
+               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
 }
 #define PF_R8(r, o) "=r"((r)[o]), "=r"((r)[o + 1]), "=r"((r)[o + 2]), "=r"((r)[o + 3]), "=r"((r)[o + 4]), "=r"((r)[o + 5]), \
                     "=r"((r)[o + 6]), "=r"((r)[o + 7])
@@ -111,11 +119,6 @@ __device__ __forceinline__ void tc_st32(uint32_t addr, const uint32_t* r) {
       "%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
       ::"r"(addr), PF_I8(r, 0), PF_I8(r, 8), PF_I8(r, 16), PF_I8(r, 24) : "memory");
 }
-__device__ __forceinline__ void tc_st16(uint32_t addr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(addr), PF_I8(r, 0), PF_I8(r, 8) : "memory");
-}
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // K-major operand in the 128-byte swizzle: rows of 128 bytes, groups of eight rows 1024 bytes apart.
@@ -124,7 +127,7 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
          ((uint64_t)2 << 61);
 }
 // kind::f16, fp16 operands (both K-major), fp32 accumulators
-__device__ __forceinline__ uint32_t f16_idesc(int M, int N) { return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24); }
+__host__ __device__ constexpr uint32_t f16_idesc(int M, int N) { return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24); }
 
 // ---- attend ----------------------------------------------------------------------------------------------------------------
 template <int D>
@@ -134,35 +137,40 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
   extern __shared__ unsigned char smem_raw[];
   const uint32_t s_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* base = smem_raw + (s_base - smem_u32(smem_raw));
-  const uint32_t sQ = s_base, sK = sQ + 2 * TB, sV = sK + NS * TB, bars = sV + NS * TB;
+  const uint32_t sQ = s_base, sK = sQ + 2 * TB, sV = sK + NS * TB, sO = sV + NS * TB, bars = sO + 8 * 32 * kPfOutRow;
   const uint32_t kfull = bars, kempty = kfull + 8 * NS, vfull = kempty + 8 * NS, vempty = vfull + 8 * NS;
-  const uint32_t qfull = vempty + 8 * NS, sfull = qfull + 16, pfull = sfull + 16, odone = pfull + 16;
-  volatile uint32_t* abort_word = reinterpret_cast<volatile uint32_t*>(base + (odone + 16 - s_base));
-  volatile uint32_t* tmem_word = abort_word + 1;
+  // per stream: queries written; S of either half computed / its P written; P V of a half done
+  const uint32_t qfull = vempty + 8 * NS, sfull = qfull + 16, pfull = sfull + 32, pvdone = pfull + 32;
+  volatile uint32_t* abort_word = reinterpret_cast<volatile uint32_t*>(base + (pvdone + 32 - s_base));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) {
-      mbar_init(kfull + 8 * i, 1); mbar_init(kempty + 8 * i, 1); mbar_init(vfull + 8 * i, 1); mbar_init(vempty + 8 * i, 1);
+      mbar_init(kfull + 8 * i, 1); mbar_init(kempty + 8 * i, p.streams); mbar_init(vfull + 8 * i, 1); mbar_init(vempty + 8 * i, p.streams);
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(qfull + 8 * s, 4); mbar_init(sfull + 8 * s, 1); mbar_init(pfull + 8 * s, 4); mbar_init(odone + 8 * s, 1);
+      mbar_init(qfull + 8 * s, 4);
+      for (int hb = 0; hb < 2; ++hb) {
+        mbar_init(sfull + 16 * s + 8 * hb, 1); mbar_init(pfull + 16 * s + 8 * hb, 4); mbar_init(pvdone + 16 * s + 8 * hb, 1);
+      }
     }
     *abort_word = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 8) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(odone + 20), "n"(kPfTmemCols) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pvdone + 36), "n"(kPfTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_word;
-  // (a wait that runs out raises the abort word: every role then stops at its next wait)
+  constexpr uint32_t tmem = 0u;               // an allocation of all columns starts at column 0
+  // (a wait that runs out raises the abort word: every role then stops at its next wait.  No suspend hint: these waits are
+  //  links of the per-tile chain, and a hinted wait was seen to wake late.)
   auto wait = [&](uint32_t bar, uint32_t parity) {
-    if (ring_wait(bar, parity, abort_word)) return true;
-    *abort_word = 1u;
-    return false;
+    for (uint32_t spins = 0; !mbar_try_wait(bar, parity);) {
+      if (++spins > kWaitLimit || ((spins & 255u) == 0u && *abort_word)) { *abort_word = 1u; return false; }
+    }
+    return true;
   };
   if (warp >= 8) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPfOtherRegs));
@@ -171,7 +179,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
     if (lane == 0) {
       PfIter it;
       PfPiece q;
-      it.init(p, (int64_t)blockIdx.x * p.L);
+      it.init(p, (int)blockIdx.x);
       uint32_t g = 0;          // tiles issued
       bool ok = true;
       while (ok && it.next(p, q)) {
@@ -200,71 +208,70 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
         while (!mbar_try_wait(vfull + 8 * st, ph) && ++spins < kWaitLimit) {}
       }
     }
-  } else if (warp == 8) {
-    // ================================ MMA issuer =================================================================
-    if (lane == 0) {
-      PfIter it;
-      PfPiece q;
-      it.init(p, (int64_t)blockIdx.x * p.L);
-      const uint32_t id_qk = f16_idesc(128, 128), id_pv = f16_idesc(128, D);
-      auto qk = [&](int s, uint32_t st) {
-        const uint64_t a0 = sw128_desc(sQ + s * TB), b0 = sw128_desc(sK + st * TB);
+  } else if ((warp - 8) / 2 < p.streams && (warp & 1) == 0) {
+    // ================================ MMA issuers: one warp per stream, converged ====================================
+    // (A ready wait costs its warp about 200 clocks; with one warp for both streams the tensor cores ran dry meanwhile.)
+    const int s = (warp - 8) / 2;
+    PfIter it;
+    PfPiece q;
+    it.init(p, (int)blockIdx.x);
+    auto wait_w = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, wait(bar, parity)) != 0; };   // one answer per warp
+    constexpr uint32_t id_qk = f16_idesc(128, 64), id_pv = f16_idesc(128, D);
+    // S of half hb of the tile in stage st; O += P V of that half
+    auto qk = [&](uint32_t st, int hb) {
+      const uint64_t a0 = sw128_desc(sQ + s * TB), b0 = sw128_desc(sK + st * TB + hb * 8192);
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t o = ((k >> 2) * 16384 + (k & 3) * 32) >> 4;
-          tc_mma_ss(tmem + 128 * s, a0 + o, b0 + o, id_qk, k > 0);
-        }
-      };
-      auto pv = [&](int s, uint32_t st, bool acc) {
-        const uint64_t b0 = sw128_desc(sV + st * TB);
+      for (int k = 0; k < D / 16; ++k) {
+        const uint32_t o = ((k >> 2) * 16384 + (k & 3) * 32) >> 4;
+        tc_mma_ss(128 * s + 64 * hb, a0 + o, b0 + o, id_qk, k > 0 ? 1u : 0u);
+      }
+      tc_commit(sfull + 16 * s + 8 * hb);
+    };
+    auto pv = [&](uint32_t st, int hb, bool acc) {
+      const uint64_t b0 = sw128_desc(sV + st * TB + hb * (D * 128));
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-          tc_mma_ts(tmem + 256 + D * s, tmem + 128 * s + 8 * k, b0 + (((k >> 2) * D * 128 + (k & 3) * 32) >> 4), id_pv, acc || k > 0);
-      };
-      uint32_t g = 0, u = 0;     // tiles whose P V is issued, units whose queries arrived
-      bool have = it.next(p, q), ok = true;
-      if (have) {
-        for (int s = 0; s < p.streams && ok; ++s) {
-          if (s == 0) ok = wait(kfull, 0);
-          if (ok) ok = wait(qfull + 8 * s, 0);
+      for (int k = 0; k < 4; ++k)
+        tc_mma_ts(256 + D * s, 128 * s + 64 * hb + 8 * k, b0 + ((k * 32) >> 4), id_pv, acc || k > 0 ? 1u : 0u);
+      tc_commit(pvdone + 16 * s + 8 * hb);
+    };
+    uint32_t g = 0, u = 0;     // tiles, units
+    bool ok = true;
+    while (ok && it.next(p, q)) {
+      // the unit's first S, both halves
+      ok = wait_w(kfull + 8 * (g % NS), (g / NS) & 1u) && wait_w(qfull + 8 * s, u & 1u);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
+        qk(g % NS, 0);
+        qk(g % NS, 1);
+        tc_commit(kempty + 8 * (g % NS));
+      }
+      // half by half: P V of this tile's half, then Q K^T of the next tile's half into the columns that P has left
+      for (int i = 0; i < q.n && ok; ++i, ++g) {
+        const bool last = i + 1 == q.n;
+        const uint32_t st = g % NS, ph = (g / NS) & 1u, st1 = (g + 1) % NS, ph1 = ((g + 1) / NS) & 1u;
+        ok = wait_w(vfull + 8 * st, ph) && (last || wait_w(kfull + 8 * st1, ph1));
+#pragma unroll
+        for (int hb = 0; hb < 2; ++hb) {
+          ok = ok && wait_w(pfull + 16 * s + 8 * hb, g & 1u);
           if (!ok) break;
           tc_fence_after();
-          qk(s, 0);
-          tc_commit(sfull + 8 * s);
-        }
-        if (ok) tc_commit(kempty);
-      }
-      while (ok && have) {
-        PfPiece nq;
-        const bool more = it.next(p, nq);
-        for (int i = 0; i < q.n && ok; ++i, ++g) {
-          const bool last = i + 1 == q.n;
-          const bool nxt = !last || more;
-          const uint32_t st = g % NS, ph = (g / NS) & 1u, st1 = (g + 1) % NS, ph1 = ((g + 1) / NS) & 1u;
-          for (int s = 0; s < p.streams; ++s) {
-            if (s == 0 && !(ok = wait(vfull + 8 * st, ph))) break;
-            if (!(ok = wait(pfull + 8 * s, g & 1u))) break;
-            tc_fence_after();
-            pv(s, st, i > 0);
-            if (last) tc_commit(odone + 8 * s);
-            if (s == p.streams - 1) tc_commit(vempty + 8 * st);
-            if (nxt) {
-              if (s == 0 && !(ok = wait(kfull + 8 * st1, ph1))) break;
-              if (last && !(ok = wait(qfull + 8 * s, (u + 1) & 1u))) break;
-              tc_fence_after();
-              qk(s, st1);
-              tc_commit(sfull + 8 * s);
-              if (s == p.streams - 1) tc_commit(kempty + 8 * st1);
+          if (elect_one()) {
+            pv(st, hb, i > 0 || hb > 0);
+            if (hb) tc_commit(vempty + 8 * st);
+            if (!last) {
+              qk(st1, hb);
+              if (hb) tc_commit(kempty + 8 * st1);
             }
           }
         }
-        q = nq; have = more; ++u;
       }
-      // the last commits must have arrived before the CTA's shared memory goes away
-      if (ok && g > 0) {
-        const uint32_t st = (g - 1) % NS, ph = ((g - 1) / NS) & 1u;
-        if (wait(vempty + 8 * st, ph)) wait(kempty + 8 * st, ph);
-      }
+      ++u;
+    }
+    // the last commits must have arrived before the CTA's shared memory goes away
+    if (ok && g > 0) {
+      const uint32_t st = (g - 1) % NS, ph = ((g - 1) / NS) & 1u;
+      if (wait(vempty + 8 * st, ph)) wait(kempty + 8 * st, ph);
     }
   }
   } else {
@@ -275,32 +282,43 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
     const int pl = row / p.G, gh = row - pl * p.G;
     const uint32_t lane_sel = (uint32_t)(warp & 3) << 21;               // TMEM lane 32 * (warp & 3), bits 31:16 of an address
     const uint32_t tS = tmem + 128 * s + lane_sel, tO = tmem + 256 + D * s + lane_sel;
-    const uint32_t q_row = sQ + s * TB + row * 128;
+    // The queries of a unit: a warp loads its 32 rows together, D / 8 lanes of 16 bytes to a row.
+    constexpr int QL = D / 8, QR = 32 / QL;      // lanes per row, rows per warp-wide load
     auto load_q = [&](const PfPiece& w) {
-      const int bh = p.bh0 + w.bh, b = bh / p.Hkv, h = bh - b * p.Hkv;
-      const int tq = (w.m * p.streams + s) * p.P + pl;
-      const bool live = pl < p.P && tq < p.Tq;
-      const int64_t o = (int64_t)b * p.qs_b + (int64_t)(h * p.G + gh) * p.qs_h + (int64_t)tq * p.qs_t;
+      const int bh = p.bh0 + w.bh, b = bh / p.Hkv, h = bh - b * p.Hkv, c = lane % QL;
+      const int64_t qb = (int64_t)b * p.qs_b + (int64_t)(h * p.G) * p.qs_h + 8 * c;
+      const int tq0 = (w.m * p.streams + s) * p.P;
+      int pw = ((warp & 3) * 32 + lane / QL) / p.G, gw = (warp & 3) * 32 + lane / QL - pw * p.G;
 #pragma unroll
-      for (int c = 0; c < D / 8; ++c) {        // 16-byte pieces of the row in fp16
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (live) {
+      for (int k0 = 0; k0 < QL; k0 += 8) {       // eight loads in flight
+        uint4 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const bool live = pw < p.P && tq0 + pw < p.Tq;
+          const int64_t o = qb + (int64_t)gw * p.qs_h + (int64_t)(tq0 + pw) * p.qs_t;
+          v[k] = make_uint4(0u, 0u, 0u, 0u);
           if (p.q_vec) {
-            v = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.Q) + o + 8 * c);
-            if (p.q_dtype == HQMQ_BF16) {
-              uint32_t* w4 = reinterpret_cast<uint32_t*>(&v);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) w4[e] = pack_half2(__uint_as_float(w4[e] << 16), __uint_as_float(w4[e] & 0xffff0000u));
-            }
-          } else {
+            if (live) v[k] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.Q) + o);
+          } else if (live) {
             float f[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = load_float(p.Q, o + 8 * c + e, p.q_dtype);
-            v = make_uint4(pack_half2(f[0], f[1]), pack_half2(f[2], f[3]), pack_half2(f[4], f[5]), pack_half2(f[6], f[7]));
+            for (int e = 0; e < 8; ++e) f[e] = load_float(p.Q, o + e, p.q_dtype);
+            v[k] = make_uint4(pack_half2(f[0], f[1]), pack_half2(f[2], f[3]), pack_half2(f[4], f[5]), pack_half2(f[6], f[7]));
           }
+          gw += QR;
+          while (gw >= p.G) { gw -= p.G; ++pw; }
         }
-        const uint32_t dst = q_row + (c >> 3) * 16384 + (((c & 7) ^ (row & 7)) << 4);
-        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          if (p.q_vec && p.q_dtype == HQMQ_BF16) {
+            uint32_t* w4 = reinterpret_cast<uint32_t*>(&v[k]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) w4[e] = pack_half2(__uint_as_float(w4[e] << 16), __uint_as_float(w4[e] & 0xffff0000u));
+          }
+          const int rw = (warp & 3) * 32 + (k0 + k) * QR + lane / QL;
+          const uint32_t dst = sQ + s * TB + rw * 128 + (c >> 3) * 16384 + (((c & 7) ^ (rw & 7)) << 4);
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(v[k].x), "r"(v[k].y), "r"(v[k].z), "r"(v[k].w) : "memory");
+        }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // the MMA reads it through the async proxy
       __syncwarp();
@@ -308,8 +326,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
     };
     PfIter it;
     PfPiece q;
-    it.init(p, (int64_t)blockIdx.x * p.L);
-    uint32_t g = 0, u = 0;
+    it.init(p, (int)blockIdx.x);
+    uint32_t g = 0;
     bool have = it.next(p, q), ok = true;
     if (have) load_q(q);
     while (ok && have) {
@@ -325,26 +343,28 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
       const bool w_live = __any_sync(0xffffffffu, live);
       const float kmul = p.kmul[bh];
       float m_run = -INFINITY, l0 = 0.f, l1 = 0.f;
-      for (int i = 0; i < q.n; ++i, ++g) {
-        ok = wait(sfull + 8 * s, g & 1u);
+      for (int i = 0; i < 2 * q.n; ++i) {
+        const int hb = i & 1;
+        const uint32_t ph = (g + (i >> 1)) & 1u, tH = tS + 64 * hb;
+        ok = wait(sfull + 16 * s + 8 * hb, ph);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
         if (w_live) {
-          uint32_t r[128];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) tc_ld32(r + 32 * c, tS + 32 * c);
+          uint32_t r[64];
+          tc_ld32(r, tH);
+          tc_ld32(r + 32, tH + 32);
           tc_wait_ld();
-          const int t0 = (q.tile0 + i) * kPfTok;
-          if (t0 < w_beg || t0 + kPfTok > w_end) {
+          const int t0 = q.tile0 * kPfTok + 64 * i;
+          if (t0 < w_beg || t0 + 64 > w_end) {
             const int lo = beg - t0, hi = end - t0;
 #pragma unroll
-            for (int c = 0; c < 128; ++c)
+            for (int c = 0; c < 64; ++c)
               if (c < lo || c >= hi) r[c] = 0xff800000u;
           }
           float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-          for (int c = 0; c < 128; c += 8)
+          for (int c = 0; c < 64; c += 8)
 #pragma unroll
             for (int e = 0; e < 4; ++e)
               mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(r[c + 2 * e]), __uint_as_float(r[c + 2 * e + 1])));
@@ -355,7 +375,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
             m_run = m_new;
             l0 *= alpha; l1 *= alpha;
             if (i > 0) {
-              // (S of this tile was issued behind the previous tile's P V: the accumulator is complete)
+              // the accumulator is rescaled once the previous half's P V is done (the one before it is: this S was issued
+              // behind it)
+              ok = wait(pvdone + 16 * s + 8 * (hb ^ 1), hb ? ph : ph ^ 1u);
+              ok = __all_sync(0xffffffffu, ok);
+              if (!ok) break;
+              tc_fence_after();
 #pragma unroll 1
               for (int c = 0; c < D; c += 32) {
                 uint32_t o[32];
@@ -368,31 +393,29 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
             }
           }
           const float nb = m_run == -INFINITY ? 0.f : -m_run;
+          uint32_t pk[32];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t pk[16];
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const float a = fast_exp2(fmaf(__uint_as_float(r[32 * c + 2 * e]), kmul, nb));
-              const float b = fast_exp2(fmaf(__uint_as_float(r[32 * c + 2 * e + 1]), kmul, nb));
-              const __half2 h = __floats2half2_rn(a, b);
-              // (the weights that are summed are the rounded ones the tensor cores see: the rounding cancels)
-              const float2 f = __half22float2(h);
-              l0 += f.x; l1 += f.y;
-              pk[e] = *reinterpret_cast<const uint32_t*>(&h);
-            }
-            tc_st16(tS + 16 * c, pk);
+          for (int e = 0; e < 32; ++e) {
+            const float a = fast_exp2(fmaf(__uint_as_float(r[2 * e]), kmul, nb));
+            const float b = fast_exp2(fmaf(__uint_as_float(r[2 * e + 1]), kmul, nb));
+            const __half2 h = __floats2half2_rn(a, b);
+            // (the weights that are summed are the rounded ones the tensor cores see: the rounding cancels)
+            const float2 f = __half22float2(h);
+            l0 += f.x; l1 += f.y;
+            pk[e] = *reinterpret_cast<const uint32_t*>(&h);
           }
+          tc_st32(tH, pk);
           tc_wait_st();
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(pfull + 8 * s);
+        if (lane == 0) mbar_arrive(pfull + 16 * s + 8 * hb);
       }
       if (!ok) break;
+      g += q.n;
       // the last Q K^T of the unit is complete: the next unit's queries may take the place of this one's
       if (more) load_q(nq);
-      ok = wait(odone + 8 * s, u & 1u);
+      ok = wait(pvdone + 16 * s + 8, (g - 1) & 1u);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
@@ -401,21 +424,28 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
         const float l = l0 + l1, vmul = p.vmul[bh];
         const bool whole = q.head && q.tail;
         const float mul = whole ? (l > 0.f ? vmul / l : 0.f) : vmul;
-        float* part = p.part + (((int64_t)blockIdx.x * 2 + (q.head ? 1 : 0)) * 256 + s * 128 + row) * (D + 2);
-        const int64_t oo = (int64_t)b * p.os_b + (int64_t)(h * p.G + gh) * p.os_h + (int64_t)tq * p.os_t;
+        // a partial is stored column by column ([d + 2][256 rows]), so that the lanes of a store are neighbours
+        float* part = p.part + ((int64_t)blockIdx.x * 2 + (q.head ? 1 : 0)) * (256 * (D + 2)) + s * 128 + row;
+        const uint32_t stage = sO + warp * (32 * kPfOutRow);
+        uint16_t* orow[4];                       // the rows this lane writes 16 bytes of (null: not a query)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int rw = (warp & 3) * 32 + 8 * k + (lane >> 2), pw = rw / p.G, gw = rw - pw * p.G;
+          const int tw = (q.m * p.streams + s) * p.P + pw;
+          orow[k] = pw < p.P && tw < p.Tq ? reinterpret_cast<uint16_t*>(p.O) + (int64_t)b * p.os_b + (int64_t)(h * p.G + gw) * p.os_h +
+                                                (int64_t)tw * p.os_t + (lane & 3) * 8 : nullptr;
+        }
 #pragma unroll 1
         for (int c = 0; c < D; c += 32) {
           uint32_t o[32];
           __syncwarp();
           tc_ld32(o, tO + c);
           tc_wait_ld();
-          if (!live) continue;
           if (!whole) {
 #pragma unroll
-            for (int e = 0; e < 32; e += 2)
-              *reinterpret_cast<float2*>(part + c + e) = make_float2(__uint_as_float(o[e]) * mul, __uint_as_float(o[e + 1]) * mul);
+            for (int e = 0; e < 32; ++e) part[(c + e) * 256] = __uint_as_float(o[e]) * mul;
           } else if (p.o_vec) {
-            uint16_t* op = reinterpret_cast<uint16_t*>(p.O) + oo + c;
+            // through shared memory: four lanes of 16 bytes to a row's 32 columns
 #pragma unroll
             for (int e = 0; e < 32; e += 8) {
               uint32_t w[4];
@@ -424,18 +454,27 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
                 const float f0 = __uint_as_float(o[e + 2 * k]) * mul, f1 = __uint_as_float(o[e + 2 * k + 1]) * mul;
                 w[k] = (uint32_t)float_to_bits16(f0, p.o_dtype) | ((uint32_t)float_to_bits16(f1, p.o_dtype) << 16);
               }
-              *reinterpret_cast<uint4*>(op + e) = make_uint4(w[0], w[1], w[2], w[3]);
+              asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(stage + lane * kPfOutRow + 2 * e), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
             }
-          } else {
+            __syncwarp();
 #pragma unroll
-            for (int e = 0; e < 32; ++e) store_float(p.O, oo + c + e, __uint_as_float(o[e]) * mul, p.o_dtype);
+            for (int k = 0; k < 4; ++k) {
+              uint4 v;
+              asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                           : "r"(stage + (8 * k + (lane >> 2)) * kPfOutRow + (lane & 3) * 16) : "memory");
+              if (orow[k]) *reinterpret_cast<uint4*>(orow[k] + c) = v;
+            }
+          } else if (live) {
+            const int64_t oo = (int64_t)b * p.os_b + (int64_t)(h * p.G + gh) * p.os_h + (int64_t)tq * p.os_t + c;
+#pragma unroll
+            for (int e = 0; e < 32; ++e) store_float(p.O, oo + e, __uint_as_float(o[e]) * mul, p.o_dtype);
           }
         }
-        if (!whole && live) *reinterpret_cast<float2*>(part + D) = make_float2(m_run, l);
+        if (!whole) { part[D * 256] = m_run; part[(D + 1) * 256] = l; }
         __syncwarp();
         tc_fence_before();
       }
-      q = nq; have = more; ++u;
+      q = nq; have = more;
     }
   }
   }
@@ -448,49 +487,53 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
 }
 
 // ---- merge of the units that were cut between CTAs: blockIdx.x + 1 = a CTA whose piece starts inside a unit ----------------
+// blockIdx.y = 32 rows of the unit: a lane per row, a warp per D / 8 columns; the result is turned in shared memory.
 template <int D>
 __global__ void __launch_bounds__(256) prefill_merge_kernel(const PrefillParams p) {
+  constexpr int E = D / 8;
+  __shared__ float tile[32][D + 1];
   const int c = blockIdx.x + 1;
-  const int64_t pos = (int64_t)c * p.L;
   PfIter it;
-  it.init(p, pos);
+  it.init(p, c);
   if (it.off == 0) return;                                  // the unit starts with the CTA
-  const int64_t s_u = pos - it.off;
+  const int64_t s_u = (int64_t)c * p.L - it.off;
   if ((int64_t)(c - 1) * p.L > s_u) return;                 // the unit's first boundary does the merge
   const int c0 = c - 1, n_parts = (int)((s_u + it.n - 1) / p.L) - c0 + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = blockIdx.y * 32 + lane;
   const int bh = p.bh0 + it.bh, b = bh / p.Hkv, h = bh - b * p.Hkv;
+  // the CTA that holds the unit's first tile wrote its second slot, the others their first
+  constexpr int64_t kSlot = 256 * (D + 2);
+  const float* part = p.part + (int64_t)c0 * 2 * kSlot + row;
+  auto slot = [&](int k) { return part + k * 2 * kSlot + (k == 0 ? kSlot : 0); };
+  float m = -INFINITY;
+  for (int k = 0; k < n_parts; ++k) m = fmaxf(m, slot(k)[D * 256]);
+  const float mu = m == -INFINITY ? 0.f : m;
+  float l = 0.f, acc[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) acc[e] = 0.f;
+  for (int k = 0; k < n_parts; ++k) {
+    const float* pp = slot(k);
+    const float w = fast_exp2(pp[D * 256] - mu);
+    l = fmaf(pp[(D + 1) * 256], w, l);
+    const float* col = pp + warp * E * 256;
+#pragma unroll
+    for (int e = 0; e < E; ++e) acc[e] = fmaf(col[e * 256], w, acc[e]);
+  }
   const bool failed = *p.status == p.epoch;                 // the attention kernel gave up on a wait
-  constexpr int E = D / 32;
-  for (int row = blockIdx.y * 32 + warp; row < (blockIdx.y + 1) * 32; row += 8) {
-    const int s = row >> 7, rl = row & 127, pl = rl / p.G, gh = rl - pl * p.G;
+  const float inv = failed ? NAN : l > 0.f ? 1.f / l : 0.f;
+#pragma unroll
+  for (int e = 0; e < E; ++e) tile[lane][warp * E + e] = acc[e] * inv;
+  __syncthreads();
+  for (int i = threadIdx.x; i < 32 * D / 2; i += 256) {
+    const int rl = i / (D / 2), x = 2 * (i - rl * (D / 2)), r = blockIdx.y * 32 + rl, s = r >> 7, pl = (r & 127) / p.G, gh = (r & 127) - pl * p.G;
     const int tq = (it.m * p.streams + s) * p.P + pl;
     if (s >= p.streams || pl >= p.P || tq >= p.Tq) continue;
-    // the CTA that holds the unit's first tile wrote its second slot, the others their first
-    const float* part = p.part + ((int64_t)c0 * 2 * 256 + row) * (D + 2);
-    constexpr int64_t kCta = (int64_t)2 * 256 * (D + 2);
-    float m = -INFINITY;
-    for (int k = lane; k < n_parts; k += 32) m = fmaxf(m, part[k * kCta + (k == 0 ? 256 * (D + 2) : 0) + D]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    const float mu = m == -INFINITY ? 0.f : m;
-    float l = 0.f, acc[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) acc[e] = 0.f;
-    for (int k = 0; k < n_parts; ++k) {
-      const float* pp = part + k * kCta + (k == 0 ? 256 * (D + 2) : 0);
-      const float w = fast_exp2(pp[D] - mu);
-      l = fmaf(pp[D + 1], w, l);
-#pragma unroll
-      for (int e = 0; e < E; e += 2) {
-        const float2 v = *reinterpret_cast<const float2*>(pp + lane * E + e);
-        acc[e] = fmaf(v.x, w, acc[e]); acc[e + 1] = fmaf(v.y, w, acc[e + 1]);
-      }
-    }
-    const float inv = failed ? NAN : l > 0.f ? 1.f / l : 0.f;
-    const int64_t oo = (int64_t)b * p.os_b + (int64_t)(h * p.G + gh) * p.os_h + (int64_t)tq * p.os_t + lane * E;
-#pragma unroll
-    for (int e = 0; e < E; ++e) store_float(p.O, oo + e, acc[e] * inv, p.o_dtype);
+    const int64_t oo = (int64_t)b * p.os_b + (int64_t)(h * p.G + gh) * p.os_h + (int64_t)tq * p.os_t + x;
+    const float f0 = tile[rl][x], f1 = tile[rl][x + 1];
+    if (p.o_vec)
+      *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(p.O) + oo) =
+          (uint32_t)float_to_bits16(f0, p.o_dtype) | ((uint32_t)float_to_bits16(f1, p.o_dtype) << 16);
+    else { store_float(p.O, oo, f0, p.o_dtype); store_float(p.O, oo + 1, f1, p.o_dtype); }
   }
 }
 
@@ -609,33 +652,49 @@ __global__ void __launch_bounds__(256) prefill_expand_kernel(const ExpandParams 
         if (outl) myflag = pk.flags[(int64_t)bh * pk.T_cap + tb + lane];
       }
       if (is_v && lane < 16) s_fac[warp * 16 + lane] = myfac;
-#pragma unroll 4
-      for (int k = 0; k < 16; k += TPW) {
-        const int tl = warp * 16 + k + half, t = t0 + tl;
-        uint32_t f = 0u;
+      // all fields of the warp's tokens first (sixteen independent loads), then the flagged ones' payload positions
+      constexpr int NF = 16 / TPW;
+      uint32_t f[NF];
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
+        const int t = tb + k * TPW + half;
+        f[k] = 0u;
         if (t < e.Tkv) {
           if constexpr (LAYOUT == 0) {
             const uint32_t raw = row_field(reinterpret_cast<const uint32_t*>(pk.codes + ((int64_t)bh * pk.T_cap + t) * pk.row_bytes), c, cb);
-            f = (raw & ((1u << e.ib) - 1u)) | ((raw >> e.ib) << 16);
+            f[k] = (raw & ((1u << e.ib) - 1u)) | ((raw >> e.ib) << 16);
           } else {
-            long long i = load_int(rf.idx, b * rf.idx_stride[0] + h * rf.idx_stride[1] + t * rf.idx_stride[2] + c, rf.idx_dtype);
-            i = i < 0 ? 0 : (i >= e.table_rows ? e.table_rows - 1 : i);
-            long long r = load_int(rf.rq, b * rf.rq_stride[0] + h * rf.rq_stride[1] + t * rf.rq_stride[2] + c, rf.rq_dtype);
-            r = r < 0 ? 0 : (r > 1023 ? 1023 : r);
-            f = (uint32_t)i | ((uint32_t)r << 16);
+            const int64_t io = b * rf.idx_stride[0] + h * rf.idx_stride[1] + t * rf.idx_stride[2] + c;
+            const int64_t ro = b * rf.rq_stride[0] + h * rf.rq_stride[1] + t * rf.rq_stride[2] + c;
+            if (rf.idx_dtype == HQMQ_I32 && rf.rq_dtype == HQMQ_I32) {
+              const int i = reinterpret_cast<const int32_t*>(rf.idx)[io], r = reinterpret_cast<const int32_t*>(rf.rq)[ro];
+              f[k] = (uint32_t)min(max(i, 0), e.table_rows - 1) | ((uint32_t)min(max(r, 0), 1023) << 16);
+            } else {
+              long long i = load_int(rf.idx, io, rf.idx_dtype), r = load_int(rf.rq, ro, rf.rq_dtype);
+              i = i < 0 ? 0 : (i >= e.table_rows ? e.table_rows - 1 : i);
+              r = r < 0 ? 0 : (r > 1023 ? 1023 : r);
+              f[k] = (uint32_t)i | ((uint32_t)r << 16);
+            }
           }
         }
-        if (outl) {
-          const uint32_t w0 = __shfl_sync(0xffffffffu, myflag, k), w1 = N == 32 ? 0u : __shfl_sync(0xffffffffu, myflag, (k + 1) & 31);
+      }
+      if (outl) {
+#pragma unroll
+        for (int k = 0; k < NF; ++k) {
+          const uint32_t w0 = __shfl_sync(0xffffffffu, myflag, k * TPW), w1 = N == 32 ? 0u : __shfl_sync(0xffffffffu, myflag, k * TPW + TPW - 1);
           const uint32_t w = half ? w1 : w0;
-          if ((w >> c) & 1u) f = 0x80000000u | (run + (half ? __popc(w0) : 0u) + __popc(w & ((1u << c) - 1u)));
+          if ((w >> c) & 1u) f[k] = 0x80000000u | (run + (half ? __popc(w0) : 0u) + __popc(w & ((1u << c) - 1u)));
           run += __popc(w0) + (N == 32 ? 0 : __popc(w1));
         }
+      }
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
+        const int tl = warp * 16 + k * TPW + half;
         if (is_v) {
-          fields[tl * (N + 1) + c] = f;
+          fields[tl * (N + 1) + c] = f[k];
         } else {
-          const float fac = __shfl_sync(0xffffffffu, myfac, k + half);
-          const uint2 v = value_of(f, fac);
+          const float fac = __shfl_sync(0xffffffffu, myfac, k * TPW + half);
+          const uint2 v = value_of(f[k], fac);
           *reinterpret_cast<uint2*>(dst + (c >> 4) * 16384 + tl * 128 + ((((c & 15) >> 1) ^ (tl & 7)) << 4) + (c & 1) * 8) = v;
         }
       }
@@ -695,7 +754,7 @@ bool prefill_plan(const hqmq_attn_args* a, PrefillPlan& pl) {
   int64_t gb = (int64_t)(kPrefillImageBytes / ((size_t)p.nt * tile));
   pl.group = gb < 1 ? 1 : gb > bh_all ? bh_all : (int)gb;
   p.total = (int64_t)pl.group * p.Wh;
-  int64_t L = (p.total + 147) / 148;
+  int64_t L = (p.total + kPfMaxCtas - 1) / kPfMaxCtas;
   p.L = L < 1 ? 1 : L;
   pl.grid = (int)((p.total + p.L - 1) / p.L);
   pl.off_mul = 16;
@@ -748,6 +807,22 @@ int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspa
     p.total = (int64_t)n_bh * p.Wh;
     p.L = (p.total + pl.grid - 1) / pl.grid;
     const int grid = (int)((p.total + p.L - 1) / p.L);
+    // where every CTA's piece starts: its unit, and the tiles of the unit before it
+    {
+      int64_t at = 0;                 // flat position of unit m of the current (b, head)
+      int m = 0, lo, n;
+      pf_unit_tiles(p, m, lo, n);
+      for (int c = 0; c < grid; ++c) {
+        const int64_t pos = (int64_t)c * p.L;
+        if (pos - at >= p.Wh) at += (pos - at) / p.Wh * p.Wh;          // whole (b, head)s at once
+        while (pos - at >= n) {
+          at += n;
+          if (++m == p.units_m) m = 0;
+          pf_unit_tiles(p, m, lo, n);
+        }
+        p.start_m[c] = m; p.start_off[c] = (int)(pos - at);
+      }
+    }
     // tiles per expand CTA: about four CTAs per SM in all, so that a CTA's table and scale scan serve several tiles
     int64_t per = ((int64_t)p.nt * n_bh * 2 + 4 * 148 - 1) / (4 * 148);
     e.per = per < 1 ? 1 : per > p.nt ? p.nt : (int)per;

@@ -6,6 +6,7 @@ namespace hqmq {
 namespace attn {
 
 constexpr int kPfTok = 128;                       // tokens per operand tile
+constexpr int kPfMaxCtas = 148;                   // one CTA per SM
 constexpr int kPrefillMinQueries = 16;
 constexpr int kPrefillMaxTable = 8192;            // codewords per head that fit the expand kernel's shared memory
 constexpr size_t kPrefillImageBytes = (size_t)512 << 20;   // operand images held at a time; larger caches go by groups of (b, head)
@@ -21,8 +22,9 @@ struct PrefillParams {
   int64_t Wh, total, L;                           // tiles per (b, head), in all, per CTA
   const unsigned char* kimg; const unsigned char* vimg;
   const float* kmul; const float* vmul;           // [B * H_kv] what a score / an output is multiplied by
-  float* part;                                    // [CTA][2][256 rows][d + 2]
+  float* part;                                    // [CTA][2][d + 2][256 rows]
   uint32_t* status; uint32_t epoch;
+  int start_m[kPfMaxCtas], start_off[kPfMaxCtas];  // first unit of every CTA's piece, the unit's tiles before it
 };
 
 struct ExpandParams {
