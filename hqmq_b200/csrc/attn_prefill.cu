@@ -55,11 +55,13 @@ __host__ __device__ inline void pf_unit_tiles(const PrefillParams& p, int m, int
 }
 
 struct PfPiece { int bh, m, tile0, n; bool head, tail; };
-// The pieces of one CTA: its stretch [c * L, (c + 1) * L) of the flat tile sequence, unit by unit.
+// The pieces of one CTA.  Cut mode (p.L > 0): its stretch [c * L, (c + 1) * L) of the flat tile sequence, unit by unit.
+// Whole mode: units in order of m falling (with a causal mask: of length falling), dealt out to the CTAs to and fro.
 struct PfIter {
-  int left;
+  int left;                      // tiles left of the piece; whole mode: index of the next unit in the CTA's hand
   int bh, m, off, lo, n;
   __device__ __forceinline__ void init(const PrefillParams& p, int cta) {
+    if (p.L == 0) { left = 0; return; }
     const int64_t pos = (int64_t)cta * p.L;
     left = (int)(p.total - pos < p.L ? p.total - pos : p.L);
     bh = (int)(pos / p.Wh);
@@ -67,6 +69,17 @@ struct PfIter {
     pf_unit_tiles(p, m, lo, n);
   }
   __device__ __forceinline__ bool next(const PrefillParams& p, PfPiece& q) {
+    if (p.L == 0) {
+      const int G = (int)gridDim.x, c = (int)blockIdx.x;
+      const int i = left * G + ((left & 1) ? G - 1 - c : c);
+      if (i >= p.units_all) return false;
+      ++left;
+      const int n_bh = p.units_all / p.units_m, j = i / n_bh;
+      q.bh = i - j * n_bh; q.m = p.units_m - 1 - j;
+      pf_unit_tiles(p, q.m, q.tile0, q.n);
+      q.head = q.tail = true;
+      return true;
+    }
     if (left <= 0) return false;
     if (off >= n) {
       off = 0;
@@ -129,6 +142,19 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
 // kind::f16, fp16 operands (both K-major), fp32 accumulators
 __host__ __device__ constexpr uint32_t f16_idesc(int M, int N) { return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24); }
 
+// Two fp32 operations per instruction.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+  return d;
+}
+
 // ---- attend ----------------------------------------------------------------------------------------------------------------
 template <int D>
 __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const PrefillParams p) {
@@ -139,25 +165,23 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
   unsigned char* base = smem_raw + (s_base - smem_u32(smem_raw));
   const uint32_t sQ = s_base, sK = sQ + 2 * TB, sV = sK + NS * TB, sO = sV + NS * TB, bars = sO + 8 * 32 * kPfOutRow;
   const uint32_t kfull = bars, kempty = kfull + 8 * NS, vfull = kempty + 8 * NS, vempty = vfull + 8 * NS;
-  // per stream: queries written; S of either half computed / its P written; P V of a half done
-  const uint32_t qfull = vempty + 8 * NS, sfull = qfull + 16, pfull = sfull + 32, pvdone = pfull + 32;
-  volatile uint32_t* abort_word = reinterpret_cast<volatile uint32_t*>(base + (pvdone + 32 - s_base));
+  // per stream: queries written, S of a tile computed, either half of its P written, the unit's last P V done
+  const uint32_t qfull = vempty + 8 * NS, sfull = qfull + 16, pfull = sfull + 16, odone = pfull + 32;
+  volatile uint32_t* abort_word = reinterpret_cast<volatile uint32_t*>(base + (odone + 16 - s_base));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) {
       mbar_init(kfull + 8 * i, 1); mbar_init(kempty + 8 * i, p.streams); mbar_init(vfull + 8 * i, 1); mbar_init(vempty + 8 * i, p.streams);
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(qfull + 8 * s, 4);
-      for (int hb = 0; hb < 2; ++hb) {
-        mbar_init(sfull + 16 * s + 8 * hb, 1); mbar_init(pfull + 16 * s + 8 * hb, 4); mbar_init(pvdone + 16 * s + 8 * hb, 1);
-      }
+      mbar_init(qfull + 8 * s, 4); mbar_init(sfull + 8 * s, 1); mbar_init(odone + 8 * s, 1);
+      mbar_init(pfull + 16 * s, 4); mbar_init(pfull + 16 * s + 8, 4);
     }
     *abort_word = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 8) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pvdone + 36), "n"(kPfTmemCols) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(odone + 20), "n"(kPfTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
@@ -216,54 +240,46 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
     PfPiece q;
     it.init(p, (int)blockIdx.x);
     auto wait_w = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, wait(bar, parity)) != 0; };   // one answer per warp
-    constexpr uint32_t id_qk = f16_idesc(128, 64), id_pv = f16_idesc(128, D);
-    // S of half hb of the tile in stage st; O += P V of that half
-    auto qk = [&](uint32_t st, int hb) {
-      const uint64_t a0 = sw128_desc(sQ + s * TB), b0 = sw128_desc(sK + st * TB + hb * 8192);
+    constexpr uint32_t id_qk = f16_idesc(128, 128), id_pv = f16_idesc(128, D);
+    // S of the tile in stage st; O += P V of half hb of its keys
+    auto qk = [&](uint32_t st) {
+      const uint64_t a0 = sw128_desc(sQ + s * TB), b0 = sw128_desc(sK + st * TB);
 #pragma unroll
       for (int k = 0; k < D / 16; ++k) {
         const uint32_t o = ((k >> 2) * 16384 + (k & 3) * 32) >> 4;
-        tc_mma_ss(128 * s + 64 * hb, a0 + o, b0 + o, id_qk, k > 0 ? 1u : 0u);
+        tc_mma_ss(128 * s, a0 + o, b0 + o, id_qk, k > 0 ? 1u : 0u);
       }
-      tc_commit(sfull + 16 * s + 8 * hb);
+      tc_commit(sfull + 8 * s);
+      tc_commit(kempty + 8 * st);
     };
     auto pv = [&](uint32_t st, int hb, bool acc) {
       const uint64_t b0 = sw128_desc(sV + st * TB + hb * (D * 128));
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        tc_mma_ts(256 + D * s, 128 * s + 64 * hb + 8 * k, b0 + ((k * 32) >> 4), id_pv, acc || k > 0 ? 1u : 0u);
-      tc_commit(pvdone + 16 * s + 8 * hb);
+        tc_mma_ts(256 + D * s, 128 * s + 32 * hb + 8 * k, b0 + ((k * 32) >> 4), id_pv, acc || k > 0 ? 1u : 0u);
     };
     uint32_t g = 0, u = 0;     // tiles, units
     bool ok = true;
     while (ok && it.next(p, q)) {
-      // the unit's first S, both halves
       ok = wait_w(kfull + 8 * (g % NS), (g / NS) & 1u) && wait_w(qfull + 8 * s, u & 1u);
       if (!ok) break;
       tc_fence_after();
-      if (elect_one()) {
-        qk(g % NS, 0);
-        qk(g % NS, 1);
-        tc_commit(kempty + 8 * (g % NS));
-      }
-      // half by half: P V of this tile's half, then Q K^T of the next tile's half into the columns that P has left
+      if (elect_one()) qk(g % NS);
       for (int i = 0; i < q.n && ok; ++i, ++g) {
         const bool last = i + 1 == q.n;
         const uint32_t st = g % NS, ph = (g / NS) & 1u, st1 = (g + 1) % NS, ph1 = ((g + 1) / NS) & 1u;
-        ok = wait_w(vfull + 8 * st, ph) && (last || wait_w(kfull + 8 * st1, ph1));
-#pragma unroll
-        for (int hb = 0; hb < 2; ++hb) {
-          ok = ok && wait_w(pfull + 16 * s + 8 * hb, g & 1u);
-          if (!ok) break;
-          tc_fence_after();
-          if (elect_one()) {
-            pv(st, hb, i > 0 || hb > 0);
-            if (hb) tc_commit(vempty + 8 * st);
-            if (!last) {
-              qk(st1, hb);
-              if (hb) tc_commit(kempty + 8 * st1);
-            }
-          }
+        ok = wait_w(vfull + 8 * st, ph) && (last || wait_w(kfull + 8 * st1, ph1)) && wait_w(pfull + 16 * s, g & 1u);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) pv(st, 0, i > 0);
+        ok = wait_w(pfull + 16 * s + 8, g & 1u);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          pv(st, 1, true);
+          if (last) tc_commit(odone + 8 * s);
+          tc_commit(vempty + 8 * st);
+          if (!last) qk(st1);
         }
       }
       ++u;
@@ -290,10 +306,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
       const int tq0 = (w.m * p.streams + s) * p.P;
       int pw = ((warp & 3) * 32 + lane / QL) / p.G, gw = (warp & 3) * 32 + lane / QL - pw * p.G;
 #pragma unroll
-      for (int k0 = 0; k0 < QL; k0 += 8) {       // eight loads in flight
-        uint4 v[8];
+      for (int k0 = 0; k0 < QL; k0 += QL) {       // all of them in flight
+        uint4 v[QL];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < QL; ++k) {
           const bool live = pw < p.P && tq0 + pw < p.Tq;
           const int64_t o = qb + (int64_t)gw * p.qs_h + (int64_t)(tq0 + pw) * p.qs_t;
           v[k] = make_uint4(0u, 0u, 0u, 0u);
@@ -309,7 +325,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
           while (gw >= p.G) { gw -= p.G; ++pw; }
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < QL; ++k) {
           if (p.q_vec && p.q_dtype == HQMQ_BF16) {
             uint32_t* w4 = reinterpret_cast<uint32_t*>(&v[k]);
 #pragma unroll
@@ -327,7 +343,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
     PfIter it;
     PfPiece q;
     it.init(p, (int)blockIdx.x);
-    uint32_t g = 0;
+    uint32_t g = 0, u = 0;
     bool have = it.next(p, q), ok = true;
     if (have) load_q(q);
     while (ok && have) {
@@ -342,29 +358,29 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
       const int w_beg = __reduce_max_sync(0xffffffffu, beg), w_end = __reduce_min_sync(0xffffffffu, end);
       const bool w_live = __any_sync(0xffffffffu, live);
       const float kmul = p.kmul[bh];
-      float m_run = -INFINITY, l0 = 0.f, l1 = 0.f;
-      for (int i = 0; i < 2 * q.n; ++i) {
-        const int hb = i & 1;
-        const uint32_t ph = (g + (i >> 1)) & 1u, tH = tS + 64 * hb;
-        ok = wait(sfull + 16 * s + 8 * hb, ph);
+      float m_run = -INFINITY;
+      float2 l2 = make_float2(0.f, 0.f);
+      const float2 kmul2 = make_float2(kmul, kmul);
+      for (int i = 0; i < q.n; ++i, ++g) {
+        ok = wait(sfull + 8 * s, g & 1u);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
         if (w_live) {
-          uint32_t r[64];
-          tc_ld32(r, tH);
-          tc_ld32(r + 32, tH + 32);
+          uint32_t r[128];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tc_ld32(r + 32 * c, tS + 32 * c);
           tc_wait_ld();
-          const int t0 = q.tile0 * kPfTok + 64 * i;
-          if (t0 < w_beg || t0 + 64 > w_end) {
+          const int t0 = (q.tile0 + i) * kPfTok;
+          if (t0 < w_beg || t0 + kPfTok > w_end) {
             const int lo = beg - t0, hi = end - t0;
 #pragma unroll
-            for (int c = 0; c < 64; ++c)
+            for (int c = 0; c < 128; ++c)
               if (c < lo || c >= hi) r[c] = 0xff800000u;
           }
           float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-          for (int c = 0; c < 64; c += 8)
+          for (int c = 0; c < 128; c += 8)
 #pragma unroll
             for (int e = 0; e < 4; ++e)
               mx[e] = fmaxf(mx[e], fmaxf(__uint_as_float(r[c + 2 * e]), __uint_as_float(r[c + 2 * e + 1])));
@@ -373,14 +389,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
             const float m_new = fmaxf(m_run, mc);
             const float alpha = m_new == -INFINITY ? 1.f : fast_exp2(m_run - m_new);
             m_run = m_new;
-            l0 *= alpha; l1 *= alpha;
+            l2.x *= alpha; l2.y *= alpha;
             if (i > 0) {
-              // the accumulator is rescaled once the previous half's P V is done (the one before it is: this S was issued
-              // behind it)
-              ok = wait(pvdone + 16 * s + 8 * (hb ^ 1), hb ? ph : ph ^ 1u);
-              ok = __all_sync(0xffffffffu, ok);
-              if (!ok) break;
-              tc_fence_after();
+              // (S of this tile was issued behind the previous tile's P V: the accumulator is complete)
 #pragma unroll 1
               for (int c = 0; c < D; c += 32) {
                 uint32_t o[32];
@@ -393,35 +404,42 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
             }
           }
           const float nb = m_run == -INFINITY ? 0.f : -m_run;
-          uint32_t pk[32];
+          const float2 nb2 = make_float2(nb, nb);
+          // P goes to the tensor cores in halves of 64 keys: the first half's P V runs under the second half's exponentials
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const float a = fast_exp2(fmaf(__uint_as_float(r[2 * e]), kmul, nb));
-            const float b = fast_exp2(fmaf(__uint_as_float(r[2 * e + 1]), kmul, nb));
-            const __half2 h = __floats2half2_rn(a, b);
-            // (the weights that are summed are the rounded ones the tensor cores see: the rounding cancels)
-            const float2 f = __half22float2(h);
-            l0 += f.x; l1 += f.y;
-            pk[e] = *reinterpret_cast<const uint32_t*>(&h);
+          for (int hb = 0; hb < 2; ++hb) {
+            uint32_t pk[32];
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+              float2 x = fma2(make_float2(__uint_as_float(r[64 * hb + 2 * e]), __uint_as_float(r[64 * hb + 2 * e + 1])), kmul2, nb2);
+              x.x = fast_exp2(x.x); x.y = fast_exp2(x.y);
+              const __half2 h = __float22half2_rn(x);
+              // (the weights that are summed are the rounded ones the tensor cores see: the rounding cancels)
+              l2 = add2(l2, __half22float2(h));
+              pk[e] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            tc_st32(tS + 32 * hb, pk);
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(pfull + 16 * s + 8 * hb);
           }
-          tc_st32(tH, pk);
-          tc_wait_st();
+        } else {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) { mbar_arrive(pfull + 16 * s); mbar_arrive(pfull + 16 * s + 8); }
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(pfull + 16 * s + 8 * hb);
       }
       if (!ok) break;
-      g += q.n;
       // the last Q K^T of the unit is complete: the next unit's queries may take the place of this one's
       if (more) load_q(nq);
-      ok = wait(pvdone + 16 * s + 8, (g - 1) & 1u);
+      ok = wait(odone + 8 * s, u & 1u);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
       if (w_live) {
         const int b = bh / p.Hkv, h = bh - b * p.Hkv;
-        const float l = l0 + l1, vmul = p.vmul[bh];
+        const float l = l2.x + l2.y, vmul = p.vmul[bh];
         const bool whole = q.head && q.tail;
         const float mul = whole ? (l > 0.f ? vmul / l : 0.f) : vmul;
         // a partial is stored column by column ([d + 2][256 rows]), so that the lanes of a store are neighbours
@@ -474,7 +492,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
         __syncwarp();
         tc_fence_before();
       }
-      q = nq; have = more;
+      q = nq; have = more; ++u;
     }
   }
   }
@@ -547,11 +565,13 @@ __device__ __forceinline__ void pf_scale_of(float big, float& mul, float& inv) {
 }
 
 // grid (tile chunks, (b, head) of the group, 2): blockIdx.z = 0 K, 1 V.  Eight warps; a warp takes the 16 tokens of one
-// outlier block of the tile with a lane per chunk (rows and flag words are read in order, so a flagged chunk's payload entry
-// is a running count).  K goes straight to its image (the lanes of a token fill whole 128-byte rows); V is unpacked to
-// shared memory first and decoded with a lane per token, so that the transposed image is written 64 bytes at a time.
+// outlier block of the tile with a lane per chunk.  K goes straight to its image (the lanes of a token fill whole 128-byte
+// rows); V is unpacked to shared memory first and decoded with a lane per token, so that the transposed image is written 64
+// bytes at a time.  Flagged chunks decode to zero (radius code 0) and are overwritten afterwards from a list of the block's
+// entries, a lane per entry: the payload is then read in order, 32 entries at a time.  (Looked up chunk by chunk inside the
+// decode loop they tripled its instructions: 46 us for 8192 tokens of 8 heads, K with 6 % flagged.)
 template <int N, int LAYOUT>
-__global__ void __launch_bounds__(256) prefill_expand_kernel(const ExpandParams e) {
+__global__ void __launch_bounds__(256, 3) prefill_expand_kernel(const ExpandParams e) {
   constexpr int D = 4 * N;
   constexpr uint32_t TB = (uint32_t)pf_tile_bytes(D);
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -559,6 +579,7 @@ __global__ void __launch_bounds__(256) prefill_expand_kernel(const ExpandParams 
   uint32_t* fields = reinterpret_cast<uint32_t*>(smem_raw + (blockIdx.z ? TB : 0));         // V only: [128][N + 1]
   uint2* tbl = reinterpret_cast<uint2*>(smem_raw + (blockIdx.z ? TB + 128 * (N + 1) * 4 : 0));
   __shared__ float s_big[8], s_fac[kPfTok];
+  __shared__ uint16_t s_list[8][16 * N];       // (token of the block) * 32 + chunk of the block's payload entries
   const bool is_v = blockIdx.z != 0;
   const hqmq_packed& pk = is_v ? e.V : e.K;
   const hqmq_ref_packed& rf = is_v ? e.Vr : e.Kr;
@@ -607,52 +628,65 @@ __global__ void __launch_bounds__(256) prefill_expand_kernel(const ExpandParams 
   pf_scale_of(big, mul, inv);
   if (blockIdx.x == 0 && threadIdx.x == 0) (is_v ? e.vmul : e.kmul)[bh] = is_v ? inv : inv * e.qscale;
 
+  // what this lane needs of the planes, as bases and 32-bit steps (a lane keeps its chunk for the whole kernel)
   const bool outl = LAYOUT == 0 && pk.flags != nullptr;
-  const int cb = e.ib + pk.radius_bits;
-  const unsigned char* vals = reinterpret_cast<const unsigned char*>(pk.out_vals) + (int64_t)bh * pk.out_cap * 4 * (pk.out_dtype == HQMQ_F32 ? 4 : 2);
-  // four fp16 values of a chunk: an outlier's payload entry (bit 31 set), or codeword and radius code
-  auto value_of = [&](uint32_t f, float fac) {
-    float x0, x1, x2, x3;
-    if (outl && (f >> 31)) {
-      const uint32_t slot = f & 0x7fffffffu;
-      x0 = x1 = x2 = x3 = 0.f;
-      if (slot < (uint32_t)pk.out_cap) {          // (an entry the encoder dropped reads as 0)
-        if (pk.out_dtype == HQMQ_F32) {
-          const float4 v = *reinterpret_cast<const float4*>(vals + (int64_t)slot * 16);
-          x0 = v.x; x1 = v.y; x2 = v.z; x3 = v.w;
-        } else {
-          const uint2 v = *reinterpret_cast<const uint2*>(vals + (int64_t)slot * 8);
-          const float2 a = pair16_to_float2(v.x, pk.out_dtype), c = pair16_to_float2(v.y, pk.out_dtype);
-          x0 = a.x; x1 = a.y; x2 = c.x; x3 = c.y;
-        }
-      }
-      fac = mul;
-    } else {
-      const uint2 cw = tbl[f & 0xffffu];
-      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&cw.x)), c = __half22float2(*reinterpret_cast<const __half2*>(&cw.y));
-      fac *= (float)(f >> 16);
-      x0 = a.x; x1 = a.y; x2 = c.x; x3 = c.y;
-    }
-    return make_uint2(pack_half2(x0 * fac, x1 * fac), pack_half2(x2 * fac, x3 * fac));
-  };
-
   constexpr int TPW = 32 / N;                 // tokens a warp takes at a time
   const int half = N == 32 ? 0 : lane >> 4, c = N == 32 ? lane : lane & 15;
+  const uint32_t* rows = nullptr;
+  int row_words = 0, w1 = 0, sh = 0;
+  uint32_t imask = 0u, fmask = 0u;
+  if constexpr (LAYOUT == 0) {
+    const int cb = e.ib + pk.radius_bits, bit = c * cb;
+    row_words = pk.row_bytes >> 2;
+    rows = reinterpret_cast<const uint32_t*>(pk.codes + (int64_t)bh * pk.T_cap * pk.row_bytes) + (bit >> 5);
+    sh = bit & 31; w1 = sh + cb > 32 ? 1 : 0;
+    imask = (1u << e.ib) - 1u; fmask = (1u << cb) - 1u;
+  }
+  const bool out32 = outl && pk.out_dtype == HQMQ_F32;
+  const unsigned char* vals = outl ? reinterpret_cast<const unsigned char*>(pk.out_vals) + (int64_t)bh * pk.out_cap * (out32 ? 16 : 8) : nullptr;
+  const uint32_t cap = outl ? (uint32_t)pk.out_cap : 0u;
+  const int out_dtype = pk.out_dtype;
+  const uint32_t* flags = outl ? pk.flags + (int64_t)bh * pk.T_cap : nullptr;
+  const uint32_t* offs = outl ? pk.out_off + (int64_t)bh * (pk.T_cap / HQMQ_OUT_BLOCK + 1) : nullptr;
+  // four fp16 values of a chunk from its codeword and radius code
+  auto value_of = [&](uint32_t f, float fac) {
+    const uint2 cw = tbl[f & 0xffffu];
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&cw.x)), c = __half22float2(*reinterpret_cast<const __half2*>(&cw.y));
+    fac *= (float)(f >> 16);
+    return make_uint2(pack_half2(a.x * fac, a.y * fac), pack_half2(c.x * fac, c.y * fac));
+  };
+  // ... of a flagged chunk from its payload entry (an entry the encoder dropped reads as 0)
+  auto payload_of = [&](uint32_t slot) {
+    if (slot >= cap) return make_uint2(0u, 0u);
+    if (out32) {
+      const float4 v = *reinterpret_cast<const float4*>(vals + (int64_t)slot * 16);
+      return make_uint2(pack_half2(v.x * mul, v.y * mul), pack_half2(v.z * mul, v.w * mul));
+    }
+    return *reinterpret_cast<const uint2*>(vals + (int64_t)slot * 8);
+  };
+  auto payload_half = [&](uint2 v) {           // (16-bit entries are converted when they are used)
+    if (out32) return v;
+    const float2 a = pair16_to_float2(v.x, out_dtype), d = pair16_to_float2(v.y, out_dtype);
+    return make_uint2(pack_half2(a.x * mul, a.y * mul), pack_half2(d.x * mul, d.y * mul));
+  };
+  // V^T image: the four dims of chunk cc of token tl
+  auto put_v = [&](int tl, int cc, uint2 v) {
+    unsigned char* im = reinterpret_cast<unsigned char*>(img) + (tl >> 6) * (D * 128) + (tl & 7) * 2 + cc * 512;
+    const int sw = ((tl & 63) >> 3) ^ ((cc & 1) * 4);
+    *reinterpret_cast<uint16_t*>(im + (sw << 4)) = (uint16_t)v.x;
+    *reinterpret_cast<uint16_t*>(im + 128 + ((sw ^ 1) << 4)) = (uint16_t)(v.x >> 16);
+    *reinterpret_cast<uint16_t*>(im + 256 + ((sw ^ 2) << 4)) = (uint16_t)v.y;
+    *reinterpret_cast<uint16_t*>(im + 384 + ((sw ^ 3) << 4)) = (uint16_t)(v.y >> 16);
+  };
   const int tile_hi = min(e.nt, (int)(blockIdx.x + 1) * e.per);
   for (int tile = blockIdx.x * e.per; tile < tile_hi; ++tile) {
     const int t0 = (e.kt0 + tile) * kPfTok;
     unsigned char* dst = (is_v ? e.vimg : e.kimg) + ((int64_t)blockIdx.y * e.nt + tile) * TB;
+    uint32_t n_ent = 0u, run = 0u;
+    uint2 ent = make_uint2(0u, 0u);
     {
       const int tb = t0 + warp * 16;
-      uint32_t run = outl && tb < e.Tkv ? pk.out_off[(int64_t)bh * (pk.T_cap / HQMQ_OUT_BLOCK + 1) + tb / HQMQ_OUT_BLOCK] : 0u;
-      float myfac = 0.f;                     // lanes 0..15: the factor of the block's tokens
-      uint32_t myflag = 0u;
-      if (lane < 16 && tb + lane < e.Tkv) {
-        myfac = scale_of(tb + lane) * e.vscale * mul;
-        if (outl) myflag = pk.flags[(int64_t)bh * pk.T_cap + tb + lane];
-      }
-      if (is_v && lane < 16) s_fac[warp * 16 + lane] = myfac;
-      // all fields of the warp's tokens first (sixteen independent loads), then the flagged ones' payload positions
+      // all fields of the warp's tokens first (independent loads), with the scales and flag words of the block
       constexpr int NF = 16 / TPW;
       uint32_t f[NF];
 #pragma unroll
@@ -661,8 +695,9 @@ __global__ void __launch_bounds__(256) prefill_expand_kernel(const ExpandParams 
         f[k] = 0u;
         if (t < e.Tkv) {
           if constexpr (LAYOUT == 0) {
-            const uint32_t raw = row_field(reinterpret_cast<const uint32_t*>(pk.codes + ((int64_t)bh * pk.T_cap + t) * pk.row_bytes), c, cb);
-            f[k] = (raw & ((1u << e.ib) - 1u)) | ((raw >> e.ib) << 16);
+            const uint32_t* r = rows + t * row_words;
+            const uint32_t raw = __funnelshift_r(r[0], r[w1], sh) & fmask;
+            f[k] = (raw & imask) | ((raw >> e.ib) << 16);
           } else {
             const int64_t io = b * rf.idx_stride[0] + h * rf.idx_stride[1] + t * rf.idx_stride[2] + c;
             const int64_t ro = b * rf.rq_stride[0] + h * rf.rq_stride[1] + t * rf.rq_stride[2] + c;
@@ -678,15 +713,27 @@ __global__ void __launch_bounds__(256) prefill_expand_kernel(const ExpandParams 
           }
         }
       }
-      if (outl) {
-#pragma unroll
-        for (int k = 0; k < NF; ++k) {
-          const uint32_t w0 = __shfl_sync(0xffffffffu, myflag, k * TPW), w1 = N == 32 ? 0u : __shfl_sync(0xffffffffu, myflag, k * TPW + TPW - 1);
-          const uint32_t w = half ? w1 : w0;
-          if ((w >> c) & 1u) f[k] = 0x80000000u | (run + (half ? __popc(w0) : 0u) + __popc(w & ((1u << c) - 1u)));
-          run += __popc(w0) + (N == 32 ? 0 : __popc(w1));
-        }
+      float myfac = 0.f;                     // lanes 0..15: the factor of the block's tokens
+      uint32_t myflag = 0u;
+      if (lane < 16 && tb + lane < e.Tkv) {
+        myfac = scale_of(tb + lane) * e.vscale * mul;
+        if (outl) myflag = flags[tb + lane];
       }
+      if (is_v && lane < 16) s_fac[warp * 16 + lane] = myfac;
+      // the block's payload entries in order; the first 32 are fetched now
+      const uint32_t mine = __popc(myflag), incl = outl ? [&] { uint32_t v = mine;
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += y; }
+        return v; }() : 0u;
+      n_ent = __shfl_sync(0xffffffffu, incl, 15);
+      if (n_ent) {
+        run = offs[tb / HQMQ_OUT_BLOCK];
+        uint32_t pos = incl - mine;
+        for (uint32_t w = myflag; w; w &= w - 1u) s_list[warp][pos++] = (uint16_t)(lane * 32 + __ffs(w) - 1);
+        __syncwarp();
+        if (lane < n_ent) ent = payload_of(run + lane);
+      }
+      unsigned char* kd = dst + (c >> 4) * 16384 + (c & 1) * 8;
 #pragma unroll
       for (int k = 0; k < NF; ++k) {
         const int tl = warp * 16 + k * TPW + half;
@@ -694,31 +741,39 @@ __global__ void __launch_bounds__(256) prefill_expand_kernel(const ExpandParams 
           fields[tl * (N + 1) + c] = f[k];
         } else {
           const float fac = __shfl_sync(0xffffffffu, myfac, k * TPW + half);
-          const uint2 v = value_of(f[k], fac);
-          *reinterpret_cast<uint2*>(dst + (c >> 4) * 16384 + tl * 128 + ((((c & 15) >> 1) ^ (tl & 7)) << 4) + (c & 1) * 8) = v;
+          *reinterpret_cast<uint2*>(kd + tl * 128 + ((((c & 15) >> 1) ^ (tl & 7)) << 4)) = value_of(f[k], fac);
         }
       }
     }
-    if (is_v) {
+    auto put_entries = [&](auto put) {         // put(token of the tile, chunk, values)
+      for (uint32_t i = lane; i < n_ent; i += 32) {
+        if (i != lane) ent = payload_of(run + i);
+        const uint32_t at = s_list[warp][i];
+        put(warp * 16 + (int)(at >> 5), (int)(at & 31u), payload_half(ent));
+      }
+      __syncwarp();
+    };
+    if (!is_v) {
+      __syncwarp();                            // (the zeros of the flagged chunks were stored by other lanes)
+      put_entries([&](int tl, int cc, uint2 v) {
+        *reinterpret_cast<uint2*>(dst + (cc >> 4) * 16384 + tl * 128 + ((((cc & 15) >> 1) ^ (tl & 7)) << 4) + (cc & 1) * 8) = v;
+      });
+    } else {
       __syncthreads();
       const int tl = (warp & 3) * 32 + lane;
       const float fac = s_fac[tl];
-      unsigned char* im = reinterpret_cast<unsigned char*>(img) + (tl >> 6) * (D * 128) + (tl & 7) * 2;
-      const int oct = (tl & 63) >> 3;
-#pragma unroll 4
+#pragma unroll 8
       for (int k = 0; k < N / 2; ++k) {
         const int cc = (warp >> 2) * (N / 2) + k;
-        const uint2 v = value_of(fields[tl * (N + 1) + cc], fac);
-        const uint32_t w[2] = {v.x, v.y};
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const int d = 4 * cc + x;
-          *reinterpret_cast<uint16_t*>(im + d * 128 + ((oct ^ (d & 7)) << 4)) = (uint16_t)(w[x >> 1] >> (16 * (x & 1)));
-        }
+        put_v(tl, cc, value_of(fields[tl * (N + 1) + cc], fac));
+      }
+      if (outl) {
+        __syncthreads();
+        put_entries(put_v);
       }
       __syncthreads();
       for (int i = threadIdx.x; i < (int)(TB / 16); i += 256) reinterpret_cast<uint4*>(dst)[i] = img[i];
-      // (a warp ahead writes the next tile's `fields` and `s_fac` meanwhile; `img` only behind the next barrier)
+      // (a warp ahead writes the next tile's `fields`, `s_fac` and list meanwhile; `img` only behind the next barrier)
     }
   }
 }
@@ -753,14 +808,31 @@ bool prefill_plan(const hqmq_attn_args* a, PrefillPlan& pl) {
   // the operand images of as many (b, head) at a time as kPrefillImageBytes hold
   int64_t gb = (int64_t)(kPrefillImageBytes / ((size_t)p.nt * tile));
   pl.group = gb < 1 ? 1 : gb > bh_all ? bh_all : (int)gb;
+  // Whole units per CTA, or equal pieces of the flat sequence?  Costs in tiles: every unit about two (its queries, pipeline
+  // fill, output), cut units one more for each partial, and the merge launch about six.
+  const int n_units = pl.group * p.units_m;
   p.total = (int64_t)pl.group * p.Wh;
-  int64_t L = (p.total + kPfMaxCtas - 1) / kPfMaxCtas;
-  p.L = L < 1 ? 1 : L;
-  pl.grid = (int)((p.total + p.L - 1) / p.L);
+  const int64_t L = (p.total + kPfMaxCtas - 1) / kPfMaxCtas;
+  const int grid_w = n_units < kPfMaxCtas ? n_units : kPfMaxCtas;
+  int64_t whole = 0;
+  for (int c = 0; c < grid_w; ++c) {
+    int64_t t = 0;
+    for (int k = 0;; ++k) {
+      const int i = k * grid_w + ((k & 1) ? grid_w - 1 - c : c);
+      if (i >= n_units) break;
+      int lo, n;
+      pf_unit_tiles(p, p.units_m - 1 - i / pl.group, lo, n);
+      t += n + 2;
+    }
+    whole = t > whole ? t : whole;
+  }
+  const int64_t cut = L + 2 * ((n_units + kPfMaxCtas - 1) / kPfMaxCtas + 1) + 2 + 6;
+  pl.whole = whole <= cut;
+  pl.grid = pl.whole ? grid_w : (int)((p.total + (L < 1 ? 1 : L) - 1) / (L < 1 ? 1 : L));
   pl.off_mul = 16;
   pl.off_img = (16 + (size_t)bh_all * 8 + 255) & ~(size_t)255;
   pl.off_part = pl.off_img + (size_t)pl.group * p.nt * tile;
-  pl.ws_bytes = pl.off_part + (size_t)pl.grid * 2 * 256 * (a->d + 2) * sizeof(float);
+  pl.ws_bytes = pl.off_part + (pl.whole ? 0 : (size_t)pl.grid * 2 * 256 * (a->d + 2) * sizeof(float));
   return true;
 }
 
@@ -805,10 +877,11 @@ int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspa
     const int n_bh = bh_all - bh0 < pl.group ? bh_all - bh0 : pl.group;
     e.bh0 = p.bh0 = bh0;
     p.total = (int64_t)n_bh * p.Wh;
-    p.L = (p.total + pl.grid - 1) / pl.grid;
-    const int grid = (int)((p.total + p.L - 1) / p.L);
+    p.units_all = n_bh * p.units_m;
+    p.L = pl.whole ? 0 : (p.total + pl.grid - 1) / pl.grid;
+    const int grid = pl.whole ? (p.units_all < pl.grid ? p.units_all : pl.grid) : (int)((p.total + p.L - 1) / p.L);
     // where every CTA's piece starts: its unit, and the tiles of the unit before it
-    {
+    if (!pl.whole) {
       int64_t at = 0;                 // flat position of unit m of the current (b, head)
       int m = 0, lo, n;
       pf_unit_tiles(p, m, lo, n);
@@ -823,14 +896,15 @@ int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspa
         p.start_m[c] = m; p.start_off[c] = (int)(pos - at);
       }
     }
-    // tiles per expand CTA: about four CTAs per SM in all, so that a CTA's table and scale scan serve several tiles
-    int64_t per = ((int64_t)p.nt * n_bh * 2 + 4 * 148 - 1) / (4 * 148);
+    // tiles per expand CTA: about six CTAs per SM in all (three at a time), so that a CTA's table and scale scan serve
+    // several tiles of a long cache
+    const int64_t per = ((int64_t)p.nt * n_bh * 2 + 6 * kPfMaxCtas - 1) / (6 * kPfMaxCtas);
     e.per = per < 1 ? 1 : per > p.nt ? p.nt : (int)per;
     void* ea[] = {&e};
     HQMQ_CHECK_CUDA(cudaLaunchKernel(ek, dim3((p.nt + e.per - 1) / e.per, n_bh, 2), dim3(256), ea, esmem, st));
     void* pa[] = {&p};
     HQMQ_CHECK_CUDA(cudaLaunchKernel(ak, dim3(grid), dim3(kPfThreads), pa, pf_smem_bytes(d), st));
-    if (grid > 1) HQMQ_CHECK_CUDA(cudaLaunchKernel(mk, dim3(grid - 1, 4 * p.streams), dim3(256), pa, 0, st));
+    if (!pl.whole && grid > 1) HQMQ_CHECK_CUDA(cudaLaunchKernel(mk, dim3(grid - 1, 4 * p.streams), dim3(256), pa, 0, st));
   }
   return HQMQ_OK;
 }

@@ -19,7 +19,8 @@ struct PrefillParams {
   int P, streams, units_m;                        // query positions per stream, row blocks per unit, units per (b, head)
   int kt0, nt;                                    // first KV tile that any query sees, tiles in the images
   int bh0;                                        // first (b, head) of the group
-  int64_t Wh, total, L;                           // tiles per (b, head), in all, per CTA
+  int64_t Wh, total, L;                           // tiles per (b, head), in all, per CTA (0: whole units, not pieces)
+  int units_all;                                  // units of the group
   const unsigned char* kimg; const unsigned char* vimg;
   const float* kmul; const float* vmul;           // [B * H_kv] what a score / an output is multiplied by
   float* part;                                    // [CTA][2][d + 2][256 rows]
@@ -41,6 +42,7 @@ struct ExpandParams {
 struct PrefillPlan {
   PrefillParams p;
   int group, grid;
+  bool whole;                                     // units are not cut
   size_t off_mul, off_img, off_part, ws_bytes;
 };
 
