@@ -120,6 +120,7 @@ def lib():
     L.hqmq_strerror.argtypes = [C.c_int]
     L.hqmq_device_check.argtypes = [C.c_int]
     L.hqmq_idx_bits.argtypes = [C.c_int]
+    L.hqmq_zero.argtypes = [C.c_void_p, C.c_size_t, C.c_void_p]
     L.hqmq_row_bytes.argtypes = [C.c_int, C.c_int, C.c_int]
     L.hqmq_native_index_maps.argtypes = [C.c_void_p, C.c_void_p]
     L.hqmq_codebook_tables.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p]

@@ -101,13 +101,16 @@ def fused_attention_packed(
     st = _lib.stream_ptr()
     T_now = K.T if T_kv is None else T_kv
     key = None
-    if Q.stride(-1) == 1 and (out is not None or partials is not None):
+    q_stride = Q.stride()
+    if q_stride[-1] == 1:
+        if out is None and partials is None:
+            out = torch.empty_like(Q)
         dst = partials if partials is not None else out
-        key = (id(V), st, Q.dtype, tuple(Q.shape), Q.stride(), dst.dtype, dst.stride(), partials is not None, causal, window,
+        key = (id(V), st, Q.dtype, Q.shape, q_stride, dst.dtype, dst.stride(), partials is not None, causal, window,
                softmax_scale, kv_splits, table_K.data_ptr(), table_V.data_ptr(), K.with_ofrag, V.with_ofrag)
         hit = K._attn_cache.get(key)
         if hit is not None:
-            a, ws, _, t_sized, _ = hit
+            a, ws_ptr, nbytes, t_sized, ref = hit[:5]
             a.Q, a.T_kv = Q.data_ptr(), T_now
             if partials is not None:
                 a.partials = partials.data_ptr()
@@ -115,17 +118,20 @@ def fused_attention_packed(
                 a.O = out.data_ptr()
             L = _lib.lib()
             with _lib.device_guard(Q.device):
-                if T_now != t_sized:
-                    nbytes = L.hqmq_attn_workspace_bytes(C.byref(a))
+                # (what a call needs depends on its key count by whole 16-key tiles)
+                if T_now != t_sized and (T_now >> 4 != t_sized >> 4 or (T_now + 15) >> 4 != (t_sized + 15) >> 4):
+                    nbytes = L.hqmq_attn_workspace_bytes(ref)
                     if nbytes == 0:
-                        _lib.check(L.hqmq_attn_decode(C.byref(a), None, 0, st), "hqmq_attn_decode")
+                        _lib.check(L.hqmq_attn_decode(ref, None, 0, st), "hqmq_attn_decode")
+                    ws = hit[5]
                     if nbytes > ws.numel():
-                        ws = torch.empty(nbytes, dtype=torch.uint8, device=Q.device)
-                    K._attn_cache[key] = (a, ws, nbytes, T_now, hit[4])
-                else:
-                    nbytes = hit[2]
-                _lib.check(L.hqmq_attn_decode(C.byref(a), ws.data_ptr(), nbytes, st), "hqmq_attn_decode")
-            return partials if partials is not None else out
+                        ws = torch.empty(nbytes + nbytes // 4, dtype=torch.uint8, device=Q.device)
+                        ws_ptr = ws.data_ptr()
+                    K._attn_cache[key] = (a, ws_ptr, nbytes, T_now, ref, ws, hit[6])
+                rc = L.hqmq_attn_decode(ref, ws_ptr, nbytes, st)
+                if rc:
+                    _lib.check(rc, "hqmq_attn_decode")
+            return dst
     _lib.check_device(Q.device)
     B, H_q, T_q, d_h = Q.shape
     if Q.stride(-1) != 1:
@@ -151,7 +157,8 @@ def fused_attention_packed(
     if key is not None:
         if len(K._attn_cache) > 64:
             K._attn_cache.clear()
-        K._attn_cache[key] = (a, ws, nbytes, T_now, (V, table_K, table_V))      # (the last item keeps what the struct points to alive)
+        # (the last item keeps what the struct points to alive)
+        K._attn_cache[key] = (a, ws.data_ptr(), nbytes, T_now, C.byref(a), ws, (V, table_K, table_V))
     return partials if partials is not None else O
 
 

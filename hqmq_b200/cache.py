@@ -90,8 +90,7 @@ class PackedKVCache:
         positions of the cache (call ``update`` first): one decode token sees everything, a prompt chunk is masked
         causally, bottom-right aligned."""
         Kp, Vp = self._layers[layer_idx]
-        dev = query_states.device
-        tk, tv = self._inner.tables(layer_idx, 0, dev), self._inner.tables(layer_idx, 1, dev)
+        tk, tv = self._inner.tables(layer_idx, 0, Kp.device), self._inner.tables(layer_idx, 1, Kp.device)
         return fused_attention_packed(query_states, Kp, Vp, tk["table16"], tv["table16"],
                                       causal="bottom_right" if query_states.shape[2] > 1 else False,
                                       softmax_scale=softmax_scale, window=self.sliding_window.get(layer_idx), out=out)

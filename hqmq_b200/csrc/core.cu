@@ -246,6 +246,12 @@ int hqmq_read_status(const void* workspace, uint32_t* status, void* stream) {
   return HQMQ_OK;
 }
 
+int hqmq_zero(void* p, size_t bytes, void* stream) {
+  if (!p) return HQMQ_ERR_ARG;
+  HQMQ_CHECK_CUDA(cudaMemsetAsync(p, 0, bytes, (cudaStream_t)stream));
+  return HQMQ_OK;
+}
+
 const char* hqmq_strerror(int code) {
   switch (code) {
     case HQMQ_OK: return "ok";

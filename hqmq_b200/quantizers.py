@@ -147,7 +147,8 @@ class HQMQQuantizer(KVQuantizer):
     def tables(self, layer_idx: int, kv: int, device) -> dict:
         """Device tables for one (layer, K|V): 'qs' (H,S,4) fp32, 'joint' (H,24S,4) fp32 in the
         reference's order, 'table16' (H,24S,4) fp16 in the native index order."""
-        device = torch.device(device)
+        if not isinstance(device, torch.device):
+            device = torch.device(device)
         key = (layer_idx, kv, device)
         t = self._tables.get(key)
         if t is None:
@@ -290,7 +291,7 @@ class HQMQQuantizer(KVQuantizer):
             if check_status and nbytes and (_lib.read_status(ws) & 1):
                 raise _lib.HqmqError(f"hqmq_b200: outlier side buffer too small (out_cap={out.out_cap} chunks per (b, h))")
         if fast_key is not None and x is x_given:
-            a._keep = (a._keep[1], out)          # the tables and the planes, not the input tensor of this call
+            a._keep = (a._keep[1],)              # the tables: not this call's input, nor the cache that holds the struct
             out._enc_cache[fast_key] = (a, ws, nbytes)
         out.T += T
         return out
@@ -301,15 +302,16 @@ class HQMQQuantizer(KVQuantizer):
         src/model_utils.py:29-32).  Same result as ``encode(k, layer_idx, 0, out=out_k)`` followed by
         ``encode(v, layer_idx, 1, out=out_v)``; a decode-time append (a few tokens per sequence) runs both tensors
         in one kernel launch (hqmq_encode_pair) instead of three per tensor."""
-        small = (k.dim() == 4 and k.shape == v.shape and k.dtype == v.dtype and k.shape[2] <= 64 and k.is_cuda and v.is_cuda
-                 and k.stride(-1) == 1 and v.stride(-1) == 1 and not any(s % 4 for s in k.stride()[:3] + v.stride()[:3]))
-        if not small or k.shape[2] == 0:
-            return (self.encode(k, layer_idx, 0, out=out_k, median_mult=median_mult, quantile=quantile),
-                    self.encode(v, layer_idx, 1, out=out_v, median_mult=median_mult, quantile=quantile))
-        T = k.shape[2]
-        key = ("pair", id(self), id(out_v), layer_idx, tuple(k.shape), k.dtype, k.stride(), v.stride(), median_mult, quantile)
+        # (one dictionary look-up on everything that decides the call's shape: a repeated append goes straight to the library)
+        shape, ks, vs = k.shape, k.stride(), v.stride()
+        key = ("pair", id(self), id(out_v), layer_idx, shape, v.shape, k.dtype, v.dtype, ks, vs, k.device, v.device, median_mult, quantile)
         hit = out_k._enc_cache.get(key)
         if hit is None:
+            small = (k.dim() == 4 and shape == v.shape and k.dtype == v.dtype and shape[2] <= 64 and k.is_cuda and v.is_cuda
+                     and ks[-1] == 1 and vs[-1] == 1 and not any(s % 4 for s in ks[:3] + vs[:3]))
+            if not small or shape[2] == 0:
+                return (self.encode(k, layer_idx, 0, out=out_k, median_mult=median_mult, quantile=quantile),
+                        self.encode(v, layer_idx, 1, out=out_v, median_mult=median_mult, quantile=quantile))
             why = self._unsupported()
             if why:
                 raise NotImplementedError(f"hqmq_b200 accelerates the unit-magnitude linear-radius path only ({why})")
@@ -325,17 +327,20 @@ class HQMQQuantizer(KVQuantizer):
             with _lib.device_guard(k.device):
                 nbytes = _lib.lib().hqmq_encode_pair_workspace_bytes(C.byref(ak), C.byref(av))
             ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=k.device)
-            ak._keep, av._keep = (ak._keep[1], out_k), (av._keep[1], out_v)     # tables and planes, not this call's inputs
-            hit = out_k._enc_cache[key] = (ak, av, ws, nbytes)
-        ak, av, ws, nbytes = hit
-        if out_k.T + T > out_k.T_cap or out_v.T + T > out_v.T_cap:
-            raise _lib.HqmqError(f"hqmq_b200: cache capacity {out_k.T_cap} exceeded ({out_k.T} + {T})")
-        ak.x, ak.t_start, av.x, av.t_start = k.data_ptr(), out_k.T, v.data_ptr(), out_v.T
+            # the tables and V's planes, not this call's inputs (nor out_k, which holds the structs: a cycle would leave the
+            # cache's memory to the garbage collector)
+            ak._keep, av._keep = (ak._keep[1],), (av._keep[1], out_v)
+            hit = out_k._enc_cache[key] = (ak, av, C.byref(ak), C.byref(av), ws.data_ptr(), nbytes, ws)
+        ak, av, rk, rv, ws_ptr, nbytes, _ = hit
+        T, tk, tv = shape[2], out_k.T, out_v.T
+        if tk + T > out_k.T_cap or tv + T > out_v.T_cap:
+            raise _lib.HqmqError(f"hqmq_b200: cache capacity {out_k.T_cap} exceeded ({tk} + {T})")
+        ak.x, ak.t_start, av.x, av.t_start = k.data_ptr(), tk, v.data_ptr(), tv
         with _lib.device_guard(k.device):
-            _lib.check(_lib.lib().hqmq_encode_pair(C.byref(ak), C.byref(av), ws.data_ptr(), nbytes, _lib.stream_ptr()),
-                       "hqmq_encode_pair")
-        out_k.T += T
-        out_v.T += T
+            rc = _lib.lib().hqmq_encode_pair(rk, rv, ws_ptr, nbytes, _lib.stream_ptr())
+            if rc:
+                _lib.check(rc, "hqmq_encode_pair")
+        out_k.T, out_v.T = tk + T, tv + T
         return out_k, out_v
 
     def decode(self, packed: PackedKV, layer_idx: int, kv: int, dtype: torch.dtype = torch.float32,
@@ -401,57 +406,72 @@ class HQMQQuantizer(KVQuantizer):
 
 
 class _OutlierStats:
-    """Running mean of the per-call outlier rates (what the reference's wrapper keeps in ``_observed_outlier_rate``),
-    from the caches' device counters, read (and synchronised) only on demand.  A call costs no device work: every
-    cache remembers how many calls of which size it took since its counters were last read, and the flagged chunks
-    of those calls are the growth of its counters.  Calls of one size on one cache share their growth evenly (exact
-    for the sum of their rates, which is all a mean needs)."""
+    """Running mean of the per-call outlier rates (what the reference's wrapper keeps in ``_observed_outlier_rate``), read
+    from the caches' device counters only on demand.  What is remembered of a cache is a small record -- its counter
+    tensor (B * H words), the count its open calls started from, their number and size -- never the cache itself, so a
+    cache that is done with gives its planes back.  Calls of one size on one cache share their growth evenly (exact for
+    the sum of their rates, which is all a mean needs); a call of another size closes the group with a copy of the
+    counter on the device.  Records are folded into two host numbers once there are ``_FOLD`` of them."""
+    _FOLD = 1024
 
     def __init__(self):
-        self._caches = []           # caches with calls that were not accounted yet
-        self._counts = []           # (0-d device tensor: flagged chunks of one finished call, chunks of that call)
+        self._open = []             # records with calls that were not accounted yet
+        self._closed = []           # (counter at the end, counter or number at the start, calls' size, calls)
         self._sum_rates, self._n = 0.0, 0   # sum of the per-call rates, number of calls
 
+    # a record: [counter tensor, count at the start (number or tensor), calls, chunks per call]
     def begin(self, pk, total_chunks: int):
-        """Before a call appends to ``pk`` (None: a fresh cache).  Calls of another size are accounted first."""
+        """Before a call appends to ``pk`` (None: a fresh cache)."""
         if pk is None:
             return
-        st = getattr(pk, "_stat_pending", None)
-        if st is not None and st[1] != total_chunks:
-            self._account(pk)
-        elif st is None and pk.T > 0 and not hasattr(pk, "_stat_base"):
-            pk._stat_base = float(pk.out_count.sum().item())      # a cache filled elsewhere: count from what it holds
+        rec = getattr(pk, "_stat_rec", None)
+        if rec is None:
+            if pk.T > 0 and pk.with_outliers:   # a cache filled elsewhere: count from what it holds
+                pk._stat_rec = [pk.out_count, pk.out_count.clone(), 0, total_chunks]
+        elif rec[2] and rec[3] != total_chunks:
+            now = rec[0].clone()
+            self._closed.append((now, rec[1], rec[3], rec[2]))
+            rec[1], rec[2] = now, 0
 
     def end(self, pk, total_chunks: int):
-        st = getattr(pk, "_stat_pending", None)
-        if st is None:
-            st = pk._stat_pending = [0, total_chunks]
-            self._caches.append(pk)
-        st[0] += 1
+        rec = getattr(pk, "_stat_rec", None)
+        if rec is None:
+            rec = pk._stat_rec = [pk.out_count, 0.0, 0, total_chunks]
+        if not rec[2]:
+            rec[3] = total_chunks
+            self._open.append(rec)
+        rec[2] += 1
+        if len(self._open) + len(self._closed) >= self._FOLD:
+            self._sync()
 
-    def _account(self, pk):
-        n_calls, total = pk._stat_pending
-        pk._stat_pending = None
-        now = float(pk.out_count.sum().item())
-        self._sum_rates += (now - getattr(pk, "_stat_base", 0.0)) / max(1, total)
-        self._n += n_calls
-        pk._stat_base = now
-
-    def push_count(self, count: torch.Tensor, total_chunks: int):
-        """A finished one-shot call (fake-quant): only its count is kept, not its cache."""
-        self._counts.append((count, total_chunks))
-        if len(self._counts) >= 1024:
+    def push_count(self, counter: torch.Tensor, total_chunks: int):
+        """A finished one-shot call (fake-quant): only its counter is kept, not its cache."""
+        self._closed.append((counter, 0.0, total_chunks, 1))
+        if len(self._open) + len(self._closed) >= self._FOLD:
             self._sync()
 
     def _sync(self):
-        for pk in self._caches:
-            if getattr(pk, "_stat_pending", None) is not None:
-                self._account(pk)
-        self._caches = []
-        for count, total in self._counts:
-            self._sum_rates += float(count.item()) / max(1, total)
-            self._n += 1
-        self._counts = []
+        done, self._closed = self._closed, []
+        recs = {id(r): r for r in self._open if r[2]}.values()
+        self._open = []
+        groups = done + [(r[0], r[1], r[3], r[2]) for r in recs]
+        tensors = [t for g in groups for t in g[:2] if isinstance(t, torch.Tensor)]
+        sums = iter(())
+        if tensors:                     # one transfer per device for all of them
+            host = {}
+            for dev in {t.device for t in tensors}:
+                host[dev] = iter(torch.cat([t.reshape(-1) for t in tensors if t.device == dev]).cpu()
+                                 .split([t.numel() for t in tensors if t.device == dev]))
+            sums = iter([float(next(host[t.device]).sum()) for t in tensors])
+        ends = []
+        for end, start, total, calls in groups:
+            e = next(sums) if isinstance(end, torch.Tensor) else end
+            b = next(sums) if isinstance(start, torch.Tensor) else start
+            self._sum_rates += (e - b) / max(1, total)
+            self._n += calls
+            ends.append(e)
+        for r, e in zip(recs, ends[len(done):]):
+            r[1], r[2] = e, 0
 
     @property
     def rate(self):
@@ -534,7 +554,7 @@ class OutlierAwareHQMQQuantizer(KVQuantizer):
         self._check_mode()
         out = self.inner._qdq(x, layer_idx, kv, **self._thr())
         if x.shape[0] and x.shape[2]:
-            self._stats.push_count(self.inner._last_packed.out_count.sum(), x.shape[0] * x.shape[1] * x.shape[2] * (x.shape[3] // 4))
+            self._stats.push_count(self.inner._last_packed.out_count, x.shape[0] * x.shape[1] * x.shape[2] * (x.shape[3] // 4))
         return out
 
     def quantize_K(self, k, layer_idx):

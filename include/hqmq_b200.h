@@ -147,6 +147,8 @@ int hqmq_abi_version(void);
 const char* hqmq_strerror(int code);
 /* HQMQ_OK if `device` has compute capability 10.x, else HQMQ_ERR_ARCH. */
 int hqmq_device_check(int device);
+/* Zero-fills device memory on the stream (planes must be zero when a cache is created). */
+int hqmq_zero(void* p, size_t bytes, void* stream);
 int hqmq_idx_bits(int S);
 int hqmq_row_bytes(int n_chunks, int S, int radius_bits);
 /* Host tables, 24 entries each: ref_to_native[p] = (a << 3) | u, native_to_ref[(a << 3) | u] = p. */
