@@ -134,6 +134,9 @@ def lib():
     L.hqmq_encode_workspace_bytes.restype = C.c_size_t
     L.hqmq_encode_workspace_bytes.argtypes = [C.POINTER(EncodeArgs)]
     L.hqmq_encode.argtypes = [C.POINTER(EncodeArgs), C.c_void_p, C.c_size_t, C.c_void_p]
+    L.hqmq_fake_quant_workspace_bytes.restype = C.c_size_t
+    L.hqmq_fake_quant_workspace_bytes.argtypes = [C.POINTER(EncodeArgs)]
+    L.hqmq_fake_quant.argtypes = [C.POINTER(EncodeArgs), C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]
     L.hqmq_med3x_state_bytes.restype = C.c_size_t
     L.hqmq_med3x_state_bytes.argtypes = [C.c_int]
     L.hqmq_med3x_hist.argtypes = [C.POINTER(EncodeArgs), C.c_int, C.c_void_p, C.c_size_t, C.c_void_p]

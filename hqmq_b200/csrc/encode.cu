@@ -12,6 +12,9 @@
 // A flagged chunk keeps its index but its stored radius code is 0: its values live in the side buffer.
 #include <string.h>
 
+#include <atomic>
+
+#include "attn_prefill.cuh"      // raise_smem_limit
 #include "common.cuh"
 
 namespace hqmq {
@@ -44,7 +47,7 @@ constexpr int kUndCap = 4096;     // undecided chunks listed per head; more -> t
 constexpr int kLutNMax = 48;
 constexpr int kLutRows = kLutNMax * kLutNMax;
 constexpr int kLutCellCap = 24576;          // stored cells (23.4 k at n = 48)
-constexpr int kLutCandCap = 65532;          // candidate entries per head (list offsets / 4 are 15-bit cell words)
+constexpr int kLutCandCap = 65528;          // candidate entries per head (list offsets / 4 are 15-bit cell words; every head's part a multiple of 16 bytes)
 constexpr int kLutMaxList = 16;             // longest list a cell may have; longer -> exhaustive search there
 constexpr float kLutBoxEps = 1e-5f;         // the boxes are grown by this much (cell assignment rounding)
 constexpr float kLutMargin = 1e-5f;         // a codeword is dropped only if it loses by more than this
@@ -387,16 +390,20 @@ constexpr int kSmallMax = 2048;          // chunks per head and call
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallTok = 512;           // tokens per head and call (kSmallMax / 4 chunks)
 
-// (the body is shared by the kernel of one tensor and by the kernel that appends K and V of a layer in one launch)
+// (the body is shared by the kernel of one tensor, by the kernel that appends K and V of a layer in one launch, and -- DENSE:
+// the fake-quantised values go to `out`, (B, H, T, 4 n) contiguous in the type of x, nothing is packed -- by the quantizer's
+// quantize calls)
+template <bool DENSE>
 __device__ __forceinline__ void
 encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __restrict__ qs_all, const hqmq_packed& dst,
                   int t_start, const Maps24& maps, const float* __restrict__ joint_all, const unsigned char* __restrict__ lut,
-                  const uint8_t* __restrict__ nmul_dev, float C, float* __restrict__ med_out, float quantile) {
+                  const uint8_t* __restrict__ nmul_dev, float C, float* __restrict__ med_out, float quantile,
+                  void* __restrict__ out = nullptr, uint32_t* __restrict__ n_flagged = nullptr) {
   __shared__ uint32_t keys[kSmallMax];                    // norm bits of every chunk of the head
   __shared__ uint32_t tokmax[kSmallTok];                  // bits of the largest radius of a token
   __shared__ uint32_t tokflags[kSmallTok];
   __shared__ uint32_t rows[kSmallTok / 8][kMaxRowWords];   // packed rows, 64 tokens at a time
-  const int h = blockIdx.x;
+  const int h = blockIdx.x, NT = blockDim.x;              // at most two chunks per thread
   const int n = g.n, per_b = g.T_new * n;                 // chunks of one batch entry
   const int N = g.B * per_b, n_tok = g.B * g.T_new;
   const int S = g.S;
@@ -417,7 +424,7 @@ encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __r
   uint32_t ni[2];
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
-    const int i = threadIdx.x + k * kSmallThreads;
+    const int i = threadIdx.x + k * NT;
     nrm[k] = 0.f; radius[k] = 0.f; ni[k] = 0u;
     if (i < N) {
       const int b = i / per_b, r = i - b * per_b, t = r / n, c = r - t * n;
@@ -446,13 +453,30 @@ encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __r
     const QRank qr = quantile_rank((uint64_t)N, quantile);
     const uint32_t lo = (uint32_t)qr.lo, hi = (uint32_t)qr.hi;
     uint32_t prefix = 0u, rank = lo;
+    if (N <= 256) {
+      // few keys: every thread counts the keys below its own; the one of rank `lo` is the key with at most lo below and
+      // more than lo at or below it (no passes, two barriers)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int i = threadIdx.x + k * NT;
+        if (i < N) {
+          const uint32_t key = keys[i];
+          uint32_t lt = 0u, le = 0u;
+          for (int j = 0; j < N; ++j) { const uint32_t y = keys[j]; lt += y < key; le += y <= key; }
+          if (lt <= lo && lo < le) s_state[0] = key;       // (every such key has the same bits)
+        }
+      }
+      __syncthreads();
+      prefix = s_state[0];
+      __syncthreads();
+    } else
     for (int pass = 0; pass < 4; ++pass) {
       const int shift = 24 - 8 * pass;
       if (threadIdx.x < 256) shist[threadIdx.x] = 0u;
       __syncthreads();
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const int i = threadIdx.x + k * kSmallThreads;
+        const int i = threadIdx.x + k * NT;
         if (i < N) {
           const uint32_t key = keys[i];
           if (pass == 0 || (key >> (shift + 8)) == (prefix >> (shift + 8))) atomicAdd(&shist[(key >> shift) & 0xffu], 1u);
@@ -493,7 +517,7 @@ encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __r
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const int i = threadIdx.x + k * kSmallThreads;
+      const int i = threadIdx.x + k * NT;
       if (i < N) {
         const uint32_t key = keys[i];
         if (key <= a_bits) atomicAdd(&s_state[2], 1u);
@@ -508,11 +532,51 @@ encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __r
     if (threadIdx.x == 0 && med_out) med_out[h] = m;
   }
 
+  if constexpr (DENSE) {
+    // ---- the dense values: codeword * (rq * (rmax / qmax)), one rounding each, or the original chunk where flagged ----
+    uint32_t fl = 0u;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int i = threadIdx.x + k * NT;
+      if (i < N) {
+        const int b = i / per_b, r = i - b * per_b, t = r / n, c = r - t * n;
+        const float rmax = fmaxf(__uint_as_float(tokmax[b * g.T_new + t]), 1e-8f);
+        const float scale = __fdiv_rn(rmax, qmaxf);
+        const float rqf = fminf(fmaxf(rintf(__fdiv_rn(radius[k], scale)), 0.f), qmaxf);
+        const int64_t o = ((((int64_t)b * g.H + h) * g.T_new + t) * n + c) * 4;
+        float v[4];
+        if (med && nrm[k] > thr) {
+          ++fl;
+          load_chunk(x, b * g.xs_b + h * g.xs_h + t * g.xs_t + 4 * c, g.x_dtype, v);
+        } else {
+          int p = 0;
+          const int au = (int)((ni[k] >> 3) / (uint32_t)S) << 3 | (int)(ni[k] & 7u);
+          for (int q = 0; q < 24; ++q) if (maps.ref_to_native[q] == au) p = q;
+          const float rad = __fmul_rn(rqf, scale);
+          const float4 cw = joint[p * S + (int)((ni[k] >> 3) % (uint32_t)S)];
+          v[0] = __fmul_rn(cw.x, rad); v[1] = __fmul_rn(cw.y, rad); v[2] = __fmul_rn(cw.z, rad); v[3] = __fmul_rn(cw.w, rad);
+        }
+        if (g.x_dtype == HQMQ_F32) {
+          *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + o) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+          uint2 w;
+          w.x = float_to_bits16(v[0], g.x_dtype) | ((uint32_t)float_to_bits16(v[1], g.x_dtype) << 16);
+          w.y = float_to_bits16(v[2], g.x_dtype) | ((uint32_t)float_to_bits16(v[3], g.x_dtype) << 16);
+          *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(out) + o) = w;
+        }
+      }
+    }
+    if (n_flagged && med) {
+      fl = __reduce_add_sync(0xffffffffu, fl);
+      if ((threadIdx.x & 31) == 0 && fl) atomicAdd(n_flagged, fl);
+    }
+  } else {
+
   // ---- phase C: radius codes, flags -------------------------------------------------------------------------
   uint32_t field[2];
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
-    const int i = threadIdx.x + k * kSmallThreads;
+    const int i = threadIdx.x + k * NT;
     field[k] = 0u;
     if (i < N) {
       const int b = i / per_b, r = i - b * per_b, t = r / n, c = r - t * n;
@@ -536,7 +600,7 @@ encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __r
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const int i = threadIdx.x + k * kSmallThreads;
+      const int i = threadIdx.x + k * NT;
       if (i < N) {
         const int b = i / per_b, r = i - b * per_b, t = r / n, c = r - t * n;
         const int tok = b * g.T_new + t - tok0;
@@ -563,6 +627,7 @@ encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __r
     store_scale(dst, row, fmaxf(__uint_as_float(tokmax[tok]), 1e-8f));
     if (dst.flags) dst.flags[row] = tokflags[tok];
   }
+  }
 }
 
 // Everything one tensor of a small call needs; two of them make the K + V append of a layer.
@@ -580,12 +645,22 @@ struct SmallArgs {
   float quantile;
   uint32_t* status;     // first word of the tensor's workspace: cleared here, set by scan_kernel on an overflow
   int blk0, nblk, scan, payload, side;
+  void* out;            // dense calls: the fake-quantised tensor, and the counter that its flagged chunks are added to
+  uint32_t* n_flagged;
 };
+// Threads of a small call's CTA: two chunks each (fewer threads, cheaper barriers).
+inline int small_threads(int64_t chunks) {
+  return chunks <= 128 ? 128 : chunks <= 512 ? 256 : chunks <= 1024 ? 512 : kSmallThreads;
+}
 struct SmallPair { SmallArgs t[2]; Maps24 maps; };
 
 __global__ void __launch_bounds__(kSmallThreads) encode_small_kernel(SmallArgs a, Maps24 maps) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0u;
-  encode_small_body(a.g, a.x, a.qs, a.dst, a.t_start, maps, a.joint, a.lut, a.nmul, a.C, a.med_out, a.quantile);
+  encode_small_body<false>(a.g, a.x, a.qs, a.dst, a.t_start, maps, a.joint, a.lut, a.nmul, a.C, a.med_out, a.quantile);
+}
+
+__global__ void __launch_bounds__(kSmallThreads) fake_quant_small_kernel(SmallArgs a, Maps24 maps) {
+  encode_small_body<true>(a.g, a.x, a.qs, a.dst, a.t_start, maps, a.joint, a.lut, a.nmul, a.C, a.med_out, a.quantile, a.out, a.n_flagged);
 }
 
 // ---- main pass for the common geometry ------------------------------------------------------------------
@@ -785,6 +860,8 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
     }
   }
 }
+
+#include "encode_fused.cuh"
 
 // ---- Med3x: radix select of the two middle order statistics ------------------------------
 // Level 0 histogram (bits 31:21) is accumulated by encode_main_kernel into query slot 0.
@@ -1707,15 +1784,15 @@ scan_small_warp(const hqmq_packed& dst, int bh, int t_start, int T_new, int blk0
 // another CTA has started.
 __global__ void __launch_bounds__(kSmallThreads) append_pair_kernel(SmallPair p) {
   const SmallArgs& a = p.t[blockIdx.y];
-  encode_small_body(a.g, a.x, a.qs, a.dst, a.t_start, p.maps, a.joint, a.lut, a.nmul, a.C, a.med_out, a.quantile);
+  encode_small_body<false>(a.g, a.x, a.qs, a.dst, a.t_start, p.maps, a.joint, a.lut, a.nmul, a.C, a.med_out, a.quantile);
   if (!a.scan) return;
   __syncthreads();          // the head's flag words and scales are in global memory for the other warps of the CTA
   const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int b = warp; b < a.g.B; b += kSmallThreads / 32)
+  for (int b = warp; b < a.g.B; b += (int)(blockDim.x >> 5))
     scan_small_warp(a.dst, b * a.g.H + h, a.t_start, a.g.T_new, a.blk0, a.nblk, a.payload, a.status, lane);
   if (!a.side) return;
   __syncthreads();          // ... and so are the offsets
-  for (int w = warp; w < a.g.B * a.nblk; w += kSmallThreads / 32) {
+  for (int w = warp; w < a.g.B * a.nblk; w += (int)(blockDim.x >> 5)) {
     const int b = w / a.nblk, i = w - b * a.nblk;
     side_block(a.g, a.x, a.dst, a.t_start, a.blk0, a.nblk, b * a.g.H + h, i, lane);
   }
@@ -2186,6 +2263,7 @@ static int fill_small(const hqmq_encode_args* a, const WsPlan& wp, uint32_t* ws,
   const hqmq_packed& d = a->dst;
   const bool med = a->median_mult > 0.f;
   const bool lut_ok = a->search == 0 && a->lut != nullptr && a->lut_footprint >= 0;
+  sa.out = nullptr; sa.n_flagged = nullptr;
   if (lut_ok && ((uintptr_t)a->lut & 15)) return HQMQ_ERR_ALIGN;
   const unsigned char* lut_b = reinterpret_cast<const unsigned char*>(a->lut);
   sa.g = geom_of(a);
@@ -2197,6 +2275,114 @@ static int fill_small(const hqmq_encode_args* a, const WsPlan& wp, uint32_t* ws,
   sa.blk0 = wp.blk0; sa.nblk = wp.nblk;
   sa.scan = (med || d.ofrag) ? 1 : 0; sa.payload = med ? 1 : 0; sa.side = med ? 1 : 0;
   return HQMQ_OK;
+}
+
+// The one-launch encoder: whether a call takes it, and its launch.
+static int sm_count() {
+  static std::atomic<int> cached{0};
+  int n = cached.load(std::memory_order_relaxed);
+  if (!n) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+    cached.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+static bool fused_call(const hqmq_encode_args* a) {
+  const hqmq_packed& d = a->dst;
+  const int ib = idx_bits_for(d.S), rb = d.radius_bits;
+  const bool layout = (ib == 10 && rb == 3) || (ib == 12 && rb == 4) || (ib == 13 && rb == 6);
+  // (two 64-wide tokens per warp need rows of whole words, which 16-bit fields give)
+  const bool geom = d.n_chunks == 32 || (d.n_chunks == 16 && ib + rb == 16);
+  if (!layout || !geom || !is_half_dtype(a->x_dtype) || a->search != 0 || !a->lut || a->lut_footprint <= 0 || ((uintptr_t)a->lut & 15)) return false;
+  if (d.H > sm_count() || (uint64_t)d.B * a->T_new * d.n_chunks >= ((uint64_t)1 << 32)) return false;
+  return fused_smem_bytes(d.S, ((size_t)a->lut_footprint + 15) & ~(size_t)15) <= (size_t)226 * 1024;
+}
+static int launch_fused(const hqmq_encode_args* a, uint32_t* status, uint32_t* hist, uint32_t* bars, void* out, uint32_t* n_flagged,
+                        cudaStream_t st) {
+  const hqmq_packed& d = a->dst;
+  FusedArgs f;
+  f.g = geom_of(a);
+  f.x = reinterpret_cast<const uint16_t*>(a->x); f.qs = a->qs; f.joint = a->joint;
+  f.lut = reinterpret_cast<const unsigned char*>(a->lut);
+  f.dst = d; f.t_start = a->t_start; f.out = reinterpret_cast<uint16_t*>(out); f.n_flagged = n_flagged;
+  f.C = a->median_mult; f.quantile = a->quantile; f.med_in = a->med_in; f.med_out = a->med_out;
+  f.hist = hist; f.bars = bars; f.status = status;
+  // one CTA per SM in all, no fewer than a round of its warps each
+  const int64_t W = (int64_t)d.B * (d.n_chunks == 16 ? (a->T_new + 1) / 2 : a->T_new);
+  int64_t cph = sm_count() / d.H;
+  if (cph > (W + kEnc32Warps - 1) / kEnc32Warps) cph = (W + kEnc32Warps - 1) / kEnc32Warps;
+  f.per = (int)((W + cph - 1) / cph);
+  f.cph = (int)((W + f.per - 1) / f.per);
+  const bool h16 = a->x_dtype == HQMQ_F16, dense = out != nullptr;
+  const void* k = nullptr;
+#define HQMQ_PICK(IB_, RB_)                                                                                    \
+  if (f.g.ib == IB_ && f.g.rbits == RB_)                                                                         \
+    k = dense ? (h16 ? (const void*)&encode_fused_kernel<HQMQ_F16, IB_, RB_, true> : (const void*)&encode_fused_kernel<HQMQ_BF16, IB_, RB_, true>)   \
+              : (h16 ? (const void*)&encode_fused_kernel<HQMQ_F16, IB_, RB_, false> : (const void*)&encode_fused_kernel<HQMQ_BF16, IB_, RB_, false>);
+  HQMQ_PICK(10, 3) HQMQ_PICK(12, 4) HQMQ_PICK(13, 6)
+#undef HQMQ_PICK
+  const size_t smem = fused_smem_bytes(d.S, ((size_t)a->lut_footprint + 15) & ~(size_t)15);
+  HQMQ_CHECK_CUDA(attn::raise_smem_limit(k, smem));
+  Maps24 maps;
+  memcpy(maps.ref_to_native, index_maps().ref_to_native, 24);
+  const Mul24& nmul = mul24_native();
+  void* args[] = {&f, &maps, (void*)&nmul};
+  // (the CTAs of a head wait for one another only for a threshold of the call's own)
+  const bool waits = a->median_mult > 0.f && !a->med_in && f.cph > 1;
+  if (waits) HQMQ_CHECK_CUDA(cudaLaunchCooperativeKernel(k, dim3(f.cph * d.H), dim3(kEnc32Threads), args, smem, st));
+  else HQMQ_CHECK_CUDA(cudaLaunchKernel(k, dim3(f.cph * d.H), dim3(kEnc32Threads), args, smem, st));
+  return HQMQ_OK;
+}
+
+// ---- fake-quantised tensor straight from x ----------------------------------------------------------------------------
+// words of a call's workspace: status [4], histograms, arrivals
+static size_t fake_quant_ws_words(int H) { return 4 + (size_t)H * 3 * 2 * kHistBins + (size_t)H * 8; }
+static int validate_fake_quant(const hqmq_encode_args* a) {
+  if (!a || a->struct_size != sizeof(hqmq_encode_args) || a->dst.struct_size != sizeof(hqmq_packed)) return HQMQ_ERR_ARG;
+  if (!a->x || !a->qs || !a->joint) return HQMQ_ERR_ARG;
+  if (!is_float_dtype(a->x_dtype)) return HQMQ_ERR_DTYPE;
+  const hqmq_packed& d = a->dst;
+  if (d.B < 1 || d.H < 1 || d.n_chunks < 1 || d.n_chunks > 32 || d.S < 1 || 24 * d.S > 65536 || d.radius_bits < 1 || d.radius_bits > 8 ||
+      a->T_new < 1 || a->t_start != 0)
+    return HQMQ_ERR_SHAPE;
+  if (!(a->quantile >= 0.f && a->quantile < 1.f)) return HQMQ_ERR_ARG;
+  if ((uintptr_t)a->x & (a->x_dtype == HQMQ_F32 ? 15 : 7)) return HQMQ_ERR_ALIGN;
+  for (int i = 0; i < 3; ++i)
+    if (a->x_stride[i] % 4) return HQMQ_ERR_ALIGN;
+  if (((uintptr_t)a->qs & 15) || ((uintptr_t)a->joint & 15)) return HQMQ_ERR_ALIGN;
+  return small_call(a) || fused_call(a) ? HQMQ_OK : HQMQ_ERR_UNSUPPORTED;
+}
+extern "C" size_t hqmq_fake_quant_workspace_bytes(const hqmq_encode_args* a) {
+  return validate_fake_quant(a) == HQMQ_OK ? fake_quant_ws_words(a->dst.H) * 4 : 0;
+}
+extern "C" int hqmq_fake_quant(const hqmq_encode_args* a, void* out, uint32_t* n_flagged, void* workspace, size_t workspace_bytes,
+                               void* stream) {
+  const int rc = validate_fake_quant(a);
+  if (rc) return rc;
+  if (!out || ((uintptr_t)out & 15)) return HQMQ_ERR_ARG;
+  if (!workspace || workspace_bytes < fake_quant_ws_words(a->dst.H) * 4) return HQMQ_ERR_WORKSPACE;
+  if ((uintptr_t)workspace & 15) return HQMQ_ERR_ALIGN;
+  cudaStream_t st = (cudaStream_t)stream;
+  uint32_t* ws = reinterpret_cast<uint32_t*>(workspace);
+  const hqmq_packed& d = a->dst;
+  if (small_call(a)) {
+    WsPlan wp{};
+    SmallArgs sa;
+    const int e = fill_small(a, wp, ws, sa);
+    if (e) return e;
+    sa.out = out; sa.n_flagged = n_flagged;
+    Maps24 maps;
+    memcpy(maps.ref_to_native, index_maps().ref_to_native, 24);
+    fake_quant_small_kernel<<<d.H, small_threads((int64_t)d.B * a->T_new * d.n_chunks), 0, st>>>(sa, maps);
+    HQMQ_LAUNCH_CHECK();
+    return HQMQ_OK;
+  }
+  uint32_t* hist = ws + 4;
+  uint32_t* bars = hist + (size_t)d.H * 3 * 2 * kHistBins;
+  if (a->median_mult > 0.f && !a->med_in) HQMQ_CHECK_CUDA(cudaMemsetAsync(ws, 0, fake_quant_ws_words(d.H) * 4, st));
+  return launch_fused(a, ws, hist, bars, out, n_flagged, st);
 }
 
 extern "C" size_t hqmq_encode_pair_workspace_bytes(const hqmq_encode_args* k, const hqmq_encode_args* v) {
@@ -2233,7 +2419,7 @@ extern "C" int hqmq_encode_pair(const hqmq_encode_args* k, const hqmq_encode_arg
   memcpy(pr.maps.ref_to_native, index_maps().ref_to_native, 24);
   // one launch for the whole append; the two status words (first word of each tensor's part) are cleared ahead of it
   HQMQ_CHECK_CUDA(cudaMemset2DAsync(wsb, wk, 0, sizeof(uint32_t), 2, st));
-  append_pair_kernel<<<dim3(dk.H, 2), kSmallThreads, 0, st>>>(pr);
+  append_pair_kernel<<<dim3(dk.H, 2), small_threads((int64_t)dk.B * k->T_new * dk.n_chunks), 0, st>>>(pr);
   HQMQ_LAUNCH_CHECK();
   return HQMQ_OK;
 }
@@ -2259,9 +2445,20 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
     SmallArgs sa;
     rc = fill_small(a, wp, ws, sa);
     if (rc) return rc;
-    encode_small_kernel<<<d.H, kSmallThreads, 0, st>>>(sa, maps);      // (clears the status word itself)
+    encode_small_kernel<<<d.H, small_threads((int64_t)d.B * a->T_new * d.n_chunks), 0, st>>>(sa, maps);      // (clears the status word itself)
     if (sa.scan) scan_kernel<<<d.B * d.H, kScanWarps * 32, 0, st>>>(d, a->t_start, a->T_new, wp.blk0, wp.nblk, sa.payload, ws + wp.status);
     if (sa.side) side_kernel<<<dim3((wp.nblk + 7) / 8, d.B * d.H), 256, 0, st>>>(g, a->x, d, a->t_start, wp.blk0, wp.nblk);
+    HQMQ_LAUNCH_CHECK();
+    return HQMQ_OK;
+  }
+  if (fused_call(a) && !bracket_wanted(*a)) {
+    // (status, histograms and select words are the first part of the workspace; the select words serve as arrival counters)
+    HQMQ_CHECK_CUDA(cudaMemsetAsync(ws, 0, (wp.sel + (size_t)d.H * 8) * sizeof(uint32_t), st));
+    rc = launch_fused(a, ws + wp.status, ws + wp.hist, ws + wp.sel, nullptr, nullptr, st);
+    if (rc) return rc;
+    if (med || d.ofrag)
+      scan_kernel<<<d.B * d.H, kScanWarps * 32, 0, st>>>(d, a->t_start, a->T_new, wp.blk0, wp.nblk, med ? 1 : 0, ws + wp.status);
+    if (med) side_kernel<<<dim3((wp.nblk + 7) / 8, d.B * d.H), 256, 0, st>>>(g, a->x, d, a->t_start, wp.blk0, wp.nblk);
     HQMQ_LAUNCH_CHECK();
     return HQMQ_OK;
   }

@@ -1,0 +1,270 @@
+// One-launch encoder for calls between the decode-time append and the very long prompt (included by encode.cu): exact
+// threshold, nearest codewords and either packed rows or the dense fake-quantised tensor, in ONE kernel.
+//
+// The multi-pass path of such a call is a dozen launches (samples, selects, histograms, flags, fix-ups), each of a few
+// microseconds, and its main pass copies 60-150 KB of tables into shared memory per 128 tokens.  Here a head's tokens are
+// split over a few CTAs that stay resident (one per SM, cooperative launch): the tables are fetched by bulk copies while
+// the three radix-select levels run -- each CTA histograms its norms, the CTAs of the head meet at a counter in global
+// memory (bounded wait), everyone scans the head's histogram -- and the main pass then knows the exact threshold, so flags
+// and radius codes are final as they are written.  Bound: launch, three rounds of about 3 us, then the issue slots of the
+// search.
+struct FusedArgs {
+  EncGeom g;                  // the call's own geometry: n = 32 chunks per token, or 16 (two tokens per warp)
+  const uint16_t* x;
+  const float* qs;
+  const float* joint;
+  const unsigned char* lut;
+  hqmq_packed dst;            // packed rows (DENSE = false)
+  int t_start;
+  uint16_t* out;              // (B, H, T, 4 n) contiguous, element type of x (DENSE = true)
+  uint32_t* n_flagged;        // DENSE: + the call's flagged chunks (optional)
+  float C, quantile;          // C <= 0: no outliers
+  const float* med_in;        // medians given by the caller
+  float* med_out;
+  uint32_t* hist;             // [H][3][2][kHistBins], zero
+  uint32_t* bars;             // [H] arrivals, zero
+  uint32_t* status;
+  int cph, per;               // CTAs per head, warp tokens per CTA
+};
+constexpr uint32_t kFusedPolls = 1u << 20;       // about a second
+
+__device__ __forceinline__ void fused_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+// Shared memory: secondaries, two histograms, row scratch, joint table, look-up table (rows, cells, candidates, products).
+__host__ __device__ inline size_t fused_smem_bytes(int S, size_t lut_foot) {
+  return (size_t)S * 16 + 2 * kHistBins * 4 + (size_t)kEnc32Warps * kMaxRowWords * 4 + (size_t)24 * S * 16 + lut_foot + 64;
+}
+
+template <int DT, int IB, int RB, bool DENSE>
+__global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const FusedArgs a, const Maps24 maps, const Mul24 nmul) {
+  constexpr int CB = IB + RB;
+  constexpr float qmaxf = (float)((1 << RB) - 1);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t s_bar;
+  __shared__ uint32_t s_warp[32], s_sel[4], s_flagged;
+  const EncGeom& g = a.g;
+  const int S = g.S, h = blockIdx.x / a.cph, part = blockIdx.x - h * a.cph;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float4* qs = reinterpret_cast<float4*>(smem_raw);
+  uint32_t* sh = reinterpret_cast<uint32_t*>(qs + S);                      // [2][kHistBins]
+  uint32_t* rows = sh + 2 * kHistBins;                                       // [warps][kMaxRowWords]
+  float4* sjoint = reinterpret_cast<float4*>(rows + kEnc32Warps * kMaxRowWords);
+  unsigned char* slut = reinterpret_cast<unsigned char*>(sjoint + 24 * S);
+
+  // ---- tables on their way ------------------------------------------------------------------------------------------
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
+  const uint32_t* gh = reinterpret_cast<const uint32_t*>(a.lut);
+  const unsigned char* head = a.lut + kLutOffHeads + (size_t)h * kLutHeadBytes;
+  const int n = (int)gh[0], n_cells = (int)gh[1];
+  const uint32_t total = reinterpret_cast<const uint32_t*>(head)[0];
+  const uint32_t b_rows = (uint32_t)n * n * 4, b_cells = ((uint32_t)n_cells * 2 + 15) & ~15u, b_cands = (total * 2 + 15) & ~15u;
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(slut), bj = (uint32_t)(24 * S * 16);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bj + b_rows + b_cells + b_cands) : "memory");
+    fused_bulk((uint32_t)__cvta_generic_to_shared(sjoint), a.joint + (int64_t)h * 24 * S * 4, bj, bar);
+    fused_bulk(d, a.lut + kLutOffRows, b_rows, bar);
+    fused_bulk(d + b_rows, head + 16, b_cells, bar);
+    if (b_cands) fused_bulk(d + b_rows + b_cells, head + 16 + (size_t)kLutCellCap * 2, b_cands, bar);
+    s_flagged = 0u;
+  }
+  LutView L;
+  L.rows = reinterpret_cast<const uint32_t*>(slut); L.cells = reinterpret_cast<const uint16_t*>(slut + b_rows);
+  L.cands = reinterpret_cast<const uint16_t*>(slut + b_rows + b_cells);
+  uint8_t* snm = slut + b_rows + b_cells + b_cands;
+  L.nm = snm; L.n = n; L.hn = 0.5f * (float)n;
+  for (int i = threadIdx.x; i < S; i += blockDim.x) qs[i] = reinterpret_cast<const float4*>(a.qs)[(int64_t)h * S + i];
+  // (DENSE decodes with the reference-order joint table: the product table then names reference primaries)
+  for (int i = threadIdx.x; i < 576; i += blockDim.x) {
+    uint8_t v = nmul.v[i / 24][i % 24];
+    if (DENSE) { int p = 0; for (int k = 0; k < 24; ++k) if (maps.ref_to_native[k] == v) p = k; v = (uint8_t)p; }
+    snm[i] = v;
+  }
+
+  // ---- this CTA's tokens: warp token w = (b, i), i a token or (16 chunks) a pair of tokens -----------------------------
+  const bool pair = g.n == 16;
+  const int T2 = pair ? (g.T_new + 1) >> 1 : g.T_new, W = g.B * T2;
+  const int w0 = part * a.per, w1 = min(W, w0 + a.per);
+  const int sub = pair ? lane >> 4 : 0, c = pair ? lane & 15 : lane;
+  const uint16_t* xh = a.x + h * g.xs_h + 4 * c;
+  // token of this lane in warp token w (t >= T: none)
+  auto locate = [&](int w, int& b, int& t) { b = w / T2; const int i = w - b * T2; t = pair ? 2 * i + sub : i; };
+  auto fetch = [&](int w, uint2& raw) {
+    int b, t;
+    locate(w, b, t);
+    const bool live = t < g.T_new;
+    raw = make_uint2(0u, 0u);
+    if (live) raw = *reinterpret_cast<const uint2*>(xh + b * g.xs_b + (int64_t)t * g.xs_t);
+    return live;
+  };
+  auto norm_of = [&](const uint2& raw) {
+    float v[4] = {bits16_to_float(raw.x & 0xffff, DT), bits16_to_float(raw.x >> 16, DT), bits16_to_float(raw.y & 0xffff, DT),
+                  bits16_to_float(raw.y >> 16, DT)};
+    return chunk_norm(v);
+  };
+
+  // ---- exact threshold: three levels of 11, 11 and 10 bits over the head's norms ----------------------------------------
+  float thr = INFINITY;
+  if (a.C > 0.f && a.med_in) {
+    const float med = a.med_in[h];
+    thr = __fmul_rn(med, a.C);
+    if (part == 0 && threadIdx.x == 0 && a.med_out) a.med_out[h] = med;
+  } else if (a.C > 0.f) {
+    const QRank qr = quantile_rank((uint64_t)g.B * g.T_new * g.n, a.quantile);
+    uint32_t p0 = 0u, p1 = 0u, k0 = (uint32_t)qr.lo, k1 = (uint32_t)qr.hi;      // prefixes and ranks of the two statistics
+    for (int level = 0; level < 3; ++level) {
+      const int hs = level == 0 ? 31 : level == 1 ? 21 : 10, ds = level == 0 ? 21 : level == 1 ? 10 : 0;
+      const uint32_t dm = level == 2 ? 0x3ffu : 0x7ffu, q0 = p0 >> hs, q1 = p1 >> hs;
+      const bool same = q0 == q1;
+      for (int i = threadIdx.x; i < 2 * kHistBins; i += blockDim.x) sh[i] = 0u;
+      __syncthreads();
+      for (int w = w0 + warp; w < w1; w += 4 * kEnc32Warps) {
+        uint2 raw[4]; bool live[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) { live[u] = w + u * kEnc32Warps < w1; if (live[u]) live[u] = fetch(w + u * kEnc32Warps, raw[u]); }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (live[u]) {
+            const uint32_t key = __float_as_uint(norm_of(raw[u])), top = key >> hs, dig = (key >> ds) & dm;
+            if (top == q0) atomicAdd(&sh[dig], 1u);
+            else if (top == q1) atomicAdd(&sh[kHistBins + dig], 1u);
+          }
+      }
+      __syncthreads();
+      uint32_t* gl = a.hist + ((int64_t)h * 3 + level) * 2 * kHistBins;
+      for (int i = threadIdx.x; i < (same ? 1 : 2) * kHistBins; i += blockDim.x)
+        if (sh[i]) atomicAdd(&gl[i], sh[i]);
+      // the head's CTAs meet
+      __threadfence();
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        atomicAdd(&a.bars[h], 1u);
+        const uint32_t want = (uint32_t)(a.cph * (level + 1));
+        uint32_t polls = 0, seen;
+        do {
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bars + h) : "memory");
+        } while (seen < want && ++polls < kFusedPolls);
+        if (seen < want) atomicOr(a.status, 2u);
+      }
+      __syncthreads();
+      // scan: two bins per thread
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint2 cnt = __ldcg(reinterpret_cast<const uint2*>(gl + (q && !same ? kHistBins : 0)) + threadIdx.x);
+        const uint32_t mine = cnt.x + cnt.y, rank = q ? k1 : k0;
+        uint32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        uint32_t wv = s_warp[lane], ws = wv;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, ws, o); if (lane >= o) ws += y; }
+        const uint32_t before = __shfl_sync(0xffffffffu, ws - wv, warp) + incl - mine;
+        if (rank >= before && rank < before + mine) {
+          const bool hi = rank >= before + cnt.x;
+          s_sel[2 * q] = (uint32_t)(2 * threadIdx.x + (hi ? 1 : 0));
+          s_sel[2 * q + 1] = rank - before - (hi ? cnt.x : 0u);
+        }
+        __syncthreads();
+      }
+      p0 |= s_sel[0] << ds; k0 = s_sel[1]; p1 |= s_sel[2] << ds; k1 = s_sel[3];
+      __syncthreads();
+    }
+    const float va = __uint_as_float(p0), vb = __uint_as_float(p1);
+    const float med = qr.hi == qr.lo ? va : quantile_lerp(va, vb, qr.w);
+    thr = __fmul_rn(med, a.C);
+    if (part == 0 && threadIdx.x == 0 && a.med_out) a.med_out[h] = med;
+  }
+
+  // ---- main pass --------------------------------------------------------------------------------------------------------
+  __syncthreads();
+  {
+    uint32_t ok = 0u, tries = 0u;
+    while (!ok && ++tries < (1u << 24))
+      asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar) : "memory");
+    if (!ok) { if (threadIdx.x == 0) atomicOr(a.status, 2u); return; }
+  }
+  const float inv_S = 1.0f / (float)S;
+  uint32_t* myrow = rows + warp * kMaxRowWords;
+  uint32_t n_fl = 0u;
+  uint2 nxt = make_uint2(0u, 0u);
+  bool live_n = false;
+  if (w0 + warp < w1) live_n = fetch(w0 + warp, nxt);
+  for (int w = w0 + warp; w < w1; w += kEnc32Warps) {
+    const uint2 raw = nxt;
+    const bool live = live_n;
+    if (w + kEnc32Warps < w1) live_n = fetch(w + kEnc32Warps, nxt);
+    int b, t;
+    locate(w, b, t);
+    float v[4] = {bits16_to_float(raw.x & 0xffff, DT), bits16_to_float(raw.x >> 16, DT), bits16_to_float(raw.y & 0xffff, DT),
+                  bits16_to_float(raw.y >> 16, DT)};
+    const float nrm = chunk_norm(v);
+    const float radius = fmaxf(nrm, 1e-8f);
+    float rmax = radius;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+    {
+      const float other = __shfl_xor_sync(0xffffffffu, rmax, 16);
+      if (!pair) rmax = fmaxf(rmax, other);
+    }
+    const float scale = __fdiv_rn(rmax, qmaxf);
+    // (radius code: see encode_main32_kernel)
+    const float quo = radius * rcp_approx(scale);
+    float rqf = rintf(quo);
+    if (fabsf(quo - rqf) > 0.499f) rqf = rintf(__fdiv_rn(radius, scale));
+    rqf = fminf(fmaxf(rqf, 0.f), qmaxf);
+    const bool flagged = live && nrm > thr;
+    const uint32_t flag_word = __ballot_sync(0xffffffffu, flagged);
+    n_fl += __popc(flag_word);
+    const float inv_r = rcp_approx(radius);
+    int au, sidx;
+    const float u0 = v[0] * inv_r, u1 = v[1] * inv_r, u2 = v[2] * inv_r, u3 = v[3] * inv_r;
+    if (!search_fold24(sjoint, L, S, inv_S, u0, u1, u2, u3, au, sidx)) {
+      int p = 0; sidx = 0;
+      if (fmaxf(fmaxf(fabsf(u0), fabsf(u1)), fmaxf(fabsf(u2), fabsf(u3))) > 0.f) p = search_exhaustive(qs, S, u0, u1, u2, u3, sidx);
+      au = DENSE ? p : maps.ref_to_native[p];
+    }
+    if constexpr (DENSE) {
+      uint2 o = raw;
+      if (!flagged) {
+        const float rad = __fmul_rn(rqf, scale);
+        const float4 cw = sjoint[au * S + sidx];
+        o.x = float_to_bits16(__fmul_rn(cw.x, rad), DT) | ((uint32_t)float_to_bits16(__fmul_rn(cw.y, rad), DT) << 16);
+        o.y = float_to_bits16(__fmul_rn(cw.z, rad), DT) | ((uint32_t)float_to_bits16(__fmul_rn(cw.w, rad), DT) << 16);
+      }
+      if (live) *reinterpret_cast<uint2*>(a.out + ((((int64_t)b * g.H + h) * g.T_new + t) * g.n + c) * 4) = o;
+    } else {
+      const uint32_t ni = (uint32_t)((((au >> 3) * S + sidx) << 3) | (au & 7));
+      const uint32_t f = ni | ((flagged ? 0u : (uint32_t)rqf) << IB);
+      const int64_t row = ((int64_t)b * g.H + h) * a.dst.T_cap + a.t_start + t;       // (pairs: each half-warp its own)
+      if constexpr (CB == 16) {
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, f, 1);
+        if (live && !(lane & 1)) reinterpret_cast<uint32_t*>(a.dst.codes + row * a.dst.row_bytes)[c >> 1] = f | (other << 16);
+      } else {
+        constexpr int RW = CB;                         // words per row of 32 chunks (pairs have 16-bit fields)
+        if (lane < RW) myrow[lane] = 0;
+        __syncwarp();
+        const int bit = lane * CB, wd = bit >> 5, s_ = bit & 31;
+        atomicOr(&myrow[wd], f << s_);
+        if (s_ + CB > 32) atomicOr(&myrow[wd + 1], f >> (32 - s_));
+        __syncwarp();
+        if (lane < RW) reinterpret_cast<uint32_t*>(a.dst.codes + row * a.dst.row_bytes)[lane] = myrow[lane];
+        __syncwarp();
+      }
+      if (live && c == 0) {
+        store_scale(a.dst, row, rmax);
+        if (a.dst.flags) a.dst.flags[row] = pair ? (sub ? flag_word >> 16 : flag_word & 0xffffu) : flag_word;
+      }
+    }
+  }
+  if (DENSE && a.n_flagged && a.C > 0.f) {
+    if (lane == 0 && n_fl) atomicAdd(&s_flagged, n_fl);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_flagged) atomicAdd(a.n_flagged, s_flagged);
+  }
+}

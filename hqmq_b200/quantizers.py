@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 from abc import ABC, abstractmethod
 from itertools import product
 from typing import Optional, Tuple
@@ -100,6 +101,7 @@ class HQMQQuantizer(KVQuantizer):
             raise ValueError(init)
         self.secondary_raw = nn.Parameter(raw.to(device=device, dtype=torch.float32))
         self._tables: dict = {}
+        self._qdq_cache: dict = {}      # argument structs and workspaces of repeated fake-quant calls, per thread and stream
 
     # ---- reference plumbing ---------------------------------------------------------------
     def trainable_parameters(self):
@@ -109,9 +111,11 @@ class HQMQQuantizer(KVQuantizer):
         self.training = training
         if tau is not None:
             self.tau = tau
+        self._qdq_cache.clear()         # (a repeated call does not look at the flags again)
 
     def _refresh_rotations(self):
         self._tables.clear()
+        self._qdq_cache.clear()
 
     def _unsupported(self) -> Optional[str]:
         if self.magnitude_mode != "unit":
@@ -365,19 +369,80 @@ class HQMQQuantizer(KVQuantizer):
             _lib.check(_lib.lib().hqmq_dequant(C.byref(a), _lib.stream_ptr()), "hqmq_dequant")
         return out
 
-    def _qdq(self, x: torch.Tensor, layer_idx: int, kv: int, median_mult: Optional[float] = None,
-             quantile: Optional[float] = None) -> torch.Tensor:
-        """Fake-quantise: decode(encode(x)).  The scale plane is kept in fp32 and the radius is
-        rebuilt as rq * (r_max / qmax), the reference's own order (src/quantizers/hqmq.py:210-216)."""
+    def _fake_quant_args(self, x, layer_idx, kv, median_mult, quantile):
+        """(argument struct, reference to it, workspace, its address and size) of a fake-quant call, or None when the library
+        has no one-step kernel for it."""
+        tb = self.tables(layer_idx, kv, x.device)
         B, H, T, d = x.shape
+        a = _lib.EncodeArgs()
+        a.struct_size = C.sizeof(_lib.EncodeArgs)
+        a.x_dtype, a.x = _lib.dtype_enum(x.dtype), x.data_ptr()
+        a.x_stride = (C.c_int64 * 3)(*x.stride()[:3])
+        a.T_new = T
+        a.qs, a.joint = tb["qs"].data_ptr(), tb["joint"].data_ptr()
+        a.median_mult = float(median_mult) if median_mult is not None else 0.0
+        a.quantile = float(quantile) if quantile is not None else 0.0
+        a.lut, a.lut_footprint = tb["lut"].data_ptr(), tb["lut_footprint"]
+        g = a.dst
+        g.struct_size = C.sizeof(_lib.Packed)
+        g.B, g.H, g.n_chunks, g.S, g.radius_bits = B, H, d // 4, self.secondary_size, self.radius_bits
+        a._keep = tb
+        with _lib.device_guard(x.device):
+            nbytes = _lib.lib().hqmq_fake_quant_workspace_bytes(C.byref(a))
+        if not nbytes:
+            return None
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+        return a, C.byref(a), ws, ws.data_ptr(), nbytes
+
+    def _qdq(self, x: torch.Tensor, layer_idx: int, kv: int, median_mult: Optional[float] = None,
+             quantile: Optional[float] = None, count=None) -> torch.Tensor:
+        """Fake-quantise: decode(encode(x)), in one kernel where the library has it (16-bit inputs of the compiled codebook
+        formats, and every small call).  The radius is rebuilt as rq * (r_max / qmax) from the fp32 scale, the reference's
+        own order (src/quantizers/hqmq.py:210-216).  ``count``: with outliers, what takes the flagged chunks of the call
+        (``_OutlierStats``)."""
+        shape, stride = x.shape, x.stride()
+        if x.is_cuda and len(shape) == 4:
+            with _lib.device_guard(x.device):
+                st = _lib.stream_ptr()
+                key = (layer_idx, kv, shape, stride, x.dtype, x.device, median_mult, quantile, st, threading.get_ident())
+                hit = self._qdq_cache.get(key)
+                # (kept entries were made for aligned addresses: a view at another offset takes the long way round)
+                if hit is not None and x.data_ptr() & 15 == 0:
+                    a, ref, _, ws, nbytes = hit
+                    out = torch.empty(shape, dtype=x.dtype, device=x.device)
+                    a.x = x.data_ptr()
+                    rc = _lib.lib().hqmq_fake_quant(ref, out.data_ptr(), count.slot(shape, x.device) if count is not None else None,
+                                                    ws, nbytes, st)
+                    if rc:
+                        _lib.check(rc, "hqmq_fake_quant")
+                    return out
+        B, H, T, d = shape
         if d % 4 != 0:
             raise ValueError(f"d_head={d} not divisible by 4")
         if T == 0 or B == 0:
             return x.clone()
+        why = self._unsupported()
+        if why:
+            raise NotImplementedError(f"hqmq_b200 accelerates the unit-magnitude linear-radius path only ({why})")
+        _lib.require_cuda(x, "HQMQQuantizer.encode")
+        _lib.check_device(x.device)
+        if H != self.n_heads:
+            raise ValueError(f"x has {H} heads, quantizer has {self.n_heads}")
+        if x.dtype in (torch.float16, torch.bfloat16, torch.float32) and d <= 128 and x.data_ptr() & 15 == 0 and stride[-1] == 1 \
+                and not any(s % 4 for s in stride[:3]):
+            entry = self._fake_quant_args(x, layer_idx, kv, median_mult, quantile)
+            if entry is not None:
+                if len(self._qdq_cache) >= 256:
+                    self._qdq_cache.clear()
+                with _lib.device_guard(x.device):
+                    key = (layer_idx, kv, shape, stride, x.dtype, x.device, median_mult, quantile, _lib.stream_ptr(), threading.get_ident())
+                self._qdq_cache[key] = entry
+                return self._qdq(x, layer_idx, kv, median_mult, quantile, count)
         pk = self.new_cache(B, T, d, x.device, scale_dtype=torch.float32, with_outliers=median_mult is not None,
                             out_dtype=x.dtype if x.dtype != torch.float64 else torch.float32)
         self.encode(x, layer_idx, kv, out=pk, median_mult=median_mult, quantile=quantile)
-        self._last_packed = pk
+        if count is not None:
+            count.push_count(pk.out_count, B * H * T * (d // 4))
         return self.decode(pk, layer_idx, kv, dtype=x.dtype, scale_first=True)
 
     def quantize_K(self, k, layer_idx):
@@ -418,6 +483,26 @@ class _OutlierStats:
         self._open = []             # records with calls that were not accounted yet
         self._closed = []           # (counter at the end, counter or number at the start, calls' size, calls)
         self._sum_rates, self._n = 0.0, 0   # sum of the per-call rates, number of calls
+        self._slots = {}            # per device: (counters, sizes of the calls that took one each)
+        self._lock = threading.Lock()
+
+    def slot(self, shape, device) -> int:
+        """Address of a zeroed device counter for one fake-quant call of that shape."""
+        with self._lock:
+            got = self._slots.get(device)
+            if got is None or len(got[1]) >= self._FOLD:
+                if got is not None:
+                    self._fold_slots(device)
+                got = self._slots[device] = (torch.zeros(self._FOLD, dtype=torch.int32, device=device), [])
+            got[1].append(shape[0] * shape[1] * shape[2] * (shape[3] // 4))
+            return got[0].data_ptr() + 4 * (len(got[1]) - 1)
+
+    def _fold_slots(self, device):
+        counters, sizes = self._slots.pop(device)
+        torch.cuda.synchronize(device)              # (calls of other streams may still be counting)
+        for flagged, total in zip(counters[:len(sizes)].tolist(), sizes):
+            self._sum_rates += flagged / max(1, total)
+        self._n += len(sizes)
 
     # a record: [counter tensor, count at the start (number or tensor), calls, chunks per call]
     def begin(self, pk, total_chunks: int):
@@ -445,12 +530,15 @@ class _OutlierStats:
             self._sync()
 
     def push_count(self, counter: torch.Tensor, total_chunks: int):
-        """A finished one-shot call (fake-quant): only its counter is kept, not its cache."""
+        """A finished fake-quant call that went through a cache: only the counter is kept."""
         self._closed.append((counter, 0.0, total_chunks, 1))
         if len(self._open) + len(self._closed) >= self._FOLD:
             self._sync()
 
     def _sync(self):
+        with self._lock:
+            for device in list(self._slots):
+                self._fold_slots(device)
         done, self._closed = self._closed, []
         recs = {id(r): r for r in self._open if r[2]}.values()
         self._open = []
@@ -552,10 +640,7 @@ class OutlierAwareHQMQQuantizer(KVQuantizer):
 
     def _qdq(self, x, layer_idx, kv):
         self._check_mode()
-        out = self.inner._qdq(x, layer_idx, kv, **self._thr())
-        if x.shape[0] and x.shape[2]:
-            self._stats.push_count(self.inner._last_packed.out_count, x.shape[0] * x.shape[1] * x.shape[2] * (x.shape[3] // 4))
-        return out
+        return self.inner._qdq(x, layer_idx, kv, count=self._stats, **self._thr())
 
     def quantize_K(self, k, layer_idx):
         return self._qdq(k, layer_idx, kv=0)

@@ -213,6 +213,18 @@ size_t hqmq_encode_workspace_bytes(const hqmq_encode_args* args);
 int hqmq_encode(const hqmq_encode_args* args, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * The dense fake-quantised tensor straight from x: what hqmq_encode followed by hqmq_dequant(layout 0, scale_first,
+ * merge_outliers) gives on an fp32 scale plane, bit for bit, without the planes in between.  Of args->dst only the geometry
+ * (B, H, n_chunks, S, radius_bits) is read; t_start must be 0.  out: (B, H, T_new, 4 n_chunks) contiguous, element type of
+ * x, 16-byte aligned.  n_flagged (may be NULL): device uint32 that the call's flagged chunks are added to.
+ * HQMQ_ERR_UNSUPPORTED for the calls that only the two-step route takes (workspace size 0): more than a small call in fp32,
+ * without a look-up table, or in a geometry other than 32 chunks per token (16 with 16-bit fields).
+ */
+size_t hqmq_fake_quant_workspace_bytes(const hqmq_encode_args* args);
+int hqmq_fake_quant(const hqmq_encode_args* args, void* out, uint32_t* n_flagged, void* workspace, size_t workspace_bytes,
+                    void* stream);
+
+/*
  * The K and the V tensor of one layer in one call: the reference cache quantises both on every update
  * (src/model_utils.py:29-32, QuantizedCache.update).  Same results as hqmq_encode(k) followed by
  * hqmq_encode(v); each tensor keeps its own median, tables and planes.  For the decode-time append (a small
@@ -251,7 +263,8 @@ int hqmq_med3x_select(int H, int level, uint64_t n_total, float median_mult, voi
  * printed or trapped on.  This copies that word to the host after synchronising `stream`.
  *   workspace of hqmq_encode:       bit 0 = the outlier side buffer (out_cap) was too small; rows,
  *                                   flags and counts are complete, payload entries beyond the
- *                                   capacity were dropped
+ *                                   capacity were dropped; bit 1 = the call gave up on a bounded wait
+ *                                   between its thread blocks, what it wrote is not valid
  *   workspace of hqmq_attn_decode:  non-zero = some call on this workspace gave up on a bounded wait
  *                                   for a staged copy; the output rows of that call are not valid (NaN where
  *                                   a merge still ran, untouched elsewhere)

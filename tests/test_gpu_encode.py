@@ -495,3 +495,41 @@ def test_d64_rows_with_padding_bits(S, br, C):
     b = q.encode(x.float().cuda(), 0, 0, median_mult=C, scale_dtype=torch.float32).to_reference()
     for got, want in zip(a, b):
         assert got is None and want is None or torch.equal(got, want)
+
+
+@pytest.mark.parametrize("shape,S,br", [((1, 2, 97, 128), 24, 3), ((3, 3, 1001, 128), 192, 6), ((2, 8, 777, 64), 96, 4),
+                                        ((1, 1, 5000, 64), 96, 4), ((5, 4, 130, 128), 96, 4), ((70, 2, 16, 64), 96, 4)])
+@pytest.mark.parametrize("C", [None, 3.0])
+@pytest.mark.parametrize("tokens_first", [False, True])
+def test_one_launch_encoder(shape, S, br, C, tokens_first):
+    """Calls between the append and the very long prompt: several CTAs per head, odd token counts (two 64-wide tokens per
+    warp), strided inputs.  The 16-bit call must give what its fp32 upcast gives through the generic passes, and the dense
+    fake-quantised tensor what decoding that cache gives, bit for bit."""
+    x = make_kv("spiky", shape, seed=91, dtype=torch.bfloat16).cuda()
+    xs = x.transpose(1, 2).contiguous().transpose(1, 2) if tokens_first else x
+    q = hqmq.HQMQ(1, shape[1], S, br, device="cuda")
+    med = [torch.zeros(shape[1], device="cuda") for _ in range(2)] if C else [None, None]
+    a = q.encode(xs, 0, 0, median_mult=C, scale_dtype=torch.float32, med_out=med[0])
+    b = q.encode(x.float(), 0, 0, median_mult=C, scale_dtype=torch.float32, med_out=med[1])
+    for got, want in zip(a.to_reference(), b.to_reference()):
+        assert got is None and want is None or torch.equal(got, want)
+    if C:
+        assert torch.equal(med[0], med[1]) and torch.equal(a.out_off, b.out_off) and torch.equal(a.out_count, b.out_count)
+        assert torch.equal(a.out_vals.float(), b.out_vals)
+    dense = q._qdq(xs, 0, 0, median_mult=C)
+    assert torch.equal(dense, q.decode(b, 0, 0, dtype=torch.bfloat16, scale_first=True))
+    assert dense.is_contiguous()
+
+
+@pytest.mark.parametrize("shape,dtype", [((16, 2, 1, 128), torch.bfloat16), ((1, 3, 9, 48), torch.float32), ((2, 2, 2, 64), torch.float16),
+                                         ((7, 2, 9, 128), torch.bfloat16)])
+def test_small_fake_quant_counts_and_values(shape, dtype):
+    x = make_kv("spiky", shape, seed=93, dtype=dtype).cuda()
+    x[..., :4] *= 30
+    q = hqmq.with_outlier_extraction(hqmq.HQMQ(2, shape[1], 96, 4, device="cuda"), 3.0)
+    rates = []
+    for layer in (0, 1, 1):
+        pk = q.inner.encode(x, layer, 0, median_mult=3.0, scale_dtype=torch.float32)
+        assert torch.equal(q.quantize_K(x, layer), q.inner.decode(pk, layer, 0, dtype=dtype, scale_first=True))
+        rates.append(pk.n_outliers() / (x.numel() // 4))
+    assert max(rates) > 0 and abs(q._observed_outlier_rate - np.mean(rates)) < 1e-9 and q._n_observations == 3
