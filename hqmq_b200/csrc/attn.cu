@@ -10,7 +10,7 @@
 namespace hqmq {
 namespace attn {
 
-const void* fast_kernel(int n_chunks, int ib, int rb, bool outl);
+const void* fast_kernel(int n_chunks, int ib, int rb, bool outl, bool small);
 size_t fast_warp_bytes(int n_chunks, int ib, int rb, bool outl);
 bool ring_kernel(int n_chunks, int ib, int rb, bool outl, int scale_dtype, RingKernelInfo& k);
 size_t ring_smem_total(int table_rows, int repk_log2, int repv_log2, int d, bool outl, int stages, int merge_slots,
@@ -107,6 +107,7 @@ struct Plan {
   int repv_log2, ring_stages, merge_slots; // ring kernels only
   size_t ticket_bytes;                     // ring kernels: one ticket word per unit between the status word and the partials
   int ppc;   // partials a CTA writes per unit and head: 1 for the staged kernels (merged in shared memory), nw otherwise
+  int cluster;      // CTAs per unit of the cluster kernels (0: another kernel)
   int warp_units;   // staged kernels: warp mode (the warps walk through the units independently; ppc = nw)
   int units, tpu_v, L, P, grid;
   size_t ws_bytes;
@@ -199,6 +200,8 @@ cudaError_t raise_smem_limit(const void* kernel, size_t smem) {
   return rc;
 }
 
+// Rounds of tiles per warp up to which a unit is the work of one cluster.
+constexpr int kSmallMaxRounds = 2;
 // Units of at most this many tiles run the staged kernels in warp mode (every warp has at most two tiles of a unit)
 constexpr int kWarpModeMaxTiles = 32;
 
@@ -215,7 +218,7 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
     // the staged kernels copy 16-byte aligned pieces: side buffers must start on 16 bytes per (b,h)
     const bool side_ok = !outl || (((!a->K.flags || (a->K.out_cap % 2 == 0 && ((uintptr_t)a->K.out_vals & 15) == 0))) &&
                                    ((!a->V.flags || (a->V.out_cap % 2 == 0 && ((uintptr_t)a->V.out_vals & 15) == 0))));
-    if (G <= 8 && is_half_dtype(a->K.scale_dtype) && side_ok) pl.kernel = fast_kernel(n, pl.ib, a->K.radius_bits, outl);
+    if (G <= 8 && is_half_dtype(a->K.scale_dtype) && side_ok) pl.kernel = fast_kernel(n, pl.ib, a->K.radius_bits, outl, false);
     if (pl.kernel) pl.nw = outl ? kFastWarpsOutl : kFastWarps;
   } else {
     pl.ib = 16;
@@ -227,6 +230,7 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
   if (!pl.kernel) return HQMQ_ERR_UNSUPPORTED;
   pl.threads = pl.nw * 32;
   pl.repv_log2 = pl.ring_stages = pl.merge_slots = 0;
+  pl.cluster = 0;
   const int keys = a->window > 0 ? (a->window < a->T_kv ? a->window : a->T_kv) : a->T_kv;
   // Long key ranges: the kernels with one CTA-wide staging ring.  The kernels are bound by shared-memory bandwidth
   // (the random 8-byte codeword gathers), so shared memory goes first to the replication of the sign-folded tables
@@ -268,6 +272,26 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
     pl.warp_units = fast && !ring && allow_warp_mode && a->kv_splits == 0 && tpu <= kWarpModeMaxTiles && tpu < piece;
   }
   if (pl.warp_units) pl.ppc = pl.nw;
+  // Few units of few tiles: a unit per cluster.  As many CTAs per unit as the SMs allow (8 is the portable cluster size), but
+  // not under half a tile per warp; with more than two rounds of tiles per warp the flat split over all SMs with replicated
+  // tables is the better one (one sequence, 8 heads: 64 CTAs of 2 rounds win to 4096 tokens, lose at 8192).
+  if (fast && !ring && a->kv_splits == 0 && !pl.warp_units && pl.units <= 148) {
+    int c = 148 / pl.units;
+    if (c > 8) c = 8;
+    while (c > 1 && (tpu + c - 1) / c < pl.nw / 2) --c;
+    const int per = (tpu + c - 1) / c;
+    if (per <= kSmallMaxRounds * pl.nw) {
+      const size_t smem = (size_t)pl.table_rows * 16 + (outl ? (size_t)8 * (a->d + kFastQPad) * 2 : 0) + (((size_t)pl.nw * kFastStages * 8 + 15) & ~(size_t)15) +
+                          (size_t)pl.nw * fast_warp_bytes(n, pl.ib, a->K.radius_bits, outl);
+      if (smem <= 220 * 1024) {
+        pl.kernel = fast_kernel(n, pl.ib, a->K.radius_bits, outl, true);
+        pl.cluster = c; pl.smem = smem; pl.rep_log2 = 0;
+        pl.tpu_v = per * c; pl.L = per; pl.P = c; pl.grid = pl.units * c;
+        pl.ticket_bytes = 0; pl.ws_bytes = 16;
+        return HQMQ_OK;
+      }
+    }
+  }
   if (ring) {
     pl.kernel = rk.fn;
     pl.nw = rk.warps;
@@ -435,6 +459,19 @@ extern "C" int hqmq_attn_decode(const hqmq_attn_args* a, void* workspace, size_t
   }
   // (the kernel's dynamic shared-memory limit was raised when the plan asked for its occupancy: resident_ctas)
   void* kargs[] = {&p};
+  if (pl.cluster) {
+    HQMQ_CHECK_CUDA(raise_smem_limit(pl.kernel, pl.smem));
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = pl.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pl.grid); cfg.blockDim = dim3(pl.threads); cfg.dynamicSmemBytes = pl.smem; cfg.stream = st;
+    cfg.attrs = at; cfg.numAttrs = 2;
+    HQMQ_CHECK_CUDA(cudaLaunchKernelExC(&cfg, pl.kernel, kargs));
+    return HQMQ_OK;
+  }
   HQMQ_CHECK_CUDA(cudaLaunchKernel(pl.kernel, dim3(pl.grid), dim3(pl.threads), kargs, pl.smem, st));
   if (fused_merge) { HQMQ_LAUNCH_CHECK(); return HQMQ_OK; }
   const int64_t rows = (int64_t)a->B * a->H_q * a->T_q;

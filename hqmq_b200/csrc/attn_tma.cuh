@@ -57,10 +57,37 @@ struct StageLayout {
   static_assert((kTile * ROW) % 16 == 0, "tile of code rows must be a multiple of 16 bytes");
 };
 
-template <int N, int IB, int RB, int NW, bool OUTL>
+// ---- thread-block clusters and dependent launches ----------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// A float of this CTA's shared memory at the same place in CTA `rank` of the cluster.
+__device__ __forceinline__ float cluster_ld(const float* mine, uint32_t rank) {
+  float v;
+  uint32_t a = smem_u32(mine);
+  asm volatile("{\n .reg .b32 t;\n mapa.shared::cluster.u32 t, %1, %2;\n ld.shared::cluster.f32 %0, [t];\n}\n" : "=f"(v) : "r"(a), "r"(rank) : "memory");
+  return v;
+}
+// A kernel launched with programmatic stream serialisation may start before its predecessor has finished: what precedes
+// grid_dep_wait() must not touch anything the predecessor writes.  grid_dep_launch() lets the successor start likewise; it
+// comes after the wait, so that a successor's own wait still covers everything before this kernel.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// SMALL: problems of a few tiles per warp.  A unit is the work of ONE cluster, p.L tiles to a CTA, and the CTAs' results are
+// merged through distributed shared memory: no partials in global memory, no merge launch.  The codeword tables are not
+// replicated (two bulk copies in flight beside the first tiles instead of 70-150 KB of stores: with one or two tiles per
+// warp the stores cost more than the bank conflicts they save).  One sequence of 4096 tokens, 8 heads: kernel + merge
+// 18.0 us before.
+template <int N, int IB, int RB, int NW, bool OUTL, bool SMALL>
 __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32_t* status) {
   using G_ = Geo<N>;
-  constexpr bool FOLD = !OUTL;   // the outlier kernel is issue-bound: it keeps the full table and the shorter gather
+  constexpr bool FOLD = !OUTL && !SMALL;   // the outlier kernel is issue-bound: it keeps the full table and the shorter gather
   using FL = FastLoader<N, IB, RB, FOLD>;
   using SL = StageLayout<N, IB, RB, OUTL>;
   constexpr int NKS = G_::NKS, NVG = G_::NVG, NOT = 2 * G_::NVG;
@@ -93,6 +120,22 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
     for (int s = 0; s < kStages; ++s) mbar_init(bar0 + 8 * s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  const uint32_t crank = SMALL ? cluster_rank() : 0u;
+  __shared__ __align__(8) uint64_t s_tbar;
+  __shared__ float s_part[SMALL ? NHEADS * (4 * N + 2) : 1];      // this CTA's merged partial
+  if constexpr (SMALL) {
+    if (threadIdx.x == 0) {
+      const uint32_t tb = smem_u32(&s_tbar), bytes = (uint32_t)tbl_bytes;
+      mbar_init(tb, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      mbar_expect_tx(tb, 2 * bytes);
+      const int64_t row0 = (int64_t)((blockIdx.x / p.P) / (p.B * p.Tq)) * p.table_rows;
+      bulk_g2s(smem_u32(tblK), p.tblK + row0 * 4, bytes, tb);
+      bulk_g2s(smem_u32(tblV), p.tblV + row0 * 4, bytes, tb);
+    }
+    grid_dep_wait();
+    grid_dep_launch();
+  }
   __syncwarp();
   uint32_t it = 0;        // tiles this warp has consumed so far (stage = it % kStages, parity from it / kStages)
   bool failed = false, drained = false;
@@ -103,7 +146,8 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
   const int upb = p.B * p.Tq;
   int cur_h = -1;
 
-  for (int u = (int)(flat_lo / p.tpu_v); (int64_t)u * p.tpu_v < flat_hi; ++u) {
+  const int u_first = SMALL ? (int)blockIdx.x / p.P : (int)(flat_lo / p.tpu_v);
+  for (int u = u_first; SMALL ? u == u_first : (int64_t)u * p.tpu_v < flat_hi; ++u) {
     const int h = u / upb, bt = u - h * upb;
     const int b = bt / p.Tq, tq = bt - b * p.Tq;
     // CTA mode: all warps share the unit -- barriers around the tables and the staged queries of every unit, the warps'
@@ -113,8 +157,8 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
     // and the CTA meets only where the KV head, and with it the tables, changes.  (In CTA mode a unit of ten tiles kept
     // six of sixteen warps idle and every unit paid barriers, a merge and the latency of its first copies in turn:
     // 42 us for 512 units of ten tiles at d_head 64.)
-    if (wm ? h != cur_h : (h != cur_h || OUTL)) __syncthreads();
-    if (h != cur_h) {
+    if (!SMALL && (wm ? h != cur_h : (h != cur_h || OUTL))) __syncthreads();
+    if (!SMALL && h != cur_h) {
       const int reps = 1 << p.rep_log2;
       for (int i = threadIdx.x; i < rows_f; i += NW * 32) {
         const uint2 ek = (reinterpret_cast<const uint2*>(p.tblK) + (int64_t)h * p.table_rows)[FOLD ? 2 * i : i];
@@ -126,7 +170,7 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
       cur_h = h;
       if (wm) __syncthreads();
     }
-    if (!wm) {
+    auto stage_queries = [&] {
       if constexpr (OUTL) {
         for (int i = threadIdx.x; i < NHEADS * p.d; i += NW * 32) {
           const int g = i / p.d, x = i - g * p.d;
@@ -135,7 +179,8 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
         }
       }
       __syncthreads();
-    }
+    };
+    if (!SMALL && !wm) stage_queries();
 
     int t_beg, t_end;
     key_range(p.Tkv, p.Tq, p.causal, p.window, tq, t_beg, t_end);
@@ -143,8 +188,8 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
     const int64_t ubase = (int64_t)u * p.tpu_v;
     const int rel_lo = (int)(flat_lo > ubase ? flat_lo - ubase : 0);
     const int rel_hi = (int)(flat_hi < ubase + p.tpu_v ? flat_hi - ubase : p.tpu_v);
-    const int my_lo = tile_lo + rel_lo;
-    const int my_hi = min(tile_hi, tile_lo + rel_hi);
+    const int my_lo = SMALL ? min(tile_hi, tile_lo + (int)crank * p.L) : tile_lo + rel_lo;
+    const int my_hi = SMALL ? min(tile_hi, my_lo + p.L) : min(tile_hi, tile_lo + rel_hi);
     const int part = (int)blockIdx.x - (int)(ubase / p.L);   // this CTA's slot among the CTAs that share the unit
     // this warp's first tile of the piece is my_lo + w0: the warp's own index, or in warp mode its turn in the
     // round-robin over the CTA's flat range
@@ -251,6 +296,7 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
       }
     }
 
+    if constexpr (SMALL) stage_queries();
     // ---- Q as B fragments (loaded while the first copies are in flight) ------------------------------------------
     uint32_t qb[NKS][2];
     {
@@ -275,6 +321,15 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
           *reinterpret_cast<uint2*>(qh16 + r * qstride + 4 * (j * NKS + ks)) = make_uint2(qb[ks][0], qb[ks][1]);
         __syncwarp();
       }
+    }
+    if constexpr (SMALL) {
+      // (every thread waits: a CTA must not exit with a copy into it in flight)
+      uint32_t spins = 0;
+      while (!mbar_try_wait(smem_u32(&s_tbar), 0)) {
+        if (++spins > kWaitLimit) { failed = true; break; }
+      }
+      failed = __any_sync(0xffffffffu, failed);
+      if (failed && lane == 0) *status = p.epoch;
     }
     for (int k = 0; k < n_my && !failed; ++k, ++it) {
       const int tile = my_lo + w0 + k * NW;
@@ -570,10 +625,12 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
     // ---- one partial per (CTA, unit, head): the warps' results are merged in shared memory ---------------------
     // The rings are idle between units (every issued tile was consumed), so their memory holds the warps'
     // partials [warp][head][d + 2] for the merge.  A warp that gave up on a wait takes the whole CTA out here.
-    if (__syncthreads_or(failed ? 1 : 0)) break;
+    const bool cta_failed = __syncthreads_or(failed ? 1 : 0) != 0;
+    if (!SMALL && cta_failed) break;
     constexpr int PD = 4 * N + 2;
     float* mp = reinterpret_cast<float*>(warp_area);
-    {
+    const int n_act = SMALL ? min(NW, my_hi - my_lo) : NW;       // warps that had a tile
+    if (warp < n_act) {
       float* mine = mp + warp * NHEADS * PD;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
@@ -599,19 +656,47 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
       const float* col = mp + g * PD;
       float m_star = -INFINITY;
 #pragma unroll
-      for (int w = 0; w < NW; ++w) m_star = fmaxf(m_star, col[w * NHEADS * PD + 4 * N]);
+      for (int w = 0; w < NW; ++w) if (!SMALL || w < n_act) m_star = fmaxf(m_star, col[w * NHEADS * PD + 4 * N]);
       const float m_use = m_star == -INFINITY ? 0.f : m_star;
       float acc = 0.f, l_star = 0.f;
 #pragma unroll
       for (int w = 0; w < NW; ++w) {
+        if (SMALL && w >= n_act) break;
         const float wgt = fast_exp2(col[w * NHEADS * PD + 4 * N] - m_use);   // 0 for a warp that saw no key
         acc = fmaf(col[w * NHEADS * PD + x], wgt, acc);
         l_star = fmaf(col[w * NHEADS * PD + 4 * N + 1], wgt, l_star);
       }
       const int64_t row = ((int64_t)b * p.Hq + h * p.G + g) * p.Tq + tq;
-      float* dst = p.partials + (row * p.P + part) * PD;
-      dst[x] = acc;
+      float* dst = SMALL ? s_part + g * PD : p.partials + (row * p.P + part) * PD;
+      dst[x] = SMALL && cta_failed ? NAN : acc;
       if (x == 0) { dst[4 * N] = m_star; dst[4 * N + 1] = l_star; }
+    }
+    if constexpr (SMALL) {
+      // ---- the cluster's CTAs: element (g, x) of the output is merged by one of them ----------------------------------
+      cluster_sync();
+      for (int i = (int)crank * NW * 32 + threadIdx.x; i < p.G * (4 * N); i += p.P * NW * 32) {
+        const int g = i / (4 * N), x = i - g * (4 * N);
+        const float* col = s_part + g * PD;
+        float m_star = -INFINITY;
+        for (int c = 0; c < p.P; ++c) m_star = fmaxf(m_star, cluster_ld(col + 4 * N, c));
+        const float m_use = m_star == -INFINITY ? 0.f : m_star;
+        float acc = 0.f, l_star = 0.f;
+        for (int c = 0; c < p.P; ++c) {
+          const float wgt = fast_exp2(cluster_ld(col + 4 * N, c) - m_use);
+          acc = fmaf(cluster_ld(col + x, c), wgt, acc);
+          l_star = fmaf(cluster_ld(col + 4 * N + 1, c), wgt, l_star);
+        }
+        if (p.merged) {
+          const int64_t row = ((int64_t)b * p.Hq + h * p.G + g) * p.Tq + tq;
+          p.merged[row * PD + x] = acc;
+          if (x == 0) { p.merged[row * PD + 4 * N] = m_star; p.merged[row * PD + 4 * N + 1] = l_star; }
+        } else {
+          store_float(p.O, (int64_t)b * p.os_b + (int64_t)(h * p.G + g) * p.os_h + (int64_t)tq * p.os_t + x,
+                      l_star > 0.f || !(acc == acc) ? acc / l_star : 0.f, p.o_dtype);
+        }
+      }
+      cluster_sync();      // nobody leaves while its partial is being read
+      return;
     }
     __syncthreads();   // the merge is done with the ring memory before the next unit's copies land in it
   }

@@ -1,0 +1,46 @@
+"""Decode attention of small problems (a unit per thread-block cluster, merged through distributed shared memory) against a
+plain fp32 evaluation on the dense reconstruction: one to eight CTAs per unit, CTAs without a tile, warps without a tile,
+one key, windows, partial results."""
+import math
+
+import pytest
+import torch
+
+import hqmq_b200 as hqmq
+from tests.test_gpu_prefill import _check, _dense_attention
+from tests.util import make_kv
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,d,T,Tq,window", [
+    (1, 4, 1, 128, 1, 1, None),            # one key
+    (1, 8, 8, 128, 4096, 1, None),         # eight CTAs per unit, two rounds of tiles per warp
+    (1, 7, 1, 128, 4095, 1, None),
+    (2, 8, 2, 128, 2000, 1, None),         # the last CTA of a unit has fewer tiles
+    (1, 8, 1, 128, 1100, 1, None),         # 69 tiles over eight CTAs of nine: the last has six
+    (4, 64, 8, 64, 513, 1, None),          # four CTAs per unit
+    (3, 8, 1, 64, 777, 1, 128),            # one CTA per unit, nine tiles for sixteen warps
+    (1, 16, 2, 64, 3000, 3, None),         # a few query positions
+    (37, 16, 4, 64, 300, 1, None),         # 148 units
+])
+@pytest.mark.parametrize("S,br,outliers", [(96, 4, True), (96, 4, False), (24, 3, True), (192, 6, False)])
+def test_small_decode(B, Hq, Hkv, d, T, Tq, window, S, br, outliers):
+    if d == 64 and S != 96:
+        pytest.skip("rows with padding bits take the generic kernel")
+    q = hqmq.HQMQ(1, Hkv, S, br, device="cuda")
+    K = make_kv("hot" if d == 128 and outliers else "spiky", (B, Hkv, T, d), seed=71, dtype=torch.bfloat16).cuda()
+    V = make_kv("spiky" if outliers else "randn", (B, Hkv, T, d), seed=72, dtype=torch.bfloat16).cuda()
+    mult = 3.0 if outliers else None
+    Kp, Vp = q.encode(K, 0, 0, median_mult=mult), q.encode(V, 0, 1, median_mult=mult)
+    tk, tv = q.tables(0, 0, "cuda")["table16"], q.tables(0, 1, "cuda")["table16"]
+    Q = (torch.randn(B, Hq, Tq, d, generator=torch.Generator().manual_seed(73)) / math.sqrt(d)).bfloat16().cuda()
+    causal = "bottom_right" if Tq > 1 else False
+    want = _dense_attention(Q, q.decode(Kp, 0, 0), q.decode(Vp, 0, 1), causal, window)
+    O = torch.empty(Q.shape, dtype=torch.float32, device="cuda")
+    for _ in range(2):
+        hqmq.fused_attention_packed(Q, Kp, Vp, tk, tv, causal=causal, window=window, out=O.fill_(7))
+        _check(O, want)
+    parts = torch.full((1, B, Hq, Tq, d + 2), float("nan"), device="cuda")
+    hqmq.fused_attention_packed(Q, Kp, Vp, tk, tv, causal=causal, window=window, partials=parts[0])
+    _check(hqmq.combine_partials(parts), want)
