@@ -230,7 +230,7 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
   if (!pl.kernel) return HQMQ_ERR_UNSUPPORTED;
   pl.threads = pl.nw * 32;
   pl.repv_log2 = pl.ring_stages = pl.merge_slots = 0;
-  pl.cluster = 0;
+  pl.cluster = pl.warp_units = 0;
   const int keys = a->window > 0 ? (a->window < a->T_kv ? a->window : a->T_kv) : a->T_kv;
   // Long key ranges: the kernels with one CTA-wide staging ring.  The kernels are bound by shared-memory bandwidth
   // (the random 8-byte codeword gathers), so shared memory goes first to the replication of the sign-folded tables
@@ -264,18 +264,10 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
   int tpu = (keys + kTile - 1) / kTile + (a->window > 0 ? 1 : 0);
   if (tpu < 1) tpu = 1;
   pl.units = a->B * a->T_q * a->H_kv;
-  // Staged kernels, many short units: warp mode.  Every warp then writes its own partial per unit and CTA (16 times
-  // the scratch of the in-CTA merge), so a caller whose scratch is fixed can rule it out.
-  {
-    // (a CTA's piece of the flat tile sequence: at least a tile per warp; warp mode pays when it spans several units)
-    const int64_t piece = std::max<int64_t>(((int64_t)pl.units * tpu + 147) / 148, pl.nw);
-    pl.warp_units = fast && !ring && allow_warp_mode && a->kv_splits == 0 && tpu <= kWarpModeMaxTiles && tpu < piece;
-  }
-  if (pl.warp_units) pl.ppc = pl.nw;
   // Few units of few tiles: a unit per cluster.  As many CTAs per unit as the SMs allow (8 is the portable cluster size), but
-  // not under half a tile per warp; with more than two rounds of tiles per warp the flat split over all SMs with replicated
-  // tables is the better one (one sequence, 8 heads: 64 CTAs of 2 rounds win to 4096 tokens, lose at 8192).
-  if (fast && !ring && a->kv_splits == 0 && !pl.warp_units && pl.units <= 148) {
+  // not under half a tile per warp; beyond kSmallMaxRounds rounds of tiles per warp the flat split over all SMs with
+  // replicated tables takes over (see there).
+  if (fast && !ring && a->kv_splits == 0 && pl.units <= 148) {
     int c = 148 / pl.units;
     if (c > 8) c = 8;
     while (c > 1 && (tpu + c - 1) / c < pl.nw / 2) --c;
@@ -292,6 +284,14 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
       }
     }
   }
+  // Staged kernels, many short units: warp mode.  Every warp then writes its own partial per unit and CTA (16 times
+  // the scratch of the in-CTA merge), so a caller whose scratch is fixed can rule it out.
+  {
+    // (a CTA's piece of the flat tile sequence: at least a tile per warp; warp mode pays when it spans several units)
+    const int64_t piece = std::max<int64_t>(((int64_t)pl.units * tpu + 147) / 148, pl.nw);
+    pl.warp_units = fast && !ring && allow_warp_mode && a->kv_splits == 0 && tpu <= kWarpModeMaxTiles && tpu < piece;
+  }
+  if (pl.warp_units) pl.ppc = pl.nw;
   if (ring) {
     pl.kernel = rk.fn;
     pl.nw = rk.warps;

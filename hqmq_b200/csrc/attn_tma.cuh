@@ -128,6 +128,7 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
       const uint32_t tb = smem_u32(&s_tbar), bytes = (uint32_t)tbl_bytes;
       mbar_init(tb, 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      grid_dep_wait();
       mbar_expect_tx(tb, 2 * bytes);
       const int64_t row0 = (int64_t)((blockIdx.x / p.P) / (p.B * p.Tq)) * p.table_rows;
       bulk_g2s(smem_u32(tblK), p.tblK + row0 * 4, bytes, tb);

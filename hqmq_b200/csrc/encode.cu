@@ -1798,6 +1798,8 @@ __global__ void __launch_bounds__(kSmallThreads) append_pair_kernel(SmallPair p)
   }
 }
 
+#include "encode_append.cuh"
+
 // ---- look-up table construction ---------------------------------------------------------------------
 // Geometry (the same for every head): per (cx, cy) column the stored cz range = the cells whose grown box meets
 // the octahedron |w1| + |w2| + |w3| <= 1, and the index of the column's first cell.
@@ -2417,6 +2419,24 @@ extern "C" int hqmq_encode_pair(const hqmq_encode_args* k, const hqmq_encode_arg
   rc = fill_small(v, plan_ws(*v), reinterpret_cast<uint32_t*>(wsb + wk), pr.t[1]);
   if (rc) return rc;
   memcpy(pr.maps.ref_to_native, index_maps().ref_to_native, 24);
+  const int64_t chunks = (int64_t)dk.B * k->T_new * dk.n_chunks;
+  if (k->T_new == 1 && chunks <= kAppendMax) {
+    // one token per sequence: the low-latency kernel; its status words are cleared inside where a tensor's heads fit a cluster
+    AppendArgs ap;
+    ap.t[0] = pr.t[0]; ap.t[1] = pr.t[1]; ap.maps = pr.maps; ap.clear = dk.H <= 8 ? 1 : 0;
+    if (!ap.clear) HQMQ_CHECK_CUDA(cudaMemset2DAsync(wsb, wk, 0, sizeof(uint32_t), 2, st));
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = dk.H; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(dk.H, 2); cfg.blockDim = dim3(2 * (int)((chunks + 31) / 32 * 32)); cfg.stream = st;
+    cfg.attrs = at; cfg.numAttrs = ap.clear ? 2 : 1;
+    void* kargs[] = {&ap};
+    HQMQ_CHECK_CUDA(cudaLaunchKernelExC(&cfg, (const void*)&append_one_kernel, kargs));
+    return HQMQ_OK;
+  }
   // one launch for the whole append; the two status words (first word of each tensor's part) are cleared ahead of it
   HQMQ_CHECK_CUDA(cudaMemset2DAsync(wsb, wk, 0, sizeof(uint32_t), 2, st));
   append_pair_kernel<<<dim3(dk.H, 2), small_threads((int64_t)dk.B * k->T_new * dk.n_chunks), 0, st>>>(pr);

@@ -196,3 +196,32 @@ def test_prompt_chunk_attends_causally_over_the_cache(T_prompt, T_chunk, window)
                                   window=window)
         err = (O[:, :, i:i + 1].cpu() - ref).abs().max().item()
         assert err < 2e-3, f"query {i}: max-abs {err:.2e}"
+
+
+@pytest.mark.parametrize("B,H,d,S,br,dtype", [(16, 2, 128, 24, 3, torch.float16), (9, 3, 128, 192, 6, torch.bfloat16),
+                                              (5, 9, 64, 96, 4, torch.bfloat16), (100, 1, 16, 24, 3, torch.float32),
+                                              (1, 8, 64, 96, 4, torch.bfloat16), (32, 2, 64, 24, 3, torch.bfloat16)])
+@pytest.mark.parametrize("outliers", [True, False])
+def test_one_token_appends_equal_single_tensor_calls(B, H, d, S, br, dtype, outliers):
+    """The one-token append of K and V (its own kernel: up to 512 chunks per head, more than eight heads without a cluster,
+    rows with padding bits, block boundaries with records) leaves the planes that two single-tensor calls leave."""
+    inner = hqmq.HQMQ(1, H, S, br, device="cuda")
+    q = hqmq.with_outlier_extraction(inner, 3.0) if outliers else inner
+    mk = lambda kv: inner.new_cache(B, 64, d, "cuda", scale_dtype=dtype, with_outliers=outliers, out_dtype=dtype,
+                                    ofrag=outliers and kv == 0, out_cap=40)
+    pair, single = (mk(0), mk(1)), (mk(0), mk(1))
+    g = torch.Generator().manual_seed(12)
+    for step in range(35):
+        k, v = torch.randn(B, H, 1, d, generator=g), torch.randn(B, H, 1, d, generator=g)
+        k[..., 5] *= 12.0
+        v *= torch.where(torch.rand(v.shape, generator=g) < 0.02, 30.0, 1.0)
+        k, v = k.to(dtype).cuda(), v.to(dtype).cuda()
+        q.encode_pair(k, v, 0, pair[0], pair[1])
+        q.encode(k, 0, 0, out=single[0])
+        q.encode(v, 0, 1, out=single[1])
+    for a, b in zip(pair, single):
+        assert a.T == b.T == 35
+        names = ["codes", "rs"] + (["flags", "out_vals", "out_off", "out_count"] if outliers else [])
+        names += ["ofrag", "ofrag_off"] if a.with_ofrag else []
+        for name in names:
+            assert torch.equal(getattr(a, name), getattr(b, name)), name
