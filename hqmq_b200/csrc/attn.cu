@@ -25,7 +25,27 @@ constexpr int kFastQPad = 8;     // must equal kQPad of the staged kernels
 
 template <int N, bool OUTL, bool WIDE>
 __global__ void __launch_bounds__(kSlowWarps * 32) attn_slow_kernel(const AttnParams p) {
-  attn_decode_body<N, SlowLoader<N>, kSlowWarps, OUTL, WIDE>(p);
+  attn_decode_body<N, SlowLoader<N>, kSlowWarps, OUTL, WIDE, false>(p);
+}
+
+// The reference tuple at its usual types (int32 indices and radius codes): bound by HBM -- 8 bytes per chunk, 16-byte loads of
+// the next tile in flight while a tile is computed, eight warps of up to 255 registers.  One sequence of 16384 tokens, 8
+// heads (67 MB): 193 us through the generic loader, whose fields are loaded one by one, with 72 partials per row to merge.
+// Other integer types and unaligned rows keep the field-by-field loads; the work is split and summed the same way, so that a
+// result does not depend on the types the codes come in.
+constexpr int kRefWarps = 8;
+template <int N, bool VEC>
+__global__ void __launch_bounds__(kRefWarps * 32, 1) attn_ref_kernel(const AttnParams p) {
+  attn_decode_body<N, typename std::conditional<VEC, RefLoader<N>, SlowLoader<N>>::type, kRefWarps, false, false, true>(p);
+}
+template <int N>
+static const void* ref_kernel(bool vec) { return vec ? (const void*)&attn_ref_kernel<N, true> : (const void*)&attn_ref_kernel<N, false>; }
+// Whether a tuple's rows can be loaded 16 bytes at a time (8 of V at d_head 64).
+static bool ref_vec(const hqmq_ref_packed& r) {
+  if (r.idx_dtype != HQMQ_I32 || r.rq_dtype != HQMQ_I32 || (((uintptr_t)r.idx | (uintptr_t)r.rq) & 15)) return false;
+  for (int i = 0; i < 3; ++i)
+    if (r.idx_stride[i] % 4 || r.rq_stride[i] % 4) return false;
+  return true;
 }
 
 template <int N>
@@ -223,6 +243,39 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
   } else {
     pl.ib = 16;
     pl.table_rows = a->K_size;
+    if (G <= 8 && (n == 32 || n == 16) && a->kv_splits == 0 &&
+        (((uintptr_t)a->joint_K | (uintptr_t)a->joint_V) & (a->joint_dtype == HQMQ_F32 ? 15 : 7)) == 0) {
+      const size_t tbl = (size_t)pl.table_rows * 16, merge = (size_t)kRefWarps * 8 * (a->d + 2) * 4;
+      if (tbl + merge <= kSmemLimit - 1024) {
+        const bool vec = ref_vec(a->K_ref) && ref_vec(a->V_ref);
+        pl.kernel = n == 32 ? ref_kernel<32>(vec) : ref_kernel<16>(vec);
+        pl.nw = kRefWarps; pl.threads = kRefWarps * 32; pl.ppc = 1; pl.ring_stages = pl.merge_slots = pl.repv_log2 = 0;
+        pl.cluster = pl.warp_units = 0;
+        const int keys = a->window > 0 ? std::min(a->window, a->T_kv) : a->T_kv;
+        const int tpu = std::max(1, (keys + kTile - 1) / kTile + (a->window > 0 ? 1 : 0));
+        pl.units = a->B * a->T_q * a->H_kv;
+        // equal pieces, a unit cut into as many as the SMs allow when there are fewer units than SMs (no CTA then straddles
+        // two units); at least half a tile per warp
+        int64_t L;
+        if (pl.units < 148) {
+          const int c = std::min(148 / pl.units, std::max(1, tpu / (kRefWarps / 2)));
+          L = (tpu + c - 1) / c;
+          pl.tpu_v = (int)L * ((tpu + (int)L - 1) / (int)L);
+        } else {
+          pl.tpu_v = tpu;
+          L = std::max<int64_t>(((int64_t)pl.units * tpu + 147) / 148, kRefWarps);
+        }
+        pl.L = (int)L;
+        pl.grid = (int)(((int64_t)pl.units * pl.tpu_v + L - 1) / L);
+        pl.P = (pl.tpu_v - 1 + pl.L - 1) / pl.L + 1;
+        // replicas of the tables against bank conflicts where a CTA has the tiles to pay for storing them
+        while (pl.rep_log2 < 2 && pl.L >= (16 << pl.rep_log2) && (tbl << (pl.rep_log2 + 1)) + merge <= kSmemLimit - 1024) ++pl.rep_log2;
+        pl.smem = (tbl << pl.rep_log2) + merge;
+        pl.ticket_bytes = (((size_t)pl.units * 4 + 15) & ~(size_t)15);
+        pl.ws_bytes = 16 + pl.ticket_bytes + (size_t)pl.units * pl.P * 8 * (a->d + 2) * sizeof(float);
+        return HQMQ_OK;
+      }
+    }
   }
   const bool fast = pl.kernel != nullptr;
   pl.ppc = fast ? 1 : kSlowWarps;
@@ -447,7 +500,7 @@ extern "C" int hqmq_attn_decode(const hqmq_attn_args* a, void* workspace, size_t
   p.partials = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(workspace) + 16 + pl.ticket_bytes);
   p.O = a->O; p.o_dtype = a->o_dtype; p.os_b = a->o_stride[0]; p.os_h = a->o_stride[1]; p.os_t = a->o_stride[2];
   p.merged = a->partials_only ? a->partials : nullptr;
-  const bool fused_merge = pl.ring_stages > 0;   // the ring kernels merge a unit's partials themselves (last CTA of the unit)
+  const bool fused_merge = pl.ticket_bytes > 0;   // the ring and tuple kernels merge a unit's partials themselves (last CTA of the unit)
   if (fused_merge) HQMQ_CHECK_CUDA(cudaMemsetAsync(p.tickets, 0, pl.ticket_bytes, st));
   p.layout = a->layout;
   p.table_rows = pl.table_rows;
@@ -459,8 +512,8 @@ extern "C" int hqmq_attn_decode(const hqmq_attn_args* a, void* workspace, size_t
   }
   // (the kernel's dynamic shared-memory limit was raised when the plan asked for its occupancy: resident_ctas)
   void* kargs[] = {&p};
+  if (pl.cluster || pl.smem > 48 * 1024) HQMQ_CHECK_CUDA(raise_smem_limit(pl.kernel, pl.smem));
   if (pl.cluster) {
-    HQMQ_CHECK_CUDA(raise_smem_limit(pl.kernel, pl.smem));
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = pl.cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;

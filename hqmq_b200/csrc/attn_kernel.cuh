@@ -363,6 +363,69 @@ struct SlowLoader {
   __device__ __forceinline__ float vscale(const Raw& raw, int nt) const { return raw.rsv[nt]; }
 };
 
+// The reference tuple with int32 indices and radius codes on 16-byte aligned rows: one 16-byte load per four chunks, sixteen
+// in flight per lane and tile, kept as loaded until the tile is computed.
+template <int N>
+struct RefLoader {
+  static constexpr int NKS = Geo<N>::NKS, NVG = Geo<N>::NVG;
+  struct Raw { int ki[2][NKS], kr[2][NKS], vi[4][NVG], vr[4][NVG]; float rsk[2], rsv[2]; };
+  const int* ki; const int* kr; const int* vi; const int* vr;     // this lane's chunks of token 0
+  const void* krs; const void* vrs;
+  int64_t ki_t, kr_t, vi_t, vr_t, krs_o, vrs_o;
+  int rows, j, r, kdt, vdt;
+  __device__ __forceinline__ void init(const AttnParams& p, int b, int h, int lane) {
+    j = lane & 3; r = lane >> 2; rows = p.table_rows - 1;
+    auto at = [&](const void* base, const int64_t* st) { return reinterpret_cast<const int*>(base) + b * st[0] + h * st[1]; };
+    ki = at(p.Kr.idx, p.Kr.idx_stride) + j * NKS; kr = at(p.Kr.rq, p.Kr.rq_stride) + j * NKS;
+    vi = at(p.Vr.idx, p.Vr.idx_stride) + r * NVG; vr = at(p.Vr.rq, p.Vr.rq_stride) + r * NVG;
+    ki_t = p.Kr.idx_stride[2]; kr_t = p.Kr.rq_stride[2]; vi_t = p.Vr.idx_stride[2]; vr_t = p.Vr.rq_stride[2];
+    krs = p.Kr.rs; vrs = p.Vr.rs; kdt = p.Kr.rs_dtype; vdt = p.Vr.rs_dtype;
+    krs_o = b * p.Kr.rs_stride[0] + h * p.Kr.rs_stride[1]; vrs_o = b * p.Vr.rs_stride[0] + h * p.Vr.rs_stride[1];
+  }
+  template <int C>
+  static __device__ __forceinline__ void take(int* dst, const int* src, bool ok) {
+    if constexpr (C % 4 == 0) {
+#pragma unroll
+      for (int i = 0; i < C; i += 4) {
+        const int4 v = ok ? __ldcs(reinterpret_cast<const int4*>(src + i)) : make_int4(0, 0, 0, 0);
+        dst[i] = v.x; dst[i + 1] = v.y; dst[i + 2] = v.z; dst[i + 3] = v.w;
+      }
+    } else {
+      const int2 v = ok ? __ldcs(reinterpret_cast<const int2*>(src)) : make_int2(0, 0);
+      dst[0] = v.x; dst[1] = v.y;
+    }
+  }
+  __device__ __forceinline__ void fetch(Raw& raw, int tile, int t_end) const {
+    const int t0 = tile * kTile;
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+      const int t = t0 + nt * 8 + r;
+      take<NKS>(raw.ki[nt], ki + t * ki_t, t < t_end);
+      take<NKS>(raw.kr[nt], kr + t * kr_t, t < t_end);
+      raw.rsk[nt] = t < t_end ? load_float(krs, krs_o + t, kdt) : 0.f;
+      raw.rsv[nt] = t < t_end ? load_float(vrs, vrs_o + t, vdt) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = t0 + 2 * j + (i & 1) + (i >> 1) * 8;
+      take<NVG>(raw.vi[i], vi + t * vi_t, t < t_end);
+      take<NVG>(raw.vr[i], vr + t * vr_t, t < t_end);
+    }
+  }
+  __device__ __forceinline__ void split(int i, int q, uint32_t& idx, __half2& rr) const {
+    idx = (uint32_t)__vimin_s32_relu(i, rows);             // clamped to [0, rows - 1] and [0, 1023]
+    rr = radius_half2((uint32_t)__vimin_s32_relu(q, 1023));
+  }
+  template <int NT, int KS> __device__ __forceinline__ void kfield(const Raw& raw, uint32_t& idx, __half2& rr) const {
+    split(raw.ki[NT][KS], raw.kr[NT][KS], idx, rr);
+  }
+  template <int I, int GG> __device__ __forceinline__ void vfield(const Raw& raw, uint32_t& idx, __half2& rr) const {
+    split(raw.vi[I][GG], raw.vr[I][GG], idx, rr);
+  }
+  __device__ __forceinline__ float kscale(const Raw& raw, int nt) const { return raw.rsk[nt]; }
+  __device__ __forceinline__ float vscale(const Raw& raw, int nt) const { return raw.rsv[nt]; }
+};
+
 // Two packed 16-bit floats (fp16 or bf16) to fp32 with one uniform branch.
 __device__ __forceinline__ float2 pair16_to_float2(uint32_t v, int dtype) {
   if (dtype == HQMQ_BF16) return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
@@ -437,9 +500,22 @@ __device__ __forceinline__ void static_for(F&& f) {
   }
 }
 
-// Loader: FastLoader<N, IB, RB> or SlowLoader<N>.  NW: warps per CTA.  OUTL: merge Med3x outliers.
-// WIDE: 8 < G <= 16.
-template <int N, class Loader, int NW, bool OUTL, bool WIDE>
+// Four elements of a joint-table row as fp16.
+__device__ __forceinline__ uint2 joint_entry(const void* j, int64_t base, int dtype) {
+  if (dtype == HQMQ_F16) return *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(j) + base);
+  float4 f;
+  if (dtype == HQMQ_F32) f = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(j) + base);
+  else {
+    const uint2 v = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(j) + base);
+    f = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+  }
+  return make_uint2(pack_half2(f.x, f.y), pack_half2(f.z, f.w));
+}
+
+// Loader: FastLoader<N, IB, RB>, RefLoader<N> or SlowLoader<N>.  NW: warps per CTA.  OUTL: merge Med3x outliers.
+// WIDE: 8 < G <= 16.  TICKET: one partial per CTA and unit (the warps' are merged in shared memory), and the last CTA of a
+// unit merges them (a ticket per unit counts arrivals, nobody waits): no merge launch.
+template <int N, class Loader, int NW, bool OUTL, bool WIDE, bool TICKET>
 __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
   using G_ = Geo<N>;
   constexpr int NKS = G_::NKS, NVG = G_::NVG, NOT = 2 * G_::NVG;   // NOT: 16-row tiles of O^T
@@ -470,7 +546,18 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
     const int b = bt / p.Tq, tq = bt - b * p.Tq;
     // ---- codeword tables of this KV head into shared memory (fp16 x 4 per entry, replicated) ---------
     if (h != cur_h || OUTL) __syncthreads();
-    if (h != cur_h) {
+    if (TICKET && h != cur_h) {
+      // (the joint tables of the reference tuple, rows on 8- or 16-byte boundaries; replicas by consecutive lanes)
+      const int total = p.table_rows << p.rep_log2;
+#pragma unroll 4
+      for (int i = threadIdx.x; i < total; i += NW * 32) {
+        const int64_t base = ((int64_t)h * p.table_rows + (i >> p.rep_log2)) * 4;
+        reinterpret_cast<uint2*>(tblK)[i] = joint_entry(p.jK, base, p.j_dtype);
+        reinterpret_cast<uint2*>(tblV)[i] = joint_entry(p.jV, base, p.j_dtype);
+      }
+      cur_h = h;
+    }
+    if (!TICKET && h != cur_h) {
       const int reps = 1 << p.rep_log2;
       for (int i = threadIdx.x; i < p.table_rows; i += NW * 32) {
         uint2 ek, ev;
@@ -802,6 +889,79 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
         compute(rawB, oB, tile);
         tile += NW;
       }
+    }
+
+    if constexpr (TICKET) {
+      constexpr int PD = 4 * N + 2;
+      float* mp = reinterpret_cast<float*>(smem_raw + 2 * tbl_bytes);        // [NW][8][PD]
+      float* mine = mp + warp * 8 * PD;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float l = l_run[0][e];
+        l += __shfl_xor_sync(0xffffffffu, l, 4);
+        l += __shfl_xor_sync(0xffffffffu, l, 8);
+        l += __shfl_xor_sync(0xffffffffu, l, 16);
+        float* dst = mine + (2 * j + e) * PD;
+#pragma unroll
+        for (int i = 0; i < NOT; ++i) {
+          const int chunk = r * NVG + (i >> 1);
+          dst[4 * chunk + 2 * (i & 1)] = o[0][i][e];
+          dst[4 * chunk + 2 * (i & 1) + 1] = o[0][i][2 + e];
+        }
+        if (r == 0) { dst[4 * N] = m_run[0][e]; dst[4 * N + 1] = l; }
+      }
+      __syncthreads();
+      const int c0 = (int)(ubase / p.L), n_ctas = (int)((ubase + p.tpu_v - 1) / p.L) - c0 + 1, slot = (int)blockIdx.x - c0;
+      auto emit = [&](int g, int x, float v, float m_star, float l_star) {
+        const int64_t row = ((int64_t)b * p.Hq + h * p.G + g) * p.Tq + tq;
+        if (p.merged) {
+          p.merged[row * PD + x] = v;
+          if (x == 0) { p.merged[row * PD + 4 * N] = m_star; p.merged[row * PD + 4 * N + 1] = l_star; }
+        } else {
+          store_float(p.O, (int64_t)b * p.os_b + (int64_t)(h * p.G + g) * p.os_h + (int64_t)tq * p.os_t + x,
+                      l_star > 0.f ? v / l_star : 0.f, p.o_dtype);
+        }
+      };
+      // element (g, x) of [G][4 N] from `parts` partials, `stride` floats apart
+      auto merge = [&](const float* col, int x, int parts, int64_t stride, auto load, float& v, float& m_star, float& l_star) {
+        m_star = -INFINITY;
+        for (int w = 0; w < parts; ++w) m_star = fmaxf(m_star, load(col + w * stride + 4 * N));
+        const float m_use = m_star == -INFINITY ? 0.f : m_star;
+        v = l_star = 0.f;
+#pragma unroll 4
+        for (int w = 0; w < parts; ++w) {
+          const float wgt = fast_exp2(load(col + w * stride + 4 * N) - m_use);
+          v = fmaf(load(col + w * stride + x), wgt, v);
+          l_star = fmaf(load(col + w * stride + 4 * N + 1), wgt, l_star);
+        }
+      };
+      for (int i = threadIdx.x; i < p.G * 4 * N; i += NW * 32) {
+        const int g = i / (4 * N), x = i - g * (4 * N);
+        float v, m_star, l_star;
+        merge(mp + g * PD, x, NW, 8 * PD, [](const float* q) { return *q; }, v, m_star, l_star);
+        if (n_ctas == 1) { emit(g, x, v, m_star, l_star); continue; }
+        float* dst = p.partials + (((int64_t)u * p.P + slot) * 8 + g) * PD;
+        dst[x] = v;
+        if (x == 0) { dst[4 * N] = m_star; dst[4 * N + 1] = l_star; }
+      }
+      if (n_ctas > 1) {
+        __shared__ uint32_t s_last;
+        __threadfence();                      // this CTA's partial is visible device-wide before its ticket is drawn
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = atomicAdd(&p.tickets[u], 1u) == (uint32_t)(n_ctas - 1) ? 1u : 0u;
+        __syncthreads();
+        if (s_last) {
+          __threadfence();
+          for (int i = threadIdx.x; i < p.G * 4 * N; i += NW * 32) {
+            const int g = i / (4 * N), x = i - g * (4 * N);
+            float v, m_star, l_star;
+            merge(p.partials + ((int64_t)u * p.P * 8 + g) * PD, x, n_ctas, 8 * PD, [](const float* q) { return __ldcg(q); }, v, m_star, l_star);
+            emit(g, x, v, m_star, l_star);
+          }
+        }
+      }
+      __syncthreads();                        // the merge is done with its shared memory
+      continue;
     }
 
     // ---- per-warp partial: o[d], m, l for every query head of this KV head -----------------------------

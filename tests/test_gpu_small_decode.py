@@ -44,3 +44,32 @@ def test_small_decode(B, Hq, Hkv, d, T, Tq, window, S, br, outliers):
     parts = torch.full((1, B, Hq, Tq, d + 2), float("nan"), device="cuda")
     hqmq.fused_attention_packed(Q, Kp, Vp, tk, tv, causal=causal, window=window, partials=parts[0])
     _check(hqmq.combine_partials(parts), want)
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,d,T,Tq,window", [
+    (1, 1, 1, 128, 1, 1, None),            # one key
+    (1, 28, 4, 128, 3001, 1, None),        # units cut into many CTAs, the last with fewer tiles
+    (2, 16, 2, 64, 517, 3, None),
+    (40, 8, 4, 64, 75, 1, None),           # more units than SMs: CTAs that hold several
+    (1, 8, 2, 128, 900, 1, 333),
+])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+def test_tuple_decode(B, Hq, Hkv, d, T, Tq, window, dtype):
+    """The packed tuple at its usual types, and with 64-bit indices and strided planes (loaded field by field)."""
+    from hqmq_b200 import kernels
+    q = hqmq.HQMQ(1, Hkv, 192, 6, device="cuda")
+    args, dense = [], []
+    for kv in (0, 1):
+        x = make_kv("randn", (B, Hkv, T, d), seed=74 + kv, dtype=torch.bfloat16).cuda()
+        idx, rq, rs, _ = q.encode(x, 0, kv).to_reference()
+        args += [idx, rq, rs.to(dtype), q.tables(0, kv, "cuda")["joint"].to(dtype)]
+        dense.append(kernels.decode_dequant(idx, rq, args[-2].float(), args[-1].float(), 63))
+    Q = (torch.randn(B, Hq, Tq, d, generator=torch.Generator().manual_seed(76)) / math.sqrt(d)).to(dtype).cuda()
+    want = _dense_attention(Q, *dense, False, window)
+    O, O2 = torch.empty(Q.shape, dtype=torch.float32, device="cuda"), torch.empty(Q.shape, dtype=torch.float32, device="cuda")
+    for _ in range(2):
+        hqmq.fused_attention(Q, *args, 63, causal=False, window=window, out=O.fill_(7))
+        _check(O, want)
+    args[0], args[5] = args[0].long(), args[5].transpose(1, 2).contiguous().transpose(1, 2)
+    hqmq.fused_attention(Q, *args, 63, causal=False, window=window, out=O2)
+    assert torch.equal(O, O2)
