@@ -245,7 +245,7 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
     pl.table_rows = a->K_size;
     if (G <= 8 && (n == 32 || n == 16) && a->kv_splits == 0 &&
         (((uintptr_t)a->joint_K | (uintptr_t)a->joint_V) & (a->joint_dtype == HQMQ_F32 ? 15 : 7)) == 0) {
-      const size_t tbl = (size_t)pl.table_rows * 16, merge = (size_t)kRefWarps * 8 * (a->d + 2) * 4;
+      const size_t tbl = (size_t)pl.table_rows * 16, merge = (size_t)kRefWarps * 8 * (a->d + 2) * 4 + (8 * 160 + 16) * 4;   // (+ weights of up to 160 CTAs)
       if (tbl + merge <= kSmemLimit - 1024) {
         const bool vec = ref_vec(a->K_ref) && ref_vec(a->V_ref);
         pl.kernel = n == 32 ? ref_kernel<32>(vec) : ref_kernel<16>(vec);
@@ -268,9 +268,7 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
         pl.L = (int)L;
         pl.grid = (int)(((int64_t)pl.units * pl.tpu_v + L - 1) / L);
         pl.P = (pl.tpu_v - 1 + pl.L - 1) / pl.L + 1;
-        // replicas of the tables against bank conflicts where a CTA has the tiles to pay for storing them
-        while (pl.rep_log2 < 2 && pl.L >= (16 << pl.rep_log2) && (tbl << (pl.rep_log2 + 1)) + merge <= kSmemLimit - 1024) ++pl.rep_log2;
-        pl.smem = (tbl << pl.rep_log2) + merge;
+        pl.smem = tbl + merge;
         pl.ticket_bytes = (((size_t)pl.units * 4 + 15) & ~(size_t)15);
         pl.ws_bytes = 16 + pl.ticket_bytes + (size_t)pl.units * pl.P * 8 * (a->d + 2) * sizeof(float);
         return HQMQ_OK;

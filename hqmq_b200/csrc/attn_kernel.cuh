@@ -85,6 +85,26 @@ __host__ __device__ inline void key_range(int Tkv, int Tq, int causal, int windo
   beg = window > 0 ? (end - window > 0 ? end - window : 0) : 0;
 }
 
+constexpr uint32_t kWaitLimit = 1u << 24;
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+
 __device__ __forceinline__ void mma16816(float c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
   asm volatile(
@@ -368,7 +388,7 @@ struct SlowLoader {
 template <int N>
 struct RefLoader {
   static constexpr int NKS = Geo<N>::NKS, NVG = Geo<N>::NVG;
-  struct Raw { int ki[2][NKS], kr[2][NKS], vi[4][NVG], vr[4][NVG]; float rsk[2], rsv[2]; };
+  struct Raw { int ki[2][NKS], kr[2][NKS], vi[4][NVG], vr[4][NVG]; uint32_t rsk[2], rsv[2]; };
   const int* ki; const int* kr; const int* vi; const int* vr;     // this lane's chunks of token 0
   const void* krs; const void* vrs;
   int64_t ki_t, kr_t, vi_t, vr_t, krs_o, vrs_o;
@@ -395,6 +415,13 @@ struct RefLoader {
       dst[0] = v.x; dst[1] = v.y;
     }
   }
+  // (converted when the tile is computed: a conversion here would wait for the load)
+  static __device__ __forceinline__ uint32_t scale_bits(const void* p, int64_t i, int dt) {
+    return dt == HQMQ_F32 ? reinterpret_cast<const uint32_t*>(p)[i] : (uint32_t)reinterpret_cast<const uint16_t*>(p)[i];
+  }
+  static __device__ __forceinline__ float scale_of(uint32_t bits, int dt) {
+    return dt == HQMQ_F32 ? __uint_as_float(bits) : bits16_to_float((uint16_t)bits, dt);
+  }
   __device__ __forceinline__ void fetch(Raw& raw, int tile, int t_end) const {
     const int t0 = tile * kTile;
 #pragma unroll
@@ -402,8 +429,8 @@ struct RefLoader {
       const int t = t0 + nt * 8 + r;
       take<NKS>(raw.ki[nt], ki + t * ki_t, t < t_end);
       take<NKS>(raw.kr[nt], kr + t * kr_t, t < t_end);
-      raw.rsk[nt] = t < t_end ? load_float(krs, krs_o + t, kdt) : 0.f;
-      raw.rsv[nt] = t < t_end ? load_float(vrs, vrs_o + t, vdt) : 0.f;
+      raw.rsk[nt] = t < t_end ? scale_bits(krs, krs_o + t, kdt) : 0u;
+      raw.rsv[nt] = t < t_end ? scale_bits(vrs, vrs_o + t, vdt) : 0u;
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -422,8 +449,8 @@ struct RefLoader {
   template <int I, int GG> __device__ __forceinline__ void vfield(const Raw& raw, uint32_t& idx, __half2& rr) const {
     split(raw.vi[I][GG], raw.vr[I][GG], idx, rr);
   }
-  __device__ __forceinline__ float kscale(const Raw& raw, int nt) const { return raw.rsk[nt]; }
-  __device__ __forceinline__ float vscale(const Raw& raw, int nt) const { return raw.rsv[nt]; }
+  __device__ __forceinline__ float kscale(const Raw& raw, int nt) const { return scale_of(raw.rsk[nt], kdt); }
+  __device__ __forceinline__ float vscale(const Raw& raw, int nt) const { return scale_of(raw.rsv[nt], vdt); }
 };
 
 // Two packed 16-bit floats (fp16 or bf16) to fp32 with one uniform branch.
@@ -512,6 +539,54 @@ __device__ __forceinline__ uint2 joint_entry(const void* j, int64_t base, int dt
   return make_uint2(pack_half2(f.x, f.y), pack_half2(f.z, f.w));
 }
 
+// Merge of the n partials (o[D], m, l) of a unit by all `threads` threads (whole warps, at least 8) of a CTA: head g's partial c
+// starts at base + g * gs + c * cs (past the L1: other CTAs wrote them).  A warp per head turns the (m, l) pairs into weights
+// first, then every thread sums pairs of elements with eight loads in flight.  (Each thread walking all partials for itself,
+// headers included, was one chain of L2 latencies: 10 us for 18 partials.)  w_s: 8 * n floats, ms_s: 16 floats of shared memory.
+template <int D, class Bar, class Emit>
+__device__ __forceinline__ void merge_partials(int tid, int threads, int G, int n, const float* base, int64_t gs, int64_t cs,
+                                               float* w_s, float* ms_s, Bar bar, Emit emit) {
+  const int warp = tid >> 5, lane = tid & 31;
+  if (warp < G) {
+    const float* hd = base + warp * gs + D;
+    float m = -INFINITY;
+    for (int c = lane; c < n; c += 32) m = fmaxf(m, __ldcg(hd + c * cs));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float mu = m == -INFINITY ? 0.f : m;
+    float l = 0.f;
+    for (int c = lane; c < n; c += 32) {
+      const float w = fast_exp2(__ldcg(hd + c * cs) - mu);
+      w_s[warp * n + c] = w;
+      l = fmaf(__ldcg(hd + c * cs + 1), w, l);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    if (lane == 0) { ms_s[warp] = m; ms_s[8 + warp] = l; }
+  }
+  bar();
+  for (int i = tid; i < G * (D / 2); i += threads) {
+    const int g = i / (D / 2), x = 2 * (i - g * (D / 2));
+    const float* col = base + g * gs + x;
+    const float* w = w_s + g * n;
+    float2 acc = make_float2(0.f, 0.f);
+    int c = 0;
+    for (; c + 8 <= n; c += 8) {
+      float2 v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = __ldcg(reinterpret_cast<const float2*>(col + (c + k) * cs));
+#pragma unroll
+      for (int k = 0; k < 8; ++k) { acc.x = fmaf(v[k].x, w[c + k], acc.x); acc.y = fmaf(v[k].y, w[c + k], acc.y); }
+    }
+    for (; c < n; ++c) {
+      const float2 v = __ldcg(reinterpret_cast<const float2*>(col + c * cs));
+      acc.x = fmaf(v.x, w[c], acc.x); acc.y = fmaf(v.y, w[c], acc.y);
+    }
+    emit(g, x, acc.x, ms_s[g], ms_s[8 + g]);
+    emit(g, x + 1, acc.y, ms_s[g], ms_s[8 + g]);
+  }
+}
+
 // Loader: FastLoader<N, IB, RB>, RefLoader<N> or SlowLoader<N>.  NW: warps per CTA.  OUTL: merge Med3x outliers.
 // WIDE: 8 < G <= 16.  TICKET: one partial per CTA and unit (the warps' are merged in shared memory), and the last CTA of a
 // unit merges them (a ticket per unit counts arrivals, nobody waits): no merge launch.
@@ -540,20 +615,40 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
   const int64_t flat_hi = flat_lo + p.L < flat_total ? flat_lo + p.L : flat_total;
   const int upb = p.B * p.Tq;   // units per KV head
   int cur_h = -1;
+  __shared__ __align__(8) uint64_t s_tbar;
+  uint32_t tbl_phase = 0u;
+  bool gave_up = false;
+  if (TICKET && threadIdx.x == 0) {
+    mbar_init(smem_u32(&s_tbar), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
 
   for (int u = (int)(flat_lo / p.tpu_v); (int64_t)u * p.tpu_v < flat_hi; ++u) {
     const int h = u / upb, bt = u - h * upb;
     const int b = bt / p.Tq, tq = bt - b * p.Tq;
     // ---- codeword tables of this KV head into shared memory (fp16 x 4 per entry, replicated) ---------
     if (h != cur_h || OUTL) __syncthreads();
+    bool tables_due = false;                // fp16 tables on their way by bulk copy
     if (TICKET && h != cur_h) {
-      // (the joint tables of the reference tuple, rows on 8- or 16-byte boundaries; replicas by consecutive lanes)
-      const int total = p.table_rows << p.rep_log2;
-#pragma unroll 4
-      for (int i = threadIdx.x; i < total; i += NW * 32) {
-        const int64_t base = ((int64_t)h * p.table_rows + (i >> p.rep_log2)) * 4;
-        reinterpret_cast<uint2*>(tblK)[i] = joint_entry(p.jK, base, p.j_dtype);
-        reinterpret_cast<uint2*>(tblV)[i] = joint_entry(p.jV, base, p.j_dtype);
+      // the joint tables of the reference tuple, rows on 8- or 16-byte boundaries, not replicated (a CTA has a few tiles per
+      // warp; at two replicas storing them took as long as the tiles: 45 against 38 us for 16384 tokens)
+      const int64_t row0 = (int64_t)h * p.table_rows;
+      if (p.j_dtype == HQMQ_F16 && (p.table_rows & 1) == 0 && (((uintptr_t)p.jK | (uintptr_t)p.jV) & 15) == 0) {
+        tables_due = true;
+        if (threadIdx.x == 0) {
+          const uint32_t bytes = (uint32_t)p.table_rows * 8u, bar = smem_u32(&s_tbar);
+          // (the generic-proxy reads and writes of the last unit's tables are done: the barrier above)
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          mbar_expect_tx(bar, 2 * bytes);
+          bulk_g2s(smem_u32(tblK), reinterpret_cast<const uint16_t*>(p.jK) + row0 * 4, bytes, bar);
+          bulk_g2s(smem_u32(tblV), reinterpret_cast<const uint16_t*>(p.jV) + row0 * 4, bytes, bar);
+        }
+      } else {
+#pragma unroll 8
+        for (int i = threadIdx.x; i < p.table_rows; i += NW * 32) {
+          reinterpret_cast<uint2*>(tblK)[i] = joint_entry(p.jK, (row0 + i) * 4, p.j_dtype);
+          reinterpret_cast<uint2*>(tblV)[i] = joint_entry(p.jV, (row0 + i) * 4, p.j_dtype);
+        }
       }
       cur_h = h;
     }
@@ -880,6 +975,13 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
         if constexpr (OUTL) fetch_off(tile, offk_nn, offk_nn1, offv_nn, offv_nn1);
         fetch(rawA, oA, tile);
       }
+      if (TICKET && tables_due) {
+        for (uint32_t spins = 0; !mbar_try_wait(smem_u32(&s_tbar), tbl_phase);)
+          if (++spins > kWaitLimit) { gave_up = true; break; }
+        tbl_phase ^= 1u;
+        if (gave_up) { *p.status = p.epoch; tile = my_hi; }      // (a lane that gives up takes its warp along)
+        if (__any_sync(0xffffffffu, gave_up)) { gave_up = true; tile = my_hi; }
+      }
       while (tile < my_hi) {
         if (tile + NW < my_hi) fetch(rawB, oB, tile + NW);
         compute(rawA, oA, tile);
@@ -910,7 +1012,6 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
         }
         if (r == 0) { dst[4 * N] = m_run[0][e]; dst[4 * N + 1] = l; }
       }
-      __syncthreads();
       const int c0 = (int)(ubase / p.L), n_ctas = (int)((ubase + p.tpu_v - 1) / p.L) - c0 + 1, slot = (int)blockIdx.x - c0;
       auto emit = [&](int g, int x, float v, float m_star, float l_star) {
         const int64_t row = ((int64_t)b * p.Hq + h * p.G + g) * p.Tq + tq;
@@ -919,26 +1020,25 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
           if (x == 0) { p.merged[row * PD + 4 * N] = m_star; p.merged[row * PD + 4 * N + 1] = l_star; }
         } else {
           store_float(p.O, (int64_t)b * p.os_b + (int64_t)(h * p.G + g) * p.os_h + (int64_t)tq * p.os_t + x,
-                      l_star > 0.f ? v / l_star : 0.f, p.o_dtype);
+                      l_star > 0.f || l_star != l_star ? v / l_star : 0.f, p.o_dtype);
         }
       };
-      // element (g, x) of [G][4 N] from `parts` partials, `stride` floats apart
-      auto merge = [&](const float* col, int x, int parts, int64_t stride, auto load, float& v, float& m_star, float& l_star) {
-        m_star = -INFINITY;
-        for (int w = 0; w < parts; ++w) m_star = fmaxf(m_star, load(col + w * stride + 4 * N));
-        const float m_use = m_star == -INFINITY ? 0.f : m_star;
-        v = l_star = 0.f;
-#pragma unroll 4
-        for (int w = 0; w < parts; ++w) {
-          const float wgt = fast_exp2(load(col + w * stride + 4 * N) - m_use);
-          v = fmaf(load(col + w * stride + x), wgt, v);
-          l_star = fmaf(load(col + w * stride + 4 * N + 1), wgt, l_star);
-        }
-      };
+      const bool failed = __syncthreads_or(gave_up ? 1 : 0) != 0;
+      float* w_s = mp + NW * 8 * PD;              // [8][n_ctas], then m and l of the unit's heads
       for (int i = threadIdx.x; i < p.G * 4 * N; i += NW * 32) {
         const int g = i / (4 * N), x = i - g * (4 * N);
-        float v, m_star, l_star;
-        merge(mp + g * PD, x, NW, 8 * PD, [](const float* q) { return *q; }, v, m_star, l_star);
+        const float* col = mp + g * PD;
+        float m_star = -INFINITY, v = 0.f, l_star = 0.f;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) m_star = fmaxf(m_star, col[w * 8 * PD + 4 * N]);
+        const float m_use = m_star == -INFINITY ? 0.f : m_star;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+          const float wgt = fast_exp2(col[w * 8 * PD + 4 * N] - m_use);
+          v = fmaf(col[w * 8 * PD + x], wgt, v);
+          l_star = fmaf(col[w * 8 * PD + 4 * N + 1], wgt, l_star);
+        }
+        if (failed) v = l_star = NAN;
         if (n_ctas == 1) { emit(g, x, v, m_star, l_star); continue; }
         float* dst = p.partials + (((int64_t)u * p.P + slot) * 8 + g) * PD;
         dst[x] = v;
@@ -952,12 +1052,8 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
         __syncthreads();
         if (s_last) {
           __threadfence();
-          for (int i = threadIdx.x; i < p.G * 4 * N; i += NW * 32) {
-            const int g = i / (4 * N), x = i - g * (4 * N);
-            float v, m_star, l_star;
-            merge(p.partials + ((int64_t)u * p.P * 8 + g) * PD, x, n_ctas, 8 * PD, [](const float* q) { return __ldcg(q); }, v, m_star, l_star);
-            emit(g, x, v, m_star, l_star);
-          }
+          merge_partials<4 * N>(threadIdx.x, NW * 32, p.G, n_ctas, p.partials + (int64_t)u * p.P * 8 * PD, PD, 8 * PD, w_s,
+                                w_s + 8 * n_ctas, [] { __syncthreads(); }, emit);
         }
       }
       __syncthreads();                        // the merge is done with its shared memory

@@ -884,6 +884,11 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
         consumer_bar();
         if (*last_s) {
           __threadfence();
+          const int64_t row0 = ((int64_t)b * p.Hq + h * p.G) * p.Tq + tq, gstride = (int64_t)p.Tq * p.P * (D + 2);
+          const float* base = p.partials + row0 * p.P * (D + 2);
+          if (8 * n_ctas <= MS * 8 * D) {
+            merge_partials<D>(threadIdx.x, kRingConsumerThreads, p.G, n_ctas, base, gstride, D + 2, slots, ms_s, consumer_bar, emit);
+          } else {          // (more pieces than SMs: kv_splits)
 #pragma unroll
           for (int q = 0; q < PER; ++q) {
             const int i = threadIdx.x + q * kRingConsumerThreads;
@@ -904,6 +909,7 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
                 emit(g, x, v, m_star, l_star);
               }
             }
+          }
           }
         }
       }

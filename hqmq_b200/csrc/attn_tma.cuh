@@ -15,30 +15,10 @@ namespace attn {
 
 constexpr int kStages = 2;
 constexpr int kPay = 64;                 // outlier entries staged per tile and tensor (+2 alignment slack)
-constexpr uint32_t kWaitLimit = 1u << 24;
 // bytes of a stage that hold either the K payload slice or the tile's fragment records
 constexpr int kSideK = (kPay + 2) * 8 > HQMQ_OFRAG_MAX_PER_TILE * HQMQ_OFRAG_BYTES ? (kPay + 2) * 8
                                                                                   : HQMQ_OFRAG_MAX_PER_TILE * HQMQ_OFRAG_BYTES;
 constexpr int kQPad = 8;   // halves of padding per query row in shared memory (spreads the rows over banks)
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  return ok != 0;
-}
 
 // Shared-memory layout of one stage (all pieces 16-byte aligned).
 template <int N, int IB, int RB, bool OUTL>
