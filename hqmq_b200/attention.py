@@ -11,6 +11,7 @@ operation on the native bit-packed cache.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from typing import Optional
 
 import torch
@@ -29,6 +30,9 @@ def _fill_q(a: _lib.AttnArgs, Q: torch.Tensor, O: Optional[torch.Tensor]):
         a.o_dtype = _lib.dtype_enum(O.dtype)
         a.O = O.data_ptr()
         a.o_stride = (C.c_int64 * 3)(*O.stride()[:3])
+
+
+_calls = threading.local()        # per thread: argument structs of repeated fused_attention calls, by shape (bounded)
 
 
 def _run(a: _lib.AttnArgs, device):
@@ -57,6 +61,28 @@ def fused_hqmq_attention(
     """O (B, H_q, T_q, d) = softmax(scale * Q K^T + mask) V with K, V decoded on the fly from the
     reference's packed tuple.  Indices address ``joint_*`` directly (reference order)."""
     _lib.require_cuda(Q, "fused_attention")
+    # A repeated call shape only patches the addresses of a kept struct (nothing of a call is kept: no tensor, no workspace).
+    ts = (Q, K_idx, K_radius_q, K_radius_scale, joint_K, V_idx, V_radius_q, V_radius_scale, joint_V)
+    key = (tuple([(t.shape, t.stride(), t.dtype) for t in ts]), Q.device, r_qmax, causal, softmax_scale, window, kv_splits,
+           None if out is None else (out.shape, out.stride(), out.dtype))
+    known = _calls.__dict__.setdefault("by_shape", {})
+    hit = known.get(key)
+    if hit is not None:
+        a, ref, nbytes, align = hit
+        ptr = [t.data_ptr() for t in ts]
+        if out is None:
+            out = torch.empty_like(Q)
+        if _alignment(ptr, out) == align:           # (the plan depends on it)
+            a.Q, a.O = ptr[0], out.data_ptr()
+            K, V = a.K_ref, a.V_ref
+            K.idx, K.rq, K.rs, a.joint_K = ptr[1:5]
+            V.idx, V.rq, V.rs, a.joint_V = ptr[5:9]
+            with _lib.device_guard(Q.device):
+                ws = torch.empty(nbytes, dtype=torch.uint8, device=Q.device)
+                rc = _lib.lib().hqmq_attn_decode(ref, ws.data_ptr(), nbytes, _lib.stream_ptr())
+                if rc:
+                    _lib.check(rc, "hqmq_attn_decode")
+            return out
     _lib.check_device(Q.device)
     assert Q.dim() == 4 and K_idx.dim() == 4, "Q is (B,H_q,T_q,d); idx is (B,H_kv,T_kv,n_chunks)"
     B, H_q, T_q, d_h = Q.shape
@@ -81,8 +107,19 @@ def fused_hqmq_attention(
     a.V_ref = _lib.ref_packed(V_idx, V_radius_q, V_radius_scale)
     a.joint_dtype, a.K_size = _lib.dtype_enum(joint_K.dtype), joint_K.shape[1]
     a.joint_K, a.joint_V = joint_K.data_ptr(), joint_V.data_ptr()
-    _run(a, Q.device)
+    _, nbytes = _run(a, Q.device)
+    if Q is ts[0] and joint_K is ts[4] and joint_V is ts[8]:     # (no copy was made)
+        if len(known) >= 64:
+            known.clear()
+        known[key] = (a, C.byref(a), nbytes, _alignment([t.data_ptr() for t in ts], O))
     return O
+
+
+def _alignment(ptrs, out) -> int:
+    bits = out.data_ptr()
+    for p in ptrs:
+        bits |= p
+    return bits & 15
 
 
 def fused_attention_packed(
