@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 from typing import Optional
 
 import torch
@@ -24,22 +25,46 @@ def row_bytes(n_chunks: int, S: int, radius_bits: int) -> int:
     return ((bits + 31) // 32) * 4
 
 
-def _zeroed(device, *planes):
-    """Zero-filled tensors for ``planes`` ((elements, dtype) each) as slices of ONE allocation, starting at multiples of
-    256 bytes: a cache then costs one allocation and one fill instead of one per plane (a request's cache of four layers:
-    60 fills fewer)."""
-    spans, total = [], 0
-    for numel, dtype in planes:
-        nbytes = numel * dtype.itemsize
-        spans.append((total, nbytes, dtype))
-        total += (nbytes + 255) & ~255
-    buf = torch.empty(total, dtype=torch.uint8, device=device)
-    if buf.is_cuda:
+def _planes(device, planes, zeroed):
+    """Tensors for ``planes`` ((elements, dtype) each) as slices of ONE allocation, starting at multiples of 256 bytes; the
+    first ``zeroed`` of them are zero-filled.  (A cache then costs one allocation and one fill instead of one per plane.)"""
+    sizes = [numel * dtype.itemsize for numel, dtype in planes]
+    padded = [(n + 255) & ~255 for n in sizes]
+    buf = torch.empty(sum(padded), dtype=torch.uint8, device=device)
+    fill = sum(padded[:zeroed])
+    if not buf.is_cuda:
+        buf[:fill].zero_()
+    elif fill:
         with _lib.device_guard(buf.device):
-            _lib.check(_lib.lib().hqmq_zero(buf.data_ptr(), total, _lib.stream_ptr()), "hqmq_zero")
-    else:
-        buf.zero_()
-    return [buf[o:o + nb].view(dt) if dt != torch.uint8 else buf[o:o + nb] for o, nb, dt in spans]
+            _lib.check(_lib.lib().hqmq_zero(buf.data_ptr(), fill, _lib.stream_ptr()), "hqmq_zero")
+    return [t[:n] if dt is torch.uint8 else t[:n].view(dt) for t, n, (_, dt) in zip(buf.split(padded), sizes, planes)]
+
+
+class _CounterPool:
+    """Zeroed int32 counters handed out once each, from blocks that are filled once.  A block lives as long as anything
+    holds a slice of it; one block per stream is open at a time."""
+    BLOCK = 1 << 16
+
+    def __init__(self):
+        self._lock, self._open = threading.Lock(), {}
+
+    def take(self, n: int, device) -> torch.Tensor:
+        # (inside a graph capture the fill has to be part of the graph)
+        if device.type != "cuda" or n > self.BLOCK // 16 or torch.cuda.is_current_stream_capturing():
+            return torch.zeros(n, dtype=torch.int32, device=device)
+        with _lib.device_guard(device):
+            key = (device, _lib.stream_ptr())
+            with self._lock:
+                block, used = self._open.get(key, (None, 0))
+                if block is None or used + n > self.BLOCK:
+                    if len(self._open) >= 64:
+                        self._open.clear()
+                    block, used = torch.zeros(self.BLOCK, dtype=torch.int32, device=device), 0
+                self._open[key] = (block, used + ((n + 3) & ~3))
+        return block[used:used + n]
+
+
+_counters = _CounterPool()
 
 
 class PackedKV:
@@ -48,7 +73,9 @@ class PackedKV:
     def __init__(self, B: int, H: int, T_cap: int, n_chunks: int, S: int, radius_bits: int, device,
                  scale_dtype: torch.dtype = torch.bfloat16, with_outliers: bool = False,
                  out_dtype: torch.dtype = torch.bfloat16, out_cap: Optional[int] = None,
-                 ofrag: bool = False, ofrag_cap: Optional[int] = None):
+                 ofrag: bool = False, ofrag_cap: Optional[int] = None, zero: bool = True):
+        # zero=False: rows, scales, payload and records start as they come; for a cache that a call fills at once (nothing
+        # reads a row, entry or record that no call wrote)
         if n_chunks < 1 or n_chunks > 32:
             raise ValueError(f"n_chunks={n_chunks}: the native layout supports d_head <= 128")
         self.B, self.H, self.n_chunks, self.S, self.radius_bits = B, H, n_chunks, S, radius_bits
@@ -63,22 +90,24 @@ class PackedKV:
         blocks = B * H * (self.T_cap // _lib.OUT_BLOCK + 1)
         self.with_outliers = with_outliers
         # 64 bytes of slack so that whole-word reads near the end of the last row stay in bounds
-        planes = [(rows * self.row_bytes + 64, torch.uint8), (rows + 8, scale_dtype)]
+        data = [(rows * self.row_bytes + 64, torch.uint8), (rows + 8, scale_dtype)]
         if with_outliers:
             self.out_cap = (int(out_cap) + 1) & ~1 if out_cap is not None else self.T_cap * n_chunks
-            planes += [(rows + 4, torch.int32), (B * H * self.out_cap * 4 + 8, out_dtype), (blocks, torch.int32)]
-            self.codes, self.rs, self.flags, self.out_vals, self.out_off = _zeroed(dev, *planes)
-            # (an allocation of its own: what is kept of a cache that is gone is this counter, for the outlier statistics)
-            self.out_count = torch.zeros(B * H, dtype=torch.int32, device=dev)
+            data += [(B * H * self.out_cap * 4 + 8, out_dtype)]
+            index = [(rows + 4, torch.int32), (blocks, torch.int32)]
+            self.flags, self.out_off, self.codes, self.rs, self.out_vals = _planes(dev, index + data, 5 if zero else 2)
+            # (what is kept of a cache that is gone is this counter, for the outlier statistics)
+            self.out_count = _counters.take(B * H, self.codes.device)
         else:
             self.out_cap = 0
-            self.codes, self.rs = _zeroed(dev, *planes)
+            self.codes, self.rs = _planes(dev, data, 2 if zero else 0)
             self.flags = self.out_vals = self.out_off = self.out_count = None
         # optional fragment records (see include/hqmq_b200.h): by default room for one record per block
         self.with_ofrag = bool(ofrag) and with_outliers
         if self.with_ofrag:
             self.ofrag_cap = int(ofrag_cap) if ofrag_cap is not None else self.T_cap // _lib.OUT_BLOCK
-            self.ofrag, self.ofrag_off = _zeroed(dev, (B * H * self.ofrag_cap * _lib.OFRAG_BYTES + 16, torch.uint8), (blocks, torch.int32))
+            self.ofrag_off, self.ofrag = _planes(dev, [(blocks, torch.int32), (B * H * self.ofrag_cap * _lib.OFRAG_BYTES + 16, torch.uint8)],
+                                                 2 if zero else 1)
         else:
             self.ofrag_cap = 0
             self.ofrag = self.ofrag_off = None

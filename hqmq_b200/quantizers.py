@@ -21,7 +21,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib
-from .packed import PackedKV
+from .packed import PackedKV, _counters
 
 
 class KVQuantizer(ABC):
@@ -183,12 +183,12 @@ class HQMQQuantizer(KVQuantizer):
     # ---- compressed representation ---------------------------------------------------------------
     def new_cache(self, B: int, T_cap: int, d_head: int, device, scale_dtype=torch.bfloat16,
                   with_outliers: bool = False, out_dtype=torch.bfloat16, out_cap: Optional[int] = None,
-                  ofrag: bool = False, ofrag_cap: Optional[int] = None) -> PackedKV:
+                  ofrag: bool = False, ofrag_cap: Optional[int] = None, zero: bool = True) -> PackedKV:
         if d_head % 4 != 0:
             raise ValueError(f"d_head={d_head} not divisible by 4")
         return PackedKV(B, self.n_heads, T_cap, d_head // 4, self.secondary_size, self.radius_bits, device,
                         scale_dtype=scale_dtype, with_outliers=with_outliers, out_dtype=out_dtype, out_cap=out_cap,
-                        ofrag=ofrag, ofrag_cap=ofrag_cap)
+                        ofrag=ofrag, ofrag_cap=ofrag_cap, zero=zero)
 
     def _check_dst(self, x: torch.Tensor, out: PackedKV):
         """The library takes batch, heads and chunks per token from the destination planes: x must have that geometry."""
@@ -278,7 +278,7 @@ class HQMQQuantizer(KVQuantizer):
             if ofrag is None:
                 ofrag = kv == 0 and median_mult is not None
             out = self.new_cache(B, T, d, x.device, scale_dtype=sd, with_outliers=median_mult is not None,
-                                 out_dtype=od, ofrag=bool(ofrag) and median_mult is not None)
+                                 out_dtype=od, ofrag=bool(ofrag) and median_mult is not None, zero=False)
         self._check_dst(x, out)
         if median_mult is not None and not out.with_outliers:
             raise ValueError("destination cache was created without outlier planes")
@@ -439,7 +439,7 @@ class HQMQQuantizer(KVQuantizer):
                 self._qdq_cache[key] = entry
                 return self._qdq(x, layer_idx, kv, median_mult, quantile, count)
         pk = self.new_cache(B, T, d, x.device, scale_dtype=torch.float32, with_outliers=median_mult is not None,
-                            out_dtype=x.dtype if x.dtype != torch.float64 else torch.float32)
+                            out_dtype=x.dtype if x.dtype != torch.float64 else torch.float32, zero=False)
         self.encode(x, layer_idx, kv, out=pk, median_mult=median_mult, quantile=quantile)
         if count is not None:
             count.push_count(pk.out_count, B * H * T * (d // 4))
@@ -514,7 +514,8 @@ class _OutlierStats:
             if pk.T > 0 and pk.with_outliers:   # a cache filled elsewhere: count from what it holds
                 pk._stat_rec = [pk.out_count, pk.out_count.clone(), 0, total_chunks]
         elif rec[2] and rec[3] != total_chunks:
-            now = rec[0].clone()
+            now = _counters.take(rec[0].numel(), rec[0].device)
+            now.copy_(rec[0])
             self._closed.append((now, rec[1], rec[3], rec[2]))
             rec[1], rec[2] = now, 0
 
@@ -542,20 +543,22 @@ class _OutlierStats:
         done, self._closed = self._closed, []
         recs = {id(r): r for r in self._open if r[2]}.values()
         self._open = []
+        recs = list(recs)
         groups = done + [(r[0], r[1], r[3], r[2]) for r in recs]
-        tensors = [t for g in groups for t in g[:2] if isinstance(t, torch.Tensor)]
-        sums = iter(())
-        if tensors:                     # one transfer per device for all of them
-            host = {}
-            for dev in {t.device for t in tensors}:
-                host[dev] = iter(torch.cat([t.reshape(-1) for t in tensors if t.device == dev]).cpu()
-                                 .split([t.numel() for t in tensors if t.device == dev]))
-            sums = iter([float(next(host[t.device]).sum()) for t in tensors])
+        blocks = {}                     # the counters are slices of a few blocks: one transfer for each of those
+
+        def value(c):
+            if not isinstance(c, torch.Tensor):
+                return c
+            block = c._base if c._base is not None else c
+            if id(block) not in blocks:
+                blocks[id(block)] = (block.cpu().numpy(), block)
+            at = c.storage_offset() - block.storage_offset()
+            return float(blocks[id(block)][0][at:at + c.numel()].sum())
         ends = []
         for end, start, total, calls in groups:
-            e = next(sums) if isinstance(end, torch.Tensor) else end
-            b = next(sums) if isinstance(start, torch.Tensor) else start
-            self._sum_rates += (e - b) / max(1, total)
+            e = value(end)
+            self._sum_rates += (e - value(start)) / max(1, total)
             self._n += calls
             ends.append(e)
         for r, e in zip(recs, ends[len(done):]):
