@@ -1776,6 +1776,35 @@ scan_small_warp(const hqmq_packed& dst, int bh, int t_start, int T_new, int blk0
   }
 }
 
+// The same steps for one tensor or for K and V of a layer (blockIdx selects the tensor).
+struct SideArgs {
+  EncGeom g;
+  const void* x;
+  hqmq_packed dst;
+  int t_start, T_new, blk0, nblk, payload;
+  uint32_t* status;
+};
+struct SidePair { SideArgs t[2]; };
+__global__ void __launch_bounds__(kScanWarps * 32) scan_pair_kernel(const SidePair p) {
+  const SideArgs& a = p.t[blockIdx.y];
+  if (!a.payload && !a.dst.ofrag) return;
+  scan_body(a.dst, a.t_start, a.T_new, a.blk0, a.nblk, a.payload, a.status);
+}
+__global__ void __launch_bounds__(256) side_pair_kernel(const SidePair p) {
+  const SideArgs& a = p.t[blockIdx.z];
+  side_block(a.g, a.x, a.dst, a.t_start, a.blk0, a.nblk, blockIdx.y, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), threadIdx.x & 31);
+}
+// Calls of at most kScanSmallBlocks blocks per (b, h): a CTA scans and writes the side planes, a warp per block.
+__global__ void __launch_bounds__(kScanSmallBlocks * 32) side_small_kernel(const SidePair p, int side) {
+  const SideArgs& a = p.t[blockIdx.y];
+  if (!a.payload && !a.dst.ofrag) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0) scan_small_warp(a.dst, blockIdx.x, a.t_start, a.T_new, a.blk0, a.nblk, a.payload, a.status, lane);
+  if (!side) return;
+  __syncthreads();
+  side_block(a.g, a.x, a.dst, a.t_start, a.blk0, a.nblk, blockIdx.x, warp, lane);
+}
+
 // The K + V append of a layer in ONE launch, grid (H, 2): blockIdx.y = 0 the K tensor, 1 the V tensor (same batch,
 // heads, tokens and head dim).  After the head's codes, scales and flags, the same CTA scans the offsets of its batch
 // entries (a warp per entry) and writes their side planes (a warp per block) -- what scan_kernel and side_kernel do in
@@ -2301,41 +2330,66 @@ static bool fused_call(const hqmq_encode_args* a) {
   if (d.H > sm_count() || (uint64_t)d.B * a->T_new * d.n_chunks >= ((uint64_t)1 << 32)) return false;
   return fused_smem_bytes(d.S, ((size_t)a->lut_footprint + 15) & ~(size_t)15) <= (size_t)226 * 1024;
 }
-static int launch_fused(const hqmq_encode_args* a, uint32_t* status, uint32_t* hist, uint32_t* bars, void* out, uint32_t* n_flagged,
-                        cudaStream_t st) {
+static void fill_fused(const hqmq_encode_args* a, int tensors, uint32_t* status, uint32_t* hist, uint32_t* bars, void* out, uint32_t* n_flagged,
+                       FusedArgs& f) {
   const hqmq_packed& d = a->dst;
-  FusedArgs f;
   f.g = geom_of(a);
   f.x = reinterpret_cast<const uint16_t*>(a->x); f.qs = a->qs; f.joint = a->joint;
   f.lut = reinterpret_cast<const unsigned char*>(a->lut);
   f.dst = d; f.t_start = a->t_start; f.out = reinterpret_cast<uint16_t*>(out); f.n_flagged = n_flagged;
   f.C = a->median_mult; f.quantile = a->quantile; f.med_in = a->med_in; f.med_out = a->med_out;
   f.hist = hist; f.bars = bars; f.status = status;
+  // (64-wide tokens outside the paired geometry used to run the generic kernels: the same near-ties are kept)
+  f.rcp_rn = d.n_chunks == 16 && !(pair16_of(*a) && ((uintptr_t)a->x & 15) == 0 && a->x_stride[0] % 8 == 0 && a->x_stride[1] % 8 == 0);
   // one CTA per SM in all, no fewer than a round of its warps each
   const int64_t W = (int64_t)d.B * (d.n_chunks == 16 ? (a->T_new + 1) / 2 : a->T_new);
-  int64_t cph = sm_count() / d.H;
+  int64_t cph = sm_count() / (tensors * d.H);
   if (cph > (W + kEnc32Warps - 1) / kEnc32Warps) cph = (W + kEnc32Warps - 1) / kEnc32Warps;
   f.per = (int)((W + cph - 1) / cph);
   f.cph = (int)((W + f.per - 1) / f.per);
-  const bool h16 = a->x_dtype == HQMQ_F16, dense = out != nullptr;
+}
+// `tensors` of one geometry, element type and codebook size, each with its own threshold or all without.
+static int launch_fused(const FusedPair& f, int tensors, int x_dtype, size_t lut_foot, cudaStream_t st) {
+  const EncGeom& g = f.t[0].g;
+  const bool h16 = x_dtype == HQMQ_F16, dense = f.t[0].out != nullptr;
   const void* k = nullptr;
 #define HQMQ_PICK(IB_, RB_)                                                                                    \
-  if (f.g.ib == IB_ && f.g.rbits == RB_)                                                                         \
+  if (g.ib == IB_ && g.rbits == RB_)                                                                             \
     k = dense ? (h16 ? (const void*)&encode_fused_kernel<HQMQ_F16, IB_, RB_, true> : (const void*)&encode_fused_kernel<HQMQ_BF16, IB_, RB_, true>)   \
               : (h16 ? (const void*)&encode_fused_kernel<HQMQ_F16, IB_, RB_, false> : (const void*)&encode_fused_kernel<HQMQ_BF16, IB_, RB_, false>);
   HQMQ_PICK(10, 3) HQMQ_PICK(12, 4) HQMQ_PICK(13, 6)
 #undef HQMQ_PICK
-  const size_t smem = fused_smem_bytes(d.S, ((size_t)a->lut_footprint + 15) & ~(size_t)15);
+  const size_t smem = fused_smem_bytes(g.S, (lut_foot + 15) & ~(size_t)15);
   HQMQ_CHECK_CUDA(attn::raise_smem_limit(k, smem));
   Maps24 maps;
   memcpy(maps.ref_to_native, index_maps().ref_to_native, 24);
   const Mul24& nmul = mul24_native();
-  void* args[] = {&f, &maps, (void*)&nmul};
+  void* args[] = {(void*)&f, &maps, (void*)&nmul};
+  const dim3 grid(f.t[0].cph * g.H, tensors);
   // (the CTAs of a head wait for one another only for a threshold of the call's own)
-  const bool waits = a->median_mult > 0.f && !a->med_in && f.cph > 1;
-  if (waits) HQMQ_CHECK_CUDA(cudaLaunchCooperativeKernel(k, dim3(f.cph * d.H), dim3(kEnc32Threads), args, smem, st));
-  else HQMQ_CHECK_CUDA(cudaLaunchKernel(k, dim3(f.cph * d.H), dim3(kEnc32Threads), args, smem, st));
+  const bool waits = f.t[0].C > 0.f && !f.t[0].med_in && f.t[0].cph > 1;
+  if (waits) HQMQ_CHECK_CUDA(cudaLaunchCooperativeKernel(k, grid, dim3(kEnc32Threads), args, smem, st));
+  else HQMQ_CHECK_CUDA(cudaLaunchKernel(k, grid, dim3(kEnc32Threads), args, smem, st));
   return HQMQ_OK;
+}
+// Offsets and side planes behind the main kernel, of one tensor or of two.
+static int launch_side(const SidePair& sp, int tensors, bool med, cudaStream_t st) {
+  const SideArgs& a = sp.t[0];
+  const int bh = a.dst.B * a.dst.H;
+  if (a.nblk <= kScanSmallBlocks) {
+    side_small_kernel<<<dim3(bh, tensors), 32 * (med ? a.nblk : 1), 0, st>>>(sp, med ? 1 : 0);
+  } else {
+    scan_pair_kernel<<<dim3(bh, tensors), kScanWarps * 32, 0, st>>>(sp);
+    if (med) side_pair_kernel<<<dim3((a.nblk + 7) / 8, bh, tensors), 256, 0, st>>>(sp);
+  }
+  HQMQ_LAUNCH_CHECK();
+  return HQMQ_OK;
+}
+static SideArgs side_args(const hqmq_encode_args* a, const WsPlan& wp, uint32_t* ws) {
+  SideArgs s;
+  s.g = geom_of(a); s.x = a->x; s.dst = a->dst; s.t_start = a->t_start; s.T_new = a->T_new; s.blk0 = wp.blk0; s.nblk = wp.nblk;
+  s.payload = a->median_mult > 0.f ? 1 : 0; s.status = ws + wp.status;
+  return s;
 }
 
 // ---- fake-quantised tensor straight from x ----------------------------------------------------------------------------
@@ -2384,7 +2438,9 @@ extern "C" int hqmq_fake_quant(const hqmq_encode_args* a, void* out, uint32_t* n
   uint32_t* hist = ws + 4;
   uint32_t* bars = hist + (size_t)d.H * 3 * 2 * kHistBins;
   if (a->median_mult > 0.f && !a->med_in) HQMQ_CHECK_CUDA(cudaMemsetAsync(ws, 0, fake_quant_ws_words(d.H) * 4, st));
-  return launch_fused(a, ws, hist, bars, out, n_flagged, st);
+  FusedPair f;
+  fill_fused(a, 1, ws, hist, bars, out, n_flagged, f.t[0]);
+  return launch_fused(f, 1, a->x_dtype, (size_t)a->lut_footprint, st);
 }
 
 extern "C" size_t hqmq_encode_pair_workspace_bytes(const hqmq_encode_args* k, const hqmq_encode_args* v) {
@@ -2407,6 +2463,24 @@ extern "C" int hqmq_encode_pair(const hqmq_encode_args* k, const hqmq_encode_arg
   const bool same = dk.B == dv.B && dk.H == dv.H && dk.n_chunks == dv.n_chunks && k->T_new == v->T_new;
   if (!same || k->T_new == 0 || !small_call(k) || !small_call(v) || plan_ws(*k).nblk > kScanSmallBlocks ||
       plan_ws(*v).nblk > kScanSmallBlocks) {
+    const bool med = k->median_mult > 0.f;
+    if (same && k->T_new > 0 && !small_call(k) && fused_call(k) && fused_call(v) && !bracket_wanted(*k) && !bracket_wanted(*v) &&
+        2 * dk.H <= sm_count() && dk.S == dv.S && dk.radius_bits == dv.radius_bits && k->x_dtype == v->x_dtype &&
+        med == (v->median_mult > 0.f) && !k->med_in == !v->med_in && plan_ws(*k).nblk == plan_ws(*v).nblk) {
+      // a prompt of ordinary length: both tensors in each launch
+      cudaStream_t st = (cudaStream_t)stream;
+      const WsPlan pk = plan_ws(*k), pv = plan_ws(*v);
+      uint32_t *sk = reinterpret_cast<uint32_t*>(wsb), *sv = reinterpret_cast<uint32_t*>(wsb + wk);
+      HQMQ_CHECK_CUDA(cudaMemset2DAsync(wsb, wk, 0, (pk.sel + (size_t)dk.H * 8) * sizeof(uint32_t), 2, st));
+      FusedPair f;
+      fill_fused(k, 2, sk + pk.status, sk + pk.hist, sk + pk.sel, nullptr, nullptr, f.t[0]);
+      fill_fused(v, 2, sv + pv.status, sv + pv.hist, sv + pv.sel, nullptr, nullptr, f.t[1]);
+      rc = launch_fused(f, 2, k->x_dtype, (size_t)(k->lut_footprint > v->lut_footprint ? k->lut_footprint : v->lut_footprint), st);
+      if (rc || !(med || dk.ofrag || dv.ofrag)) return rc;
+      SidePair sp;
+      sp.t[0] = side_args(k, pk, sk); sp.t[1] = side_args(v, pv, sv);
+      return launch_side(sp, 2, med, st);
+    }
     // no common launch shape: one tensor after the other, each with its part of the workspace
     rc = hqmq_encode(k, wsb, wk, stream);
     if (rc) return rc;
@@ -2474,13 +2548,13 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
   if (fused_call(a) && !bracket_wanted(*a)) {
     // (status, histograms and select words are the first part of the workspace; the select words serve as arrival counters)
     HQMQ_CHECK_CUDA(cudaMemsetAsync(ws, 0, (wp.sel + (size_t)d.H * 8) * sizeof(uint32_t), st));
-    rc = launch_fused(a, ws + wp.status, ws + wp.hist, ws + wp.sel, nullptr, nullptr, st);
-    if (rc) return rc;
-    if (med || d.ofrag)
-      scan_kernel<<<d.B * d.H, kScanWarps * 32, 0, st>>>(d, a->t_start, a->T_new, wp.blk0, wp.nblk, med ? 1 : 0, ws + wp.status);
-    if (med) side_kernel<<<dim3((wp.nblk + 7) / 8, d.B * d.H), 256, 0, st>>>(g, a->x, d, a->t_start, wp.blk0, wp.nblk);
-    HQMQ_LAUNCH_CHECK();
-    return HQMQ_OK;
+    FusedPair f;
+    fill_fused(a, 1, ws + wp.status, ws + wp.hist, ws + wp.sel, nullptr, nullptr, f.t[0]);
+    rc = launch_fused(f, 1, a->x_dtype, (size_t)a->lut_footprint, st);
+    if (rc || !(med || d.ofrag)) return rc;
+    SidePair sp;
+    sp.t[0] = side_args(a, wp, ws);
+    return launch_side(sp, 1, med, st);
   }
   HQMQ_CHECK_CUDA(cudaMemsetAsync(ws, 0, wp.zero_bytes, st));
 

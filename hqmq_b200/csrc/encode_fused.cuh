@@ -25,7 +25,9 @@ struct FusedArgs {
   uint32_t* bars;             // [H] arrivals, zero
   uint32_t* status;
   int cph, per;               // CTAs per head, warp tokens per CTA
+  int rcp_rn;                 // directions are normalised with the rounded reciprocal (as the generic passes do)
 };
+struct FusedPair { FusedArgs t[2]; };            // blockIdx.y: the tensor (K and V of a layer in one launch, or one tensor)
 constexpr uint32_t kFusedPolls = 1u << 20;       // about a second
 
 __device__ __forceinline__ void fused_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -39,12 +41,13 @@ __host__ __device__ inline size_t fused_smem_bytes(int S, size_t lut_foot) {
 }
 
 template <int DT, int IB, int RB, bool DENSE>
-__global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const FusedArgs a, const Maps24 maps, const Mul24 nmul) {
+__global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const FusedPair pr, const Maps24 maps, const Mul24 nmul) {
   constexpr int CB = IB + RB;
   constexpr float qmaxf = (float)((1 << RB) - 1);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ uint32_t s_warp[32], s_sel[4], s_flagged;
+  const FusedArgs& a = pr.t[blockIdx.y];
   const EncGeom& g = a.g;
   const int S = g.S, h = blockIdx.x / a.cph, part = blockIdx.x - h * a.cph;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -221,7 +224,7 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
     const bool flagged = live && nrm > thr;
     const uint32_t flag_word = __ballot_sync(0xffffffffu, flagged);
     n_fl += __popc(flag_word);
-    const float inv_r = rcp_approx(radius);
+    const float inv_r = a.rcp_rn ? __frcp_rn(radius) : rcp_approx(radius);
     int au, sidx;
     const float u0 = v[0] * inv_r, u1 = v[1] * inv_r, u2 = v[2] * inv_r, u3 = v[3] * inv_r;
     if (!search_fold24(sjoint, L, S, inv_S, u0, u1, u2, u3, au, sidx)) {

@@ -25,21 +25,6 @@ def row_bytes(n_chunks: int, S: int, radius_bits: int) -> int:
     return ((bits + 31) // 32) * 4
 
 
-def _planes(device, planes, zeroed):
-    """Tensors for ``planes`` ((elements, dtype) each) as slices of ONE allocation, starting at multiples of 256 bytes; the
-    first ``zeroed`` of them are zero-filled.  (A cache then costs one allocation and one fill instead of one per plane.)"""
-    sizes = [numel * dtype.itemsize for numel, dtype in planes]
-    padded = [(n + 255) & ~255 for n in sizes]
-    buf = torch.empty(sum(padded), dtype=torch.uint8, device=device)
-    fill = sum(padded[:zeroed])
-    if not buf.is_cuda:
-        buf[:fill].zero_()
-    elif fill:
-        with _lib.device_guard(buf.device):
-            _lib.check(_lib.lib().hqmq_zero(buf.data_ptr(), fill, _lib.stream_ptr()), "hqmq_zero")
-    return [t[:n] if dt is torch.uint8 else t[:n].view(dt) for t, n, (_, dt) in zip(buf.split(padded), sizes, planes)]
-
-
 class _CounterPool:
     """Zeroed int32 counters handed out once each, from blocks that are filled once.  A block lives as long as anything
     holds a slice of it; one block per stream is open at a time."""
@@ -89,32 +74,66 @@ class PackedKV:
         rows = B * H * self.T_cap
         blocks = B * H * (self.T_cap // _lib.OUT_BLOCK + 1)
         self.with_outliers = with_outliers
-        # 64 bytes of slack so that whole-word reads near the end of the last row stay in bounds
-        data = [(rows * self.row_bytes + 64, torch.uint8), (rows + 8, scale_dtype)]
+        # One allocation for the planes (slices at multiples of 256 bytes) and one fill of what has to start at zero, which
+        # comes first; tensors over the slices are made when somebody asks for one (__getattr__), the library takes addresses.
+        # 64 bytes of slack so that whole-word reads near the end of the last row stay in bounds.
+        self._spans = {}
+        index, data = [], [("codes", rows * self.row_bytes + 64, torch.uint8), ("rs", rows + 8, scale_dtype)]
         if with_outliers:
             self.out_cap = (int(out_cap) + 1) & ~1 if out_cap is not None else self.T_cap * n_chunks
-            data += [(B * H * self.out_cap * 4 + 8, out_dtype)]
-            index = [(rows + 4, torch.int32), (blocks, torch.int32)]
-            self.flags, self.out_off, self.codes, self.rs, self.out_vals = _planes(dev, index + data, 5 if zero else 2)
-            # (what is kept of a cache that is gone is this counter, for the outlier statistics)
-            self.out_count = _counters.take(B * H, self.codes.device)
+            index += [("flags", rows + 4, torch.int32), ("out_off", blocks, torch.int32)]
+            data += [("out_vals", B * H * self.out_cap * 4 + 8, out_dtype)]
         else:
             self.out_cap = 0
-            self.codes, self.rs = _planes(dev, data, 2 if zero else 0)
             self.flags = self.out_vals = self.out_off = self.out_count = None
+        buf = self._allocate(dev, index, data, zero)
+        self.device = buf.device
+        if with_outliers:
+            # (what is kept of a cache that is gone is this counter, for the outlier statistics)
+            self.out_count = _counters.take(B * H, self.device)
         # optional fragment records (see include/hqmq_b200.h): by default room for one record per block
         self.with_ofrag = bool(ofrag) and with_outliers
         if self.with_ofrag:
             self.ofrag_cap = int(ofrag_cap) if ofrag_cap is not None else self.T_cap // _lib.OUT_BLOCK
-            self.ofrag_off, self.ofrag = _planes(dev, [(blocks, torch.int32), (B * H * self.ofrag_cap * _lib.OFRAG_BYTES + 16, torch.uint8)],
-                                                 2 if zero else 1)
+            self._allocate(dev, [("ofrag_off", blocks, torch.int32)],
+                           [("ofrag", B * H * self.ofrag_cap * _lib.OFRAG_BYTES + 16, torch.uint8)], zero)
         else:
             self.ofrag_cap = 0
             self.ofrag = self.ofrag_off = None
 
-    @property
-    def device(self):
-        return self.codes.device
+    def _allocate(self, device, index, data, zero) -> torch.Tensor:
+        total = fill = 0
+        spans = []
+        for planes in (index, data):
+            for name, numel, dtype in planes:
+                nbytes = numel * dtype.itemsize
+                spans.append((name, total, nbytes, dtype))
+                total += (nbytes + 255) & ~255
+            if zero or planes is index:
+                fill = total
+        buf = torch.empty(total, dtype=torch.uint8, device=device)
+        base = buf.data_ptr()
+        if not buf.is_cuda:
+            buf[:fill].zero_()
+        elif fill:
+            with _lib.device_guard(buf.device):
+                _lib.check(_lib.lib().hqmq_zero(base, fill, _lib.stream_ptr()), "hqmq_zero")
+        for name, at, nbytes, dtype in spans:
+            self._spans[name] = (buf, at, nbytes, dtype, base + at)
+        return buf
+
+    def __getattr__(self, name):
+        span = self.__dict__.get("_spans", {}).get(name)
+        if span is None:
+            raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
+        buf, at, nbytes, dtype, _ = span
+        t = buf[at:at + nbytes].view(dtype)
+        self.__dict__[name] = t
+        return t
+
+    def _ptr(self, name) -> int:
+        t = self.__dict__.get(name)
+        return self._spans[name][4] if t is None else t.data_ptr()
 
     @property
     def qmax(self) -> int:
@@ -128,18 +147,19 @@ class PackedKV:
         p.scale_dtype = _lib.dtype_enum(self.scale_dtype)
         p.out_dtype = _lib.dtype_enum(self.out_dtype)
         p.out_cap = self.out_cap
-        p.codes, p.rs = self.codes.data_ptr(), self.rs.data_ptr()
+        p.codes, p.rs = self._ptr("codes"), self._ptr("rs")
         if self.with_outliers:
-            p.flags, p.out_vals = self.flags.data_ptr(), self.out_vals.data_ptr()
-            p.out_off, p.out_count = self.out_off.data_ptr(), self.out_count.data_ptr()
+            p.flags, p.out_vals = self._ptr("flags"), self._ptr("out_vals")
+            p.out_off, p.out_count = self._ptr("out_off"), self.out_count.data_ptr()
         if self.with_ofrag:
             p.ofrag_cap = self.ofrag_cap
-            p.ofrag, p.ofrag_off = self.ofrag.data_ptr(), self.ofrag_off.data_ptr()
+            p.ofrag, p.ofrag_off = self._ptr("ofrag"), self._ptr("ofrag_off")
         return p
 
     def drop_ofrag(self) -> None:
         """Forget the fragment records: attention then merges K outliers from flags / out_vals."""
         self.with_ofrag, self.ofrag_cap, self.ofrag, self.ofrag_off = False, 0, None, None
+        self._spans.pop("ofrag", None), self._spans.pop("ofrag_off", None)
         self._enc_cache.clear()
         self._attn_cache.clear()
 
