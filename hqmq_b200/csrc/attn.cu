@@ -15,6 +15,7 @@ size_t fast_warp_bytes(int n_chunks, int ib, int rb, bool outl);
 bool ring_kernel(int n_chunks, int ib, int rb, bool outl, int scale_dtype, RingKernelInfo& k);
 size_t ring_smem_total(int table_rows, int repk_log2, int repv_log2, int d, bool outl, int stages, int merge_slots,
                        size_t stage_bytes, int warps);
+constexpr int kRingManyPieces = 4;       // see attn_ring_body
 constexpr int kRingMinKeys = 1024;       // shorter key ranges keep the per-warp staging rings
 // ... and so do small problems: below about four stages per SM the ring kernel's set-up (it replicates the tables
 // up to sixteen times) outweighs its faster tile loop (B1, 8 KV heads, 4096 keys: 42 against 26 us per step)
@@ -344,7 +345,7 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
   }
   if (pl.warp_units) pl.ppc = pl.nw;
   if (ring) {
-    pl.kernel = rk.fn;
+    pl.kernel = rk.fn[0];
     pl.nw = rk.warps;
     pl.threads = (rk.warps + 1) * 32;
     pl.smem = ring_smem_total(pl.table_rows, pl.rep_log2, pl.repv_log2, a->d, outl, pl.ring_stages, pl.merge_slots, rk.stage_bytes, rk.warps);
@@ -407,6 +408,11 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
       pl.grid = pl.units * c;
       pl.P = c;
     }
+  }
+  // (the merge of many pieces keeps 8 weights per piece in the merge slots)
+  if (pl.ring_stages && pl.P > kRingManyPieces && pl.P <= pl.merge_slots * a->d) {
+    pl.kernel = rk.fn[1];
+    if (query_device) resident_ctas(pl.kernel, pl.smem, pl.threads);
   }
   const int64_t rows = (int64_t)a->B * a->H_q * a->T_q;
   pl.ticket_bytes = pl.ring_stages ? (((size_t)pl.units * 4 + 15) & ~(size_t)15) : 0;

@@ -6,15 +6,21 @@ namespace hqmq {
 namespace attn {
 
 // SDT: element type of the per-token scale planes (HQMQ_F16 or HQMQ_BF16), fixed at compile time like the field layout.
-template <int N, int IB, int RB, bool OUTL, int SDT>
+// MANY: how the pieces of a unit are merged (see attn_ring_body).
+template <int N, int IB, int RB, bool OUTL, int SDT, bool MANY>
 __global__ void __launch_bounds__((ring_warps(N) + 1) * 32, 1) attn_ring_kernel(const AttnParams p) {
-  attn_ring_body<N, IB, RB, OUTL, SDT>(p);
+  attn_ring_body<N, IB, RB, OUTL, SDT, MANY>(p);
 }
 
+template <int N, int IB, int RB, bool OUTL, bool MANY>
+static const void* fn(int sdt) {
+  return sdt == HQMQ_F16 ? reinterpret_cast<const void*>(&attn_ring_kernel<N, IB, RB, OUTL, HQMQ_F16, MANY>)
+                         : reinterpret_cast<const void*>(&attn_ring_kernel<N, IB, RB, OUTL, HQMQ_BF16, MANY>);
+}
 template <int N, int IB, int RB, bool OUTL>
 static void fill(int sdt, RingKernelInfo& k) {
-  k.fn = sdt == HQMQ_F16 ? reinterpret_cast<const void*>(&attn_ring_kernel<N, IB, RB, OUTL, HQMQ_F16>)
-                         : reinterpret_cast<const void*>(&attn_ring_kernel<N, IB, RB, OUTL, HQMQ_BF16>);
+  k.fn[0] = fn<N, IB, RB, OUTL, false>(sdt);
+  k.fn[1] = fn<N, IB, RB, OUTL, true>(sdt);
   k.stage_bytes = RingLayout<N, IB, RB, OUTL>::BYTES;
   k.warps = ring_warps(N);
 }

@@ -164,7 +164,10 @@ __device__ __forceinline__ bool ring_wait_producer(uint32_t bar, uint32_t parity
   }
 }
 
-template <int N, int IB, int RB, bool OUTL, int SDT>
+// MANY: units are cut into more than kRingManyPieces pieces, merged with a warp per head for the weights (8 units over 148 CTAs:
+// 119.3 -> 115.9 us).  With two or three pieces every thread walks them itself; that kernel does not carry the other merge,
+// whose mere presence cost the main loop 1.3 % (113.8 against 115.3 us for 128 units).
+template <int N, int IB, int RB, bool OUTL, int SDT, bool MANY>
 __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
   using G_ = Geo<N>;
   using FL = FastLoader<N, IB, RB, true>;
@@ -884,12 +887,10 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
         consumer_bar();
         if (*last_s) {
           __threadfence();
-          const int64_t row0 = ((int64_t)b * p.Hq + h * p.G) * p.Tq + tq, gstride = (int64_t)p.Tq * p.P * (D + 2);
-          const float* base = p.partials + row0 * p.P * (D + 2);
-          // (few pieces: every thread walks them itself, one barrier and the header pass less; 115.3 against 113.6 us for 128
-          //  units cut in two or three)
-          if (n_ctas > 4 && 8 * n_ctas <= MS * 8 * D) {
-            merge_partials<D>(threadIdx.x, kRingConsumerThreads, p.G, n_ctas, base, gstride, D + 2, slots, ms_s, consumer_bar, emit);
+          if constexpr (MANY) {
+            const int64_t row0 = ((int64_t)b * p.Hq + h * p.G) * p.Tq + tq, gstride = (int64_t)p.Tq * p.P * (D + 2);
+            merge_partials<D>(threadIdx.x, kRingConsumerThreads, p.G, n_ctas, p.partials + row0 * p.P * (D + 2), gstride, D + 2,
+                              slots, ms_s, consumer_bar, emit);
           } else {
 #pragma unroll
           for (int q = 0; q < PER; ++q) {
