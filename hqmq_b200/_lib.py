@@ -212,18 +212,20 @@ def device_guard(device: torch.device):
     """torch.cuda.device(device), or nothing when that device is already current (saves the switch on the
     decode-time hot path)."""
     idx = device.index
-    if idx is None or idx == torch.cuda.current_device():
+    if idx is None or idx == _current_device():
         return _NO_GUARD
     return torch.cuda.device(device)
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+# (torch.cuda.current_device() asks three more functions first whether CUDA is up; callers here hold a CUDA tensor)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def stream_ptr() -> int:
     """cudaStream_t of torch's current stream on the current device."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_current_device())
     return torch.cuda.current_stream().cuda_stream
 
 

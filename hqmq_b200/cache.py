@@ -52,8 +52,10 @@ class PackedKVCache:
         cap = max(1024, int(self.outlier_capacity * self.max_tokens * (d // 4))) if self._with_outliers else None
         mk = lambda kv: self._inner.new_cache(B, self.max_tokens, d, k.device, scale_dtype=sd,
                                               with_outliers=self._with_outliers, out_dtype=k.dtype, out_cap=cap,
-                                              ofrag=self._with_outliers and kv == 0)
-        return mk(0), mk(1)
+                                              ofrag=self._with_outliers and kv == 0, place=False)
+        pair = mk(0), mk(1)
+        PackedKV.place(k.device, *pair)
+        return pair
 
     def update(self, key_states: torch.Tensor, value_states: torch.Tensor, layer_idx: int,
                cache_kwargs=None) -> Tuple[PackedKV, PackedKV]:

@@ -52,15 +52,31 @@ class _CounterPool:
 _counters = _CounterPool()
 
 
+def _plane(name):
+    """A plane as a tensor (None where the cache has no such plane)."""
+    def get(self):
+        t = self._tensors.get(name)
+        if t is None and name in self._spans:
+            buf, at, nbytes, dtype, _ = self._spans[name]
+            t = self._tensors[name] = buf[at:at + nbytes].view(dtype)
+        return t
+
+    def put(self, t):
+        self._tensors[name], self._struct = t, None
+    return property(get, put)
+
+
 class PackedKV:
     """Bit-packed cache planes for one tensor of shape (B, H, T<=T_cap, 4*n_chunks)."""
+    codes, rs, flags, out_off, out_vals, out_count, ofrag, ofrag_off = map(_plane, (
+        "codes", "rs", "flags", "out_off", "out_vals", "out_count", "ofrag", "ofrag_off"))
 
     def __init__(self, B: int, H: int, T_cap: int, n_chunks: int, S: int, radius_bits: int, device,
                  scale_dtype: torch.dtype = torch.bfloat16, with_outliers: bool = False,
                  out_dtype: torch.dtype = torch.bfloat16, out_cap: Optional[int] = None,
-                 ofrag: bool = False, ofrag_cap: Optional[int] = None, zero: bool = True):
+                 ofrag: bool = False, ofrag_cap: Optional[int] = None, zero: bool = True, place: bool = True):
         # zero=False: rows, scales, payload and records start as they come; for a cache that a call fills at once (nothing
-        # reads a row, entry or record that no call wrote)
+        # reads a row, entry or record that no call wrote).  place=False: no memory yet, see place().
         if n_chunks < 1 or n_chunks > 32:
             raise ValueError(f"n_chunks={n_chunks}: the native layout supports d_head <= 128")
         self.B, self.H, self.n_chunks, self.S, self.radius_bits = B, H, n_chunks, S, radius_bits
@@ -75,64 +91,59 @@ class PackedKV:
         blocks = B * H * (self.T_cap // _lib.OUT_BLOCK + 1)
         self.with_outliers = with_outliers
         # One allocation for the planes (slices at multiples of 256 bytes) and one fill of what has to start at zero, which
-        # comes first; tensors over the slices are made when somebody asks for one (__getattr__), the library takes addresses.
+        # comes first; tensors over the slices are made when somebody asks for one, the library takes addresses.
         # 64 bytes of slack so that whole-word reads near the end of the last row stay in bounds.
-        self._spans = {}
         index, data = [], [("codes", rows * self.row_bytes + 64, torch.uint8), ("rs", rows + 8, scale_dtype)]
+        self.out_cap = self.ofrag_cap = 0
         if with_outliers:
             self.out_cap = (int(out_cap) + 1) & ~1 if out_cap is not None else self.T_cap * n_chunks
             index += [("flags", rows + 4, torch.int32), ("out_off", blocks, torch.int32)]
             data += [("out_vals", B * H * self.out_cap * 4 + 8, out_dtype)]
-        else:
-            self.out_cap = 0
-            self.flags = self.out_vals = self.out_off = self.out_count = None
-        buf = self._allocate(dev, index, data, zero)
-        self.device = buf.device
-        if with_outliers:
-            # (what is kept of a cache that is gone is this counter, for the outlier statistics)
-            self.out_count = _counters.take(B * H, self.device)
         # optional fragment records (see include/hqmq_b200.h): by default room for one record per block
         self.with_ofrag = bool(ofrag) and with_outliers
         if self.with_ofrag:
             self.ofrag_cap = int(ofrag_cap) if ofrag_cap is not None else self.T_cap // _lib.OUT_BLOCK
-            self._allocate(dev, [("ofrag_off", blocks, torch.int32)],
-                           [("ofrag", B * H * self.ofrag_cap * _lib.OFRAG_BYTES + 16, torch.uint8)], zero)
-        else:
-            self.ofrag_cap = 0
-            self.ofrag = self.ofrag_off = None
+            index += [("ofrag_off", blocks, torch.int32)]
+            data += [("ofrag", B * H * self.ofrag_cap * _lib.OFRAG_BYTES + 16, torch.uint8)]
+        self._layout, at = [], 0
+        for name, numel, dtype in index + data:
+            self._layout.append((name, at, numel * dtype.itemsize, dtype))
+            at += (numel * dtype.itemsize + 255) & ~255
+        self._bytes, self._fill = at, at if zero else self._layout[len(index)][1]
+        self._spans, self._tensors, self._struct = {}, {}, None
+        if place:
+            PackedKV.place(dev, self)
 
-    def _allocate(self, device, index, data, zero) -> torch.Tensor:
-        total = fill = 0
-        spans = []
-        for planes in (index, data):
-            for name, numel, dtype in planes:
-                nbytes = numel * dtype.itemsize
-                spans.append((name, total, nbytes, dtype))
-                total += (nbytes + 255) & ~255
-            if zero or planes is index:
-                fill = total
-        buf = torch.empty(total, dtype=torch.uint8, device=device)
-        base = buf.data_ptr()
-        if not buf.is_cuda:
-            buf[:fill].zero_()
-        elif fill:
-            with _lib.device_guard(buf.device):
-                _lib.check(_lib.lib().hqmq_zero(base, fill, _lib.stream_ptr()), "hqmq_zero")
-        for name, at, nbytes, dtype in spans:
-            self._spans[name] = (buf, at, nbytes, dtype, base + at)
-        return buf
-
-    def __getattr__(self, name):
-        span = self.__dict__.get("_spans", {}).get(name)
-        if span is None:
-            raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
-        buf, at, nbytes, dtype, _ = span
-        t = buf[at:at + nbytes].view(dtype)
-        self.__dict__[name] = t
-        return t
+    @staticmethod
+    def place(device, *caches) -> None:
+        """Give the planes of caches made with ``place=False`` their memory, one buffer for all of them."""
+        buf = torch.empty(sum(pk._bytes for pk in caches), dtype=torch.uint8, device=device)
+        base, at, fills = buf.data_ptr(), 0, []
+        for pk in caches:
+            pk.device = buf.device
+            pk._spans = {name: (buf, at + off, nbytes, dtype, base + at + off) for name, off, nbytes, dtype in pk._layout}
+            if fills and fills[-1][1] == at:
+                fills[-1][1] = at + pk._fill
+            else:
+                fills.append([at, at + pk._fill])
+            at += pk._bytes
+        for lo, hi in fills:
+            if not buf.is_cuda:
+                buf[lo:hi].zero_()
+            elif hi > lo:
+                with _lib.device_guard(buf.device):
+                    _lib.check(_lib.lib().hqmq_zero(base + lo, hi - lo, _lib.stream_ptr()), "hqmq_zero")
+        # (what is kept of a cache that is gone is its counter, for the outlier statistics)
+        n = [pk.B * pk.H if pk.with_outliers else 0 for pk in caches]
+        if any(n):
+            counters, lo = _counters.take(sum(n), buf.device), 0
+            for pk, k in zip(caches, n):
+                if k:
+                    pk.out_count = counters if k == counters.numel() else counters[lo:lo + k]
+                lo += k
 
     def _ptr(self, name) -> int:
-        t = self.__dict__.get(name)
+        t = self._tensors.get(name)
         return self._spans[name][4] if t is None else t.data_ptr()
 
     @property
@@ -140,6 +151,10 @@ class PackedKV:
         return (1 << self.radius_bits) - 1
 
     def c_struct(self) -> _lib.Packed:
+        """The library's descriptor of the planes (kept: copy it before changing a field)."""
+        kept, state = self._struct, (self.with_outliers, self.with_ofrag, self.out_cap, self.ofrag_cap)
+        if kept is not None and kept[0] == state:
+            return kept[1]
         p = _lib.Packed()
         p.struct_size = C.sizeof(_lib.Packed)
         p.B, p.H, p.T_cap, p.n_chunks = self.B, self.H, self.T_cap, self.n_chunks
@@ -154,12 +169,14 @@ class PackedKV:
         if self.with_ofrag:
             p.ofrag_cap = self.ofrag_cap
             p.ofrag, p.ofrag_off = self._ptr("ofrag"), self._ptr("ofrag_off")
+        self._struct = (state, p)
         return p
 
     def drop_ofrag(self) -> None:
         """Forget the fragment records: attention then merges K outliers from flags / out_vals."""
-        self.with_ofrag, self.ofrag_cap, self.ofrag, self.ofrag_off = False, 0, None, None
-        self._spans.pop("ofrag", None), self._spans.pop("ofrag_off", None)
+        self.with_ofrag, self.ofrag_cap = False, 0
+        for name in ("ofrag", "ofrag_off"):
+            self._spans.pop(name, None), self._tensors.pop(name, None)
         self._enc_cache.clear()
         self._attn_cache.clear()
 

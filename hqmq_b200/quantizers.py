@@ -183,12 +183,12 @@ class HQMQQuantizer(KVQuantizer):
     # ---- compressed representation ---------------------------------------------------------------
     def new_cache(self, B: int, T_cap: int, d_head: int, device, scale_dtype=torch.bfloat16,
                   with_outliers: bool = False, out_dtype=torch.bfloat16, out_cap: Optional[int] = None,
-                  ofrag: bool = False, ofrag_cap: Optional[int] = None, zero: bool = True) -> PackedKV:
+                  ofrag: bool = False, ofrag_cap: Optional[int] = None, zero: bool = True, place: bool = True) -> PackedKV:
         if d_head % 4 != 0:
             raise ValueError(f"d_head={d_head} not divisible by 4")
         return PackedKV(B, self.n_heads, T_cap, d_head // 4, self.secondary_size, self.radius_bits, device,
                         scale_dtype=scale_dtype, with_outliers=with_outliers, out_dtype=out_dtype, out_cap=out_cap,
-                        ofrag=ofrag, ofrag_cap=ofrag_cap, zero=zero)
+                        ofrag=ofrag, ofrag_cap=ofrag_cap, zero=zero, place=place)
 
     def _check_dst(self, x: torch.Tensor, out: PackedKV):
         """The library takes batch, heads and chunks per token from the destination planes: x must have that geometry."""
@@ -305,15 +305,17 @@ class HQMQQuantizer(KVQuantizer):
         """Append the keys and the values of one layer (the reference cache quantises both on every update,
         src/model_utils.py:29-32).  Same result as ``encode(k, layer_idx, 0, out=out_k)`` followed by
         ``encode(v, layer_idx, 1, out=out_v)``; a decode-time append (a few tokens per sequence) runs both tensors
-        in one kernel launch (hqmq_encode_pair) instead of three per tensor."""
+        in one kernel launch (hqmq_encode_pair) instead of three per tensor, a prompt of ordinary length shares each of its
+        launches between them."""
         # (one dictionary look-up on everything that decides the call's shape: a repeated append goes straight to the library)
         shape, ks, vs = k.shape, k.stride(), v.stride()
         key = ("pair", id(self), id(out_v), layer_idx, shape, v.shape, k.dtype, v.dtype, ks, vs, k.device, v.device, median_mult, quantile)
         hit = out_k._enc_cache.get(key)
         if hit is None:
-            small = (k.dim() == 4 and shape == v.shape and k.dtype == v.dtype and shape[2] <= 64 and k.is_cuda and v.is_cuda
-                     and ks[-1] == 1 and vs[-1] == 1 and not any(s % 4 for s in ks[:3] + vs[:3]))
-            if not small or shape[2] == 0:
+            # (beyond 16 M values a tensor's own launches fill the chip, and two workspaces would be held instead of one)
+            paired = (k.dim() == 4 and shape == v.shape and k.dtype == v.dtype and 0 < k.numel() <= 1 << 24 and k.is_cuda and v.is_cuda
+                      and ks[-1] == 1 and vs[-1] == 1 and not any(s % 4 for s in ks[:3] + vs[:3]))
+            if not paired:
                 return (self.encode(k, layer_idx, 0, out=out_k, median_mult=median_mult, quantile=quantile),
                         self.encode(v, layer_idx, 1, out=out_v, median_mult=median_mult, quantile=quantile))
             why = self._unsupported()
@@ -334,7 +336,9 @@ class HQMQQuantizer(KVQuantizer):
             # the tables and V's planes, not this call's inputs (nor out_k, which holds the structs: a cycle would leave the
             # cache's memory to the garbage collector)
             ak._keep, av._keep = (ak._keep[1],), (av._keep[1], out_v)
-            hit = out_k._enc_cache[key] = (ak, av, C.byref(ak), C.byref(av), ws.data_ptr(), nbytes, ws)
+            hit = (ak, av, C.byref(ak), C.byref(av), ws.data_ptr(), nbytes, ws)
+            if shape[2] <= 64:          # (a prompt is not repeated on its cache)
+                out_k._enc_cache[key] = hit
         ak, av, rk, rv, ws_ptr, nbytes, _ = hit
         T, tk, tv = shape[2], out_k.T, out_v.T
         if tk + T > out_k.T_cap or tv + T > out_v.T_cap:
@@ -530,6 +534,34 @@ class _OutlierStats:
         if len(self._open) + len(self._closed) >= self._FOLD:
             self._sync()
 
+    # the same for the two caches of a layer: a repeated append only counts its calls, and the counters of a pair that was
+    # placed together are copied together
+    def begin_pair(self, pk, pv, total_chunks: int):
+        rk, rv = getattr(pk, "_stat_rec", None), getattr(pv, "_stat_rec", None)
+        if rk is not None and rv is not None and rk[2] and rv[2]:
+            if rk[3] == total_chunks and rv[3] == total_chunks:
+                return
+            ck, cv, n = rk[0], rv[0], rk[0].numel()
+            if (rk[3] != total_chunks and rv[3] != total_chunks and ck._base is not None and ck._base is cv._base
+                    and cv.storage_offset() == ck.storage_offset() + n and cv.numel() == n and ck.is_contiguous()):
+                now = _counters.take(2 * n, ck.device)
+                now.copy_(ck.as_strided((2 * n,), (1,)))
+                for rec, c in ((rk, now[:n]), (rv, now[n:])):
+                    self._closed.append((c, rec[1], rec[3], rec[2]))
+                    rec[1], rec[2] = c, 0
+                return
+        self.begin(pk, total_chunks)
+        self.begin(pv, total_chunks)
+
+    def end_pair(self, pk, pv, total_chunks: int):
+        rk, rv = getattr(pk, "_stat_rec", None), getattr(pv, "_stat_rec", None)
+        if rk is not None and rv is not None and rk[2] and rv[2] and len(self._open) + len(self._closed) < self._FOLD:
+            rk[2] += 1
+            rv[2] += 1
+            return
+        self.end(pk, total_chunks)
+        self.end(pv, total_chunks)
+
     def push_count(self, counter: torch.Tensor, total_chunks: int):
         """A finished fake-quant call that went through a cache: only the counter is kept."""
         self._closed.append((counter, 0.0, total_chunks, 1))
@@ -628,14 +660,12 @@ class OutlierAwareHQMQQuantizer(KVQuantizer):
     def encode_pair(self, k, v, layer_idx, out_k: PackedKV, out_v: PackedKV):
         """Keys and values of one layer in one call (see ``HQMQQuantizer.encode_pair``), each with its own median."""
         self._check_mode()
-        total = k.shape[0] * k.shape[1] * k.shape[2] * (k.shape[3] // 4)
-        if total:
-            self._stats.begin(out_k, total)
-            self._stats.begin(out_v, total)
+        total = math.prod(k.shape) // 4
+        if not total:
+            return self.inner.encode_pair(k, v, layer_idx, out_k, out_v, **self._thr())
+        self._stats.begin_pair(out_k, out_v, total)
         pair = self.inner.encode_pair(k, v, layer_idx, out_k, out_v, **self._thr())
-        if total:
-            self._stats.end(out_k, total)
-            self._stats.end(out_v, total)
+        self._stats.end_pair(out_k, out_v, total)
         return pair
 
     def decode(self, packed, layer_idx, kv, **kw):

@@ -225,3 +225,26 @@ def test_one_token_appends_equal_single_tensor_calls(B, H, d, S, br, dtype, outl
         names += ["ofrag", "ofrag_off"] if a.with_ofrag else []
         for name in names:
             assert torch.equal(getattr(a, name), getattr(b, name)), name
+
+
+@pytest.mark.parametrize("B,H,T,d,S,br", [(1, 8, 513, 128, 24, 3), (2, 3, 200, 128, 192, 6), (1, 80, 65, 128, 96, 4),
+                                          (2, 2, 511, 64, 96, 4), (1, 2, 1025, 64, 24, 3)])
+@pytest.mark.parametrize("outliers", [True, False])
+def test_paired_prompts_equal_single_tensor_calls(B, H, T, d, S, br, outliers):
+    """A prompt and a second chunk behind it (up to 32 blocks per head and more, more heads than half of the SMs, rows with
+    padding bits): encode_pair leaves the planes that two single-tensor calls leave."""
+    inner = hqmq.HQMQ(1, H, S, br, device="cuda")
+    q = hqmq.with_outlier_extraction(inner, 3.0) if outliers else inner
+    mk = lambda kv: inner.new_cache(B, 2 * T, d, "cuda", with_outliers=outliers, ofrag=outliers and kv == 0)
+    pair, single = (mk(0), mk(1)), (mk(0), mk(1))
+    for step in range(2):
+        k = make_kv("hot", (B, H, T, d), seed=70 + step, dtype=torch.bfloat16).cuda()
+        v = make_kv("spiky", (B, H, T, d), seed=80 + step, dtype=torch.bfloat16).cuda()
+        q.encode_pair(k, v, 0, pair[0], pair[1])
+        q.encode(k, 0, 0, out=single[0])
+        q.encode(v, 0, 1, out=single[1])
+    for a, b in zip(pair, single):
+        names = ["codes", "rs"] + (["flags", "out_vals", "out_off", "out_count"] if outliers else [])
+        names += ["ofrag", "ofrag_off"] if a.with_ofrag else []
+        for name in names:
+            assert torch.equal(getattr(a, name), getattr(b, name)), name
