@@ -183,24 +183,24 @@ __device__ __forceinline__ bool search_fold24(const float4* __restrict__ joint, 
   if (a3 > am) { am = a3; ax = 3; }
   if (!(am > 0.f)) return false;
   const float hs = ((a0 + a1) + a2) + a3;          // twice the similarity of the nearest half-integer unit
-  int gp; float v0, v1, v2, v3;
-  if (hs > 2.f * am) {
-    // g = (s0, s1, s2, s3) / 2 with s_i = sign(u_i); 2 conj(g) u in terms of the |u_i|
-    const uint32_t b0 = __float_as_uint(u0), b1 = __float_as_uint(u1), b2 = __float_as_uint(u2), b3 = __float_as_uint(u3);
-    gp = 8 + (int)(((b0 >> 31) << 3) | ((b1 >> 31) << 2) | ((b2 >> 31) << 1) | (b3 >> 31));
-    v0 = hs;
-    v1 = xor_sign(a1 - a0, (b0 ^ b1) & 0x80000000u) + xor_sign(a2 - a3, (b2 ^ b3) & 0x80000000u);
-    v2 = xor_sign(a2 - a0, (b0 ^ b2) & 0x80000000u) + xor_sign(a3 - a1, (b1 ^ b3) & 0x80000000u);
-    v3 = xor_sign(a3 - a0, (b0 ^ b3) & 0x80000000u) + xor_sign(a1 - a2, (b1 ^ b2) & 0x80000000u);
-  } else {
-    if (ax == 0) { v0 = u0; v1 = u1; v2 = u2; v3 = u3; }
-    else if (ax == 1) { v0 = u1; v1 = -u0; v2 = u3; v3 = -u2; }
-    else if (ax == 2) { v0 = u2; v1 = -u3; v2 = -u0; v3 = u1; }
-    else { v0 = u3; v1 = u2; v2 = -u1; v3 = -u0; }
-    const bool neg = v0 < 0.f;
-    if (neg) { v0 = -v0; v1 = -v1; v2 = -v2; v3 = -v3; }
-    gp = 2 * ax + (neg ? 1 : 0);
-  }
+  // Both folds are taken and one is selected: the lanes of a warp need either and all four axes, and as branches they were a
+  // quarter of the kernel's instructions (28 BRA, 30 BSSY / BSYNC of 411 per token).
+  // g = (s0, s1, s2, s3) / 2 with s_i = sign(u_i); 2 conj(g) u in terms of the |u_i|
+  const uint32_t b0 = __float_as_uint(u0), b1 = __float_as_uint(u1), b2 = __float_as_uint(u2), b3 = __float_as_uint(u3);
+  const bool half = hs > 2.f * am;
+  const float h1 = xor_sign(a1 - a0, (b0 ^ b1) & 0x80000000u) + xor_sign(a2 - a3, (b2 ^ b3) & 0x80000000u);
+  const float h2 = xor_sign(a2 - a0, (b0 ^ b2) & 0x80000000u) + xor_sign(a3 - a1, (b1 ^ b3) & 0x80000000u);
+  const float h3 = xor_sign(a3 - a0, (b0 ^ b3) & 0x80000000u) + xor_sign(a1 - a2, (b1 ^ b2) & 0x80000000u);
+  // g = the axis of the largest |u_i| with its sign: conj(g) u swaps neighbours (ax & 1), pairs (ax & 2), and signs
+  const bool o = ax & 1, w = ax & 2;
+  const uint32_t q0 = o ? b1 : b0, q1 = o ? b0 : b1, q2 = o ? b3 : b2, q3 = o ? b2 : b3;
+  const uint32_t e0 = w ? q2 : q0, e1 = w ? q3 : q1, e2 = w ? q0 : q2, e3 = w ? q1 : q3;
+  const uint32_t neg = e0 & 0x80000000u, f3 = (uint32_t)ax << 31, f2 = ((uint32_t)ax << 30) & 0x80000000u;
+  const float v0 = half ? hs : am;
+  const float v1 = half ? h1 : __uint_as_float(e1 ^ neg ^ f2 ^ f3);
+  const float v2 = half ? h2 : __uint_as_float(e2 ^ neg ^ f2);
+  const float v3 = half ? h3 : __uint_as_float(e3 ^ neg ^ f3);
+  const int gp = half ? 8 + (int)(((b0 >> 31) << 3) | ((b1 >> 31) << 2) | ((b2 >> 31) << 1) | (b3 >> 31)) : 2 * ax + (int)(neg >> 31);
   const float inv = rcp_approx(v0) * L.hn;
   const int cx = min(L.n - 1, max(0, (int)fmaf(v1, inv, L.hn)));
   const int cy = min(L.n - 1, max(0, (int)fmaf(v2, inv, L.hn)));
@@ -745,13 +745,9 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
     v[2] = bits16_to_float(raw.y & 0xffff, DT); v[3] = bits16_to_float(raw.y >> 16, DT);
     const float nrm = chunk_norm(v);
     const float radius = fmaxf(nrm, 1e-8f);
-    float rmax = radius;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-    {
-      const float other = __shfl_xor_sync(0xffffffffu, rmax, 16);
-      if (!g.pair16) rmax = fmaxf(rmax, other);       // (pairs: each half-warp is a token of its own)
-    }
+    // (radii are positive: their bits order like the values)
+    const float rmax = __uint_as_float(g.pair16 ? __reduce_max_sync(lane & 16 ? 0xffff0000u : 0xffffu, __float_as_uint(radius))
+                                          : __reduce_max_sync(0xffffffffu, __float_as_uint(radius)));
     const float scale = __fdiv_rn(rmax, qmaxf);
     // radius code: the quotient is first taken with an approximate reciprocal; only a lane whose quotient
     // lies close to a rounding boundary repeats it with the IEEE division the contract names

@@ -208,13 +208,9 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
                   bits16_to_float(raw.y >> 16, DT)};
     const float nrm = chunk_norm(v);
     const float radius = fmaxf(nrm, 1e-8f);
-    float rmax = radius;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-    {
-      const float other = __shfl_xor_sync(0xffffffffu, rmax, 16);
-      if (!pair) rmax = fmaxf(rmax, other);
-    }
+    // (radii are positive: their bits order like the values)
+    const float rmax = __uint_as_float(pair ? __reduce_max_sync(lane & 16 ? 0xffff0000u : 0xffffu, __float_as_uint(radius))
+                                          : __reduce_max_sync(0xffffffffu, __float_as_uint(radius)));
     const float scale = __fdiv_rn(rmax, qmaxf);
     // (radius code: see encode_main32_kernel)
     const float quo = radius * rcp_approx(scale);
