@@ -693,7 +693,7 @@ template <int DT, int IB, int RB, bool BR>
 __global__ void __launch_bounds__(kEnc32Threads, 1)
 encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __restrict__ qs_all, hqmq_packed dst,
                      int t_start, uint32_t* __restrict__ hist, Maps24 maps, const float* __restrict__ joint_all,
-                     const unsigned char* __restrict__ lut, Mul24 nmul, int iters,
+                     const unsigned char* __restrict__ lut, Mul24 nmul, int64_t per,
                      const uint32_t* __restrict__ sel_s, BracketArgs br) {
   if (!BR && br.run_if && *br.run_if == 0u) return;
   __shared__ uint32_t s_below, s_rcount;
@@ -707,21 +707,29 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
   uint32_t* sh1 = shist + kHistBins;                                  // [2][kHistBins]: next digit inside the predicted bins
   float4* sjoint = reinterpret_cast<float4*>(sh1 + 2 * kHistBins);    // [24 S], then the look-up table of the head
 
-  const int bh = blockIdx.y;
-  const int h = bh % g.H, b = bh / g.H;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = g.S;
+  const float inv_S = 1.0f / (float)S;
+  uint32_t* myrow = rows + warp * kMaxRowWords;
+  // The tokens of all heads form one sequence, head by head, cut into equal pieces, one per CTA and SM: the tables are
+  // loaded once or twice per CTA, and all SMs finish together.  (Cut per (batch, head), 384 CTAs of 16 x 8 heads x 8192
+  // tokens were 2.6 rounds with a table load and an exit each: 547 us.)
+  const int64_t W = (int64_t)g.B * g.T_new, f1 = min((int64_t)g.H * W, (int64_t)(blockIdx.x + 1) * per);
+  for (int64_t f0 = (int64_t)blockIdx.x * per; f0 < f1;) {
+  const int h = (int)(f0 / W);
+  const int64_t f_end = min(f1, (int64_t)(h + 1) * W);
+  const int w0 = (int)(f0 - (int64_t)h * W), w1 = (int)(f_end - (int64_t)h * W);
+  f0 = f_end;
   for (int i = threadIdx.x; i < S; i += blockDim.x) qs[i] = reinterpret_cast<const float4*>(qs_all)[(int64_t)h * S + i];
   if (hist || BR) for (int i = threadIdx.x; i < 3 * kHistBins; i += blockDim.x) shist[i] = 0;   // shist and sh1
   for (int i = threadIdx.x; i < 24 * S; i += blockDim.x) sjoint[i] = reinterpret_cast<const float4*>(joint_all)[(int64_t)h * 24 * S + i];
   const LutView L = lut_to_smem(lut, h, reinterpret_cast<unsigned char*>(sjoint + 24 * S), nmul);
-  const float inv_S = 1.0f / (float)S;
   // Bins (norm bits 31:21) that a sample of the call says hold the two middle order statistics: their next
   // 11-bit digit is histogrammed here too, which spares a pass over x when the sample was right.
   const uint32_t pb0 = sel_s ? sel_s[h * 8 + 0] >> 21 : 0xffffffffu, pb1 = sel_s ? sel_s[h * 8 + 2] >> 21 : 0xffffffffu;
   uint32_t r_lo = 0u, r_hi = 0u, n_below = 0u, s1 = 0u;
   float thr_lo = 0.f, thr_hi = 0.f;
-  const int region = blockIdx.y * gridDim.x + blockIdx.x;
+  const int region = blockIdx.x + h;              // (the next piece has the next CTA or the next head, or both)
   if constexpr (BR) {
     r_lo = br.bp[h * kBpWords + 0]; r_hi = br.bp[h * kBpWords + 1];
     thr_lo = __uint_as_float(br.bp[h * kBpWords + 2]); thr_hi = __uint_as_float(br.bp[h * kBpWords + 3]);
@@ -730,16 +738,22 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
   }
   __syncthreads();
 
-  uint32_t* myrow = rows + warp * kMaxRowWords;
-  const int t_block0 = blockIdx.x * kEnc32Warps * iters;
-  const uint16_t* xp = x + b * g.xs_b + h * g.xs_h + 4 * lane;
-  int t = t_block0 + warp;
+  // this warp's token w = b * T_new + t of the head, its chunks in x and its row, advanced by kEnc32Warps tokens
+  const int rpt = g.pair16 ? 2 : 1;
+  int w = w0 + warp;
+  int b = w / g.T_new, t = w - b * g.T_new;
+  const uint16_t* xp = x + b * g.xs_b + h * g.xs_h + (int64_t)t * g.xs_t + 4 * lane;
+  int64_t row = ((int64_t)b * g.H + h) * dst.T_cap + t_start + (int64_t)rpt * t;
+  const int64_t xstep = kEnc32Warps * g.xs_t, xwrap = g.xs_b - g.T_new * g.xs_t;
+  const int64_t rwrap = (int64_t)g.H * dst.T_cap - (int64_t)rpt * g.T_new;
   uint2 raw_n = make_uint2(0u, 0u);
-  if (t < g.T_new) raw_n = *reinterpret_cast<const uint2*>(xp + (int64_t)t * g.xs_t);
-  for (int it = 0; it < iters && t < g.T_new; ++it, t += kEnc32Warps) {
+  if (w < w1) raw_n = *reinterpret_cast<const uint2*>(xp);
+  for (int bn = b, tn = t; w < w1; w += kEnc32Warps, b = bn, t = tn) {
     const uint2 raw = raw_n;
-    if (it + 1 < iters && t + kEnc32Warps < g.T_new)
-      raw_n = *reinterpret_cast<const uint2*>(xp + (int64_t)(t + kEnc32Warps) * g.xs_t);
+    const int64_t row_now = row;
+    tn += kEnc32Warps; xp += xstep; row += rpt * kEnc32Warps;
+    while (tn >= g.T_new) { tn -= g.T_new; ++bn; xp += xwrap; row += rwrap; }
+    if (w + kEnc32Warps < w1) raw_n = *reinterpret_cast<const uint2*>(xp);
     float v[4];
     v[0] = bits16_to_float(raw.x & 0xffff, DT); v[1] = bits16_to_float(raw.x >> 16, DT);
     v[2] = bits16_to_float(raw.y & 0xffff, DT); v[3] = bits16_to_float(raw.y >> 16, DT);
@@ -799,8 +813,7 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
     const uint32_t f = ni | ((uint32_t)rqf << IB);
 
     // ---- packed row, scale, flag word ---------------------------------------------------------------------
-    const int64_t row = (int64_t)bh * dst.T_cap + t_start + (g.pair16 ? 2 * t : t);   // (pairs: two rows, contiguous)
-    uint32_t* out = reinterpret_cast<uint32_t*>(dst.codes + row * dst.row_bytes);
+    uint32_t* out = reinterpret_cast<uint32_t*>(dst.codes + row_now * dst.row_bytes);   // (pairs: two rows, contiguous)
     if constexpr (CB == 16) {
       const uint32_t other = __shfl_xor_sync(0xffffffffu, f, 1);
       if (!(lane & 1)) out[lane >> 1] = f | (other << 16);
@@ -816,8 +829,8 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
     }
     if (lane == 0 || (g.pair16 && lane == 16)) {
       const int half = lane >> 4;
-      store_scale(dst, row + half, rmax);
-      if (dst.flags) dst.flags[row + half] = g.pair16 ? (half ? flag_word >> 16 : flag_word & 0xffffu) : flag_word;
+      store_scale(dst, row_now + half, rmax);
+      if (dst.flags) dst.flags[row_now + half] = g.pair16 ? (half ? flag_word >> 16 : flag_word & 0xffffu) : flag_word;
     }
     if (!BR && hist) {
       const uint32_t key = __float_as_uint(nrm), top = key >> 21;
@@ -854,6 +867,8 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
         if (c1) atomicAdd(&g1[kHistBins + i], c1);
       }
     }
+  }
+  __syncthreads();          // the next head's tables and counters replace these
   }
 }
 
@@ -1197,13 +1212,15 @@ list_pickA_kernel(uint32_t* __restrict__ bp, const uint32_t* __restrict__ histA,
   }
 }
 
-// grid = the main pass's grid (one CTA per list region)
+// grid (CTAs of the main pass that can share a head, heads): one CTA per list region
 __global__ void __launch_bounds__(256)
 list_histB_kernel(const uint32_t* __restrict__ bp, const uint32_t* __restrict__ rcnt, const uint32_t* __restrict__ rlist, int rcap,
-                  int H, uint32_t* __restrict__ histB, const uint32_t* __restrict__ gate) {
+                  int64_t per, int64_t W, uint32_t* __restrict__ histB, const uint32_t* __restrict__ gate) {
   if (*gate) return;
-  const int bh = blockIdx.y, h = bh % H;
-  const int region = blockIdx.y * gridDim.x + blockIdx.x;
+  const int h = blockIdx.y;
+  const int64_t cta = h * W / per + blockIdx.x;
+  if (cta > ((h + 1) * W - 1) / per) return;
+  const int region = (int)cta + h;
   const uint32_t r_lo = bp[h * kBpWords + 0], s1 = bp[h * kBpWords + 5];
   const uint32_t bin0 = bp[h * kBpWords + 6], bin1 = bp[h * kBpWords + 7];
   const uint32_t lowmask = (1u << s1) - 1u;
@@ -2036,14 +2053,13 @@ inline size_t lut_ws_bytes(int H) { return (size_t)H * kLutCellCap * 4 + (size_t
 // shared memory a main-pass kernel can give to a table next to its other arrays (fp32 joint table, histograms, rows)
 inline size_t lut_smem_budget(int S) { return (size_t)226 * 1024 - (size_t)24 * S * 16 - (size_t)S * 16 - 3 * kHistBins * 4 - 4096; }
 
-// Geometry of the main pass for the common case (d_head 128, 16-bit input): tokens per CTA and CTAs per (b, h).
-struct MainGrid { int iters, gx; };
+// Geometry of the main pass for the common case (d_head 128, 16-bit input): tokens per CTA, CTAs (one per SM).
+struct MainGrid { int64_t per; int ctas; };
 static MainGrid main_grid(int T_new, int B, int H) {
   MainGrid m;
-  // tokens per CTA: long enough to amortise loading the tables, short enough to fill the machine twice
-  int64_t it = ((int64_t)T_new * B * H + (int64_t)2 * 148 * kEnc32Warps - 1) / ((int64_t)2 * 148 * kEnc32Warps);
-  m.iters = it < 1 ? 1 : it > 128 ? 128 : (int)it;
-  m.gx = (T_new + kEnc32Warps * m.iters - 1) / (kEnc32Warps * m.iters);
+  const int64_t total = (int64_t)T_new * B * H;
+  m.per = (((total + 147) / 148 + kEnc32Warps - 1) / kEnc32Warps) * kEnc32Warps;
+  m.ctas = (int)((total + m.per - 1) / m.per);
   return m;
 }
 // The bracket pass pays when the sample predicts well: the statistic's sampling error falls with the square root of
@@ -2090,8 +2106,8 @@ WsPlan plan_ws(const hqmq_encode_args& a) {
   if (bracket_wanted(a)) {
     const int T32 = pair16_of(a) ? a.T_new / 2 : a.T_new;
     const MainGrid mg = main_grid(T32, a.dst.B, H);
-    w.regions = mg.gx * a.dst.B * H;
-    w.rcap = kEnc32Warps * mg.iters * 32 / 16;        // a sixteenth of a CTA's chunks (the range holds about 2 %)
+    w.regions = mg.ctas + H - 1;
+    w.rcap = (int)(mg.per * 32 / 16);                  // a sixteenth of a CTA's chunks (the range holds about 2 %)
     w.gate = o; o += 4;
     w.bp = o; o += (size_t)H * kBpWords;
     w.histA = o; o += (size_t)H * kHistBins;
@@ -2599,18 +2615,18 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
     const size_t smem_fast = (size_t)g.S * 16 + (size_t)kEnc32Warps * kMaxRowWords * 4 + 3 * kHistBins * 4 + (size_t)24 * g.S * 16 +
                              lut_foot + 16;
     const MainGrid mg = main_grid(T32, d.B, d.H);
-    int iters = mg.iters;
+    int64_t per32 = mg.per;
     if (smem_fast > 48 * 1024) {
       HQMQ_CHECK_CUDA(cudaFuncSetAttribute(fastk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fast));
       HQMQ_CHECK_CUDA(cudaFuncSetAttribute(fastk_br, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fast));
     }
-    dim3 fgrid(mg.gx, d.B * d.H);
+    const dim3 fgrid(mg.ctas);
     // Med3x: a sample of the tokens predicts the threshold statistic.  Two select levels over the sample give it
     // to 22 bits, the bracket pass then needs x only once; should the prediction fail, the multi-pass kernels
     // below (gated on a word the bracket's check raises) redo the call, with the sample's first level telling the
     // main pass which bins to refine.
     predicted = med && !ext_med && fast32 && T32 >= 1024;
-    const bool bracket = predicted && bracket_wanted(*a) && wp.regions == (int)(fgrid.x * fgrid.y);
+    const bool bracket = predicted && bracket_wanted(*a);
     const uint16_t* x16 = reinterpret_cast<const uint16_t*>(a->x);
     const unsigned char* lut_arg = reinterpret_cast<const unsigned char*>(a->lut);
     int t_start_arg = a->t_start;
@@ -2646,11 +2662,13 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
       uint32_t* no_hist = nullptr;
       const uint32_t* no_sel = nullptr;
       void* kargs_b[] = {(void*)&g32, (void*)&x16, (void*)&a->qs, (void*)&d, (void*)&t_start_arg, (void*)&no_hist, (void*)&maps,
-                         (void*)&a->joint, (void*)&lut_arg, (void*)&nmul, (void*)&iters, (void*)&no_sel, (void*)&brargs};
+                         (void*)&a->joint, (void*)&lut_arg, (void*)&nmul, (void*)&per32, (void*)&no_sel, (void*)&brargs};
       HQMQ_CHECK_CUDA(cudaLaunchKernel(fastk_br, fgrid, dim3(kEnc32Threads), kargs_b, smem_fast, st));
       const uint64_t N_all = (uint64_t)d.B * a->T_new * d.n_chunks;
       list_pickA_kernel<<<d.H, 256, 0, st>>>(bp, ws + wp.histA, N_all, a->quantile, ws + wp.gate);
-      list_histB_kernel<<<fgrid, 256, 0, st>>>(bp, ws + wp.rcnt, ws + wp.rlist, wp.rcap, d.H, ws + wp.histB, gate);
+      const int64_t W32 = (int64_t)d.B * T32;
+      const int shares = (int)((W32 - 1 + mg.per - 1) / mg.per) + 1;         // most CTAs that share a head
+      list_histB_kernel<<<dim3(shares, d.H), 256, 0, st>>>(bp, ws + wp.rcnt, ws + wp.rlist, wp.rcap, mg.per, W32, ws + wp.histB, gate);
       list_pickB_kernel<<<d.H, 256, 0, st>>>(bp, ws + wp.histB, N_all, a->median_mult, a->quantile, ws + wp.sel_b, a->med_out, gate);
       int fg = (148 * 32 + d.B * d.H - 1) / (d.B * d.H);
       const int fg_max = (T32 + kF32Tok - 1) / kF32Tok;
@@ -2668,7 +2686,7 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
     const uint32_t* sel_s_arg = predicted ? ws + wp.sel_s : nullptr;
     uint32_t* hist_arg = med && !ext_med ? ws + wp.hist : nullptr;
     void* kargs[] = {(void*)&g32, (void*)&x16, (void*)&a->qs, (void*)&d, (void*)&t_start_arg, (void*)&hist_arg, (void*)&maps,
-                     (void*)&a->joint, (void*)&lut_arg, (void*)&nmul, (void*)&iters, (void*)&sel_s_arg, (void*)&brargs};
+                     (void*)&a->joint, (void*)&lut_arg, (void*)&nmul, (void*)&per32, (void*)&sel_s_arg, (void*)&brargs};
     HQMQ_CHECK_CUDA(cudaLaunchKernel(fastk, fgrid, dim3(kEnc32Threads), kargs, smem_fast, st));
   } else if (use_lut) {
     if (smem_lut > 48 * 1024)
