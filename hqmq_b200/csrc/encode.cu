@@ -27,7 +27,7 @@ constexpr int kEncIters = 8;      // token groups per block
 constexpr int kHistBins = 2048;   // 11-bit digits: bits [31:21], [20:10], then 10 bits [9:0]
 constexpr int kMaxRowWords = 20;
 constexpr int kBandWords = 4;     // per head: thr_lo bits, thr_hi bits, undecided chunks seen, spare
-constexpr int kUndCap = 4096;     // undecided chunks listed per head; more -> the fix-up re-scans x instead
+constexpr int kUndCap = 4096;     // undecided chunks listed per head at least; more -> the fix-up re-scans x instead
 
 // ---- nearest-codeword look-up table -------------------------------------------------------------------
 // The joint codebook {p * q_s} is invariant under left multiplication by any of the 24 Hurwitz units g, so the
@@ -668,34 +668,30 @@ __global__ void __launch_bounds__(kSmallThreads) fake_quant_small_kernel(SmallAr
 // one lane per chunk, no run-time geometry in the loop.  Results are the ones encode_main_kernel gives.
 constexpr int kEnc32Threads = 1024;   // one CTA per SM (the tables fill half of shared memory): 32 warps hide the search latency
 constexpr int kEnc32Warps = kEnc32Threads / 32;
-// Bracket mode (BR): a two-level select over a sample of the tokens has predicted the threshold statistic to a
-// relative 2^-13; the main pass then does everything that needs x in its one read.  Per head, `bp` holds a range
-// [R_lo, R_hi] of norm bits around the predicted statistic (+-1 %) and the bounds thr_lo / thr_hi of the threshold
-// that follow from it.  A chunk above thr_hi is flagged here (radius code 0, bit in the token's flag word), a chunk
-// at or below thr_lo is not, the few in between are listed for the fix-up; the norms inside the range are appended
-// to a list (one region per CTA) and the norms below it are counted, from which list_select_kernel takes the exact
-// order statistics -- and finds out whether the prediction held: if not, it raises the gate word and the
-// multi-pass kernels, which otherwise return at once, redo the call.
+// A two-level select over a sample of the tokens has predicted the threshold statistic to a relative 2^-13; this pass then
+// does everything that needs x in its one read.  Per head, `bp` holds a range [R_lo, R_hi] of norm bits around the predicted
+// statistic (+-1 %) and the bounds thr_lo / thr_hi of the threshold that follow from it.  A chunk above thr_hi is flagged
+// here (radius code 0, bit in the token's flag word), a chunk at or below thr_lo is not, the few in between are listed for
+// the fix-up; the norms inside the range are appended to a list (one region per CTA and head) and the norms below it are
+// counted, from which list_select_kernel takes the exact order statistics -- and finds out whether the prediction held: if
+// not, it raises the gate word and the one-launch encoder, which otherwise returns at once, redoes the call.
 struct BracketArgs {
   const uint32_t* bp;       // [H][8]: R_lo, R_hi, thr_lo, thr_hi (float bits), norms below R_lo, ...
   uint32_t* bp_count;       // same array, for the atomics
   uint32_t* band;           // [H][kBandWords]: word 2 counts the undecided chunks
-  uint32_t* und;            // [H][kUndCap] undecided chunks
+  uint32_t* und;            // [H][und_cap] undecided chunks
   uint32_t* rcnt;           // [regions] norms appended per region (may exceed rcap: the list then overflowed)
   uint32_t* rlist;          // [regions][rcap]
   uint32_t* histA;          // [H][kHistBins] top digit of (norm bits - R_lo) of the norms inside the range
   int rcap, und_cap;
-  const uint32_t* run_if;   // multi-pass (non-bracket) launch: return unless this word is non-zero (nullptr: run)
 };
 constexpr int kBpWords = 16;
 
-template <int DT, int IB, int RB, bool BR>
+template <int DT, int IB, int RB>
 __global__ void __launch_bounds__(kEnc32Threads, 1)
 encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __restrict__ qs_all, hqmq_packed dst,
-                     int t_start, uint32_t* __restrict__ hist, Maps24 maps, const float* __restrict__ joint_all,
-                     const unsigned char* __restrict__ lut, Mul24 nmul, int64_t per,
-                     const uint32_t* __restrict__ sel_s, BracketArgs br) {
-  if (!BR && br.run_if && *br.run_if == 0u) return;
+                     int t_start, Maps24 maps, const float* __restrict__ joint_all, const unsigned char* __restrict__ lut, Mul24 nmul,
+                     int64_t per, BracketArgs br) {
   __shared__ uint32_t s_below, s_rcount;
   constexpr int CB = IB + RB;
   constexpr int RW = 32 * CB / 32;                       // words per row
@@ -704,8 +700,7 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
   float4* qs = reinterpret_cast<float4*>(smem_raw);
   uint32_t* rows = reinterpret_cast<uint32_t*>(qs + g.S);            // [warps][kMaxRowWords]
   uint32_t* shist = rows + kEnc32Warps * kMaxRowWords;                  // [kHistBins]
-  uint32_t* sh1 = shist + kHistBins;                                  // [2][kHistBins]: next digit inside the predicted bins
-  float4* sjoint = reinterpret_cast<float4*>(sh1 + 2 * kHistBins);    // [24 S], then the look-up table of the head
+  float4* sjoint = reinterpret_cast<float4*>(shist + kHistBins);    // [24 S], then the look-up table of the head
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = g.S;
@@ -721,21 +716,14 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
   const int w0 = (int)(f0 - (int64_t)h * W), w1 = (int)(f_end - (int64_t)h * W);
   f0 = f_end;
   for (int i = threadIdx.x; i < S; i += blockDim.x) qs[i] = reinterpret_cast<const float4*>(qs_all)[(int64_t)h * S + i];
-  if (hist || BR) for (int i = threadIdx.x; i < 3 * kHistBins; i += blockDim.x) shist[i] = 0;   // shist and sh1
+  for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) shist[i] = 0;
   for (int i = threadIdx.x; i < 24 * S; i += blockDim.x) sjoint[i] = reinterpret_cast<const float4*>(joint_all)[(int64_t)h * 24 * S + i];
   const LutView L = lut_to_smem(lut, h, reinterpret_cast<unsigned char*>(sjoint + 24 * S), nmul);
-  // Bins (norm bits 31:21) that a sample of the call says hold the two middle order statistics: their next
-  // 11-bit digit is histogrammed here too, which spares a pass over x when the sample was right.
-  const uint32_t pb0 = sel_s ? sel_s[h * 8 + 0] >> 21 : 0xffffffffu, pb1 = sel_s ? sel_s[h * 8 + 2] >> 21 : 0xffffffffu;
-  uint32_t r_lo = 0u, r_hi = 0u, n_below = 0u, s1 = 0u;
-  float thr_lo = 0.f, thr_hi = 0.f;
   const int region = blockIdx.x + h;              // (the next piece has the next CTA or the next head, or both)
-  if constexpr (BR) {
-    r_lo = br.bp[h * kBpWords + 0]; r_hi = br.bp[h * kBpWords + 1];
-    thr_lo = __uint_as_float(br.bp[h * kBpWords + 2]); thr_hi = __uint_as_float(br.bp[h * kBpWords + 3]);
-    s1 = br.bp[h * kBpWords + 5];
-    if (threadIdx.x == 0) { s_below = 0u; s_rcount = 0u; }
-  }
+  const uint32_t r_lo = br.bp[h * kBpWords + 0], r_hi = br.bp[h * kBpWords + 1], s1 = br.bp[h * kBpWords + 5];
+  const float thr_lo = __uint_as_float(br.bp[h * kBpWords + 2]), thr_hi = __uint_as_float(br.bp[h * kBpWords + 3]);
+  uint32_t n_below = 0u;
+  if (threadIdx.x == 0) { s_below = 0u; s_rcount = 0u; }
   __syncthreads();
 
   // this warp's token w = b * T_new + t of the head, its chunks in x and its row, advanced by kEnc32Warps tokens
@@ -769,8 +757,8 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
     float rqf = rintf(quo);
     if (fabsf(quo - rqf) > 0.499f) rqf = rintf(__fdiv_rn(radius, scale));
     rqf = fminf(fmaxf(rqf, 0.f), qmaxf);
-    uint32_t flag_word = 0u;
-    if constexpr (BR) {
+    uint32_t flag_word;
+    {
       const uint32_t key = __float_as_uint(nrm);
       const bool certain = nrm > thr_hi;
       if (certain) rqf = 0.f;                       // a flagged chunk's values live in the side buffer
@@ -832,42 +820,17 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
       store_scale(dst, row_now + half, rmax);
       if (dst.flags) dst.flags[row_now + half] = g.pair16 ? (half ? flag_word >> 16 : flag_word & 0xffffu) : flag_word;
     }
-    if (!BR && hist) {
-      const uint32_t key = __float_as_uint(nrm), top = key >> 21;
-      atomicAdd(&shist[top], 1u);
-      if (top == pb0) atomicAdd(&sh1[(key >> 10) & 0x7ffu], 1u);
-      else if (top == pb1) atomicAdd(&sh1[kHistBins + ((key >> 10) & 0x7ffu)], 1u);
-    }
   }
-  if constexpr (BR) {
-    if (lane == 0 && n_below) atomicAdd(&s_below, n_below);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      if (s_below) atomicAdd(&br.bp_count[h * kBpWords + 4], s_below);
-      br.rcnt[region] = s_rcount;
-      if (s_rcount > (uint32_t)br.rcap) atomicOr(&br.bp_count[h * kBpWords + 10], 1u);
-    }
-    uint32_t* gA = br.histA + (int64_t)h * kHistBins;
-    for (int i = threadIdx.x; i < kHistBins; i += blockDim.x)
-      if (shist[i]) atomicAdd(&gA[i], shist[i]);
+  if (lane == 0 && n_below) atomicAdd(&s_below, n_below);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (s_below) atomicAdd(&br.bp_count[h * kBpWords + 4], s_below);
+    br.rcnt[region] = s_rcount;
+    if (s_rcount > (uint32_t)br.rcap) atomicOr(&br.bp_count[h * kBpWords + 10], 1u);
   }
-  if (!BR && hist) {
-    __syncthreads();
-    uint32_t* gh = hist + (int64_t)h * 3 * 2 * kHistBins;  // level 0, query 0
-    for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) {
-      uint32_t cnt = shist[i];
-      if (cnt) atomicAdd(&gh[i], cnt);
-    }
-    if (sel_s) {
-      uint32_t* g1 = gh + 2 * kHistBins;                   // level 1, both queries
-      const bool same = pb0 == pb1;
-      for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) {
-        const uint32_t c0 = sh1[i], c1 = same ? c0 : sh1[kHistBins + i];
-        if (c0) atomicAdd(&g1[i], c0);
-        if (c1) atomicAdd(&g1[kHistBins + i], c1);
-      }
-    }
-  }
+  uint32_t* gA = br.histA + (int64_t)h * kHistBins;
+  for (int i = threadIdx.x; i < kHistBins; i += blockDim.x)
+    if (shist[i]) atomicAdd(&gA[i], shist[i]);
   __syncthreads();          // the next head's tables and counters replace these
   }
 }
@@ -876,22 +839,14 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
 
 // ---- Med3x: radix select of the two middle order statistics ------------------------------
 // Level 0 histogram (bits 31:21) is accumulated by encode_main_kernel into query slot 0.
-__global__ void __launch_bounds__(256)
-select_kernel(uint32_t* __restrict__ hist, uint32_t* __restrict__ sel, int level, uint64_t N, float C,
-              float* __restrict__ med_out, uint32_t* __restrict__ band, const uint32_t* __restrict__ sel_s,
-              const uint32_t* __restrict__ hist_fb, float quantile, const uint32_t* __restrict__ gate, int gate_want) {
+// One level for head h by a CTA of 256 threads.  The histograms may have been completed by other CTAs of this launch.
+__device__ __forceinline__ void select_level(const uint32_t* hist, uint32_t* sel, int h, int level, uint64_t N, float quantile) {
   __shared__ uint64_t wtot[8];
-  if (gate && (*gate != 0u) != (gate_want != 0)) return;   // (this launch belongs to the other of the two paths)
-
-  const int h = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;   // launched with 256 threads
   uint32_t* st = sel + h * 8;
-  // level 1 with a sampled prediction: the main pass filled the level-1 histograms if the sample named the
-  // right bins, else hist32_kernel filled the fallback ones
-  const bool use_fb = level == 1 && sel_s && !(sel_s[h * 8 + 0] == st[0] && sel_s[h * 8 + 2] == st[2]);
   const QRank qr = quantile_rank(N, quantile);
   const uint64_t lo = qr.lo, hi = qr.hi;
-  uint32_t* hl = hist + ((int64_t)h * 3 + level) * 2 * kHistBins;
+  const uint32_t* hl = hist + ((int64_t)h * 3 + level) * 2 * kHistBins;
   const int shift = level == 0 ? 21 : level == 1 ? 10 : 0;
   const int bins = level == 2 ? 1024 : kHistBins;
   const int per = bins / 256;         // bins per thread: 8 or 4
@@ -899,12 +854,12 @@ select_kernel(uint32_t* __restrict__ hist, uint32_t* __restrict__ sel, int level
     const uint64_t rank = level == 0 ? (q == 0 ? lo : hi) : st[2 * q + 1];
     const uint32_t prefix = level == 0 ? 0u : st[2 * q];
     // level 0 has one histogram (slot 0); deeper levels have one per query
-    const uint32_t* hq = use_fb ? hist_fb + ((int64_t)h * 2 + q) * kHistBins : hl + (level == 0 ? 0 : q * kHistBins);
+    const uint32_t* hq = hl + (level == 0 ? 0 : q * kHistBins);
     uint32_t cnt[8];
 #pragma unroll
     for (int i = 0; i < 8; i += 4) {
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (i < per) v = *reinterpret_cast<const uint4*>(hq + tid * per + i);
+      if (i < per) v = __ldcg(reinterpret_cast<const uint4*>(hq + tid * per + i));
       cnt[i] = v.x; cnt[i + 1] = v.y; cnt[i + 2] = v.z; cnt[i + 3] = v.w;
     }
     uint64_t mine = 0;
@@ -939,16 +894,18 @@ select_kernel(uint32_t* __restrict__ hist, uint32_t* __restrict__ sel, int level
     }
   }
   __syncthreads();
-  if (tid != 0) return;
-  if (level == 1 && band) {
-    // 22 bits of both order statistics are known: a >= prefix_a, b <= prefix_b | 0x3ff, a <= med <= b, and
-    // thr = fl(med * C) is monotone in med, so it lies in [fl(a_lo * C), fl(b_hi * C)]
-    band[h * kBandWords + 0] = __float_as_uint(__fmul_rn(__uint_as_float(st[0]), C));
-    band[h * kBandWords + 1] = __float_as_uint(__fmul_rn(__uint_as_float(st[2] | 0x3ffu), C));
-  }
+}
+__global__ void __launch_bounds__(256)
+select_kernel(const uint32_t* __restrict__ hist, uint32_t* __restrict__ sel, int level, uint64_t N, float C,
+              float* __restrict__ med_out, float quantile) {
+  const int h = blockIdx.x;
+  select_level(hist, sel, h, level, N, quantile);
+  if (threadIdx.x != 0) return;
+  uint32_t* st = sel + h * 8;
+  const QRank qr = quantile_rank(N, quantile);
   if (level == 2) {
     const float a = __uint_as_float(st[0]), b = __uint_as_float(st[2]);
-    float med = hi == lo ? a : quantile_lerp(a, b, qr.w);
+    float med = qr.hi == qr.lo ? a : quantile_lerp(a, b, qr.w);
     const float thr = __fmul_rn(med, C);
     st[4] = st[0]; st[5] = st[2];
     st[6] = __float_as_uint(thr);
@@ -1028,74 +985,28 @@ __device__ __forceinline__ void norms_of_two(const uint4& r, float& n0, float& n
   n0 = chunk_norm(a); n1 = chunk_norm(b);
 }
 
-template <int DT>
-__global__ void __launch_bounds__(256)
-hist32_kernel(Fast32 f, uint32_t* __restrict__ hist, const uint32_t* __restrict__ sel, int level,
-              const uint32_t* __restrict__ sel_s, uint32_t* __restrict__ hist_fb, const uint32_t* __restrict__ gate, int gate_want) {
-  __shared__ uint32_t sh[2][kHistBins];
-  if (gate && (*gate != 0u) != (gate_want != 0)) return;   // (this launch belongs to the other of the two paths)
-
-  const int bh = blockIdx.y;
-  const int h = bh % f.H, b = bh / f.H;
-  // with a sampled prediction this pass is only the fallback: nothing to do when the sample named the right bins
-  if (sel_s && sel_s[h * 8 + 0] == sel[h * 8 + 0] && sel_s[h * 8 + 2] == sel[h * 8 + 2]) return;
-  for (int i = threadIdx.x; i < 2 * kHistBins; i += blockDim.x) (&sh[0][0])[i] = 0;
-  __syncthreads();
-  const uint32_t p0 = sel[h * 8 + 0], p1 = sel[h * 8 + 2];
-  // level 0 (used when the histograms of several GPUs are summed between the levels): nothing is fixed yet; a
-  // norm has sign bit 0 and `sel` starts zeroed, so comparing bit 31 alone lets every key through
-  const int hs = level == 0 ? 31 : level == 1 ? 21 : 10;   // bits already fixed are above hs
-  const int ds = level == 0 ? 21 : level == 1 ? 10 : 0;
-  const uint32_t dm = level == 2 ? 0x3ffu : 0x7ffu;
-  const uint32_t q0 = p0 >> hs, q1 = p1 >> hs;
-  const bool same = q0 == q1;                            // both order statistics share the prefix: one histogram
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l16 = lane & 15;
-  int per = (f.T_new + gridDim.x - 1) / gridDim.x;
-  per = (per + kF32Tok - 1) / kF32Tok * kF32Tok;
-  const int t0 = blockIdx.x * per, t1 = min(f.T_new, t0 + per);
-  const uint16_t* base = f.x + b * f.xs_b + h * f.xs_h + 8 * l16;
-  for (int t = t0 + warp * 2 + (lane >> 4); t < t1; t += kF32Tok) {
-    uint4 r[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (t + 16 * u < t1) r[u] = *reinterpret_cast<const uint4*>(base + (int64_t)(t + 16 * u) * f.xs_t);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (t + 16 * u < t1) {
-        float n[2];
-        norms_of_two<DT>(r[u], n[0], n[1]);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const uint32_t key = __float_as_uint(n[e]);
-          const uint32_t dig = (key >> ds) & dm, top = key >> hs;
-          if (top == q0) atomicAdd(&sh[0][dig], 1u);
-          else if (top == q1) atomicAdd(&sh[1][dig], 1u);
-        }
-      }
-    }
-  }
-  __syncthreads();
-  uint32_t* gh = sel_s ? hist_fb + (int64_t)h * 2 * kHistBins : hist + ((int64_t)h * 3 + level) * 2 * kHistBins;
-  for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) {
-    const uint32_t c0 = sh[0][i], c1 = same ? c0 : sh[1][i];
-    if (c0) atomicAdd(&gh[i], c0);
-    if (c1) atomicAdd(&gh[kHistBins + i], c1);
-  }
-}
-
-// Histogram of every kSampleStride-th token: level 0 (norm bits 31:21) predicts the bins of the two order
-// statistics before the main pass runs; level 1 (bits 20:10 of the sampled norms inside those bins, `sel_s` holding
-// the level-0 result) refines the prediction to 22 bits for the bracket mode of the main pass.
+// Histogram of every kSampleStride-th token, and from it the two order statistics of the sample: level 0 (norm bits 31:21)
+// finds their bins, level 1 (bits 20:10 of the sampled norms inside those) gives them to 22 bits, and the bracket of the
+// main pass with them.  The last CTA of a head to arrive (a ticket, nobody waits) does the select.
+// The order statistics a <= b of the whole call are expected inside [R_lo, R_hi] = [a_s (1 - delta), b_s (1 + delta)], where
+// a_s / b_s are the sample's (low bits 0 / all ones).  The threshold is fl(lerp(a, b, w) * C) with lerp(a, b, w) in [a, b]
+// and fl monotone, so it then lies in [fl(R_lo * C), fl(R_hi * C)].  Whether the expectation held is checked exactly by
+// list_select_kernel.
 constexpr int kSampleStride = 32;
+struct SampleArgs {
+  uint32_t* hist; uint32_t* sel; uint32_t* tickets;     // laid out like the full ones; [H][2] arrivals
+  uint64_t N; float quantile, C, delta;
+  uint32_t* bp; uint32_t* band;
+};
 template <int DT>
-__global__ void __launch_bounds__(256)
-sample32_kernel(Fast32 f, uint32_t* __restrict__ hist_s, int level, const uint32_t* __restrict__ sel_s) {
+__global__ void __launch_bounds__(256) sample32_kernel(Fast32 f, const SampleArgs a, int level) {
   __shared__ uint32_t sh[2][kHistBins];
+  __shared__ uint32_t s_last;
   const int bh = blockIdx.y;
   const int h = bh % f.H, b = bh / f.H;
   for (int i = threadIdx.x; i < 2 * kHistBins; i += blockDim.x) (&sh[0][0])[i] = 0;
   __syncthreads();
-  const uint32_t q0 = level ? sel_s[h * 8 + 0] >> 21 : 0u, q1 = level ? sel_s[h * 8 + 2] >> 21 : 0u;
+  const uint32_t q0 = level ? a.sel[h * 8 + 0] >> 21 : 0u, q1 = level ? a.sel[h * 8 + 2] >> 21 : 0u;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l16 = lane & 15;
   const int n_s = (f.T_new + kSampleStride - 1) / kSampleStride;       // sampled tokens of this (b, h)
   const uint16_t* base = f.x + b * f.xs_b + h * f.xs_h + 8 * l16;
@@ -1113,7 +1024,7 @@ sample32_kernel(Fast32 f, uint32_t* __restrict__ hist_s, int level, const uint32
   }
   __syncthreads();
   // laid out like the full histograms: level 0 has one slot, level 1 one per order statistic
-  uint32_t* gh = hist_s + ((int64_t)h * 3 + level) * 2 * kHistBins;
+  uint32_t* gh = a.hist + ((int64_t)h * 3 + level) * 2 * kHistBins;
   const bool same = q0 == q1;
   for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) {
     const uint32_t c0 = sh[0][i];
@@ -1123,149 +1034,141 @@ sample32_kernel(Fast32 f, uint32_t* __restrict__ hist_s, int level, const uint32
       if (c1) atomicAdd(&gh[kHistBins + i], c1);
     }
   }
-}
-
-// Bracket of the main pass from the sample's two-level select: the order statistics a <= b of the whole call are
-// expected inside [R_lo, R_hi] = [a_s (1 - delta), b_s (1 + delta)], where a_s / b_s are the sample's statistics known to
-// 22 bits (low bits 0 / all ones).  The threshold is fl(lerp(a, b, w) * C) with lerp(a, b, w) in [a, b] and fl
-// monotone, so it then lies in [fl(R_lo * C), fl(R_hi * C)].  Whether the expectation held is checked exactly by
-// list_select_kernel.
-__global__ void bracket_kernel(const uint32_t* __restrict__ sel_s, float C, float delta, int H, uint32_t* __restrict__ bp,
-                               uint32_t* __restrict__ band) {
-  const int h = blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= H) return;
-  const float a_s = __uint_as_float(sel_s[h * 8 + 0]), b_s = __uint_as_float(sel_s[h * 8 + 2] | 0x3ffu);
-  const float r_lo = __fmul_rn(a_s, 1.f - delta), r_hi = __fmul_rn(b_s, 1.f + delta);
-  bp[h * kBpWords + 0] = __float_as_uint(r_lo);
-  bp[h * kBpWords + 1] = __float_as_uint(r_hi);
-  bp[h * kBpWords + 2] = __float_as_uint(__fmul_rn(r_lo, C));
-  bp[h * kBpWords + 3] = __float_as_uint(__fmul_rn(r_hi, C));
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&a.tickets[2 * h + level], 1u) == gridDim.x * (gridDim.y / f.H) - 1u ? 1u : 0u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  select_level(a.hist, a.sel, h, level, a.N, a.quantile);
+  if (level == 0 || threadIdx.x != 0) return;
+  uint32_t* bp = a.bp + h * kBpWords;
+  const float a_s = __uint_as_float(a.sel[h * 8 + 0]), b_s = __uint_as_float(a.sel[h * 8 + 2] | 0x3ffu);
+  const float r_lo = __fmul_rn(a_s, 1.f - a.delta), r_hi = __fmul_rn(b_s, 1.f + a.delta);
+  bp[0] = __float_as_uint(r_lo);
+  bp[1] = __float_as_uint(r_hi);
+  a.band[h * kBandWords + 0] = bp[2] = __float_as_uint(__fmul_rn(r_lo, a.C));
+  a.band[h * kBandWords + 1] = bp[3] = __float_as_uint(__fmul_rn(r_hi, a.C));
   // top digit of (norm bits - R_lo): 2048 bins of 2^s1 keys cover the range (a range wider than 2^22 keys -- a
-  // statistic next to zero -- is left to the multi-pass path)
+  // statistic next to zero -- is left to the one-launch encoder)
   const uint32_t width = __float_as_uint(r_hi) - __float_as_uint(r_lo);
   const int bits = 32 - __clz(width | 1u);
-  bp[h * kBpWords + 5] = (uint32_t)(bits > 11 ? bits - 11 : 0);
-  band[h * kBandWords + 0] = bp[h * kBpWords + 2];
-  band[h * kBandWords + 1] = bp[h * kBpWords + 3];
+  bp[5] = (uint32_t)(bits > 11 ? bits - 11 : 0);
 }
 
-// ---- exact order statistics of a head from what the bracket pass left ------------------------------------------
+// ---- exact order statistics of a head from what the main pass left ---------------------------------------------
 // The pass counted the norms below the range, histogrammed the top digit of (norm bits - R_lo) for the norms inside
-// it (`histA`, 2048 bins of 2^s1 keys each) and listed those norms per CTA region.  list_pickA_kernel checks that both
-// order statistics fall inside the range (else the prediction failed and the gate word is raised) and names the bin
-// of the lower one and the next non-empty bin; list_histB_kernel histograms the low s1 bits of the listed norms
-// of those two bins; list_pickB_kernel then has both statistics exactly and writes the select words of the head
-// (a, b, threshold, statistic) like the last level of select_kernel.
-// bp words: 0 R_lo, 1 R_hi, 2 thr_lo, 3 thr_hi, 4 norms below R_lo, 5 s1, 6 bin of a, 7 next non-empty bin (or ~0),
-// 8 rank of a inside its bin, 9 listed norms before the bin of a, 10 a region overflowed
-template <int NT>
-__device__ __forceinline__ void block_find_rank(const uint32_t* __restrict__ hist, int nbins, uint32_t rank, uint32_t* s_part,
-                                                int& bin, uint32_t& before, int& next_bin) {
-  // hist in shared or global memory; every thread sums its stretch, thread 0 walks the stretch sums
-  const int tid = threadIdx.x, per = (nbins + NT - 1) / NT;
-  uint32_t mine = 0;
-  for (int i = tid * per; i < min(nbins, (tid + 1) * per); ++i) mine += hist[i];
-  s_part[tid] = mine;
+// it (`histA`, 2048 bins of 2^s1 keys each) and listed those norms per region.  Every CTA of list_select_kernel checks that
+// both order statistics of its head fall inside the range (else the prediction failed and the gate word is raised), finds
+// the bin of the lower one and the next non-empty bin, and histograms the low s1 bits of one region's listed norms of
+// those two bins; the last CTA of the head then has both statistics exactly and writes the select words (a, b, threshold,
+// statistic) like the last level of select_kernel.  (As three launches, ranks found by one thread: 20 us.)
+// bp words: 0 R_lo, 1 R_hi, 2 thr_lo, 3 thr_hi, 4 norms below R_lo, 5 s1, 6 arrivals, 10 a region overflowed
+// Bin of `rank` in a histogram of at most 8 * 256 bins, the entries before it and the next non-empty bin (~0: none), by a
+// CTA of 256 threads; s: 11 words.
+__device__ __forceinline__ void block_find_rank(const uint32_t* hist, int nbins, uint32_t rank, uint32_t* s, int& bin,
+                                                uint32_t& before, int& next_bin) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, per = (nbins + 255) / 256;
+  uint32_t c[8], mine = 0u;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int at = tid * per + i;
+    c[i] = i < per && at < nbins ? __ldcg(hist + at) : 0u;
+    mine += c[i];
+  }
+  uint32_t incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+  if (lane == 31) s[warp] = incl;
+  if (tid == 0) { s[8] = (uint32_t)nbins - 1u; s[9] = 0u; s[10] = 0xffffffffu; }
   __syncthreads();
-  if (tid == 0) {
-    uint32_t acc = 0; int t = 0;
-    while (t < NT - 1 && acc + s_part[t] <= rank) acc += s_part[t++];
-    int i = t * per;
-    const int end = min(nbins, (t + 1) * per);
-    while (i < end - 1 && acc + hist[i] <= rank) acc += hist[i++];
-    int nx = i + 1;
-    while (nx < nbins && hist[nx] == 0u) ++nx;
-    s_part[NT] = (uint32_t)i; s_part[NT + 1] = acc; s_part[NT + 2] = nx < nbins ? (uint32_t)nx : 0xffffffffu;
+  uint32_t acc = incl - mine;
+  for (int w = 0; w < warp; ++w) acc += s[w];
+  if (rank >= acc && rank < acc + mine) {
+    bool found = false;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (!found && rank < acc + c[i]) { s[8] = (uint32_t)(tid * per + i); s[9] = acc; found = true; }
+      acc += c[i];
+    }
   }
   __syncthreads();
-  bin = (int)s_part[NT]; before = s_part[NT + 1]; next_bin = (int)s_part[NT + 2];
+  bin = (int)s[8]; before = s[9];
+#pragma unroll
+  for (int i = 7; i >= 0; --i)
+    if (c[i] && tid * per + i > bin) incl = (uint32_t)(tid * per + i), mine = 0xffffffffu;
+  if (mine == 0xffffffffu) atomicMin(&s[10], incl);
+  __syncthreads();
+  next_bin = (int)s[10];
   __syncthreads();
 }
 
+// grid (CTAs of the main pass that can share a head, heads): one CTA per list region
 __global__ void __launch_bounds__(256)
-list_pickA_kernel(uint32_t* __restrict__ bp, const uint32_t* __restrict__ histA, uint64_t N, float quantile,
-                  uint32_t* __restrict__ gate) {
-  __shared__ uint32_t s_part[256 + 4];
-  __shared__ uint32_t s_tot;
-  const int h = blockIdx.x, tid = threadIdx.x;
+list_select_kernel(uint32_t* __restrict__ bp_all, const uint32_t* __restrict__ histA, const uint32_t* __restrict__ rcnt,
+                   const uint32_t* __restrict__ rlist, int rcap, int64_t per, int64_t W, uint32_t* histB, uint64_t N, float C,
+                   float quantile, uint32_t* __restrict__ sel, float* __restrict__ med_out, uint32_t* __restrict__ gate) {
+  __shared__ uint32_t s_w[11], s_tot, s_last;
+  const int h = blockIdx.y, tid = threadIdx.x;
+  const int64_t cta0 = h * W / per, ctas = ((h + 1) * W - 1) / per - cta0 + 1;
+  if ((int64_t)blockIdx.x >= ctas) return;
+  uint32_t* bp = bp_all + h * kBpWords;
   const uint32_t* hA = histA + (int64_t)h * kHistBins;
   if (tid == 0) s_tot = 0u;
   __syncthreads();
   uint32_t mine = 0;
   for (int i = tid; i < kHistBins; i += 256) mine += hA[i];
-  if (mine) atomicAdd(&s_tot, mine);
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if ((tid & 31) == 0 && mine) atomicAdd(&s_tot, mine);
   __syncthreads();
   const QRank qr = quantile_rank(N, quantile);
-  const uint64_t below = bp[h * kBpWords + 4];
-  const bool ok = !bp[h * kBpWords + 10] && bp[h * kBpWords + 5] <= 11u && qr.lo >= below && qr.hi < below + s_tot;
-  if (!ok) {
+  const uint64_t below = bp[4];
+  const uint32_t r_lo = bp[0], s1 = bp[5];
+  if (bp[10] || s1 > 11u || qr.lo < below || qr.hi >= below + s_tot) {
     if (tid == 0) atomicExch(gate, 1u);
     return;
   }
-  int bin, next_bin; uint32_t before;
-  block_find_rank<256>(hA, kHistBins, (uint32_t)(qr.lo - below), s_part, bin, before, next_bin);
-  if (tid == 0) {
-    bp[h * kBpWords + 6] = (uint32_t)bin;
-    bp[h * kBpWords + 7] = (uint32_t)next_bin;
-    bp[h * kBpWords + 8] = (uint32_t)(qr.lo - below) - before;
-    bp[h * kBpWords + 9] = before;
-  }
-}
-
-// grid (CTAs of the main pass that can share a head, heads): one CTA per list region
-__global__ void __launch_bounds__(256)
-list_histB_kernel(const uint32_t* __restrict__ bp, const uint32_t* __restrict__ rcnt, const uint32_t* __restrict__ rlist, int rcap,
-                  int64_t per, int64_t W, uint32_t* __restrict__ histB, const uint32_t* __restrict__ gate) {
-  if (*gate) return;
-  const int h = blockIdx.y;
-  const int64_t cta = h * W / per + blockIdx.x;
-  if (cta > ((h + 1) * W - 1) / per) return;
-  const int region = (int)cta + h;
-  const uint32_t r_lo = bp[h * kBpWords + 0], s1 = bp[h * kBpWords + 5];
-  const uint32_t bin0 = bp[h * kBpWords + 6], bin1 = bp[h * kBpWords + 7];
+  int bin0, bin1; uint32_t before0;
+  block_find_rank(hA, kHistBins, (uint32_t)(qr.lo - below), s_w, bin0, before0, bin1);
+  const uint32_t rank = (uint32_t)(qr.lo - below) - before0;
   const uint32_t lowmask = (1u << s1) - 1u;
+  const int region = (int)(cta0 + blockIdx.x) + h;
   uint32_t c = rcnt[region];
   if (c > (uint32_t)rcap) c = rcap;
   const uint32_t* keys = rlist + (int64_t)region * rcap;
   uint32_t* hB = histB + (int64_t)h * 2 * kHistBins;
   // (the bins hold few keys: straight to the global histograms)
-  for (uint32_t i0 = threadIdx.x; i0 < c; i0 += 4 * 256) {
-    uint32_t k[4];
+  for (uint32_t i0 = tid; i0 < c; i0 += 8 * 256) {
+    uint32_t k[8];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) k[u] = i0 + u * 256 < c ? keys[i0 + u * 256] : 0xffffffffu;
+    for (int u = 0; u < 8; ++u) k[u] = i0 + u * 256 < c ? keys[i0 + u * 256] : 0xffffffffu;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < 8; ++u) {
       if (i0 + u * 256 < c) {
         const uint32_t off = k[u] - r_lo, top = off >> s1;
-        if (top == bin0) atomicAdd(&hB[off & lowmask], 1u);
-        else if (top == bin1) atomicAdd(&hB[kHistBins + (off & lowmask)], 1u);
+        if (top == (uint32_t)bin0) atomicAdd(&hB[off & lowmask], 1u);
+        else if (top == (uint32_t)bin1) atomicAdd(&hB[kHistBins + (off & lowmask)], 1u);
       }
     }
   }
-}
-
-__global__ void __launch_bounds__(256)
-list_pickB_kernel(const uint32_t* __restrict__ bp, const uint32_t* __restrict__ histB, uint64_t N, float C, float quantile,
-                  uint32_t* __restrict__ sel, float* __restrict__ med_out, const uint32_t* __restrict__ gate) {
-  __shared__ uint32_t s_part[256 + 4];
-  if (*gate) return;
-  const int h = blockIdx.x, tid = threadIdx.x;
-  const uint32_t r_lo = bp[h * kBpWords + 0], s1 = bp[h * kBpWords + 5];
-  const uint32_t bin0 = bp[h * kBpWords + 6], bin1 = bp[h * kBpWords + 7], rank = bp[h * kBpWords + 8];
-  const uint32_t* hB = histB + (int64_t)h * 2 * kHistBins;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&bp[6], 1u) == (uint32_t)ctas - 1u ? 1u : 0u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
   const int nb = 1 << s1;
   int bin, next_bin; uint32_t before;
-  block_find_rank<256>(hB, nb, rank, s_part, bin, before, next_bin);
+  block_find_rank(hB, nb, rank, s_w, bin, before, next_bin);
   // smallest key of the next non-empty top bin (the upper statistic when a is the last key of its bin)
   int first1 = 0, dummy_n; uint32_t dummy_b;
-  if (bin1 != 0xffffffffu) block_find_rank<256>(hB + kHistBins, nb, 0u, s_part, first1, dummy_b, dummy_n);
+  if (bin1 != -1) block_find_rank(hB + kHistBins, nb, 0u, s_w, first1, dummy_b, dummy_n);
   if (tid == 0) {
-    const QRank qr = quantile_rank(N, quantile);
-    const uint32_t a_bits = r_lo + (bin0 << s1) + (uint32_t)bin;
+    const uint32_t a_bits = r_lo + ((uint32_t)bin0 << s1) + (uint32_t)bin;
     uint32_t b_bits = a_bits;
-    if (qr.hi != qr.lo && before + hB[bin] <= rank + 1u) {      // the key after a's run of equal keys
-      if (next_bin != -1) b_bits = r_lo + (bin0 << s1) + (uint32_t)next_bin;
-      else b_bits = r_lo + (bin1 << s1) + (uint32_t)first1;      // (pickA made sure the statistic exists in the list)
+    if (qr.hi != qr.lo && before + __ldcg(hB + bin) <= rank + 1u) {      // the key after a's run of equal keys
+      if (next_bin != -1) b_bits = r_lo + ((uint32_t)bin0 << s1) + (uint32_t)next_bin;
+      else b_bits = r_lo + ((uint32_t)bin1 << s1) + (uint32_t)first1;      // (the statistic exists in the list)
     }
     const float a = __uint_as_float(a_bits), b = __uint_as_float(b_bits);
     const float med = qr.hi == qr.lo ? a : quantile_lerp(a, b, qr.w);
@@ -1294,150 +1197,51 @@ __device__ __forceinline__ void flag_late(const hqmq_packed& dst, int64_t row, i
   clear_radius(reinterpret_cast<uint32_t*>(dst.codes + row * dst.row_bytes), c, ib, rbits);
 }
 
-// Last histogram level and the flags in ONE pass over x.  After level 1 the threshold is known to lie in
-// [thr_lo, thr_hi] (a relative width of 2^-13): a chunk above thr_hi is an outlier whatever the last ten
-// bits of the median turn out to be, a chunk at or below thr_lo is not, and the (normally empty) set in
-// between is listed for fixup_list_kernel; if the list overflows, fixup_scan_kernel re-reads x for that head.
-// A flagged chunk is stored in the side buffer: its radius code in the packed row becomes 0 so that decoding
-// the row contributes nothing for it.
+// The undecided chunks of a head against the exact threshold, kFixupCtas CTAs per head: the listed ones, or, when the list
+// overflowed, x is read again and every chunk between the two bounds settled.
+constexpr int kFixupCtas = 32;
 template <int DT>
 __global__ void __launch_bounds__(256)
-histflags32_kernel(Fast32 f, hqmq_packed dst, int t_start, int ib, int rbits, uint32_t* __restrict__ hist,
-                   const uint32_t* __restrict__ sel, uint32_t* __restrict__ band, uint32_t* __restrict__ und,
-                   const uint32_t* __restrict__ gate, int gate_want) {
-  __shared__ uint32_t sh[2][1024];
-  if (gate && (*gate != 0u) != (gate_want != 0)) return;   // (this launch belongs to the other of the two paths)
-
-  const int bh = blockIdx.y;
-  const int h = bh % f.H, b = bh / f.H;
-  for (int i = threadIdx.x; i < 2 * 1024; i += blockDim.x) (&sh[0][0])[i] = 0;
-  __syncthreads();
-  const uint32_t q0 = sel[h * 8 + 0] >> 10, q1 = sel[h * 8 + 2] >> 10;
-  const bool same = q0 == q1;
-  const float thr_lo = __uint_as_float(band[h * kBandWords + 0]), thr_hi = __uint_as_float(band[h * kBandWords + 1]);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l16 = lane & 15;
-  int per = (f.T_new + gridDim.x - 1) / gridDim.x;
-  per = (per + kF32Tok - 1) / kF32Tok * kF32Tok;
-  const int t0 = blockIdx.x * per, t1 = min(f.T_new, t0 + per);
-  const uint16_t* base = f.x + b * f.xs_b + h * f.xs_h + 8 * l16;
-  const bool cb16 = ib + rbits == 16;
-  const uint32_t rmask16 = (0xffffu >> ib) << ib;             // radius bits of a 16-bit field
-  for (int tb = t0 + warp * 2; tb < t1; tb += kF32Tok) {      // warp-uniform trip count: the halves shuffle below
-    const int t = tb + (lane >> 4);
-    uint4 r[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (t + 16 * u < t1) r[u] = *reinterpret_cast<const uint4*>(base + (int64_t)(t + 16 * u) * f.xs_t);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int tu = t + 16 * u;
-      const bool live = tu < t1;
-      uint32_t m = 0;
-      if (live) {
-        float n[2];
-        norms_of_two<DT>(r[u], n[0], n[1]);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const uint32_t key = __float_as_uint(n[e]);
-          const uint32_t top = key >> 10;
-          if (top == q0) atomicAdd(&sh[0][key & 0x3ffu], 1u);
-          else if (top == q1) atomicAdd(&sh[1][key & 0x3ffu], 1u);
-          if (n[e] > thr_hi) m |= 1u << e;
-          else if (n[e] > thr_lo) {
-            const uint32_t pos = atomicAdd(&band[h * kBandWords + 2], 1u);
-            const int c32 = 2 * l16 + e;
-            if (pos < (uint32_t)kUndCap)
-              und[(int64_t)h * kUndCap + pos] =
-                  f.pair ? (uint32_t)(((int64_t)b * (2 * f.T_new) + 2 * tu + (c32 >> 4)) * 32 + (c32 & 15))
-                         : (uint32_t)(((int64_t)b * f.T_new + tu) * 32 + c32);
-          }
-        }
-      }
-      // the token's flag word: OR of the 16 lanes that share it (bits 2*l16 and 2*l16 + 1 each)
-      uint32_t word = m << (2 * l16);
-      word |= __shfl_xor_sync(0xffffffffu, word, 1);
-      word |= __shfl_xor_sync(0xffffffffu, word, 2);
-      word |= __shfl_xor_sync(0xffffffffu, word, 4);
-      word |= __shfl_xor_sync(0xffffffffu, word, 8);
-      if (live) {
-        const int64_t row = (int64_t)bh * dst.T_cap + t_start + (f.pair ? 2 * tu : tu);   // (pairs: two contiguous rows)
-        if (m) {
-          uint32_t* rowp = reinterpret_cast<uint32_t*>(dst.codes + row * dst.row_bytes);
-          if (cb16) {
-            // 16-bit fields: both chunks of this lane live in word l16 of the row, one atomic clears either or both
-            atomicAnd(&rowp[l16], ~(((m & 1u) ? rmask16 : 0u) | ((m & 2u) ? rmask16 << 16 : 0u)));
-          } else {
-            if (m & 1u) clear_radius(rowp, 2 * l16, ib, rbits);
-            if (m & 2u) clear_radius(rowp, 2 * l16 + 1, ib, rbits);
-          }
-        }
-        if (l16 == 0) {
-          if (f.pair) { dst.flags[row] = word & 0xffffu; dst.flags[row + 1] = word >> 16; }
-          else dst.flags[row] = word;
-        }
-      }
-    }
-  }
-  __syncthreads();
-  uint32_t* gh = hist + ((int64_t)h * 3 + 2) * 2 * kHistBins;
-  for (int i = threadIdx.x; i < 1024; i += blockDim.x) {
-    const uint32_t c0 = sh[0][i], c1 = same ? c0 : sh[1][i];
-    if (c0) atomicAdd(&gh[i], c0);
-    if (c1) atomicAdd(&gh[kHistBins + i], c1);
-  }
-}
-
-// The undecided chunks of one head against the exact threshold (one CTA per head).
-template <int DT>
-__global__ void __launch_bounds__(256)
-fixup_list_kernel(Fast32 f, hqmq_packed dst, int t_start, int ib, int rbits, const uint32_t* __restrict__ sel,
-                  const uint32_t* __restrict__ band, const uint32_t* __restrict__ und, const uint32_t* __restrict__ gate,
-                  int gate_want, int und_cap) {
-  if (gate && (*gate != 0u) != (gate_want != 0)) return;   // (this launch belongs to the other of the two paths)
-  const int h = blockIdx.x;
+fixup_kernel(Fast32 f, hqmq_packed dst, int t_start, int ib, int rbits, int B, const uint32_t* __restrict__ sel,
+             const uint32_t* __restrict__ band, const uint32_t* __restrict__ und, const uint32_t* __restrict__ gate, int und_cap) {
+  if (*gate) return;                  // (the one-launch encoder redoes the call)
+  const int h = blockIdx.y;
   const uint32_t n = band[h * kBandWords + 2];
-  if (n == 0 || n > (uint32_t)und_cap) return;
+  if (n == 0) return;
   const float thr = __uint_as_float(sel[h * 8 + 6]);
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const uint32_t e = und[(int64_t)h * und_cap + i];
-    const int c = e & 31;
-    const int64_t bt = e >> 5;
-    const int b = (int)(bt / f.T_new), t = (int)(bt - (int64_t)b * f.T_new);
-    const uint2 raw = *reinterpret_cast<const uint2*>(f.x + b * f.xs_b + h * f.xs_h + (int64_t)t * f.xs_t + 4 * c);
-    float v[4];
-    v[0] = bits16_to_float(raw.x & 0xffff, DT); v[1] = bits16_to_float(raw.x >> 16, DT);
-    v[2] = bits16_to_float(raw.y & 0xffff, DT); v[3] = bits16_to_float(raw.y >> 16, DT);
-    if (chunk_norm(v) > thr) flag_late(dst, ((int64_t)b * f.H + h) * dst.T_cap + t_start + t, c, ib, rbits);
+  if (n <= (uint32_t)und_cap) {
+    const int tokens = f.pair ? 2 * f.T_new : f.T_new;
+    const int64_t xs_t = f.pair ? f.xs_t / 2 : f.xs_t;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+      const uint32_t e = und[(int64_t)h * und_cap + i];
+      const int c = e & 31;
+      const int64_t bt = e >> 5;
+      const int b = (int)(bt / tokens), t = (int)(bt - (int64_t)b * tokens);
+      const uint2 raw = *reinterpret_cast<const uint2*>(f.x + b * f.xs_b + h * f.xs_h + (int64_t)t * xs_t + 4 * c);
+      float v[4];
+      v[0] = bits16_to_float(raw.x & 0xffff, DT); v[1] = bits16_to_float(raw.x >> 16, DT);
+      v[2] = bits16_to_float(raw.y & 0xffff, DT); v[3] = bits16_to_float(raw.y >> 16, DT);
+      if (chunk_norm(v) > thr) flag_late(dst, ((int64_t)b * f.H + h) * dst.T_cap + t_start + t, c, ib, rbits);
+    }
+    return;
   }
-}
-
-// Fallback when a head's list overflowed: re-read x and settle every chunk between the two bounds.
-template <int DT>
-__global__ void __launch_bounds__(256)
-fixup_scan_kernel(Fast32 f, hqmq_packed dst, int t_start, int ib, int rbits, const uint32_t* __restrict__ sel,
-                  const uint32_t* __restrict__ band, const uint32_t* __restrict__ gate, int gate_want, int und_cap) {
-  if (gate && (*gate != 0u) != (gate_want != 0)) return;   // (this launch belongs to the other of the two paths)
-  const int bh = blockIdx.y;
-  const int h = bh % f.H, b = bh / f.H;
-  if (band[h * kBandWords + 2] <= (uint32_t)und_cap) return;
-  const float thr = __uint_as_float(sel[h * 8 + 6]);
   const float thr_lo = __uint_as_float(band[h * kBandWords + 0]), thr_hi = __uint_as_float(band[h * kBandWords + 1]);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l16 = lane & 15;
-  int per = (f.T_new + gridDim.x - 1) / gridDim.x;
-  per = (per + kF32Tok - 1) / kF32Tok * kF32Tok;
-  const int t0 = blockIdx.x * per, t1 = min(f.T_new, t0 + per);
-  const uint16_t* base = f.x + b * f.xs_b + h * f.xs_h + 8 * l16;
-  for (int t = t0 + warp * 2 + (lane >> 4); t < t1; t += 16) {
-    const uint4 r = *reinterpret_cast<const uint4*>(base + (int64_t)t * f.xs_t);
-    float n[2];
-    norms_of_two<DT>(r, n[0], n[1]);
+  for (int b = 0; b < B; ++b) {
+    const uint16_t* base = f.x + b * f.xs_b + h * f.xs_h + 8 * l16;
+    const int64_t row0 = ((int64_t)b * f.H + h) * dst.T_cap + t_start;
+    for (int t = blockIdx.x * 16 + warp * 2 + (lane >> 4); t < f.T_new; t += gridDim.x * 16) {
+      const uint4 r = *reinterpret_cast<const uint4*>(base + (int64_t)t * f.xs_t);
+      float nv[2];
+      norms_of_two<DT>(r, nv[0], nv[1]);
 #pragma unroll
-    for (int e = 0; e < 2; ++e)
-      if (n[e] > thr_lo && !(n[e] > thr_hi) && n[e] > thr) {
-        const int c32 = 2 * l16 + e;
-        if (f.pair) flag_late(dst, (int64_t)bh * dst.T_cap + t_start + 2 * t + (c32 >> 4), c32 & 15, ib, rbits);
-        else flag_late(dst, (int64_t)bh * dst.T_cap + t_start + t, c32, ib, rbits);
-      }
+      for (int e = 0; e < 2; ++e)
+        if (nv[e] > thr_lo && !(nv[e] > thr_hi) && nv[e] > thr) {
+          const int c32 = 2 * l16 + e;
+          if (f.pair) flag_late(dst, row0 + 2 * t + (c32 >> 4), c32 & 15, ib, rbits);
+          else flag_late(dst, row0 + t, c32, ib, rbits);
+        }
+    }
   }
 }
 
@@ -2082,11 +1886,11 @@ static bool bracket_wanted(const hqmq_encode_args& a) {
 }
 
 struct WsPlan {
-  size_t status, hist, sel, band, und, hist_s, sel_s, hist_fb, gate, bp, histA, histB, band_b, und_b, sel_b, rcnt, rlist, zero_bytes, total;
-  int blk0, nblk, rcap, regions, und_cap;
+  size_t status, hist, sel, hist_s, sel_s, tickets, gate, bp, histA, histB, band, und, sel_b, rcnt, rlist, zero_bytes, total;
+  int blk0, nblk, rcap, und_cap;
 };
 WsPlan plan_ws(const hqmq_encode_args& a) {
-  WsPlan w;
+  WsPlan w = {};
   const int H = a.dst.H;
   w.blk0 = a.t_start / HQMQ_OUT_BLOCK;
   w.nblk = a.T_new > 0 ? (a.t_start + a.T_new - 1) / HQMQ_OUT_BLOCK - w.blk0 + 1 : 0;
@@ -2094,34 +1898,28 @@ WsPlan plan_ws(const hqmq_encode_args& a) {
   w.status = o; o += 4;
   w.hist = o; o += (size_t)H * 3 * 2 * kHistBins;
   w.sel = o; o += (size_t)H * 8;
-  w.band = o; o += (size_t)H * kBandWords;
-  w.und = o; o += (size_t)H * kUndCap;
-  w.hist_s = o; o += (size_t)H * 3 * 2 * kHistBins;   // sampled histograms (level-0 slot used)
-  w.sel_s = o; o += (size_t)H * 8;
-  w.hist_fb = o; o += (size_t)H * 2 * kHistBins;      // level 1 when the sample mispredicted
-  // bracket mode of the main pass (reserved whenever the call could take it)
-  w.gate = w.bp = w.histA = w.histB = w.band_b = w.und_b = w.sel_b = w.rcnt = w.rlist = 0;
-  w.rcap = w.regions = w.und_cap = 0;
   w.zero_bytes = o * sizeof(uint32_t);
   if (bracket_wanted(a)) {
     const int T32 = pair16_of(a) ? a.T_new / 2 : a.T_new;
     const MainGrid mg = main_grid(T32, a.dst.B, H);
-    w.regions = mg.ctas + H - 1;
+    const int regions = mg.ctas + H - 1;
     w.rcap = (int)(mg.per * 32 / 16);                  // a sixteenth of a CTA's chunks (the range holds about 2 %)
+    w.hist_s = o; o += (size_t)H * 3 * 2 * kHistBins;   // the sample's histograms (two levels)
+    w.sel_s = o; o += (size_t)H * 8;
+    w.tickets = o; o += ((size_t)H * 2 + 3) & ~(size_t)3;
     w.gate = o; o += 4;
     w.bp = o; o += (size_t)H * kBpWords;
     w.histA = o; o += (size_t)H * kHistBins;
     w.histB = o; o += (size_t)H * 2 * kHistBins;
-    w.band_b = o; o += (size_t)H * kBandWords;
+    w.band = o; o += (size_t)H * kBandWords;
     w.sel_b = o; o += (size_t)H * 8;
-    w.rcnt = o; o += (size_t)w.regions;
+    w.rcnt = o; o += (size_t)regions;
     w.zero_bytes = o * sizeof(uint32_t);              // everything up to here starts at zero; the lists need not
-    // the undecided list: the bracket is wider than the multi-pass path's band (a few per mille of the chunks of a
-    // head with many outliers fall inside it)
+    // (a few per mille of the chunks of a head with many outliers fall inside the bracket)
     const int64_t per_head = (int64_t)a.dst.B * T32 * 32;
     w.und_cap = (int)(per_head / 256 > kUndCap ? (per_head / 256 < (1 << 20) ? per_head / 256 : (1 << 20)) : kUndCap);
-    w.und_b = o; o += (size_t)H * w.und_cap;
-    w.rlist = o; o += (size_t)w.regions * w.rcap;
+    w.und = o; o += (size_t)H * w.und_cap;
+    w.rlist = o; o += (size_t)regions * w.rcap;
   }
   w.total = o * sizeof(uint32_t);
   return w;
@@ -2271,8 +2069,7 @@ extern "C" int hqmq_med3x_select(int H, int level, uint64_t n_total, float media
   if ((uintptr_t)state & 15) return HQMQ_ERR_ALIGN;
   uint32_t* hist = reinterpret_cast<uint32_t*>(state);
   uint32_t* sel = hist + (size_t)H * 3 * 2 * kHistBins;
-  select_kernel<<<H, 256, 0, (cudaStream_t)stream>>>(hist, sel, level, n_total, median_mult, level == 2 ? med_out : nullptr,
-                                                     nullptr, nullptr, nullptr, 0.f, nullptr, 0);
+  select_kernel<<<H, 256, 0, (cudaStream_t)stream>>>(hist, sel, level, n_total, median_mult, level == 2 ? med_out : nullptr, 0.f);
   HQMQ_LAUNCH_CHECK();
   return HQMQ_OK;
 }
@@ -2332,15 +2129,28 @@ static int sm_count() {
   }
   return n;
 }
+// Shared-memory bytes of the largest head's table, from hqmq_encode_lut_footprint (0 = unknown: the largest a table can be).
+static size_t lut_foot_of(const hqmq_encode_args* a) {
+  return a->lut_footprint > 0 ? ((size_t)a->lut_footprint + 15) & ~(size_t)15 : lut_smem_bytes(kLutNMax, kLutCellCap, kLutCandCap);
+}
 static bool fused_call(const hqmq_encode_args* a) {
   const hqmq_packed& d = a->dst;
   const int ib = idx_bits_for(d.S), rb = d.radius_bits;
-  const bool layout = (ib == 10 && rb == 3) || (ib == 12 && rb == 4) || (ib == 13 && rb == 6);
   // (two 64-wide tokens per warp need rows of whole words, which 16-bit fields give)
   const bool geom = d.n_chunks == 32 || (d.n_chunks == 16 && ib + rb == 16);
-  if (!layout || !geom || !is_half_dtype(a->x_dtype) || a->search != 0 || !a->lut || a->lut_footprint <= 0 || ((uintptr_t)a->lut & 15)) return false;
-  if (d.H > sm_count() || (uint64_t)d.B * a->T_new * d.n_chunks >= ((uint64_t)1 << 32)) return false;
-  return fused_smem_bytes(d.S, ((size_t)a->lut_footprint + 15) & ~(size_t)15) <= (size_t)226 * 1024;
+  if (!geom || ib < 1 || ib + rb > kMaxRowWords || !is_half_dtype(a->x_dtype) || a->search != 0 || !a->lut || a->lut_footprint <= 0 || ((uintptr_t)a->lut & 15)) return false;
+  if ((uint64_t)d.B * a->T_new * d.n_chunks >= ((uint64_t)1 << 32)) return false;
+  return fused_smem_bytes(d.S, lut_foot_of(a)) <= (size_t)226 * 1024;
+}
+// Calls for the one-read main pass: token rows on 16-byte boundaries, and the one-launch encoder able to take over where the
+// prediction fails.
+static bool common_layout(const hqmq_encode_args* a) {
+  const int ib = idx_bits_for(a->dst.S), rb = a->dst.radius_bits;
+  return (ib == 10 && rb == 3) || (ib == 12 && rb == 4) || (ib == 13 && rb == 6);
+}
+static bool bracket_call(const hqmq_encode_args* a) {
+  return bracket_wanted(*a) && common_layout(a) && fused_call(a) && ((uintptr_t)a->x & 15) == 0 && a->x_stride[0] % 8 == 0 && a->x_stride[1] % 8 == 0 &&
+         a->x_stride[2] % 8 == 0;
 }
 static void fill_fused(const hqmq_encode_args* a, int tensors, uint32_t* status, uint32_t* hist, uint32_t* bars, void* out, uint32_t* n_flagged,
                        FusedArgs& f) {
@@ -2350,12 +2160,14 @@ static void fill_fused(const hqmq_encode_args* a, int tensors, uint32_t* status,
   f.lut = reinterpret_cast<const unsigned char*>(a->lut);
   f.dst = d; f.t_start = a->t_start; f.out = reinterpret_cast<uint16_t*>(out); f.n_flagged = n_flagged;
   f.C = a->median_mult; f.quantile = a->quantile; f.med_in = a->med_in; f.med_out = a->med_out;
-  f.hist = hist; f.bars = bars; f.status = status;
-  // (64-wide tokens outside the paired geometry used to run the generic kernels: the same near-ties are kept)
-  f.rcp_rn = d.n_chunks == 16 && !(pair16_of(*a) && ((uintptr_t)a->x & 15) == 0 && a->x_stride[0] % 8 == 0 && a->x_stride[1] % 8 == 0);
+  f.hist = hist; f.bars = bars; f.status = status; f.gate = nullptr;
+  // (the near-ties of the generic kernels, which divide with the rounded reciprocal, are kept where those used to run: other
+  //  field widths, 64-wide tokens outside the paired geometry)
+  f.rcp_rn = !common_layout(a) || (d.n_chunks == 16 && !(pair16_of(*a) && ((uintptr_t)a->x & 15) == 0 && a->x_stride[0] % 8 == 0 && a->x_stride[1] % 8 == 0));
   // one CTA per SM in all, no fewer than a round of its warps each
   const int64_t W = (int64_t)d.B * (d.n_chunks == 16 ? (a->T_new + 1) / 2 : a->T_new);
   int64_t cph = sm_count() / (tensors * d.H);
+  if (cph < 1) cph = 1;                 // (a CTA per head meets nobody: any number of them)
   if (cph > (W + kEnc32Warps - 1) / kEnc32Warps) cph = (W + kEnc32Warps - 1) / kEnc32Warps;
   f.per = (int)((W + cph - 1) / cph);
   f.cph = (int)((W + f.per - 1) / f.per);
@@ -2371,6 +2183,9 @@ static int launch_fused(const FusedPair& f, int tensors, int x_dtype, size_t lut
               : (h16 ? (const void*)&encode_fused_kernel<HQMQ_F16, IB_, RB_, false> : (const void*)&encode_fused_kernel<HQMQ_BF16, IB_, RB_, false>);
   HQMQ_PICK(10, 3) HQMQ_PICK(12, 4) HQMQ_PICK(13, 6)
 #undef HQMQ_PICK
+  if (!k)
+    k = dense ? (h16 ? (const void*)&encode_fused_kernel<HQMQ_F16, 0, 0, true> : (const void*)&encode_fused_kernel<HQMQ_BF16, 0, 0, true>)
+              : (h16 ? (const void*)&encode_fused_kernel<HQMQ_F16, 0, 0, false> : (const void*)&encode_fused_kernel<HQMQ_BF16, 0, 0, false>);
   const size_t smem = fused_smem_bytes(g.S, (lut_foot + 15) & ~(size_t)15);
   HQMQ_CHECK_CUDA(attn::raise_smem_limit(k, smem));
   Maps24 maps;
@@ -2390,6 +2205,9 @@ static int launch_side(const SidePair& sp, int tensors, bool med, cudaStream_t s
   const int bh = a.dst.B * a.dst.H;
   if (a.nblk <= kScanSmallBlocks) {
     side_small_kernel<<<dim3(bh, tensors), 32 * (med ? a.nblk : 1), 0, st>>>(sp, med ? 1 : 0);
+  } else if (tensors == 1) {        // (arguments picked by blockIdx cost the side kernel a quarter of its time)
+    scan_kernel<<<bh, kScanWarps * 32, 0, st>>>(a.dst, a.t_start, a.T_new, a.blk0, a.nblk, a.payload, a.status);
+    if (med) side_kernel<<<dim3((a.nblk + 7) / 8, bh), 256, 0, st>>>(a.g, a.x, a.dst, a.t_start, a.blk0, a.nblk);
   } else {
     scan_pair_kernel<<<dim3(bh, tensors), kScanWarps * 32, 0, st>>>(sp);
     if (med) side_pair_kernel<<<dim3((a.nblk + 7) / 8, bh, tensors), 256, 0, st>>>(sp);
@@ -2452,7 +2270,7 @@ extern "C" int hqmq_fake_quant(const hqmq_encode_args* a, void* out, uint32_t* n
   if (a->median_mult > 0.f && !a->med_in) HQMQ_CHECK_CUDA(cudaMemsetAsync(ws, 0, fake_quant_ws_words(d.H) * 4, st));
   FusedPair f;
   fill_fused(a, 1, ws, hist, bars, out, n_flagged, f.t[0]);
-  return launch_fused(f, 1, a->x_dtype, (size_t)a->lut_footprint, st);
+  return launch_fused(f, 1, a->x_dtype, lut_foot_of(a), st);
 }
 
 extern "C" size_t hqmq_encode_pair_workspace_bytes(const hqmq_encode_args* k, const hqmq_encode_args* v) {
@@ -2476,7 +2294,7 @@ extern "C" int hqmq_encode_pair(const hqmq_encode_args* k, const hqmq_encode_arg
   if (!same || k->T_new == 0 || !small_call(k) || !small_call(v) || plan_ws(*k).nblk > kScanSmallBlocks ||
       plan_ws(*v).nblk > kScanSmallBlocks) {
     const bool med = k->median_mult > 0.f;
-    if (same && k->T_new > 0 && !small_call(k) && fused_call(k) && fused_call(v) && !bracket_wanted(*k) && !bracket_wanted(*v) &&
+    if (same && k->T_new > 0 && !small_call(k) && fused_call(k) && fused_call(v) && !bracket_call(k) && !bracket_call(v) &&
         2 * dk.H <= sm_count() && dk.S == dv.S && dk.radius_bits == dv.radius_bits && k->x_dtype == v->x_dtype &&
         med == (v->median_mult > 0.f) && !k->med_in == !v->med_in && plan_ws(*k).nblk == plan_ws(*v).nblk) {
       // a prompt of ordinary length: both tensors in each launch
@@ -2487,7 +2305,7 @@ extern "C" int hqmq_encode_pair(const hqmq_encode_args* k, const hqmq_encode_arg
       FusedPair f;
       fill_fused(k, 2, sk + pk.status, sk + pk.hist, sk + pk.sel, nullptr, nullptr, f.t[0]);
       fill_fused(v, 2, sv + pv.status, sv + pv.hist, sv + pv.sel, nullptr, nullptr, f.t[1]);
-      rc = launch_fused(f, 2, k->x_dtype, (size_t)(k->lut_footprint > v->lut_footprint ? k->lut_footprint : v->lut_footprint), st);
+      rc = launch_fused(f, 2, k->x_dtype, lut_foot_of(k) > lut_foot_of(v) ? lut_foot_of(k) : lut_foot_of(v), st);
       if (rc || !(med || dk.ofrag || dv.ofrag)) return rc;
       SidePair sp;
       sp.t[0] = side_args(k, pk, sk); sp.t[1] = side_args(v, pv, sv);
@@ -2557,159 +2375,103 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
     HQMQ_LAUNCH_CHECK();
     return HQMQ_OK;
   }
-  if (fused_call(a) && !bracket_wanted(*a)) {
+  const bool bracket = bracket_call(a);
+  if (fused_call(a) && !bracket) {
     // (status, histograms and select words are the first part of the workspace; the select words serve as arrival counters)
     HQMQ_CHECK_CUDA(cudaMemsetAsync(ws, 0, (wp.sel + (size_t)d.H * 8) * sizeof(uint32_t), st));
     FusedPair f;
     fill_fused(a, 1, ws + wp.status, ws + wp.hist, ws + wp.sel, nullptr, nullptr, f.t[0]);
-    rc = launch_fused(f, 1, a->x_dtype, (size_t)a->lut_footprint, st);
+    rc = launch_fused(f, 1, a->x_dtype, lut_foot_of(a), st);
     if (rc || !(med || d.ofrag)) return rc;
     SidePair sp;
     sp.t[0] = side_args(a, wp, ws);
     return launch_side(sp, 1, med, st);
   }
   HQMQ_CHECK_CUDA(cudaMemsetAsync(ws, 0, wp.zero_bytes, st));
+  const uint64_t N = (uint64_t)d.B * a->T_new * d.n_chunks;
+  const Mul24& nmul = mul24_native();
+  const bool h16 = a->x_dtype == HQMQ_F16;
+  if (bracket) {
+    // A sample of the tokens predicts the threshold statistic, the main pass needs x only once; should the prediction fail,
+    // the one-launch encoder (gated on a word that the check raises) redoes the call.
+    const bool pair16 = pair16_of(*a);
+    const int T32 = pair16 ? a->T_new / 2 : a->T_new;
+    EncGeom g32 = g;
+    if (pair16) { g32.n = 32; g32.npl = 32; g32.tpw = 1; g32.T_new = T32; g32.xs_t = 2 * g.xs_t; g32.pair16 = 1; }
+    const uint16_t* x16 = reinterpret_cast<const uint16_t*>(a->x);
+    const unsigned char* lut_arg = reinterpret_cast<const unsigned char*>(a->lut);
+    const Fast32 f32{x16, g.xs_b, g.xs_h, g32.xs_t, d.H, T32, pair16 ? 1 : 0};
+    const int n_s = (T32 + kSampleStride - 1) / kSampleStride;
+    int gs = (148 * 8 + d.B * d.H - 1) / (d.B * d.H);
+    if (gs > (n_s + 15) / 16) gs = (n_s + 15) / 16;
+    if (gs < 1) gs = 1;
+    float delta = 3.0f / sqrtf((float)d.B * (float)n_s * 32.f);
+    delta = delta < 0.002f ? 0.002f : delta > 0.012f ? 0.012f : delta;
+    uint32_t* bp = ws + wp.bp;
+    uint32_t* gate = ws + wp.gate;
+    const SampleArgs sa{ws + wp.hist_s, ws + wp.sel_s, ws + wp.tickets, (uint64_t)d.B * n_s * 32, a->quantile, a->median_mult, delta, bp, ws + wp.band};
+    for (int level = 0; level < 2; ++level) {
+      if (h16) sample32_kernel<HQMQ_F16><<<dim3(gs, d.B * d.H), 256, 0, st>>>(f32, sa, level);
+      else sample32_kernel<HQMQ_BF16><<<dim3(gs, d.B * d.H), 256, 0, st>>>(f32, sa, level);
+    }
+    const void* k = nullptr;
+#define HQMQ_PICK(IB_, RB_) \
+    if (g.ib == IB_ && g.rbits == RB_) k = h16 ? (const void*)&encode_main32_kernel<HQMQ_F16, IB_, RB_> : (const void*)&encode_main32_kernel<HQMQ_BF16, IB_, RB_>;
+    HQMQ_PICK(10, 3) HQMQ_PICK(12, 4) HQMQ_PICK(13, 6)
+#undef HQMQ_PICK
+    const size_t smem = (size_t)g.S * 16 + (size_t)kEnc32Warps * kMaxRowWords * 4 + kHistBins * 4 + (size_t)24 * g.S * 16 + lut_foot_of(a) + 16;
+    HQMQ_CHECK_CUDA(attn::raise_smem_limit(k, smem));
+    const MainGrid mg = main_grid(T32, d.B, d.H);
+    int64_t per = mg.per;
+    int t_start = a->t_start;
+    BracketArgs br{bp, bp, ws + wp.band, ws + wp.und, ws + wp.rcnt, ws + wp.rlist, ws + wp.histA, wp.rcap, wp.und_cap};
+    void* kargs[] = {(void*)&g32, (void*)&x16, (void*)&a->qs, (void*)&d, (void*)&t_start, (void*)&maps, (void*)&a->joint, (void*)&lut_arg,
+                     (void*)&nmul, (void*)&per, (void*)&br};
+    HQMQ_CHECK_CUDA(cudaLaunchKernel(k, dim3(mg.ctas), dim3(kEnc32Threads), kargs, smem, st));
+    const int64_t W32 = (int64_t)d.B * T32;
+    const int shares = (int)((W32 + mg.per - 2) / mg.per) + 1;             // most CTAs that share a head
+    list_select_kernel<<<dim3(shares, d.H), 256, 0, st>>>(bp, ws + wp.histA, ws + wp.rcnt, ws + wp.rlist, wp.rcap, mg.per, W32, ws + wp.histB, N,
+                                                          a->median_mult, a->quantile, ws + wp.sel_b, a->med_out, gate);
+    if (h16) fixup_kernel<HQMQ_F16><<<dim3(kFixupCtas, d.H), 256, 0, st>>>(f32, d, a->t_start, g.ib, g.rbits, d.B, ws + wp.sel_b, ws + wp.band, ws + wp.und, gate, wp.und_cap);
+    else fixup_kernel<HQMQ_BF16><<<dim3(kFixupCtas, d.H), 256, 0, st>>>(f32, d, a->t_start, g.ib, g.rbits, d.B, ws + wp.sel_b, ws + wp.band, ws + wp.und, gate, wp.und_cap);
+    FusedPair f;
+    fill_fused(a, 1, ws + wp.status, ws + wp.hist, ws + wp.sel, nullptr, nullptr, f.t[0]);
+    f.t[0].gate = gate;
+    rc = launch_fused(f, 1, a->x_dtype, lut_foot_of(a), st);
+    if (rc) return rc;
+    SidePair sp;
+    sp.t[0] = side_args(a, wp, ws);
+    return launch_side(sp, 1, true, st);
+  }
 
+  // any other geometry: the main pass, then two more passes over x for the exact threshold and one for the flags
   const int tok_per_block = kEncWarps * g.tpw * kEncIters;
   dim3 grid((a->T_new + tok_per_block - 1) / tok_per_block, d.B * d.H);
   const size_t smem_base = (size_t)g.S * 16 + (size_t)kEncWarps * g.tpw * kMaxRowWords * 4 + kHistBins * 4;
   if (smem_base > 200 * 1024) return HQMQ_ERR_UNSUPPORTED;
   // look-up-table search when a table is given and it fits shared memory next to the joint codebook
-  // (lut_footprint: shared-memory bytes of the largest head's table, from hqmq_encode_lut_footprint; 0 = unknown:
-  //  assume the largest a table can be)
-  const size_t lut_foot = a->lut_footprint > 0 ? ((size_t)a->lut_footprint + 15) & ~(size_t)15
-                                                : lut_smem_bytes(kLutNMax, kLutCellCap, kLutCandCap);
-  const size_t smem_lut = smem_base + (size_t)24 * g.S * 16 + lut_foot;
+  const size_t smem_lut = smem_base + (size_t)24 * g.S * 16 + lut_foot_of(a);
   const bool use_lut = a->search == 0 && a->lut != nullptr && a->lut_footprint >= 0 && smem_lut <= 226 * 1024;
-  // fast passes: d_head 128, 16-bit input, token rows on 16-byte boundaries (the fused last pass lists
-  // undecided chunks by a 32-bit index over the (batch, token, chunk) grid of a head)
-  // (d_head 64 with contiguous tokens runs the same kernels on pairs of tokens)
-  const bool pair16 = pair16_of(*a);
-  const int T32 = pair16 ? a->T_new / 2 : a->T_new;
-  EncGeom g32 = g;
-  if (pair16) { g32.n = 32; g32.npl = 32; g32.tpw = 1; g32.T_new = T32; g32.xs_t = 2 * g.xs_t; g32.pair16 = 1; }
-  const bool fast32 = (g.n == 32 || pair16) && is_half_dtype(a->x_dtype) && ((uintptr_t)a->x & 15) == 0 && g.xs_b % 8 == 0 &&
-                      g.xs_h % 8 == 0 && g.xs_t % 8 == 0 && (int64_t)d.B * a->T_new * 32 < ((int64_t)1 << 32);
-  Fast32 f32{reinterpret_cast<const uint16_t*>(a->x), g.xs_b, g.xs_h, g32.xs_t, d.H, T32, pair16 ? 1 : 0};
-  Fast32 f32_tok{reinterpret_cast<const uint16_t*>(a->x), g.xs_b, g.xs_h, g.xs_t, d.H, a->T_new, 0};   // per real token (the fix-up list)
-  const Mul24& nmul = mul24_native();
   if (use_lut && (uintptr_t)a->lut & 15) return HQMQ_ERR_ALIGN;
-  // specialised kernel: d_head 128, 16-bit input, one of the compiled field layouts
-  const void* fastk = nullptr;
-  const void* fastk_br = nullptr;
-  bool predicted = false;
-  const uint32_t* gate = nullptr;      // bracket mode: the word that sends the call through the multi-pass kernels after all
-  if (use_lut && is_half_dtype(a->x_dtype) && (g.n == 32 || (pair16 && fast32))) {
-    const bool h16 = a->x_dtype == HQMQ_F16;
-#define HQMQ_PICK(IB_, RB_)                                                                              \
-    if (g.ib == IB_ && g.rbits == RB_) {                                                                   \
-      fastk = h16 ? (const void*)&encode_main32_kernel<HQMQ_F16, IB_, RB_, false>                          \
-                  : (const void*)&encode_main32_kernel<HQMQ_BF16, IB_, RB_, false>;                        \
-      fastk_br = h16 ? (const void*)&encode_main32_kernel<HQMQ_F16, IB_, RB_, true>                        \
-                     : (const void*)&encode_main32_kernel<HQMQ_BF16, IB_, RB_, true>;                      \
-    }
-    HQMQ_PICK(10, 3) HQMQ_PICK(12, 4) HQMQ_PICK(13, 6)
-#undef HQMQ_PICK
-  }
-  if (fastk) {
-    const size_t smem_fast = (size_t)g.S * 16 + (size_t)kEnc32Warps * kMaxRowWords * 4 + 3 * kHistBins * 4 + (size_t)24 * g.S * 16 +
-                             lut_foot + 16;
-    const MainGrid mg = main_grid(T32, d.B, d.H);
-    int64_t per32 = mg.per;
-    if (smem_fast > 48 * 1024) {
-      HQMQ_CHECK_CUDA(cudaFuncSetAttribute(fastk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fast));
-      HQMQ_CHECK_CUDA(cudaFuncSetAttribute(fastk_br, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fast));
-    }
-    const dim3 fgrid(mg.ctas);
-    // Med3x: a sample of the tokens predicts the threshold statistic.  Two select levels over the sample give it
-    // to 22 bits, the bracket pass then needs x only once; should the prediction fail, the multi-pass kernels
-    // below (gated on a word the bracket's check raises) redo the call, with the sample's first level telling the
-    // main pass which bins to refine.
-    predicted = med && !ext_med && fast32 && T32 >= 1024;
-    const bool bracket = predicted && bracket_wanted(*a);
-    const uint16_t* x16 = reinterpret_cast<const uint16_t*>(a->x);
-    const unsigned char* lut_arg = reinterpret_cast<const unsigned char*>(a->lut);
-    int t_start_arg = a->t_start;
-    BracketArgs brargs{};
-    if (predicted) {
-      const int n_s = (T32 + kSampleStride - 1) / kSampleStride;
-      const uint64_t N_s = (uint64_t)d.B * n_s * 32;
-      int gs = (148 * 8 + d.B * d.H - 1) / (d.B * d.H);
-      if (gs > (n_s + 15) / 16) gs = (n_s + 15) / 16;
-      if (gs < 1) gs = 1;
-      const bool h16s = a->x_dtype == HQMQ_F16;
-      uint32_t* hist_s = ws + wp.hist_s;
-      uint32_t* sel_s_w = ws + wp.sel_s;
-      for (int level = 0; level < (bracket ? 2 : 1); ++level) {
-        if (h16s) sample32_kernel<HQMQ_F16><<<dim3(gs, d.B * d.H), 256, 0, st>>>(f32, hist_s, level, sel_s_w);
-        else sample32_kernel<HQMQ_BF16><<<dim3(gs, d.B * d.H), 256, 0, st>>>(f32, hist_s, level, sel_s_w);
-        select_kernel<<<d.H, 256, 0, st>>>(hist_s, sel_s_w, level, N_s, a->median_mult, nullptr, nullptr, nullptr, nullptr,
-                                           a->quantile, nullptr, 0);
-      }
-    }
-    if (bracket) {
-      const bool h16s = a->x_dtype == HQMQ_F16;
-      uint32_t* sel_s_w = ws + wp.sel_s;
-      const int n_s = (T32 + kSampleStride - 1) / kSampleStride;
-      float delta = 3.0f / sqrtf((float)d.B * (float)n_s * 32.f);
-      delta = delta < 0.002f ? 0.002f : delta > 0.012f ? 0.012f : delta;
-      uint32_t* bp = ws + wp.bp;
-      bracket_kernel<<<(d.H + 63) / 64, 64, 0, st>>>(sel_s_w, a->median_mult, delta, d.H, bp, ws + wp.band_b);
-      gate = ws + wp.gate;
-      brargs.bp = bp; brargs.bp_count = bp; brargs.band = ws + wp.band_b; brargs.und = ws + wp.und_b;
-      brargs.rcnt = ws + wp.rcnt; brargs.rlist = ws + wp.rlist; brargs.histA = ws + wp.histA; brargs.rcap = wp.rcap; brargs.und_cap = wp.und_cap;
-      brargs.run_if = nullptr;
-      uint32_t* no_hist = nullptr;
-      const uint32_t* no_sel = nullptr;
-      void* kargs_b[] = {(void*)&g32, (void*)&x16, (void*)&a->qs, (void*)&d, (void*)&t_start_arg, (void*)&no_hist, (void*)&maps,
-                         (void*)&a->joint, (void*)&lut_arg, (void*)&nmul, (void*)&per32, (void*)&no_sel, (void*)&brargs};
-      HQMQ_CHECK_CUDA(cudaLaunchKernel(fastk_br, fgrid, dim3(kEnc32Threads), kargs_b, smem_fast, st));
-      const uint64_t N_all = (uint64_t)d.B * a->T_new * d.n_chunks;
-      list_pickA_kernel<<<d.H, 256, 0, st>>>(bp, ws + wp.histA, N_all, a->quantile, ws + wp.gate);
-      const int64_t W32 = (int64_t)d.B * T32;
-      const int shares = (int)((W32 - 1 + mg.per - 1) / mg.per) + 1;         // most CTAs that share a head
-      list_histB_kernel<<<dim3(shares, d.H), 256, 0, st>>>(bp, ws + wp.rcnt, ws + wp.rlist, wp.rcap, mg.per, W32, ws + wp.histB, gate);
-      list_pickB_kernel<<<d.H, 256, 0, st>>>(bp, ws + wp.histB, N_all, a->median_mult, a->quantile, ws + wp.sel_b, a->med_out, gate);
-      int fg = (148 * 32 + d.B * d.H - 1) / (d.B * d.H);
-      const int fg_max = (T32 + kF32Tok - 1) / kF32Tok;
-      if (fg > fg_max) fg = fg_max;
-      if (fg < 1) fg = 1;
-      if (h16s) {
-        fixup_list_kernel<HQMQ_F16><<<d.H, 256, 0, st>>>(f32_tok, d, a->t_start, g.ib, g.rbits, ws + wp.sel_b, ws + wp.band_b, ws + wp.und_b, gate, 0, wp.und_cap);
-        fixup_scan_kernel<HQMQ_F16><<<dim3(fg, d.B * d.H), 256, 0, st>>>(f32, d, a->t_start, g.ib, g.rbits, ws + wp.sel_b, ws + wp.band_b, gate, 0, wp.und_cap);
-      } else {
-        fixup_list_kernel<HQMQ_BF16><<<d.H, 256, 0, st>>>(f32_tok, d, a->t_start, g.ib, g.rbits, ws + wp.sel_b, ws + wp.band_b, ws + wp.und_b, gate, 0, wp.und_cap);
-        fixup_scan_kernel<HQMQ_BF16><<<dim3(fg, d.B * d.H), 256, 0, st>>>(f32, d, a->t_start, g.ib, g.rbits, ws + wp.sel_b, ws + wp.band_b, gate, 0, wp.und_cap);
-      }
-      brargs.run_if = gate;       // the multi-pass launch below runs only if the check raised the gate
-    }
-    const uint32_t* sel_s_arg = predicted ? ws + wp.sel_s : nullptr;
-    uint32_t* hist_arg = med && !ext_med ? ws + wp.hist : nullptr;
-    void* kargs[] = {(void*)&g32, (void*)&x16, (void*)&a->qs, (void*)&d, (void*)&t_start_arg, (void*)&hist_arg, (void*)&maps,
-                     (void*)&a->joint, (void*)&lut_arg, (void*)&nmul, (void*)&per32, (void*)&sel_s_arg, (void*)&brargs};
-    HQMQ_CHECK_CUDA(cudaLaunchKernel(fastk, fgrid, dim3(kEnc32Threads), kargs, smem_fast, st));
-  } else if (use_lut) {
+  uint32_t* hist = ws + wp.hist;
+  uint32_t* sel = ws + wp.sel;
+  uint32_t* hist_arg = med && !ext_med ? hist : nullptr;
+  if (use_lut) {
     if (smem_lut > 48 * 1024)
       HQMQ_CHECK_CUDA(cudaFuncSetAttribute(encode_main_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_lut));
-    encode_main_kernel<true><<<grid, kEncThreads, smem_lut, st>>>(g, a->x, a->qs, d, a->t_start, med && !ext_med ? ws + wp.hist : nullptr,
-                                                                  maps, a->joint, reinterpret_cast<const unsigned char*>(a->lut), nmul);
+    encode_main_kernel<true><<<grid, kEncThreads, smem_lut, st>>>(g, a->x, a->qs, d, a->t_start, hist_arg, maps, a->joint,
+                                                                  reinterpret_cast<const unsigned char*>(a->lut), nmul);
   } else {
     if (smem_base > 48 * 1024)
       HQMQ_CHECK_CUDA(cudaFuncSetAttribute(encode_main_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_base));
-    encode_main_kernel<false><<<grid, kEncThreads, smem_base, st>>>(g, a->x, a->qs, d, a->t_start, med && !ext_med ? ws + wp.hist : nullptr,
-                                                                    maps, a->joint, nullptr, nmul);
+    encode_main_kernel<false><<<grid, kEncThreads, smem_base, st>>>(g, a->x, a->qs, d, a->t_start, hist_arg, maps, a->joint, nullptr, nmul);
   }
   HQMQ_LAUNCH_CHECK();
-  if (!med) {
-    // no chunk of this call is flagged: the record offsets of its blocks just carry the running total on
-    if (d.ofrag) {
-      scan_kernel<<<d.B * d.H, kScanWarps * 32, 0, st>>>(d, a->t_start, a->T_new, wp.blk0, wp.nblk, 0, ws + wp.status);
-      HQMQ_LAUNCH_CHECK();
-    }
-    return HQMQ_OK;
-  }
+  SidePair sp;
+  sp.t[0] = side_args(a, wp, ws);
+  // (without a threshold no chunk of this call is flagged: the record offsets of its blocks just carry the running total on)
+  if (!med) return d.ofrag ? launch_side(sp, 1, false, st) : HQMQ_OK;
 
-  const uint64_t N = (uint64_t)d.B * a->T_new * d.n_chunks;
   const int64_t per_bh = (int64_t)a->T_new * d.n_chunks;
   // about 16 resident CTAs per SM in total; each CTA amortises zeroing and flushing its private histograms
   const int bh_count = d.B * d.H;
@@ -2717,61 +2479,22 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
   const int hb_max = (int)((per_bh + 256 * 16 - 1) / (256 * 16));
   if (hb > hb_max) hb = hb_max;
   if (hb < 1) hb = 1;
-  uint32_t* hist = ws + wp.hist;
-  uint32_t* sel = ws + wp.sel;
-  int fgrid = (148 * 32 + bh_count - 1) / bh_count;
-  const int fgrid_max = (T32 + kF32Tok - 1) / kF32Tok;
-  if (fgrid > fgrid_max) fgrid = fgrid_max;
-  if (fgrid < 1) fgrid = 1;
-  const dim3 f32_grid(fgrid, d.B * d.H);
-  const bool h16 = a->x_dtype == HQMQ_F16;
-  uint32_t* band = ws + wp.band;
-  uint32_t* und = ws + wp.und;
-  const uint32_t* sel_s = predicted ? ws + wp.sel_s : nullptr;
-  uint32_t* hist_fb = ws + wp.hist_fb;
   if (ext_med) {
-    // threshold from the caller's medians, then the plain flag pass (any geometry)
+    // threshold from the caller's medians, then the plain flag pass
     thr_from_median_kernel<<<(d.H + 63) / 64, 64, 0, st>>>(a->med_in, a->median_mult, d.H, sel, a->med_out);
-    const int tok_per_fblock = 8 * g.tpw;
-    int fb = (a->T_new + 4 * tok_per_fblock - 1) / (4 * tok_per_fblock);
-    const int fb_cap = (148 * 32 + bh_count - 1) / bh_count;
-    if (fb > fb_cap) fb = fb_cap;
-    if (fb < 1) fb = 1;
-    flags_kernel<<<dim3(fb, d.B * d.H), 256, 0, st>>>(g, a->x, d, a->t_start, sel);
   } else {
-  select_kernel<<<d.H, 256, 0, st>>>(hist, sel, 0, N, a->median_mult, nullptr, nullptr, nullptr, nullptr, a->quantile, gate, 1);
-  if (fast32) {
-    // (with a prediction this launch returns at once unless the sample named the wrong bins)
-    if (h16) hist32_kernel<HQMQ_F16><<<f32_grid, 256, 0, st>>>(f32, hist, sel, 1, sel_s, hist_fb, gate, 1);
-    else hist32_kernel<HQMQ_BF16><<<f32_grid, 256, 0, st>>>(f32, hist, sel, 1, sel_s, hist_fb, gate, 1);
-    select_kernel<<<d.H, 256, 0, st>>>(hist, sel, 1, N, a->median_mult, nullptr, band, sel_s, hist_fb, a->quantile, gate, 1);
-    // last histogram level and provisional flags in one pass, exact threshold, then the (normally empty) fix-up
-    if (h16) histflags32_kernel<HQMQ_F16><<<f32_grid, 256, 0, st>>>(f32, d, a->t_start, g.ib, g.rbits, hist, sel, band, und, gate, 1);
-    else histflags32_kernel<HQMQ_BF16><<<f32_grid, 256, 0, st>>>(f32, d, a->t_start, g.ib, g.rbits, hist, sel, band, und, gate, 1);
-    select_kernel<<<d.H, 256, 0, st>>>(hist, sel, 2, N, a->median_mult, a->med_out, nullptr, nullptr, nullptr, a->quantile, gate, 1);
-    if (h16) {
-      fixup_list_kernel<HQMQ_F16><<<d.H, 256, 0, st>>>(f32_tok, d, a->t_start, g.ib, g.rbits, sel, band, und, gate, 1, kUndCap);
-      fixup_scan_kernel<HQMQ_F16><<<f32_grid, 256, 0, st>>>(f32, d, a->t_start, g.ib, g.rbits, sel, band, gate, 1, kUndCap);
-    } else {
-      fixup_list_kernel<HQMQ_BF16><<<d.H, 256, 0, st>>>(f32_tok, d, a->t_start, g.ib, g.rbits, sel, band, und, gate, 1, kUndCap);
-      fixup_scan_kernel<HQMQ_BF16><<<f32_grid, 256, 0, st>>>(f32, d, a->t_start, g.ib, g.rbits, sel, band, gate, 1, kUndCap);
-    }
-  } else {
-    hist_kernel<<<dim3(hb, d.B * d.H), 256, 0, st>>>(g, a->x, hist, sel, 1);
-    select_kernel<<<d.H, 256, 0, st>>>(hist, sel, 1, N, a->median_mult, nullptr, nullptr, nullptr, nullptr, a->quantile, nullptr, 0);
-    hist_kernel<<<dim3(hb, d.B * d.H), 256, 0, st>>>(g, a->x, hist, sel, 2);
-    select_kernel<<<d.H, 256, 0, st>>>(hist, sel, 2, N, a->median_mult, a->med_out, nullptr, nullptr, nullptr, a->quantile, nullptr, 0);
-    const int tok_per_fblock = 8 * g.tpw;
-    int fb = (a->T_new + 4 * tok_per_fblock - 1) / (4 * tok_per_fblock);
-    const int fb_cap = (148 * 32 + bh_count - 1) / bh_count;
-    if (fb > fb_cap) fb = fb_cap;
-    if (fb < 1) fb = 1;
-    flags_kernel<<<dim3(fb, d.B * d.H), 256, 0, st>>>(g, a->x, d, a->t_start, sel);
+    select_kernel<<<d.H, 256, 0, st>>>(hist, sel, 0, N, a->median_mult, nullptr, a->quantile);
+    hist_kernel<<<dim3(hb, bh_count), 256, 0, st>>>(g, a->x, hist, sel, 1);
+    select_kernel<<<d.H, 256, 0, st>>>(hist, sel, 1, N, a->median_mult, nullptr, a->quantile);
+    hist_kernel<<<dim3(hb, bh_count), 256, 0, st>>>(g, a->x, hist, sel, 2);
+    select_kernel<<<d.H, 256, 0, st>>>(hist, sel, 2, N, a->median_mult, a->med_out, a->quantile);
   }
-  }
+  const int tok_per_fblock = 8 * g.tpw;
+  int fb = (a->T_new + 4 * tok_per_fblock - 1) / (4 * tok_per_fblock);
+  const int fb_cap = (148 * 32 + bh_count - 1) / bh_count;
+  if (fb > fb_cap) fb = fb_cap;
+  if (fb < 1) fb = 1;
+  flags_kernel<<<dim3(fb, bh_count), 256, 0, st>>>(g, a->x, d, a->t_start, sel);
   HQMQ_LAUNCH_CHECK();
-  scan_kernel<<<d.B * d.H, kScanWarps * 32, 0, st>>>(d, a->t_start, a->T_new, wp.blk0, wp.nblk, 1, ws + wp.status);
-  side_kernel<<<dim3((wp.nblk + 7) / 8, d.B * d.H), 256, 0, st>>>(g, a->x, d, a->t_start, wp.blk0, wp.nblk);
-  HQMQ_LAUNCH_CHECK();
-  return HQMQ_OK;
+  return launch_side(sp, 1, true, st);
 }

@@ -24,6 +24,7 @@ struct FusedArgs {
   uint32_t* hist;             // [H][3][2][kHistBins], zero
   uint32_t* bars;             // [H] arrivals, zero
   uint32_t* status;
+  const uint32_t* gate;       // return unless this word is set (nullptr: run)
   int cph, per;               // CTAs per head, warp tokens per CTA
   int rcp_rn;                 // directions are normalised with the rounded reciprocal (as the generic passes do)
 };
@@ -40,15 +41,17 @@ __host__ __device__ inline size_t fused_smem_bytes(int S, size_t lut_foot) {
   return (size_t)S * 16 + 2 * kHistBins * 4 + (size_t)kEnc32Warps * kMaxRowWords * 4 + (size_t)24 * S * 16 + lut_foot + 64;
 }
 
+// IB, RB: field widths of the layouts in common use, or 0: any other, from the geometry.
 template <int DT, int IB, int RB, bool DENSE>
 __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const FusedPair pr, const Maps24 maps, const Mul24 nmul) {
-  constexpr int CB = IB + RB;
-  constexpr float qmaxf = (float)((1 << RB) - 1);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ uint32_t s_warp[32], s_sel[4], s_flagged;
   const FusedArgs& a = pr.t[blockIdx.y];
+  if (a.gate && *a.gate == 0u) return;
   const EncGeom& g = a.g;
+  const int ib = IB ? IB : g.ib, CB = IB ? IB + RB : g.ib + g.rbits;
+  const float qmaxf = (float)(IB ? (1 << RB) - 1 : g.qmax);
   const int S = g.S, h = blockIdx.x / a.cph, part = blockIdx.x - h * a.cph;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float4* qs = reinterpret_cast<float4*>(smem_raw);
@@ -239,13 +242,13 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
       if (live) *reinterpret_cast<uint2*>(a.out + ((((int64_t)b * g.H + h) * g.T_new + t) * g.n + c) * 4) = o;
     } else {
       const uint32_t ni = (uint32_t)((((au >> 3) * S + sidx) << 3) | (au & 7));
-      const uint32_t f = ni | ((flagged ? 0u : (uint32_t)rqf) << IB);
+      const uint32_t f = ni | ((flagged ? 0u : (uint32_t)rqf) << ib);
       const int64_t row = ((int64_t)b * g.H + h) * a.dst.T_cap + a.t_start + t;       // (pairs: each half-warp its own)
-      if constexpr (CB == 16) {
+      if (CB == 16) {
         const uint32_t other = __shfl_xor_sync(0xffffffffu, f, 1);
         if (live && !(lane & 1)) reinterpret_cast<uint32_t*>(a.dst.codes + row * a.dst.row_bytes)[c >> 1] = f | (other << 16);
       } else {
-        constexpr int RW = CB;                         // words per row of 32 chunks (pairs have 16-bit fields)
+        const int RW = CB;                             // words per row of 32 chunks (pairs have 16-bit fields)
         if (lane < RW) myrow[lane] = 0;
         __syncwarp();
         const int bit = lane * CB, wd = bit >> 5, s_ = bit & 31;

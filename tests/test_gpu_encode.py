@@ -535,3 +535,27 @@ def test_small_fake_quant_counts_and_values(shape, dtype):
         assert torch.equal(q.quantize_K(x, layer), q.inner.decode(pk, layer, 0, dtype=dtype, scale_first=True))
         rates.append(pk.n_outliers() / (x.numel() // 4))
     assert max(rates) > 0 and abs(q._observed_outlier_rate - np.mean(rates)) < 1e-9 and q._n_observations == 3
+
+
+@pytest.mark.parametrize("shape,S,br", [((1, 3, 161, 128), 48, 4), ((2, 2, 700, 128), 12, 5), ((1, 2, 333, 64), 85, 5)])
+@pytest.mark.parametrize("C", [None, 3.0])
+def test_one_launch_encoder_other_field_widths(shape, S, br, C):
+    """Field widths without a compiled layout (15, 14 and, at head dim 64, 16 bits)."""
+    test_one_launch_encoder(shape, S, br, C, False)
+
+
+@pytest.mark.parametrize("B,H,T,d,kind", [(64, 2, 1024, 128, "hot"), (37, 3, 1801, 128, "spiky"), (1, 149, 512, 128, "hot"),
+                                          (33, 2, 4000, 64, "spiky"), (64, 2, 1024, 128, "constant"), (64, 2, 1024, 128, "drift")])
+def test_large_call_pieces(B, H, T, d, kind):
+    """The equal pieces of the one-read pass: a head over many CTAs, pieces across heads and odd batch boundaries, calls whose
+    prediction fails and that the one-launch encoder redoes; more heads than SMs in the latter."""
+    if kind == "constant":
+        x = torch.ones(B, H, T, d).bfloat16()
+    elif kind == "drift":                              # the sampled tokens are unlike the rest
+        x = make_kv("randn", (B, H, T, d), seed=5, dtype=torch.float32)
+        x[:, :, ::32] *= 5.0
+        x = x.bfloat16()
+    else:
+        x = make_kv(kind, (B, H, T, d), seed=5, dtype=torch.bfloat16)
+    S, br = (24, 3) if d == 128 else (96, 4)
+    _threshold_compare(x, S, br, 3.0)
