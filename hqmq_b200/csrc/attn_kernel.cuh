@@ -539,6 +539,12 @@ __device__ __forceinline__ uint2 joint_entry(const void* j, int64_t base, int dt
   return make_uint2(pack_half2(f.x, f.y), pack_half2(f.z, f.w));
 }
 
+// A kernel launched with programmatic stream serialisation may start before its predecessor has finished: what precedes
+// grid_dep_wait() must not touch anything the predecessor writes.  grid_dep_launch() lets the successor start likewise; it
+// comes after the wait, so that a successor's own wait still covers everything before this kernel.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Merge of the n partials (o[D], m, l) of a unit by all `threads` threads (whole warps, at least 8) of a CTA: head g's partial c
 // starts at base + g * gs + c * cs (past the L1: other CTAs wrote them).  A warp per head turns the (m, l) pairs into weights
 // first, then every thread sums pairs of elements with eight loads in flight.  (Each thread walking all partials for itself,

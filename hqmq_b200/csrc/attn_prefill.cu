@@ -187,6 +187,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // (launched while the expansion still runs: nothing before this line touches what a kernel wrote)
+  grid_dep_wait();
+  grid_dep_launch();
   constexpr uint32_t tmem = 0u;               // an allocation of all columns starts at column 0
   // (a wait that runs out raises the abort word: every role then stops at its next wait.  No suspend hint: these waits are
   //  links of the per-tile chain, and a hinted wait was seen to wake late.)
@@ -514,6 +517,7 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const PrefillParams 
   PfIter it;
   it.init(p, c);
   if (it.off == 0) return;                                  // the unit starts with the CTA
+  grid_dep_wait();
   const int64_t s_u = (int64_t)c * p.L - it.off;
   if ((int64_t)(c - 1) * p.L > s_u) return;                 // the unit's first boundary does the merge
   const int c0 = c - 1, n_parts = (int)((s_u + it.n - 1) / p.L) - c0 + 1;
@@ -580,6 +584,7 @@ __global__ void __launch_bounds__(256, 3) prefill_expand_kernel(const ExpandPara
   uint2* tbl = reinterpret_cast<uint2*>(smem_raw + (blockIdx.z ? TB + 128 * (N + 1) * 4 : 0));
   __shared__ float s_big[8], s_fac[kPfTok];
   __shared__ uint16_t s_list[8][16 * N];       // (token of the block) * 32 + chunk of the block's payload entries
+  grid_dep_launch();
   const bool is_v = blockIdx.z != 0;
   const hqmq_packed& pk = is_v ? e.V : e.K;
   const hqmq_ref_packed& rf = is_v ? e.Vr : e.Kr;
@@ -836,6 +841,15 @@ bool prefill_plan(const hqmq_attn_args* a, PrefillPlan& pl) {
   return true;
 }
 
+// Launch that may start while its predecessor on the stream finishes (see grid_dep_wait).
+static cudaError_t launch_dependent(const void* k, dim3 grid, int threads, void** args, size_t smem, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = &at; cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, k, args);
+}
 int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspace, float qscale, uint32_t epoch, cudaStream_t st) {
   PrefillParams p = pl.p;
   unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
@@ -903,8 +917,8 @@ int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspa
     void* ea[] = {&e};
     HQMQ_CHECK_CUDA(cudaLaunchKernel(ek, dim3((p.nt + e.per - 1) / e.per, n_bh, 2), dim3(256), ea, esmem, st));
     void* pa[] = {&p};
-    HQMQ_CHECK_CUDA(cudaLaunchKernel(ak, dim3(grid), dim3(kPfThreads), pa, pf_smem_bytes(d), st));
-    if (!pl.whole && grid > 1) HQMQ_CHECK_CUDA(cudaLaunchKernel(mk, dim3(grid - 1, 4 * p.streams), dim3(256), pa, 0, st));
+    HQMQ_CHECK_CUDA(launch_dependent(ak, dim3(grid), kPfThreads, pa, pf_smem_bytes(d), st));
+    if (!pl.whole && grid > 1) HQMQ_CHECK_CUDA(launch_dependent(mk, dim3(grid - 1, 4 * p.streams), 256, pa, 0, st));
   }
   return HQMQ_OK;
 }

@@ -53,12 +53,6 @@ __device__ __forceinline__ float cluster_ld(const float* mine, uint32_t rank) {
   asm volatile("{\n .reg .b32 t;\n mapa.shared::cluster.u32 t, %1, %2;\n ld.shared::cluster.f32 %0, [t];\n}\n" : "=f"(v) : "r"(a), "r"(rank) : "memory");
   return v;
 }
-// A kernel launched with programmatic stream serialisation may start before its predecessor has finished: what precedes
-// grid_dep_wait() must not touch anything the predecessor writes.  grid_dep_launch() lets the successor start likewise; it
-// comes after the wait, so that a successor's own wait still covers everything before this kernel.
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // SMALL: problems of a few tiles per warp.  A unit is the work of ONE cluster, p.L tiles to a CTA, and the CTAs' results are
 // merged through distributed shared memory: no partials in global memory, no merge launch.  The codeword tables are not
 // replicated (two bulk copies in flight beside the first tiles instead of 70-150 KB of stores: with one or two tiles per
