@@ -121,6 +121,21 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
     if (part == 0 && threadIdx.x == 0 && a.med_out) a.med_out[h] = med;
   } else if (a.C > 0.f) {
     const QRank qr = quantile_rank((uint64_t)g.B * g.T_new * g.n, a.quantile);
+    // the norms of a warp's first tokens stay in registers for all three levels (each level used to read them again: 4.6 us of
+    // load latency and norm arithmetic a level; what differs from every prefix, as 0xffffffff does, is not counted)
+    constexpr int kKeep = 8;
+    uint32_t keys[kKeep];
+    {
+      uint2 raw[kKeep];
+#pragma unroll
+      for (int u = 0; u < kKeep; ++u) {
+        const int w = w0 + warp + u * kEnc32Warps;
+        raw[u] = make_uint2(0u, 0u);
+        keys[u] = w < w1 && fetch(w, raw[u]) ? 0u : 0xffffffffu;
+      }
+#pragma unroll
+      for (int u = 0; u < kKeep; ++u) keys[u] |= __float_as_uint(norm_of(raw[u]));
+    }
     uint32_t p0 = 0u, p1 = 0u, k0 = (uint32_t)qr.lo, k1 = (uint32_t)qr.hi;      // prefixes and ranks of the two statistics
     for (int level = 0; level < 3; ++level) {
       const int hs = level == 0 ? 31 : level == 1 ? 21 : 10, ds = level == 0 ? 21 : level == 1 ? 10 : 0;
@@ -128,7 +143,13 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
       const bool same = q0 == q1;
       for (int i = threadIdx.x; i < 2 * kHistBins; i += blockDim.x) sh[i] = 0u;
       __syncthreads();
-      for (int w = w0 + warp; w < w1; w += 4 * kEnc32Warps) {
+#pragma unroll
+      for (int u = 0; u < kKeep; ++u) {
+        const uint32_t top = keys[u] >> hs, dig = (keys[u] >> ds) & dm;
+        if (top == q0) atomicAdd(&sh[dig], 1u);
+        else if (top == q1) atomicAdd(&sh[kHistBins + dig], 1u);
+      }
+      for (int w = w0 + warp + kKeep * kEnc32Warps; w < w1; w += 4 * kEnc32Warps) {
         uint2 raw[4]; bool live[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) { live[u] = w + u * kEnc32Warps < w1; if (live[u]) live[u] = fetch(w + u * kEnc32Warps, raw[u]); }
