@@ -86,6 +86,12 @@ __host__ __device__ inline void key_range(int Tkv, int Tq, int causal, int windo
 }
 
 constexpr uint32_t kWaitLimit = 1u << 24;
+// A kernel launched with programmatic stream serialisation may start before its predecessor has finished: what precedes
+// grid_dep_wait() must not touch anything the predecessor writes.  grid_dep_launch() lets the successor start likewise; it
+// comes after the wait, so that a successor's own wait still covers everything before this kernel.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -538,12 +544,6 @@ __device__ __forceinline__ uint2 joint_entry(const void* j, int64_t base, int dt
   }
   return make_uint2(pack_half2(f.x, f.y), pack_half2(f.z, f.w));
 }
-
-// A kernel launched with programmatic stream serialisation may start before its predecessor has finished: what precedes
-// grid_dep_wait() must not touch anything the predecessor writes.  grid_dep_launch() lets the successor start likewise; it
-// comes after the wait, so that a successor's own wait still covers everything before this kernel.
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Merge of the n partials (o[D], m, l) of a unit by all `threads` threads (whole warps, at least 8) of a CTA: head g's partial c
 // starts at base + g * gs + c * cs (past the L1: other CTAs wrote them).  A warp per head turns the (m, l) pairs into weights
@@ -1054,7 +1054,10 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
         __shared__ uint32_t s_last;
         __threadfence();                      // this CTA's partial is visible device-wide before its ticket is drawn
         __syncthreads();
-        if (threadIdx.x == 0) s_last = atomicAdd(&p.tickets[u], 1u) == (uint32_t)(n_ctas - 1) ? 1u : 0u;
+        if (threadIdx.x == 0) {
+          grid_dep_wait();                    // (the tickets are zero, see ticket_zero_kernel)
+          s_last = atomicAdd(&p.tickets[u], 1u) == (uint32_t)(n_ctas - 1) ? 1u : 0u;
+        }
         __syncthreads();
         if (s_last) {
           __threadfence();
@@ -1091,6 +1094,7 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
         if (r == 0) { dst[p.d] = m_run[nh][e]; dst[p.d + 1] = l; }
       }
   }
+  if (TICKET) grid_dep_wait();      // (no CTA may outlive the kernel ahead of it)
 }
 
 }  // namespace attn

@@ -110,6 +110,8 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
     }
     grid_dep_wait();
     grid_dep_launch();
+  } else {
+    grid_dep_launch();      // (the merge kernel may be brought up while this one runs out)
   }
   __syncwarp();
   uint32_t it = 0;        // tiles this warp has consumed so far (stage = it % kStages, parity from it / kStages)
