@@ -966,14 +966,13 @@ hist_kernel(EncGeom g, const void* __restrict__ x, uint32_t* __restrict__ hist, 
 
 // ---- Med3x passes for the common geometry -----------------------------------------------------------------
 // 32 chunks per token (d_head 128), 16-bit inputs, token rows 16-byte aligned: one lane reads two chunks
-// (16 bytes), half a warp reads a token, and every thread keeps four such loads in flight.
+// (16 bytes), half a warp reads a token.
 struct Fast32 {
   const uint16_t* x;
   int64_t xs_b, xs_h, xs_t;
   int H, T_new;
   int pair;      // 1: every "token" here is two consecutive tokens of 16 chunks (d_head 64), see EncGeom::pair16
 };
-constexpr int kF32Tok = 64;   // tokens per CTA iteration: 8 warps x 2 tokens x 4 loads
 
 template <int DT>
 __device__ __forceinline__ void norms_of_two(const uint4& r, float& n0, float& n1) {
@@ -1869,7 +1868,7 @@ static MainGrid main_grid(int T_new, int B, int H) {
 // The bracket pass pays when the sample predicts well: the statistic's sampling error falls with the square root of
 // the sampled norms per head (a 1/32 sample of B * T_new tokens, 32 norms each), so the bracket's half-width is
 // 3 / sqrt(norms) (about six standard errors of a median), at least 0.2 % and at most 1.2 %; calls too small for that,
-// and quantiles out in the tails (few norms nearby: a much larger error), take the multi-pass path as before.
+// and quantiles out in the tails (few norms nearby: a much larger error), take the one-launch encoder.
 // d_head 64 as pairs of tokens (see EncGeom::pair16): the call's geometry must allow it, and a token's row must be whole
 // words without padding (16-bit fields; rows of 13- and 19-bit fields are padded, so two of them are not one longer row).
 static bool pair16_of(const hqmq_encode_args& a) {

@@ -1,8 +1,8 @@
 // One-launch encoder for calls between the decode-time append and the very long prompt (included by encode.cu): exact
 // threshold, nearest codewords and either packed rows or the dense fake-quantised tensor, in ONE kernel.
 //
-// The multi-pass path of such a call is a dozen launches (samples, selects, histograms, flags, fix-ups), each of a few
-// microseconds, and its main pass copies 60-150 KB of tables into shared memory per 128 tokens.  Here a head's tokens are
+// As separate passes such a call was a dozen launches (samples, selects, histograms, flags, fix-ups), each of a few
+// microseconds, and its main pass copied 60-150 KB of tables into shared memory per 128 tokens.  Here a head's tokens are
 // split over a few CTAs that stay resident (one per SM, cooperative launch): the tables are fetched by bulk copies while
 // the three radix-select levels run -- each CTA histograms its norms, the CTAs of the head meet at a counter in global
 // memory (bounded wait), everyone scans the head's histogram -- and the main pass then knows the exact threshold, so flags
