@@ -227,6 +227,15 @@ constexpr int kSmallMaxRounds = 2;
 // Units of at most this many tiles run the staged kernels in warp mode (every warp has at most two tiles of a unit)
 constexpr int kWarpModeMaxTiles = 32;
 
+// The staged kernel of a call, or nullptr where it takes the generic one.
+const void* staged_kernel(const hqmq_attn_args* a) {
+  if (a->layout != 0 || a->H_q / a->H_kv > 8 || !is_half_dtype(a->K.scale_dtype)) return nullptr;
+  // the staged kernels copy 16-byte aligned pieces: side buffers must start on 16 bytes per (b,h)
+  auto side_ok = [](const hqmq_packed& k) { return !k.flags || (k.out_cap % 2 == 0 && ((uintptr_t)k.out_vals & 15) == 0); };
+  if (!side_ok(a->K) || !side_ok(a->V)) return nullptr;
+  return fast_kernel(a->d / 4, idx_bits_for(a->K.S), a->K.radius_bits, a->K.flags != nullptr || a->V.flags != nullptr, false);
+}
+
 static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, bool allow_warp_mode) {
   const int n = a->d / 4;
   const int G = a->H_q / a->H_kv;
@@ -237,10 +246,7 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
   if (a->layout == 0) {
     pl.ib = idx_bits_for(a->K.S);
     pl.table_rows = 24 * a->K.S;
-    // the staged kernels copy 16-byte aligned pieces: side buffers must start on 16 bytes per (b,h)
-    const bool side_ok = !outl || (((!a->K.flags || (a->K.out_cap % 2 == 0 && ((uintptr_t)a->K.out_vals & 15) == 0))) &&
-                                   ((!a->V.flags || (a->V.out_cap % 2 == 0 && ((uintptr_t)a->V.out_vals & 15) == 0))));
-    if (G <= 8 && is_half_dtype(a->K.scale_dtype) && side_ok) pl.kernel = fast_kernel(n, pl.ib, a->K.radius_bits, outl, false);
+    pl.kernel = staged_kernel(a);
     if (pl.kernel) pl.nw = outl ? kFastWarpsOutl : kFastWarps;
   } else {
     pl.ib = 16;

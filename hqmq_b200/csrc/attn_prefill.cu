@@ -647,8 +647,7 @@ __global__ void __launch_bounds__(256, 3) prefill_expand_kernel(const ExpandPara
     sh = bit & 31; w1 = sh + cb > 32 ? 1 : 0;
     imask = (1u << e.ib) - 1u; fmask = (1u << cb) - 1u;
   }
-  const bool out32 = outl && pk.out_dtype == HQMQ_F32;
-  const unsigned char* vals = outl ? reinterpret_cast<const unsigned char*>(pk.out_vals) + (int64_t)bh * pk.out_cap * (out32 ? 16 : 8) : nullptr;
+  const unsigned char* vals = outl ? reinterpret_cast<const unsigned char*>(pk.out_vals) + (int64_t)bh * pk.out_cap * 8 : nullptr;   // (16-bit entries)
   const uint32_t cap = outl ? (uint32_t)pk.out_cap : 0u;
   const int out_dtype = pk.out_dtype;
   const uint32_t* flags = outl ? pk.flags + (int64_t)bh * pk.T_cap : nullptr;
@@ -663,14 +662,9 @@ __global__ void __launch_bounds__(256, 3) prefill_expand_kernel(const ExpandPara
   // ... of a flagged chunk from its payload entry (an entry the encoder dropped reads as 0)
   auto payload_of = [&](uint32_t slot) {
     if (slot >= cap) return make_uint2(0u, 0u);
-    if (out32) {
-      const float4 v = *reinterpret_cast<const float4*>(vals + (int64_t)slot * 16);
-      return make_uint2(pack_half2(v.x * mul, v.y * mul), pack_half2(v.z * mul, v.w * mul));
-    }
     return *reinterpret_cast<const uint2*>(vals + (int64_t)slot * 8);
   };
-  auto payload_half = [&](uint2 v) {           // (16-bit entries are converted when they are used)
-    if (out32) return v;
+  auto payload_half = [&](uint2 v) {           // (converted when they are used)
     const float2 a = pair16_to_float2(v.x, out_dtype), d = pair16_to_float2(v.y, out_dtype);
     return make_uint2(pack_half2(a.x * mul, a.y * mul), pack_half2(d.x * mul, d.y * mul));
   };
@@ -792,6 +786,12 @@ bool prefill_plan(const hqmq_attn_args* a, PrefillPlan& pl) {
   const int rows = a->layout == 0 ? 24 * a->K.S : a->K_size;
   if ((a->d != 64 && a->d != 128) || a->T_q < kPrefillMinQueries || a->T_kv < 1 || a->partials_only || a->kv_splits > 0) return false;
   if (rows > kPrefillMaxTable) return false;
+  // Outliers are fp16 operands here: exact for a 16-bit side buffer, 11 of 24 bits of one in fp32, which the decode kernels
+  // add in fp32.  The generic one of those also keeps fp32 queries for the outliers of K.  Such calls stay with them.
+  if (a->layout == 0) {
+    if ((a->K.flags && a->K.out_dtype == HQMQ_F32) || (a->V.flags && a->V.out_dtype == HQMQ_F32)) return false;
+    if (a->K.flags && a->q_dtype == HQMQ_F32 && !staged_kernel(a)) return false;
+  }
   PrefillParams& p = pl.p;
   memset(&p, 0, sizeof(p));
   p.Hkv = a->H_kv; p.G = G; p.Tq = a->T_q; p.Tkv = a->T_kv; p.causal = a->causal; p.window = a->window;

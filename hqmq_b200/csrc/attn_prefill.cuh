@@ -49,6 +49,8 @@ struct PrefillPlan {
 // The plan of a call that takes this path, or false.
 bool prefill_plan(const hqmq_attn_args* a, PrefillPlan& pl);
 int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspace, float qscale, uint32_t epoch, cudaStream_t st);
+// The staged decode kernel that a call would take, or nullptr where that is the generic one (attn.cu).
+const void* staged_kernel(const hqmq_attn_args* a);
 // Raises a kernel's dynamic shared-memory limit to the device's maximum, once per kernel and device (attn.cu).
 cudaError_t raise_smem_limit(const void* kernel, size_t smem);
 

@@ -144,6 +144,35 @@ def test_validation_returns_error_codes_without_launching(built_lib):
     assert L.hqmq_unpack(C.byref(p), 0, 1, None, None, None, None, None) == -1
 
 
+def _prompt_args(T_kv=65536, T_q=16, G=4, S=96, br=4, out_dtype=_lib.BF16, q_dtype=_lib.BF16, flags=True):
+    """Arguments of a prompt call (addresses are never read: only its workspace is asked for)."""
+    a = _lib.AttnArgs()
+    a.struct_size = C.sizeof(_lib.AttnArgs)
+    a.q_dtype, a.o_dtype, a.Q, a.O = q_dtype, q_dtype, 4096, 4096
+    a.B, a.H_q, a.H_kv, a.T_q, a.T_kv, a.d, a.causal, a.r_qmax = 1, 2 * G, 2, T_q, T_kv, 128, 2, (1 << br) - 1
+    for p in (a.K, a.V):
+        p.struct_size = C.sizeof(_lib.Packed)
+        p.B, p.H, p.T_cap, p.n_chunks, p.S, p.radius_bits = 1, 2, (T_kv + 63) & ~63, 32, S, br
+        p.row_bytes, p.scale_dtype, p.out_dtype = packed.row_bytes(32, S, br), _lib.BF16, out_dtype
+        p.codes = p.rs = 4096
+        if flags:
+            p.out_cap, p.flags, p.out_vals, p.out_off, p.out_count = 1024, 4096, 4096, 4096, 4096
+    a.table_K = a.table_V = 4096
+    return a
+
+
+def test_prompts_decode_the_cache_once_only_where_nothing_is_rounded_further(built_lib):
+    """The path that decodes the cache into fp16 operands once per call (its workspace holds them) takes 16-bit outliers, and
+    fp32 queries where the decode kernel would round them as well; the others stay with the decode kernels."""
+    images = 2 * 2 * 65536 * 256
+    need = lambda **kw: _lib.lib().hqmq_attn_workspace_bytes(C.byref(_prompt_args(**kw)))
+    assert need() >= images and need(out_dtype=_lib.F16) >= images and need(flags=False, out_dtype=_lib.F32) >= images
+    assert need(q_dtype=_lib.F32) >= images and need(G=16) >= images and need(S=48) >= images
+    assert need(flags=False, q_dtype=_lib.F32, S=48) >= images
+    for kw in (dict(out_dtype=_lib.F32), dict(q_dtype=_lib.F32, G=16), dict(q_dtype=_lib.F32, S=48)):
+        assert 0 < need(**kw) < images, kw
+
+
 def test_packed_cache_has_no_cpu_path(built_lib):
     """The cache mirrors the reference cache's update() call but never falls back: CPU tensors raise."""
     import hqmq_b200 as hqmq

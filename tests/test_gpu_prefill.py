@@ -74,3 +74,28 @@ def test_tuple_prompt_attention(Hq, Hkv, d, T, Tq, causal, dtype):
     O = torch.empty(Q.shape, dtype=torch.float32, device="cuda")
     hqmq.fused_attention(Q, *args, 63, causal=causal, out=O)
     _check(O, _dense_attention(Q, *dense, causal, None))
+
+
+@pytest.mark.parametrize("scale_dtype,G", [(torch.bfloat16, 4), (torch.float32, 4), (torch.bfloat16, 16)])
+def test_prompt_keeps_fp32_outliers(scale_dtype, G):
+    """Outliers kept in fp32 (without fp16 records) weigh into scores and sums in fp32 whatever the number of query positions.
+    The keys differ by about 1 around 1000 in a flagged chunk: rounding them to 11 bits moves the scores by 2e-2."""
+    B, Hkv, T, Tq, d = 1, 2, 1100, 70, 128
+    g = torch.Generator().manual_seed(87)
+    K, V = torch.randn(B, Hkv, T, d, generator=g), torch.randn(B, Hkv, T, d, generator=g)
+    K[..., :4] += 1000.0
+    V[..., 20:24] *= 50.0
+    q = hqmq.HQMQ(1, Hkv, 96, 4, device="cuda")
+    Kp, Vp = (q.encode(x.cuda(), 0, kv, median_mult=3.0, scale_dtype=scale_dtype, ofrag=False) for kv, x in ((0, K), (1, V)))
+    assert Kp.out_dtype == torch.float32 and Kp.n_outliers() >= B * Hkv * T
+    Q = torch.randn(B, Hkv * G, Tq, d, generator=g).half().float().cuda()
+    O = torch.empty(Q.shape, dtype=torch.float32, device="cuda")
+    hqmq.fused_attention_packed(Q, Kp, Vp, q.tables(0, 0, "cuda")["table16"], q.tables(0, 1, "cuda")["table16"], causal=True, out=O)
+    Kd, Vd = (q.decode(pk, 0, kv).double().repeat_interleave(G, 1) for kv, pk in ((0, Kp), (1, Vp)))
+    s = Q.double() @ Kd.transpose(-1, -2) / math.sqrt(d)
+    want = torch.softmax(s.masked_fill(~torch.ones(Tq, T, dtype=torch.bool, device="cuda").tril(), float("-inf")), -1) @ Vd
+    assert rel_l2(O, want) < 1e-3
+    if scale_dtype == torch.bfloat16 and G == 4:
+        # the first position returns its one key's values; of a flagged chunk all 24 bits but the roundings of P x / P
+        x = V[:, :, 0, 20:24].repeat_interleave(G, 1).cuda()
+        assert ((O[:, :, 0, 20:24] - x).abs() <= 2e-6 * x.abs()).all()
