@@ -71,9 +71,9 @@ __global__ void combine_kernel(const float* __restrict__ parts, int n_parts, int
                                void* __restrict__ out, int64_t os_b, int64_t os_h, int64_t os_t, int Hq, int Tq, int G,
                                int B, int tpu_v, int L, int nw, float* __restrict__ merged,
                                const uint32_t* __restrict__ status, uint32_t epoch, int part_major) {
+  grid_dep_wait();
   const int64_t row = blockIdx.x;
   if (row >= rows) return;
-  grid_dep_wait();
   const bool failed = status != nullptr && *status == epoch;   // the attention kernel gave up on a wait
   const int64_t tq = row % Tq, bh = row / Tq, hq = bh % Hq, b = bh / Hq;
   int n_valid = n_parts;

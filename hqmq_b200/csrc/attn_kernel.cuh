@@ -88,7 +88,9 @@ __host__ __device__ inline void key_range(int Tkv, int Tq, int causal, int windo
 constexpr uint32_t kWaitLimit = 1u << 24;
 // A kernel launched with programmatic stream serialisation may start before its predecessor has finished: what precedes
 // grid_dep_wait() must not touch anything the predecessor writes.  grid_dep_launch() lets the successor start likewise; it
-// comes after the wait, so that a successor's own wait still covers everything before this kernel.
+// comes after the wait, so that a successor's own wait still covers everything before this kernel.  Every CTA waits before it
+// returns: a kernel none of whose CTAs waited could be complete while its predecessor still runs, and what follows on the stream
+// would be ordered behind neither.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -516,8 +516,8 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const PrefillParams 
   const int c = blockIdx.x + 1;
   PfIter it;
   it.init(p, c);
+  grid_dep_wait();                                          // (no CTA may outlive the kernel ahead of it)
   if (it.off == 0) return;                                  // the unit starts with the CTA
-  grid_dep_wait();
   const int64_t s_u = (int64_t)c * p.L - it.off;
   if ((int64_t)(c - 1) * p.L > s_u) return;                 // the unit's first boundary does the merge
   const int c0 = c - 1, n_parts = (int)((s_u + it.n - 1) / p.L) - c0 + 1;

@@ -144,6 +144,31 @@ def test_validation_returns_error_codes_without_launching(built_lib):
     assert L.hqmq_unpack(C.byref(p), 0, 1, None, None, None, None, None) == -1
 
 
+def _kernels():
+    """(file, name, body) of every __global__ function of the library's sources."""
+    csrc = os.path.join(ROOT, "hqmq_b200", "csrc")
+    for f in sorted(os.listdir(csrc)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, f)).read())
+        for m in re.finditer(r"__global__\s+void(?:\s+__launch_bounds__\((?:[^()]|\([^()]*\))*\))?\s*(\w+)\s*\(", text):
+            at = text.index("{", m.end())
+            depth, end = 1, at + 1
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[end], 0)
+                end += 1
+            yield f, m.group(1), text[at:end]
+
+
+def test_dependent_kernels_wait_before_they_return():
+    """A CTA of a kernel that may start ahead of its predecessor's end must not return without having waited for it."""
+    seen = []
+    for f, name, body in _kernels():
+        m = re.search(r"grid_dep_wait\(\)|griddepcontrol\.wait", body)
+        if m:
+            seen.append(name)
+            assert not re.search(r"\breturn\s*;", body[:m.start()]), f"{f}: {name} can return before its wait"
+    assert {"combine_kernel", "prefill_attn_kernel", "prefill_merge_kernel", "append_one_kernel"} <= set(seen), seen
+
+
 def _prompt_args(T_kv=65536, T_q=16, G=4, S=96, br=4, out_dtype=_lib.BF16, q_dtype=_lib.BF16, flags=True):
     """Arguments of a prompt call (addresses are never read: only its workspace is asked for)."""
     a = _lib.AttnArgs()
