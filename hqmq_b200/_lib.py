@@ -18,6 +18,7 @@ OUT_BLOCK = 16
 OFRAG_BYTES = 528
 T_ALIGN = 64
 ATTN_STATIC_SCRATCH_BYTES = 16 << 20
+ATTN_PROMPT_QUERIES = 16
 
 _TORCH_TO_ENUM = {
     torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16, torch.int32: I32,

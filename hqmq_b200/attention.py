@@ -155,8 +155,9 @@ def fused_attention_packed(
                 a.O = out.data_ptr()
             L = _lib.lib()
             with _lib.device_guard(Q.device):
-                # (what a call needs depends on its key count by whole 16-key tiles)
-                if T_now != t_sized and (T_now >> 4 != t_sized >> 4 or (T_now + 15) >> 4 != (t_sized + 15) >> 4):
+                # (what a call of few query positions needs depends on its key count by whole 16-key tiles)
+                if T_now != t_sized and (Q.shape[2] >= _lib.ATTN_PROMPT_QUERIES or T_now >> 4 != t_sized >> 4
+                                         or (T_now + 15) >> 4 != (t_sized + 15) >> 4):
                     nbytes = L.hqmq_attn_workspace_bytes(ref)
                     if nbytes == 0:
                         _lib.check(L.hqmq_attn_decode(ref, None, 0, st), "hqmq_attn_decode")

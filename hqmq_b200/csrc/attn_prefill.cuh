@@ -7,7 +7,7 @@ namespace attn {
 
 constexpr int kPfTok = 128;                       // tokens per operand tile
 constexpr int kPfMaxCtas = 148;                   // one CTA per SM
-constexpr int kPrefillMinQueries = 16;
+constexpr int kPrefillMinQueries = HQMQ_ATTN_PROMPT_QUERIES;
 constexpr int kPrefillMaxTable = 8192;            // codewords per head that fit the expand kernel's shared memory
 constexpr size_t kPrefillImageBytes = (size_t)512 << 20;   // operand images held at a time; larger caches go by groups of (b, head)
 

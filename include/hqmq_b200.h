@@ -343,6 +343,10 @@ typedef struct hqmq_attn_args {
  * Replaces fused_hqmq_attention_triton (src/quantizers/hqmq_attention.py:425-518; kernel
  * :120-265) with the semantics of its oracle fused_hqmq_attention_torch (:68-101).
  */
+/* What a call needs depends on T_kv: below HQMQ_ATTN_PROMPT_QUERIES query positions by its whole 16-key tiles only (equal
+ * T_kv / 16 and (T_kv + 15) / 16 need the same), from there on in no simple way: ask for every T_kv.  A call of that many
+ * positions needs room for its decoded cache; with less, it takes the slower path of fewer positions if that path's need is met. */
+#define HQMQ_ATTN_PROMPT_QUERIES 16
 size_t hqmq_attn_workspace_bytes(const hqmq_attn_args* args);
 int hqmq_attn_decode(const hqmq_attn_args* args, void* workspace, size_t workspace_bytes, void* stream);
 

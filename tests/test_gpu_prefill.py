@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import hqmq_b200 as hqmq
-from hqmq_b200 import kernels
+from hqmq_b200 import _lib, kernels
 from tests.util import make_kv, rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -99,3 +99,23 @@ def test_prompt_keeps_fp32_outliers(scale_dtype, G):
         # the first position returns its one key's values; of a flagged chunk all 24 bits but the roundings of P x / P
         x = V[:, :, 0, 20:24].repeat_interleave(G, 1).cuda()
         assert ((O[:, :, 0, 20:24] - x).abs() <= 2e-6 * x.abs()).all()
+
+
+@pytest.mark.parametrize("Tq", [1, 100])
+def test_repeated_calls_pass_the_workspace_that_their_key_count_needs(Tq, monkeypatch):
+    """One call shape over a growing cache, a key at a time: the cut of the work changes with single keys."""
+    L, Hkv = _lib.lib(), 8
+    q = hqmq.HQMQ(1, Hkv, 96, 4, device="cuda")
+    Kp, Vp = (q.encode(make_kv("randn", (1, Hkv, 1700, 128), seed=88 + kv, dtype=torch.bfloat16).cuda(), 0, kv) for kv in (0, 1))
+    tk, tv = q.tables(0, 0, "cuda")["table16"], q.tables(0, 1, "cuda")["table16"]
+    Q = torch.randn(1, 32, Tq, 128, device="cuda").bfloat16()
+    short, real = [], L.hqmq_attn_decode
+
+    def attn_decode(a, ws, nbytes, st):
+        if nbytes < L.hqmq_attn_workspace_bytes(a):
+            short.append(T)
+        return real(a, ws, nbytes, st)
+    monkeypatch.setattr(L, "hqmq_attn_decode", attn_decode)
+    for T in list(range(1520, 1700)) + [1600, 1100, 1023, 1024]:
+        hqmq.fused_attention_packed(Q, Kp, Vp, tk, tv, causal="bottom_right", T_kv=T)
+    assert not short
