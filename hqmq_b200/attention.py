@@ -134,7 +134,8 @@ def fused_attention_packed(
     _lib.require_cuda(Q, "fused_attention_packed")
     # A decode loop repeats one call shape on one pair of caches: the argument struct and the workspace of such a call
     # are kept with the K cache (per stream: calls on one stream are ordered, calls on different streams get their
-    # own workspace), and a repeat only patches the addresses and the key count.
+    # own workspace), and a repeat only patches the addresses and the key count.  The workspace of a prompt call holds the
+    # whole decoded cache: it comes from the allocator for each call and goes back.
     st = _lib.stream_ptr()
     T_now = K.T if T_kv is None else T_kv
     key = None
@@ -147,7 +148,8 @@ def fused_attention_packed(
                softmax_scale, kv_splits, table_K.data_ptr(), table_V.data_ptr(), K.with_ofrag, V.with_ofrag)
         hit = K._attn_cache.get(key)
         if hit is not None:
-            a, ws_ptr, nbytes, t_sized, ref = hit[:5]
+            a, ws_ptr, nbytes, t_sized, ref, ws = hit[:6]
+            prompt = Q.shape[2] >= _lib.ATTN_PROMPT_QUERIES
             a.Q, a.T_kv = Q.data_ptr(), T_now
             if partials is not None:
                 a.partials = partials.data_ptr()
@@ -156,16 +158,17 @@ def fused_attention_packed(
             L = _lib.lib()
             with _lib.device_guard(Q.device):
                 # (what a call of few query positions needs depends on its key count by whole 16-key tiles)
-                if T_now != t_sized and (Q.shape[2] >= _lib.ATTN_PROMPT_QUERIES or T_now >> 4 != t_sized >> 4
-                                         or (T_now + 15) >> 4 != (t_sized + 15) >> 4):
+                if T_now != t_sized and (prompt or T_now >> 4 != t_sized >> 4 or (T_now + 15) >> 4 != (t_sized + 15) >> 4):
                     nbytes = L.hqmq_attn_workspace_bytes(ref)
                     if nbytes == 0:
                         _lib.check(L.hqmq_attn_decode(ref, None, 0, st), "hqmq_attn_decode")
-                    ws = hit[5]
-                    if nbytes > ws.numel():
+                    if not prompt and nbytes > ws.numel():
                         ws = torch.empty(nbytes + nbytes // 4, dtype=torch.uint8, device=Q.device)
                         ws_ptr = ws.data_ptr()
                     K._attn_cache[key] = (a, ws_ptr, nbytes, T_now, ref, ws, hit[6])
+                if prompt:
+                    ws = torch.empty(nbytes, dtype=torch.uint8, device=Q.device)
+                    ws_ptr = ws.data_ptr()
                 rc = L.hqmq_attn_decode(ref, ws_ptr, nbytes, st)
                 if rc:
                     _lib.check(rc, "hqmq_attn_decode")
@@ -195,8 +198,10 @@ def fused_attention_packed(
     if key is not None:
         if len(K._attn_cache) > 64:
             K._attn_cache.clear()
+        if T_q >= _lib.ATTN_PROMPT_QUERIES:
+            ws = None
         # (the last item keeps what the struct points to alive)
-        K._attn_cache[key] = (a, ws.data_ptr(), nbytes, T_now, C.byref(a), ws, (V, table_K, table_V))
+        K._attn_cache[key] = (a, ws.data_ptr() if ws is not None else 0, nbytes, T_now, C.byref(a), ws, (V, table_K, table_V))
     return partials if partials is not None else O
 
 

@@ -119,3 +119,17 @@ def test_repeated_calls_pass_the_workspace_that_their_key_count_needs(Tq, monkey
     for T in list(range(1520, 1700)) + [1600, 1100, 1023, 1024]:
         hqmq.fused_attention_packed(Q, Kp, Vp, tk, tv, causal="bottom_right", T_kv=T)
     assert not short
+
+
+def test_prompt_calls_leave_no_workspace_behind():
+    """A cache that exists to save memory holds no dense copy of itself after a prompt attended over it."""
+    q = hqmq.HQMQ(1, 8, 96, 4, device="cuda")
+    Kp, Vp = (q.encode(make_kv("randn", (1, 8, 4096, 128), seed=88 + kv, dtype=torch.bfloat16).cuda(), 0, kv) for kv in (0, 1))
+    tk, tv = q.tables(0, 0, "cuda")["table16"], q.tables(0, 1, "cuda")["table16"]
+    for Tq in (200, 300, 200):
+        Q = (torch.randn(1, 32, Tq, 128, device="cuda") / 11).bfloat16()
+        O = [torch.empty_like(Q), torch.empty_like(Q)]
+        before = torch.cuda.memory_allocated()
+        for out in O:
+            hqmq.fused_attention_packed(Q, Kp, Vp, tk, tv, causal=False, out=out)
+        assert torch.cuda.memory_allocated() - before < 1 << 20 and torch.equal(*O)
