@@ -415,10 +415,12 @@ class HQMQQuantizer(KVQuantizer):
                     a, ref, _, ws, nbytes = hit
                     out = torch.empty(shape, dtype=x.dtype, device=x.device)
                     a.x = x.data_ptr()
-                    rc = _lib.lib().hqmq_fake_quant(ref, out.data_ptr(), count.slot(shape, x.device) if count is not None else None,
-                                                    ws, nbytes, st)
+                    block, at = count.slot(x.device, st) if count is not None else (None, 0)
+                    rc = _lib.lib().hqmq_fake_quant(ref, out.data_ptr(), None if block is None else block.address + 4 * at, ws, nbytes, st)
                     if rc:
                         _lib.check(rc, "hqmq_fake_quant")
+                    if block is not None:
+                        count.counted(block, at, shape)
                     return out
         B, H, T, d = shape
         if d % 4 != 0:
@@ -474,39 +476,67 @@ class HQMQQuantizer(KVQuantizer):
         return "_".join(parts)
 
 
+class _CounterBlock:
+    """Zeroed device counters, taken one by one for the calls of one stream (``key``; None: of a graph)."""
+
+    def __init__(self, n, device, key=None):
+        self.counters = torch.zeros(n, dtype=torch.int32, device=device)
+        self.address, self.size, self.taken, self.key = self.counters.data_ptr(), n, 0, key
+
+
 class _OutlierStats:
     """Running mean of the per-call outlier rates (what the reference's wrapper keeps in ``_observed_outlier_rate``), read
     from the caches' device counters only on demand.  What is remembered of a cache is a small record -- its counter
     tensor (B * H words), the count its open calls started from, their number and size -- never the cache itself, so a
     cache that is done with gives its planes back.  Calls of one size on one cache share their growth evenly (exact for
     the sum of their rates, which is all a mean needs); a call of another size closes the group with a copy of the
-    counter on the device.  Records are folded into two host numbers once there are ``_FOLD`` of them."""
+    counter on the device.  Records are folded into two host numbers once there are ``_FOLD`` of them.  Nothing is folded
+    while the calling stream is being captured."""
     _FOLD = 1024
 
     def __init__(self):
         self._open = []             # records with calls that were not accounted yet
         self._closed = []           # (counter at the end, counter or number at the start, calls' size, calls)
         self._sum_rates, self._n = 0.0, 0   # sum of the per-call rates, number of calls
-        self._slots = {}            # per device: (counters, sizes of the calls that took one each)
+        self._blocks = {}           # per device and stream: the block that its fake-quant calls take counters from
+        self._counted = []          # (block, index, chunks) of the fake-quant calls that were launched
         self._lock = threading.Lock()
 
-    def slot(self, shape, device) -> int:
-        """Address of a zeroed device counter for one fake-quant call of that shape."""
+    # A fake-quant call adds its flagged chunks to a counter of its own.  The counters of a stream are filled on that stream;
+    # a call is accounted only once it is launched, and its record holds the block.  A captured call's counter belongs to the
+    # graph, which zeroes it at every replay: what is read is the last one's count (nothing meaningful before the first).
+    def slot(self, device, stream):
+        """(block, index) of a zeroed counter for one call on the current stream, ``stream``."""
+        if torch.cuda.is_current_stream_capturing():
+            return _CounterBlock(1, device), 0
+        key, rolled = (device, stream), False
         with self._lock:
-            got = self._slots.get(device)
-            if got is None or len(got[1]) >= self._FOLD:
-                if got is not None:
-                    self._fold_slots(device)
-                got = self._slots[device] = (torch.zeros(self._FOLD, dtype=torch.int32, device=device), [])
-            got[1].append(shape[0] * shape[1] * shape[2] * (shape[3] // 4))
-            return got[0].data_ptr() + 4 * (len(got[1]) - 1)
+            block = self._blocks.get(key)
+            if block is None or block.taken == block.size:
+                if len(self._blocks) >= 64:
+                    self._blocks.clear()
+                rolled = block is not None
+                block = self._blocks[key] = _CounterBlock(self._FOLD, device, key)
+            at, block.taken = block.taken, block.taken + 1
+        if rolled:
+            self._fold(key)             # (this is the stream of those calls: the copy is behind their kernels)
+        return block, at
 
-    def _fold_slots(self, device):
-        counters, sizes = self._slots.pop(device)
-        torch.cuda.synchronize(device)              # (calls of other streams may still be counting)
-        for flagged, total in zip(counters[:len(sizes)].tolist(), sizes):
-            self._sum_rates += flagged / max(1, total)
-        self._n += len(sizes)
+    def counted(self, block, at, shape):
+        """The call that took the counter is launched."""
+        with self._lock:
+            self._counted.append((block, at, shape[0] * shape[1] * shape[2] * (shape[3] // 4)))
+
+    def _fold(self, key=None):
+        """Account the launched calls of one stream (None: of all); their kernels are complete or ahead on this stream."""
+        with self._lock:
+            done = [r for r in self._counted if key is None or r[0].key == key]
+            self._counted = [r for r in self._counted if not (key is None or r[0].key == key)]
+        values = {b: b.counters.tolist() for b in {r[0] for r in done}}
+        with self._lock:
+            for block, at, total in done:
+                self._sum_rates += values[block][at] / max(1, total)
+            self._n += len(done)
 
     # a record: [counter tensor, count at the start (number or tensor), calls, chunks per call]
     def begin(self, pk, total_chunks: int):
@@ -531,7 +561,7 @@ class _OutlierStats:
             rec[3] = total_chunks
             self._open.append(rec)
         rec[2] += 1
-        if len(self._open) + len(self._closed) >= self._FOLD:
+        if len(self._open) + len(self._closed) >= self._FOLD and not torch.cuda.is_current_stream_capturing():
             self._sync()
 
     # the same for the two caches of a layer: a repeated append only counts its calls, and the counters of a pair that was
@@ -565,13 +595,21 @@ class _OutlierStats:
     def push_count(self, counter: torch.Tensor, total_chunks: int):
         """A finished fake-quant call that went through a cache: only the counter is kept."""
         self._closed.append((counter, 0.0, total_chunks, 1))
-        if len(self._open) + len(self._closed) >= self._FOLD:
+        if len(self._open) + len(self._closed) >= self._FOLD and not torch.cuda.is_current_stream_capturing():
             self._sync()
 
-    def _sync(self):
+    def _read(self):
+        if torch.cuda.is_available() and torch.cuda.is_current_stream_capturing():
+            return
         with self._lock:
-            for device in list(self._slots):
-                self._fold_slots(device)
+            devices = {r[0].counters.device for r in self._counted}
+        devices |= {t.device for t in [r[0] for r in self._open + self._closed] if t.is_cuda}
+        for device in devices:
+            torch.cuda.synchronize(device)              # (calls of other streams may still be counting)
+        self._fold()
+        self._sync()
+
+    def _sync(self):
         done, self._closed = self._closed, []
         recs = {id(r): r for r in self._open if r[2]}.values()
         self._open = []
@@ -598,12 +636,12 @@ class _OutlierStats:
 
     @property
     def rate(self):
-        self._sync()
+        self._read()
         return self._sum_rates / self._n if self._n else 0.0
 
     @property
     def n(self):
-        self._sync()
+        self._read()
         return self._n
 
 
