@@ -230,6 +230,11 @@ def stream_ptr() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+# Whether torch's current stream is being captured.  A captured call takes its workspace from the graph's own pool: one that is
+# kept with a cache may be replaced or dropped while the graph still replays.
+capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", torch.cuda.is_current_stream_capturing)
+
+
 def read_status(workspace: torch.Tensor) -> int:
     """First word of a workspace after synchronising the current stream (see hqmq_read_status)."""
     st = C.c_uint32(0)

@@ -248,3 +248,43 @@ def test_paired_prompts_equal_single_tensor_calls(B, H, T, d, S, br, outliers):
         names += ["ofrag", "ofrag_off"] if a.with_ofrag else []
         for name in names:
             assert torch.equal(getattr(a, name), getattr(b, name)), name
+
+
+def test_captured_calls_own_their_workspaces():
+    """A graph of an append, an attention and a fake-quant call replays with the same results after the buffers kept for
+    repeated calls are gone, and writes nothing into memory that was handed out again."""
+    B, H, d, S, br = 2, 2, 128, 96, 4
+    q = hqmq.HQMQ(1, H, S, br, device="cuda")
+    Kp, Vp = (q.new_cache(B, 1024, d, "cuda", with_outliers=True, ofrag=kv == 0) for kv in (0, 1))
+    x = [make_kv("spiky", (B, H, T, d), seed=120 + T, dtype=torch.bfloat16).cuda() for T in (600, 40, 700)]
+    q.encode_pair(x[0], x[0], 0, Kp, Vp, median_mult=3.0)
+    tk, tv = q.tables(0, 0, "cuda")["table16"], q.tables(0, 1, "cuda")["table16"]
+    Q = (torch.randn(B, 8, 1, d, device="cuda") / math.sqrt(d)).bfloat16()
+
+    def step():
+        at = Kp.T, Vp.T
+        q.encode_pair(x[1], x[1], 0, Kp, Vp, median_mult=3.0)
+        q.encode(x[1], 0, 0, out=Kp, median_mult=3.0)
+        o = hqmq.fused_attention_packed(Q, Kp, Vp, tk, tv, kv_splits=4, T_kv=640), q._qdq(x[2], 0, 0, median_mult=3.0)
+        Kp.T, Vp.T = at
+        return o
+    counts = Kp.out_count.clone(), Vp.out_count.clone()
+
+    def rewind():
+        Kp.out_count.copy_(counts[0]), Vp.out_count.copy_(counts[1])
+    want = step()
+    rewind()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step()
+    kept = [t for c in (Kp._enc_cache, Kp._attn_cache, q._qdq_cache) for e in c.values() for t in e if isinstance(t, torch.Tensor)]
+    sizes = [t.numel() for t in kept]
+    assert len(sizes) >= 4
+    del kept
+    Kp._enc_cache.clear(), Kp._attn_cache.clear(), q._qdq_cache.clear()
+    canaries = [torch.zeros(n, dtype=torch.uint8, device="cuda") for n in sizes for _ in range(4)]
+    for _ in range(2):
+        rewind()
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert not any(c.any() for c in canaries)
