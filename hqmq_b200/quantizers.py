@@ -14,7 +14,7 @@ import ctypes as C
 import math
 import threading
 from abc import ABC, abstractmethod
-from itertools import product
+from itertools import count, product
 from typing import Optional, Tuple
 
 import torch
@@ -70,6 +70,12 @@ def _norm4(v: torch.Tensor) -> torch.Tensor:
     return ssq.double().sqrt().float()
 
 
+_states = count()
+# what a kept call was validated and laid out for
+_CALL_STATE = frozenset(("training", "magnitude_mode", "jl_dim", "log_radius", "robust_radius_scale", "n_heads", "secondary_size",
+                         "radius_bits"))
+
+
 class HQMQQuantizer(KVQuantizer):
     """Hurwitz quaternion multiplicative quantizer; direction of each 4-chunk = q_p * q_s."""
 
@@ -103,6 +109,16 @@ class HQMQQuantizer(KVQuantizer):
         self._tables: dict = {}
         self._qdq_cache: dict = {}      # argument structs and workspaces of repeated fake-quant calls, per thread and stream
 
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        if name in _CALL_STATE:
+            self._new_state()
+
+    def _new_state(self):
+        """Calls kept so far are void: those of caches are found by this number, which no other quantizer or state has."""
+        self._state = next(_states)
+        self.__dict__.get("_qdq_cache", {}).clear()
+
     # ---- reference plumbing ---------------------------------------------------------------
     def trainable_parameters(self):
         return [self.secondary_raw]
@@ -111,11 +127,10 @@ class HQMQQuantizer(KVQuantizer):
         self.training = training
         if tau is not None:
             self.tau = tau
-        self._qdq_cache.clear()         # (a repeated call does not look at the flags again)
 
     def _refresh_rotations(self):
         self._tables.clear()
-        self._qdq_cache.clear()
+        self._new_state()
 
     def _unsupported(self) -> Optional[str]:
         if self.magnitude_mode != "unit":
@@ -247,7 +262,7 @@ class HQMQQuantizer(KVQuantizer):
         # (calls on one cache are ordered on a stream anyway, since they append to the same planes).
         fast_key = None
         if out is not None and med_out is None and med_in is None and not check_status and x.dim() == 4 and x.shape[2] <= 64:
-            fast_key = (id(self), layer_idx, kv, tuple(x.shape), x.dtype, x.stride(), median_mult, search, quantile)
+            fast_key = (self._state, layer_idx, kv, tuple(x.shape), x.dtype, x.stride(), median_mult, search, quantile)
             hit = out._enc_cache.get(fast_key)
             if hit is not None:
                 a, ws, nbytes = hit
@@ -311,7 +326,7 @@ class HQMQQuantizer(KVQuantizer):
         launches between them."""
         # (one dictionary look-up on everything that decides the call's shape: a repeated append goes straight to the library)
         shape, ks, vs = k.shape, k.stride(), v.stride()
-        key = ("pair", id(self), id(out_v), layer_idx, shape, v.shape, k.dtype, v.dtype, ks, vs, k.device, v.device, median_mult, quantile)
+        key = ("pair", self._state, id(out_v), layer_idx, shape, v.shape, k.dtype, v.dtype, ks, vs, k.device, v.device, median_mult, quantile)
         hit = out_k._enc_cache.get(key)
         if hit is None:
             # (beyond 16 M values a tensor's own launches fill the chip, and two workspaces would be held instead of one)

@@ -288,3 +288,44 @@ def test_captured_calls_own_their_workspaces():
         graph.replay()
         assert all(torch.equal(a, b) for a, b in zip(got, want))
     assert not any(c.any() for c in canaries)
+
+
+def test_kept_calls_end_with_the_state_they_were_made_for():
+    """A repeated call is refused once the quantizer trains (its attribute set directly or by set_training), and uses the
+    codebook of the moment: after its rotations were refreshed, and for another quantizer at the same address."""
+    B, H, d = 2, 2, 64
+    x = torch.randn(B, H, 1, d, generator=torch.Generator().manual_seed(9)).bfloat16().cuda()
+
+    def appended(q, dst, pair):
+        t0 = dst[0].T
+        if pair:
+            q.encode_pair(x, x, 0, *dst)
+        else:
+            q.encode(x, 0, 0, out=dst[0])
+        return dst[0].to_reference(t0, 1)[0]
+    for pair in (False, True):
+        q = hqmq.HQMQ(1, H, 96, 4, device="cuda", seed=1)
+        dst = q.new_cache(B, 64, d, "cuda"), q.new_cache(B, 64, d, "cuda")
+        first = appended(q, dst, pair)
+        assert torch.equal(appended(q, dst, pair), first)
+        dense = q.quantize_K(x, 0)
+        for start, stop in ((lambda: setattr(q, "training", True), lambda: setattr(q, "training", False)),
+                            (lambda: q.set_training(True), lambda: q.set_training(False)),
+                            (lambda: setattr(q, "log_radius", True), lambda: setattr(q, "log_radius", False))):
+            start()
+            with pytest.raises(NotImplementedError):
+                appended(q, dst, pair)
+            with pytest.raises(NotImplementedError):
+                q.quantize_K(x, 0)
+            stop()
+        assert torch.equal(appended(q, dst, pair), first) and torch.equal(q.quantize_K(x, 0), dense)
+        other = hqmq.HQMQ(1, H, 96, 4, device="cuda", seed=2)
+        want = other.encode(x, 0, 0).to_reference()[0]
+        assert not torch.equal(want, first)
+        q.secondary_raw.data.copy_(other.secondary_raw)
+        q._refresh_rotations()
+        assert torch.equal(appended(q, dst, pair), want) and torch.equal(q.quantize_K(x, 0), other.quantize_K(x, 0))
+        for seed in range(3, 20):               # (a freed quantizer's address is taken again soon)
+            del q
+            q = hqmq.HQMQ(1, H, 96, 4, device="cuda", seed=seed)
+            assert torch.equal(appended(q, dst, pair), q.encode(x, 0, 0).to_reference()[0]), seed
