@@ -133,8 +133,8 @@ def fused_attention_packed(
     (o[d], m, l) is written there instead of O, for merging across sequence shards."""
     _lib.require_cuda(Q, "fused_attention_packed")
     # A decode loop repeats one call shape on one pair of caches: the argument struct and the workspace of such a call
-    # are kept with the K cache (per stream: calls on one stream are ordered, calls on different streams get their
-    # own workspace), and a repeat only patches the addresses and the key count.  The workspace of a prompt call holds the
+    # are kept with the K cache (per stream and thread: calls on one stream are ordered, calls on different streams get their
+    # own workspace, and a thread patches no struct that another one's call is reading), and a repeat only patches the addresses and the key count.  The workspace of a prompt call holds the
     # whole decoded cache: it comes from the allocator for each call and goes back.
     st = _lib.stream_ptr()
     T_now = K.T if T_kv is None else T_kv
@@ -144,7 +144,7 @@ def fused_attention_packed(
         if out is None and partials is None:
             out = torch.empty_like(Q)
         dst = partials if partials is not None else out
-        key = (id(V), st, Q.dtype, Q.shape, q_stride, dst.dtype, dst.stride(), partials is not None, causal, window,
+        key = (id(V), st, threading.get_ident(), Q.dtype, Q.shape, q_stride, dst.dtype, dst.stride(), partials is not None, causal, window,
                softmax_scale, kv_splits, table_K.data_ptr(), table_V.data_ptr(), K.with_ofrag, V.with_ofrag)
         hit = K._attn_cache.get(key)
         if hit is not None:

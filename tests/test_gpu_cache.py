@@ -2,11 +2,13 @@
 planes.  Attention over the cache must match the oracle run on the oracle's own encoding of the same calls, and
 the dense view must equal what the reference's cache would hold (its fake-quantised tensors)."""
 import math
+import threading
 
 import pytest
 import torch
 
 import hqmq_b200 as hqmq
+from hqmq_b200 import _lib
 from hqmq_b200.cache import PackedKVCache
 from oracle import hqmq_oracle as orc
 from tests.util import make_kv
@@ -329,3 +331,35 @@ def test_kept_calls_end_with_the_state_they_were_made_for():
             del q
             q = hqmq.HQMQ(1, H, 96, 4, device="cuda", seed=seed)
             assert torch.equal(appended(q, dst, pair), q.encode(x, 0, 0).to_reference()[0]), seed
+
+
+def test_threads_of_one_stream_attend_over_one_cache(monkeypatch):
+    """A repeated call of one thread while another thread's repeated call of the same shape is on its way into the library."""
+    q = hqmq.HQMQ(1, 2, 96, 4, device="cuda")
+    Kp, Vp = (q.encode(make_kv("randn", (1, 2, 300, 128), seed=130 + kv, dtype=torch.bfloat16).cuda(), 0, kv) for kv in (0, 1))
+    tk, tv = q.tables(0, 0, "cuda")["table16"], q.tables(0, 1, "cuda")["table16"]
+    Qs = [(torch.randn(1, 4, 1, 128, device="cuda") / 11).bfloat16() for _ in range(2)]
+    want = [hqmq.fused_attention_packed(Q, Kp, Vp, tk, tv) for Q in Qs]
+    go, gone, got = threading.Event(), threading.Event(), {}
+
+    def second():
+        got["warm"] = hqmq.fused_attention_packed(Qs[1], Kp, Vp, tk, tv)
+        go.wait()
+        got["out"] = hqmq.fused_attention_packed(Qs[1], Kp, Vp, tk, tv)
+        gone.set()
+    L = _lib.lib()
+    real, thread, me = L.hqmq_attn_decode, threading.Thread(target=second), threading.get_ident()
+    thread.start()
+    while "warm" not in got:
+        pass
+
+    def attn_decode(*args):
+        if threading.get_ident() == me:
+            go.set()
+            gone.wait()
+        return real(*args)
+    monkeypatch.setattr(L, "hqmq_attn_decode", attn_decode)
+    out = torch.full_like(Qs[0], 7)
+    hqmq.fused_attention_packed(Qs[0], Kp, Vp, tk, tv, out=out)
+    thread.join()
+    assert torch.equal(got["out"], want[1]) and torch.equal(out, want[0])
