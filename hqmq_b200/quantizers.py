@@ -168,6 +168,8 @@ class HQMQQuantizer(KVQuantizer):
         reference's order, 'table16' (H,24S,4) fp16 in the native index order."""
         if not isinstance(device, torch.device):
             device = torch.device(device)
+        if device.index is None and device.type == "cuda":       # ("cuda" and "cuda:0" name one set of tables)
+            device = torch.device("cuda", torch.cuda.current_device())
         key = (layer_idx, kv, device)
         t = self._tables.get(key)
         if t is None:

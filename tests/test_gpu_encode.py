@@ -559,3 +559,10 @@ def test_large_call_pieces(B, H, T, d, kind):
         x = make_kv(kind, (B, H, T, d), seed=5, dtype=torch.bfloat16)
     S, br = (24, 3) if d == 128 else (96, 4)
     _threshold_compare(x, S, br, 3.0)
+
+
+def test_tables_are_built_once_per_device():
+    q = hqmq.HQMQ(1, 2, 24, 3, device="cuda")
+    t = q.tables(0, 0, "cuda")
+    q.quantize_K(torch.randn(1, 2, 3, 32, device="cuda"), 0)
+    assert q.tables(0, 0, "cuda:0") is t and q.tables(0, 0, torch.device("cuda")) is t and len(q._tables) == 1
