@@ -230,9 +230,13 @@ def stream_ptr() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
-# Whether torch's current stream is being captured.  A captured call takes its workspace from the graph's own pool: one that is
-# kept with a cache may be replaced or dropped while the graph still replays.
-capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", torch.cuda.is_current_stream_capturing)
+_current_is_capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", torch.cuda.is_current_stream_capturing)
+
+
+def capturing(stream: int) -> bool:
+    """Whether torch's current stream, ``stream``, is being captured.  A captured call takes its workspace from the graph's
+    own pool: one that is kept with a cache may be replaced or dropped while the graph still replays."""
+    return stream != 0 and _current_is_capturing()          # (the legacy default stream cannot be captured)
 
 
 def read_status(workspace: torch.Tensor) -> int:

@@ -166,7 +166,7 @@ def fused_attention_packed(
                         ws = torch.empty(nbytes + nbytes // 4, dtype=torch.uint8, device=Q.device)
                         ws_ptr = ws.data_ptr()
                     K._attn_cache[key] = (a, ws_ptr, nbytes, T_now, ref, ws, hit[6])
-                if prompt or _lib.capturing():
+                if prompt or (st and _lib.capturing(st)):
                     ws = torch.empty(nbytes, dtype=torch.uint8, device=Q.device)
                     ws_ptr = ws.data_ptr()
                 rc = L.hqmq_attn_decode(ref, ws_ptr, nbytes, st)
@@ -195,7 +195,7 @@ def fused_attention_packed(
     if partials is not None:
         a.partials_only, a.partials = 1, partials.data_ptr()
     ws, nbytes = _run(a, Q.device)
-    if key is not None and not _lib.capturing():
+    if key is not None and not _lib.capturing(st):
         if len(K._attn_cache) > 64:
             K._attn_cache.clear()
         if T_q >= _lib.ATTN_PROMPT_QUERIES:

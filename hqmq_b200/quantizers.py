@@ -273,9 +273,10 @@ class HQMQQuantizer(KVQuantizer):
                     raise _lib.HqmqError(f"hqmq_b200: cache capacity {out.T_cap} exceeded ({out.T} + {T})")
                 a.x, a.t_start = x.data_ptr(), out.T
                 with _lib.device_guard(x.device):
-                    if _lib.capturing():
+                    st = _lib.stream_ptr()
+                    if _lib.capturing(st):
                         ws = torch.empty_like(ws)
-                    _lib.check(_lib.lib().hqmq_encode(C.byref(a), ws.data_ptr(), nbytes, _lib.stream_ptr()), "hqmq_encode")
+                    _lib.check(_lib.lib().hqmq_encode(C.byref(a), ws.data_ptr(), nbytes, st), "hqmq_encode")
                 out.T += T
                 return out
         why = self._unsupported()
@@ -313,7 +314,7 @@ class HQMQQuantizer(KVQuantizer):
             _lib.check(L.hqmq_encode(C.byref(a), ws.data_ptr(), nbytes, _lib.stream_ptr()), "hqmq_encode")
             if check_status and nbytes and (_lib.read_status(ws) & 1):
                 raise _lib.HqmqError(f"hqmq_b200: outlier side buffer too small (out_cap={out.out_cap} chunks per (b, h))")
-        if fast_key is not None and x is x_given and not _lib.capturing():
+        if fast_key is not None and x is x_given and not _lib.capturing(_lib.stream_ptr()):
             a._keep = (a._keep[1],)              # the tables: not this call's input, nor the cache that holds the struct
             out._enc_cache[fast_key] = (a, ws, nbytes)
         out.T += T
@@ -356,7 +357,7 @@ class HQMQQuantizer(KVQuantizer):
             # cache's memory to the garbage collector)
             ak._keep, av._keep = (ak._keep[1],), (av._keep[1], out_v)
             hit = (ak, av, C.byref(ak), C.byref(av), ws.data_ptr(), nbytes, ws)
-            if shape[2] <= 64 and not _lib.capturing():          # (a prompt is not repeated on its cache)
+            if shape[2] <= 64 and not _lib.capturing(_lib.stream_ptr()):         # (a prompt is not repeated on its cache)
                 out_k._enc_cache[key] = hit
         ak, av, rk, rv, ws_ptr, nbytes, ws = hit
         T, tk, tv = shape[2], out_k.T, out_v.T
@@ -364,10 +365,11 @@ class HQMQQuantizer(KVQuantizer):
             raise _lib.HqmqError(f"hqmq_b200: cache capacity {out_k.T_cap} exceeded ({tk} + {T})")
         ak.x, ak.t_start, av.x, av.t_start = k.data_ptr(), tk, v.data_ptr(), tv
         with _lib.device_guard(k.device):
-            if _lib.capturing():
+            st = _lib.stream_ptr()
+            if st and _lib.capturing(st):
                 ws = torch.empty_like(ws)
                 ws_ptr = ws.data_ptr()
-            rc = _lib.lib().hqmq_encode_pair(rk, rv, ws_ptr, nbytes, _lib.stream_ptr())
+            rc = _lib.lib().hqmq_encode_pair(rk, rv, ws_ptr, nbytes, st)
             if rc:
                 _lib.check(rc, "hqmq_encode_pair")
         out_k.T, out_v.T = tk + T, tv + T
@@ -435,7 +437,7 @@ class HQMQQuantizer(KVQuantizer):
                 # (kept entries were made for aligned addresses: a view at another offset takes the long way round)
                 if hit is not None and x.data_ptr() & 15 == 0:
                     a, ref, buf, ws, nbytes = hit
-                    capturing = _lib.capturing()
+                    capturing = st and _lib.capturing(st)
                     if capturing:
                         buf = torch.empty_like(buf)
                         ws = buf.data_ptr()
@@ -587,7 +589,7 @@ class _OutlierStats:
             rec[3] = total_chunks
             self._open.append(rec)
         rec[2] += 1
-        if len(self._open) + len(self._closed) >= self._FOLD and not _lib.capturing():
+        if len(self._open) + len(self._closed) >= self._FOLD and not _lib.capturing(_lib.stream_ptr()):
             self._sync()
 
     # the same for the two caches of a layer: a repeated append only counts its calls, and the counters of a pair that was
@@ -621,11 +623,11 @@ class _OutlierStats:
     def push_count(self, counter: torch.Tensor, total_chunks: int):
         """A finished fake-quant call that went through a cache: only the counter is kept."""
         self._closed.append((counter, 0.0, total_chunks, 1))
-        if len(self._open) + len(self._closed) >= self._FOLD and not _lib.capturing():
+        if len(self._open) + len(self._closed) >= self._FOLD and not _lib.capturing(_lib.stream_ptr()):
             self._sync()
 
     def _read(self):
-        if torch.cuda.is_available() and _lib.capturing():
+        if torch.cuda.is_available() and torch.cuda.is_current_stream_capturing():
             return
         with self._lock:
             devices = {r[0].counters.device for r in self._counted}
