@@ -70,10 +70,13 @@ class PackedKVCache:
 
     def check(self) -> None:
         """Synchronise and raise if some side buffer was too small for the outliers it was given (rows, flags
-        and counts are complete then, but payload entries beyond the capacity were dropped)."""
+        and counts are complete then, but payload entries beyond the capacity were dropped), or if an update gave up on
+        a bounded wait of the encoder (its tokens have a scale of NaN, which no input gives)."""
         from ._lib import HqmqError
         for layer, pair in self._layers.items():
             for name, pk in zip("KV", pair):
+                if bool(pk.rs[:pk.B * pk.H * pk.T_cap].view(pk.B, pk.H, -1)[:, :, :pk.T].isnan().any()):
+                    raise HqmqError(f"hqmq_b200: an update of layer {layer} {name} gave up on a bounded wait")
                 if pk.with_outliers and int(pk.out_count.max()) > pk.out_cap:
                     raise HqmqError(f"hqmq_b200: outlier side buffer of layer {layer} {name} overflowed "
                                     f"({int(pk.out_count.max())} > {pk.out_cap} chunks per (b, h)); raise outlier_capacity")

@@ -46,7 +46,7 @@ template <int DT, int IB, int RB, bool DENSE>
 __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const FusedPair pr, const Maps24 maps, const Mul24 nmul) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t s_bar;
-  __shared__ uint32_t s_warp[32], s_sel[4], s_flagged;
+  __shared__ uint32_t s_warp[32], s_sel[4], s_flagged, s_gave_up;
   const FusedArgs& a = pr.t[blockIdx.y];
   if (a.gate && *a.gate == 0u) return;
   const EncGeom& g = a.g;
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
     fused_bulk(d, a.lut + kLutOffRows, b_rows, bar);
     fused_bulk(d + b_rows, head + 16, b_cells, bar);
     if (b_cands) fused_bulk(d + b_rows + b_cells, head + 16 + (size_t)kLutCellCap * 2, b_cands, bar);
-    s_flagged = 0u;
+    s_flagged = s_gave_up = 0u;
   }
   LutView L;
   L.rows = reinterpret_cast<const uint32_t*>(slut); L.cells = reinterpret_cast<const uint16_t*>(slut + b_rows);
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
         do {
           asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bars + h) : "memory");
         } while (seen < want && ++polls < kFusedPolls);
-        if (seen < want) atomicOr(a.status, 2u);
+        if (seen < want) s_gave_up = 1u;
       }
       __syncthreads();
       // scan: two bins per thread
@@ -214,7 +214,29 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
     uint32_t ok = 0u, tries = 0u;
     while (!ok && ++tries < (1u << 24))
       asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar) : "memory");
-    if (!ok) { if (threadIdx.x == 0) atomicOr(a.status, 2u); return; }
+    if (__syncthreads_or(!ok || s_gave_up)) {
+      // a bounded wait ran out: what this CTA's tokens decode to is NaN (rows of index 0, nothing flagged), and the status says so
+      if (threadIdx.x == 0) {
+        atomicOr(a.status, 2u);
+        if (part == 0 && a.med_out) a.med_out[h] = NAN;
+      }
+      for (int w = w0 + warp; w < w1; w += kEnc32Warps) {
+        int b, t;
+        locate(w, b, t);
+        if (t >= g.T_new) continue;
+        if constexpr (DENSE) {
+          *reinterpret_cast<uint2*>(a.out + ((((int64_t)b * g.H + h) * g.T_new + t) * g.n + c) * 4) = make_uint2(0x7fff7fffu, 0x7fff7fffu);
+        } else {
+          const int64_t row = ((int64_t)b * g.H + h) * a.dst.T_cap + a.t_start + t;
+          for (int i = c; i < a.dst.row_bytes >> 2; i += g.n) reinterpret_cast<uint32_t*>(a.dst.codes + row * a.dst.row_bytes)[i] = 0u;
+          if (c == 0) {
+            store_scale(a.dst, row, NAN);
+            if (a.dst.flags) a.dst.flags[row] = 0u;
+          }
+        }
+      }
+      return;
+    }
   }
   const float inv_S = 1.0f / (float)S;
   uint32_t* myrow = rows + warp * kMaxRowWords;

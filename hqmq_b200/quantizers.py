@@ -254,7 +254,8 @@ class HQMQQuantizer(KVQuantizer):
         ``ofrag``: also keep the flagged chunks of every complete 16-token block as tensor-core operand
         records for the decode-attention kernel (K tensors only use them).  Default: on for a fresh K
         cache with Med3x, off otherwise.  ``check_status``: synchronise and raise if the outlier side buffer
-        overflowed (otherwise the caller may compare ``out_count`` with ``out_cap`` itself).  ``quantile``: flag
+        overflowed (otherwise the caller may compare ``out_count`` with ``out_cap`` itself) or the encoder gave up on a
+        bounded wait (the scales of the tokens concerned are NaN).  ``quantile``: flag
         against ``median_mult`` times ``torch.quantile(norms, quantile)`` per head instead of the median (the
         reference wrapper's "fraction" mode: quantile = 1 - fraction, median_mult = 1).  ``med_in``: (H,) fp32
         medians to flag against instead of this call's own (``hqmq_b200.dist.split_batch_median`` computes them
@@ -312,7 +313,10 @@ class HQMQQuantizer(KVQuantizer):
             nbytes = L.hqmq_encode_workspace_bytes(C.byref(a))
             ws = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=x.device)
             _lib.check(L.hqmq_encode(C.byref(a), ws.data_ptr(), nbytes, _lib.stream_ptr()), "hqmq_encode")
-            if check_status and nbytes and (_lib.read_status(ws) & 1):
+            status = _lib.read_status(ws) if check_status and nbytes else 0
+            if status & 2:
+                raise _lib.HqmqError("hqmq_b200: the encoder gave up on a bounded wait; the tokens concerned decode to NaN")
+            if status & 1:
                 raise _lib.HqmqError(f"hqmq_b200: outlier side buffer too small (out_cap={out.out_cap} chunks per (b, h))")
         if fast_key is not None and x is x_given and not _lib.capturing(_lib.stream_ptr()):
             a._keep = (a._keep[1],)              # the tables: not this call's input, nor the cache that holds the struct

@@ -263,8 +263,10 @@ int hqmq_med3x_select(int H, int level, uint64_t n_total, float median_mult, voi
  * printed or trapped on.  This copies that word to the host after synchronising `stream`.
  *   workspace of hqmq_encode:       bit 0 = the outlier side buffer (out_cap) was too small; rows,
  *                                   flags and counts are complete, payload entries beyond the
- *                                   capacity were dropped; bit 1 = the call gave up on a bounded wait
- *                                   between its thread blocks, what it wrote is not valid
+ *                                   capacity were dropped; bit 1 = the call gave up on a bounded wait;
+ *                                   the tokens concerned have a scale of NaN (and the dense tensor of
+ *                                   hqmq_fake_quant NaN in their place; its status word is defined for
+ *                                   calls with a threshold of their own)
  *   workspace of hqmq_attn_decode:  non-zero = some call on this workspace gave up on a bounded wait
  *                                   for a staged copy; the output rows of that call are not valid (NaN where
  *                                   a merge still ran, untouched elsewhere)

@@ -363,3 +363,27 @@ def test_threads_of_one_stream_attend_over_one_cache(monkeypatch):
     hqmq.fused_attention_packed(Qs[0], Kp, Vp, tk, tv, out=out)
     thread.join()
     assert torch.equal(got["out"], want[1]) and torch.equal(out, want[0])
+
+
+def test_an_encoder_that_gave_up_is_reported(monkeypatch):
+    """Bit 1 of an encode call's status (a bounded wait ran out) raises where the caller asks for the status, and the NaN
+    scales it leaves are found by the cache's check; inputs of any value give a scale that is a number."""
+    q = hqmq.HQMQ(1, 2, 96, 4, device="cuda")
+    x = make_kv("spiky", (1, 2, 200, 128), seed=140, dtype=torch.bfloat16).cuda()
+    for status, message in ((2, "bounded wait"), (1, "side buffer"), (3, "bounded wait")):
+        monkeypatch.setattr(_lib, "read_status", lambda ws: status)
+        with pytest.raises(hqmq.HqmqError, match=message):
+            q.encode(x, 0, 0, median_mult=3.0, check_status=True)
+    monkeypatch.undo()
+    q.encode(x, 0, 0, median_mult=3.0, check_status=True)
+    cache = PackedKVCache(hqmq.with_outlier_extraction(q, 3.0), max_tokens=512)
+    for T in (200, 1):
+        y = x[:, :, :T].clone()
+        y[0, 0, 0, 5], y[0, 1, 0, 6], y[0, 0, 0, 70] = float("nan"), float("inf"), float("-inf")
+        cache.update(y, y, 0)
+        cache.update(y.zero_(), y, 0)
+    cache.check()
+    k, v = cache._layers[0]
+    v.rs[v.T_cap + v.T - 1] = float("nan")
+    with pytest.raises(hqmq.HqmqError, match="bounded wait"):
+        cache.check()
