@@ -202,6 +202,35 @@ static int resident_ctas(const void* kernel, size_t smem, int threads) {
   return val;
 }
 
+// Clusters of `c` CTAs of `kernel` that the current device holds at once (a cluster lies within a GPC, and the GPCs of a chip
+// differ in SMs: 15 clusters of eight, 33 of four of one CTA per SM).  Cached like resident_ctas; without a device: any number.
+static int resident_clusters(const void* kernel, size_t smem, int threads, int c) {
+  struct Entry { const void* k; size_t smem; int dev, c, val; };
+  static Entry cache[256];
+  static int n_cache = 0;
+  static std::mutex mu;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    for (int i = 0; i < n_cache; ++i)
+      if (cache[i].k == kernel && cache[i].smem == smem && cache[i].dev == dev && cache[i].c == c) return cache[i].val;
+  }
+  int val = 0;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = c; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(c); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.attrs = &at; cfg.numAttrs = 1;
+  if (raise_smem_limit(kernel, smem) != cudaSuccess || cudaOccupancyMaxActiveClusters(&val, kernel, &cfg) != cudaSuccess || val < 1) {
+    cudaGetLastError();
+    return 1 << 20;
+  }
+  std::lock_guard<std::mutex> lock(mu);
+  if (n_cache < 256) cache[n_cache++] = {kernel, smem, dev, c, val};
+  return val;
+}
+
 cudaError_t raise_smem_limit(const void* kernel, size_t smem) {
   struct Entry { const void* k; int dev; };
   static Entry done[64];
@@ -324,18 +353,21 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
   if (tpu < 1) tpu = 1;
   pl.units = a->B * a->T_q * a->H_kv;
   // Few units of few tiles: a unit per cluster.  As many CTAs per unit as the SMs allow (8 is the portable cluster size), but
-  // not under half a tile per warp; beyond kSmallMaxRounds rounds of tiles per warp the flat split over all SMs with
-  // replicated tables takes over (see there).
+  // not under half a tile per warp, and no more than let all clusters run at once (1900 tokens, s96: 16 units as clusters of eight were two
+  // rounds of them, 26.6 us, and are 16.4 as clusters of six; 20 units 30.7 -> 18.1, 20.5 by the flat split; 48 units of 1000
+  // tokens 30.0 -> 18.4).  Beyond kSmallMaxRounds rounds of tiles per warp the flat split over all SMs with replicated tables takes over.
   if (fast && !ring && a->kv_splits == 0 && pl.units <= 148) {
+    const size_t smem = (size_t)pl.table_rows * 16 + (outl ? (size_t)8 * (a->d + kFastQPad) * 2 : 0) + (((size_t)pl.nw * kFastStages * 8 + 15) & ~(size_t)15) +
+                        (size_t)pl.nw * fast_warp_bytes(n, pl.ib, a->K.radius_bits, outl);
+    const void* small = fast_kernel(n, pl.ib, a->K.radius_bits, outl, true);
     int c = 148 / pl.units;
     if (c > 8) c = 8;
     while (c > 1 && (tpu + c - 1) / c < pl.nw / 2) --c;
-    const int per = (tpu + c - 1) / c;
-    if (per <= kSmallMaxRounds * pl.nw) {
-      const size_t smem = (size_t)pl.table_rows * 16 + (outl ? (size_t)8 * (a->d + kFastQPad) * 2 : 0) + (((size_t)pl.nw * kFastStages * 8 + 15) & ~(size_t)15) +
-                          (size_t)pl.nw * fast_warp_bytes(n, pl.ib, a->K.radius_bits, outl);
-      if (smem <= 220 * 1024) {
-        pl.kernel = fast_kernel(n, pl.ib, a->K.radius_bits, outl, true);
+    if (smem <= 220 * 1024 && (tpu + c - 1) / c <= kSmallMaxRounds * pl.nw) {
+      while (c > 1 && query_device && resident_clusters(small, smem, pl.threads, c) < pl.units) --c;
+      const int per = (tpu + c - 1) / c;
+      if (per <= kSmallMaxRounds * pl.nw) {
+        pl.kernel = small;
         pl.cluster = c; pl.smem = smem; pl.rep_log2 = 0;
         pl.tpu_v = per * c; pl.L = per; pl.P = c; pl.grid = pl.units * c;
         pl.ticket_bytes = 0; pl.ws_bytes = 16;

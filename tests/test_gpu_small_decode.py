@@ -23,6 +23,11 @@ pytestmark = pytest.mark.gpu
     (3, 8, 1, 64, 777, 1, 128),            # one CTA per unit, nine tiles for sixteen warps
     (1, 16, 2, 64, 3000, 3, None),         # a few query positions
     (37, 16, 4, 64, 300, 1, None),         # 148 units
+    (2, 8, 8, 128, 1900, 1, None),         # 16, 20, 29, 37 and 48 units: more than clusters of 148 / units CTAs fit at once
+    (5, 8, 4, 128, 1000, 1, None),
+    (29, 4, 1, 128, 700, 1, None),
+    (37, 4, 1, 64, 1001, 1, None),
+    (12, 8, 4, 128, 640, 1, None),
 ])
 @pytest.mark.parametrize("S,br,outliers", [(96, 4, True), (96, 4, False), (24, 3, True), (192, 6, False)])
 def test_small_decode(B, Hq, Hkv, d, T, Tq, window, S, br, outliers):
