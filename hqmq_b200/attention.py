@@ -149,7 +149,7 @@ def fused_attention_packed(
         hit = K._attn_cache.get(key)
         if hit is not None:
             a, ws_ptr, nbytes, t_sized, ref, ws = hit[:6]
-            prompt = Q.shape[2] >= _lib.ATTN_PROMPT_QUERIES
+            prompt = ws is None
             a.Q, a.T_kv = Q.data_ptr(), T_now
             if partials is not None:
                 a.partials = partials.data_ptr()

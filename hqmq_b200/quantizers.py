@@ -168,10 +168,10 @@ class HQMQQuantizer(KVQuantizer):
         reference's order, 'table16' (H,24S,4) fp16 in the native index order."""
         if not isinstance(device, torch.device):
             device = torch.device(device)
-        if device.index is None and device.type == "cuda":       # ("cuda" and "cuda:0" name one set of tables)
+        t = self._tables.get((layer_idx, kv, device))
+        if t is None and device.index is None and device.type == "cuda":       # ("cuda" and "cuda:0" name one set of tables)
             device = torch.device("cuda", torch.cuda.current_device())
-        key = (layer_idx, kv, device)
-        t = self._tables.get(key)
+            t = self._tables.get((layer_idx, kv, device))
         if t is None:
             qs, joint = self._codebook_fp32(layer_idx, kv)
             t = {"qs": qs.to(device), "joint": joint.to(device)}
@@ -194,7 +194,7 @@ class HQMQQuantizer(KVQuantizer):
                     _lib.check(L.hqmq_encode_lut_footprint(lut.data_ptr(), H, C.byref(mc), _lib.stream_ptr()),
                                "hqmq_encode_lut_footprint")
                 t["lut"], t["lut_footprint"] = lut, mc.value
-            self._tables[key] = t
+            self._tables[layer_idx, kv, device] = t
         return t
 
     # ---- compressed representation ---------------------------------------------------------------
