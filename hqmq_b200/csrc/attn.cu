@@ -251,8 +251,11 @@ cudaError_t raise_smem_limit(const void* kernel, size_t smem) {
   return rc;
 }
 
-// Rounds of tiles per warp up to which a unit is the work of one cluster.
-constexpr int kSmallMaxRounds = 2;
+// Rounds of tiles per warp up to which a unit is the work of one cluster.  Flat split / cluster, us, 8 heads of 128 (s96 with
+// outliers; s24): 4000 tokens 26.7 / 18.4 (29.1 / 14.3), 6000 28.7 / 22.5 (30.8 / 16.4), 10000 32.8 / 28.7 (34.1 / 22.5), 16000
+// 36.9 / 36.9 (36.9 / 28.7).  The fewer the units, the more SMs a cluster each leaves idle: two to four units (s96) 8000 tokens
+// 26.6 / 24.6, 10000 28.7 / 26.6, 12000 28.7 / 30.7; one unit 4000 18.4 / 18.4, 6000 18.9 / 22.5.
+constexpr int kSmallMaxRounds = 5, kSmallMaxRoundsOneUnit = 2;
 // Units of at most this many tiles run the staged kernels in warp mode (every warp has at most two tiles of a unit)
 constexpr int kWarpModeMaxTiles = 32;
 
@@ -355,18 +358,20 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
   // Few units of few tiles: a unit per cluster.  As many CTAs per unit as the SMs allow (8 is the portable cluster size), but
   // not under half a tile per warp, and no more than let all clusters run at once (1900 tokens, s96: 16 units as clusters of eight were two
   // rounds of them, 26.6 us, and are 16.4 as clusters of six; 20 units 30.7 -> 18.1, 20.5 by the flat split; 48 units of 1000
-  // tokens 30.0 -> 18.4).  Beyond kSmallMaxRounds rounds of tiles per warp the flat split over all SMs with replicated tables takes over.
+  // tokens 30.0 -> 18.4).  Beyond kSmallMaxRounds rounds of tiles per warp the flat split over all SMs with replicated tables
+  // takes over.
   if (fast && !ring && a->kv_splits == 0 && pl.units <= 148) {
     const size_t smem = (size_t)pl.table_rows * 16 + (outl ? (size_t)8 * (a->d + kFastQPad) * 2 : 0) + (((size_t)pl.nw * kFastStages * 8 + 15) & ~(size_t)15) +
                         (size_t)pl.nw * fast_warp_bytes(n, pl.ib, a->K.radius_bits, outl);
     const void* small = fast_kernel(n, pl.ib, a->K.radius_bits, outl, true);
+    const int most = (pl.units > 1 ? kSmallMaxRounds : kSmallMaxRoundsOneUnit) * pl.nw;        // tiles per CTA
     int c = 148 / pl.units;
     if (c > 8) c = 8;
     while (c > 1 && (tpu + c - 1) / c < pl.nw / 2) --c;
-    if (smem <= 220 * 1024 && (tpu + c - 1) / c <= kSmallMaxRounds * pl.nw) {
+    if (smem <= 220 * 1024 && (tpu + c - 1) / c <= most) {
       while (c > 1 && query_device && resident_clusters(small, smem, pl.threads, c) < pl.units) --c;
       const int per = (tpu + c - 1) / c;
-      if (per <= kSmallMaxRounds * pl.nw) {
+      if (per <= most) {
         pl.kernel = small;
         pl.cluster = c; pl.smem = smem; pl.rep_log2 = 0;
         pl.tpu_v = per * c; pl.L = per; pl.P = c; pl.grid = pl.units * c;

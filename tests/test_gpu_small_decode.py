@@ -28,6 +28,11 @@ pytestmark = pytest.mark.gpu
     (29, 4, 1, 128, 700, 1, None),
     (37, 4, 1, 64, 1001, 1, None),
     (12, 8, 4, 128, 640, 1, None),
+    (1, 8, 2, 128, 10239, 1, None),        # five rounds of tiles per warp, the most of a cluster, and one tile more
+    (1, 8, 2, 128, 10241, 1, None),
+    (1, 8, 1, 64, 4097, 1, None),          # one unit: two rounds and one tile
+    (6, 16, 8, 64, 2600, 1, None),         # four rounds in clusters of three
+    (1, 32, 8, 128, 7001, 1, 5001),        # a window that starts inside a tile
 ])
 @pytest.mark.parametrize("S,br,outliers", [(96, 4, True), (96, 4, False), (24, 3, True), (192, 6, False)])
 def test_small_decode(B, Hq, Hkv, d, T, Tq, window, S, br, outliers):
