@@ -15,7 +15,10 @@ size_t fast_warp_bytes(int n_chunks, int ib, int rb, bool outl);
 bool ring_kernel(int n_chunks, int ib, int rb, bool outl, int scale_dtype, RingKernelInfo& k);
 size_t ring_smem_total(int table_rows, int repk_log2, int repv_log2, int d, bool outl, int stages, int merge_slots,
                        size_t stage_bytes, int warps);
-constexpr int kRingManyPieces = 4;       // see attn_ring_body
+// Pieces of a unit beyond which the ring kernel with the wide merge runs (see attn_ring_body).  Wide / narrow merge, us: 18 pieces
+// (8 units) 92.2 / 97.8, 9 (16 units) 88.0 / 88.3, s192 78.8 / 80.6, 6 (24) 84.1 / 85.4, s192 100.7 / 103.1, 4 (32) 95.1 / 94.2,
+// 3 (48) 117.6 / 116.7, 2 (64) 153.8 / 152.1.
+constexpr int kRingManyPieces = 4;
 constexpr int kRingMinKeys = 1024;       // shorter key ranges keep the per-warp staging rings
 // ... and so do small problems: below about four stages per SM the ring kernel's set-up (it replicates the tables
 // up to sixteen times) outweighs its faster tile loop (B1, 8 KV heads, 4096 keys: 42 against 26 us per step)

@@ -7,6 +7,14 @@ namespace attn {
 
 constexpr int kPfTok = 128;                       // tokens per operand tile
 constexpr int kPfMaxCtas = 148;                   // one CTA per SM
+// Query positions from which a call decodes the cache once instead of once per position.  This path / the decode kernels, us:
+//   16 positions  8 heads of 128, G 4, s96 with outliers, 1 sequence: 300 tokens 21 / 16, 1000 29 / 25, 4000 46 / 45, 16000
+//                 136 / 144, 64000 347 / 469; 16 sequences: 300 35 / 169, 4000 297 / 556, 16000 1122 / 2006
+//                 4 heads, G 7, s192, 4 sequences: 1000 31 / 67, 16000 191 / 345;  8 heads of 64, G 8, 4 sequences: 1000 27 / 61
+//   8 positions   1 sequence: 1000 29 / 18, 16000 136 / 87; 16 sequences: 1000 85 / 159, 4000 296 / 288, 16000 1118 / 1014
+//   24 positions  1 sequence: 300 20 / 35, 4000 46 / 75, 64000 348 / 704
+// (The decode kernels stay shorter while every position and head can have a cluster of its own, 148 in all, up to about 2000
+// tokens: 2 heads, 48 positions, 1000 tokens 33 / 24.  The line does not look at that.)
 constexpr int kPrefillMinQueries = HQMQ_ATTN_PROMPT_QUERIES;
 constexpr int kPrefillMaxTable = 8192;            // codewords per head that fit the expand kernel's shared memory
 constexpr size_t kPrefillImageBytes = (size_t)512 << 20;   // operand images held at a time; larger caches go by groups of (b, head)

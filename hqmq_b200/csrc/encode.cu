@@ -668,9 +668,9 @@ __global__ void __launch_bounds__(kSmallThreads) fake_quant_small_kernel(SmallAr
 // one lane per chunk, no run-time geometry in the loop.  Results are the ones encode_main_kernel gives.
 constexpr int kEnc32Threads = 1024;   // one CTA per SM (the tables fill half of shared memory): 32 warps hide the search latency
 constexpr int kEnc32Warps = kEnc32Threads / 32;
-// A two-level select over a sample of the tokens has predicted the threshold statistic to a relative 2^-13; this pass then
-// does everything that needs x in its one read.  Per head, `bp` holds a range [R_lo, R_hi] of norm bits around the predicted
-// statistic (+-1 %) and the bounds thr_lo / thr_hi of the threshold that follow from it.  A chunk above thr_hi is flagged
+// A two-level select over a sample of the tokens predicts the threshold statistic; this pass then does everything that needs x
+// in its one read.  Per head, `bp` holds a range [R_lo, R_hi] of norm bits around the prediction (0.2 to 1.2 % either way, by the
+// sample's size, see bracket_wanted) and the bounds thr_lo / thr_hi of the threshold that follow from it.  A chunk above thr_hi is flagged
 // here (radius code 0, bit in the token's flag word), a chunk at or below thr_lo is not, the few in between are listed for
 // the fix-up; the norms inside the range are appended to a list (one region per CTA and head) and the norms below it are
 // counted, from which list_select_kernel takes the exact order statistics -- and finds out whether the prediction held: if
@@ -1865,16 +1865,20 @@ static MainGrid main_grid(int T_new, int B, int H) {
   m.ctas = (int)((total + m.per - 1) / m.per);
   return m;
 }
-// The bracket pass pays when the sample predicts well: the statistic's sampling error falls with the square root of
-// the sampled norms per head (a 1/32 sample of B * T_new tokens, 32 norms each), so the bracket's half-width is
-// 3 / sqrt(norms) (about six standard errors of a median), at least 0.2 % and at most 1.2 %; calls too small for that,
-// and quantiles out in the tails (few norms nearby: a much larger error), take the one-launch encoder.
 // d_head 64 as pairs of tokens (see EncGeom::pair16): the call's geometry must allow it, and a token's row must be whole
 // words without padding (16-bit fields; rows of 13- and 19-bit fields are padded, so two of them are not one longer row).
 static bool pair16_of(const hqmq_encode_args& a) {
   return a.dst.n_chunks == 16 && (16 * (idx_bits_for(a.dst.S) + a.dst.radius_bits)) % 32 == 0 && is_half_dtype(a.x_dtype) && a.x_stride[2] == 64 && a.T_new >= 2 && a.T_new % 2 == 0 &&
          a.t_start % 2 == 0;
 }
+// The bracket pass pays when the sample predicts well: the statistic's sampling error falls with the square root of
+// the sampled norms per head (a 1/32 sample of B * T_new tokens, 32 norms each), so the bracket's half-width is
+// 3 / sqrt(norms) (about six standard errors of a median), at least 0.2 % and at most 1.2 %; calls too small for that,
+// and quantiles out in the tails (few norms nearby: a much larger error), take the one-launch encoder.
+// 65536 tokens are where 1.2 % still holds six standard errors.  One read / one launch, us a tensor, s96, 8 heads of 128 with 6 %
+// flagged: 65536 tokens a head 359 / 480, 98304 487 / 705, 131072 612 / 933 (s24, none flagged: 65536 331 / 457; four heads, s192:
+// 337 / 362; heads of 64: 131072 362 / 477).  Below the line the one read would still be the shorter at 8 heads (32768: 217 / 247,
+// 49152: 295 / 362; four heads 220 / 219; 16384: 134 / 135), but its bracket would hold four standard errors, three at 16384.
 constexpr int64_t kBracketMinTokens = 65536;     // B * T_new per head (of 32 chunks each)
 static bool bracket_wanted(const hqmq_encode_args& a) {
   const bool pair = pair16_of(a);
