@@ -119,6 +119,14 @@ class HQMQQuantizer(KVQuantizer):
         self._state = next(_states)
         self.__dict__.get("_qdq_cache", {}).clear()
 
+    # (a copy keeps no calls, and is found by a number of its own)
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k not in ("_qdq_cache", "_state")}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state, _qdq_cache={})
+        self._new_state()
+
     # ---- reference plumbing ---------------------------------------------------------------
     def trainable_parameters(self):
         return [self.secondary_raw]
@@ -533,6 +541,15 @@ class _OutlierStats:
         self._blocks = {}           # per device and stream: the block that its fake-quant calls take counters from
         self._counted = []          # (block, index, chunks) of the fake-quant calls that were launched
         self._lock = threading.Lock()
+
+    # (a copy carries the two numbers on)
+    def __getstate__(self):
+        self._read()
+        return {"_sum_rates": self._sum_rates, "_n": self._n}
+
+    def __setstate__(self, state):
+        self.__init__()
+        self.__dict__.update(state)
 
     # A fake-quant call adds its flagged chunks to a counter of its own.  The counters of a stream are filled on that stream;
     # a call is accounted only once it is launched, and its record holds the block.  A captured call's counter belongs to the

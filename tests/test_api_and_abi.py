@@ -1,8 +1,10 @@
 """CPU checks of the host layer: the reference's public surface, bit accounting, constructors,
 the C ABI (library loads, every declared symbol is exported, argument validation returns error
 codes before anything is launched)."""
+import copy
 import ctypes as C
 import os
+import pickle
 import re
 
 import pytest
@@ -55,6 +57,15 @@ def test_constructors_and_wrappers():
         hqmq.HQMQ(1, 1, magnitude_mode="bogus", device="cpu")
     with pytest.raises(AssertionError):
         hqmq.OutlierAwareHQMQQuantizer(object())
+
+
+@pytest.mark.parametrize("how", [copy.deepcopy, lambda q: pickle.loads(pickle.dumps(q))])
+def test_quantizers_can_be_copied(how):
+    q = hqmq.with_outlier_extraction(hqmq.HQMQ(2, 2, 24, 3, device="cpu"), C=3.0)
+    q._stats._sum_rates, q._stats._n = 0.5, 2
+    c = how(q)
+    assert c.name == q.name and torch.equal(c.inner.secondary_raw, q.inner.secondary_raw) and c.inner._state != q.inner._state
+    assert (c._n_observations, c._observed_outlier_rate) == (2, 0.25) and c.bits_per_value() == q.bits_per_value()
 
 
 def test_seeded_codebook_matches_oracle():

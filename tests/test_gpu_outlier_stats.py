@@ -1,5 +1,6 @@
 """The outlier rate that the wrapper observes over fake-quant calls of several streams and threads, read between calls, and
 with calls captured in a graph."""
+import copy
 import threading
 
 import pytest
@@ -60,6 +61,14 @@ def test_the_rate_is_read_between_a_call_and_its_launch(monkeypatch):
         q.quantize_K(x, 0)
     assert q._n_observations == 20 and abs(q._observed_outlier_rate - sum(rates) / 20) < 1e-9
     assert not any(h.any() for h in held)
+
+
+def test_a_copy_made_between_calls_goes_on_by_itself():
+    q, (xs, rates) = _quantizer(), _inputs(8)
+    want = [q.quantize_K(x, 0) for x in xs]
+    c = copy.deepcopy(q)
+    assert all(torch.equal(c.quantize_K(x, 0), w) for x, w in zip(xs, want))
+    assert c._n_observations == 16 and q._n_observations == 8 and abs(c._observed_outlier_rate - sum(rates) / 8) < 1e-9
 
 
 def test_threads_on_streams_of_their_own_and_a_reader():
