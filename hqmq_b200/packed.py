@@ -142,6 +142,17 @@ class PackedKV:
                     pk.out_count = counters if k == counters.numel() else counters[lo:lo + k]
                 lo += k
 
+    # (a copy has planes of its own and keeps no calls; its outlier statistics start from what it holds)
+    def __getstate__(self):
+        state = {k: v for k, v in self.__dict__.items() if k not in ("_enc_cache", "_attn_cache", "_struct", "_stat_rec")}
+        state["_tensors"] = {name: t for name, t in self._tensors.items()
+                             if name not in self._spans or t.data_ptr() != self._spans[name][4]}    # (not the views of the buffer)
+        return state
+
+    def __setstate__(self, state):
+        self.__dict__.update(state, _enc_cache={}, _attn_cache={}, _struct=None)
+        self._spans = {name: (buf, at, nbytes, dtype, buf.data_ptr() + at) for name, (buf, at, nbytes, dtype, _) in self._spans.items()}
+
     def _ptr(self, name) -> int:
         t = self._tensors.get(name)
         return self._spans[name][4] if t is None else t.data_ptr()

@@ -68,6 +68,29 @@ def test_quantizers_can_be_copied(how):
     assert (c._n_observations, c._observed_outlier_rate) == (2, 0.25) and c.bits_per_value() == q.bits_per_value()
 
 
+@pytest.mark.parametrize("how", [copy.deepcopy, lambda c: pickle.loads(pickle.dumps(c))])
+def test_copied_planes_are_the_copys_own(how):
+    q = hqmq.HQMQ(1, 2, 24, 3, device="cpu")
+    pair = q.new_cache(2, 100, 64, "cpu", with_outliers=True, place=False), q.new_cache(2, 100, 64, "cpu", place=False)
+    packed.PackedKV.place(torch.device("cpu"), *pair)
+    for pk in pair:
+        pk.codes.random_(0, 256)
+        pk.T = 37
+        pk.c_struct()
+    own = torch.arange(len(pair[1].rs)).to(pair[1].rs.dtype)
+    pair[1].rs = own                             # a plane that a caller has put in the place of the cache's own
+    for pk, c in zip(pair, how(pair)):
+        names = ["codes", "rs"] + (["flags", "out_vals", "out_off"] if pk.with_outliers else [])
+        before = {n: getattr(pk, n).clone() for n in names}
+        for n in names:
+            t, s = getattr(c, n), c.c_struct()
+            assert torch.equal(t.view(torch.uint8), before[n].view(torch.uint8)) and t.data_ptr() != getattr(pk, n).data_ptr()
+            assert getattr(s, n) == t.data_ptr() == c._ptr(n)
+            t.zero_()
+            assert torch.equal(getattr(pk, n).view(torch.uint8), before[n].view(torch.uint8))
+        assert c.T == 37 and c.out_cap == pk.out_cap and c._enc_cache == {} == c._attn_cache
+
+
 def test_seeded_codebook_matches_oracle():
     from oracle import hqmq_oracle as orc
     q = hqmq.HQMQ(n_layers=2, n_heads=3, secondary_size=96, radius_bits=4, device="cpu", seed=42)

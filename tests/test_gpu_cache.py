@@ -1,6 +1,7 @@
 """PackedKVCache: the reference cache's call pattern (a prompt, then one token per step and layer) on compressed
 planes.  Attention over the cache must match the oracle run on the oracle's own encoding of the same calls, and
 the dense view must equal what the reference's cache would hold (its fake-quantised tensors)."""
+import copy
 import math
 import threading
 
@@ -387,3 +388,31 @@ def test_an_encoder_that_gave_up_is_reported(monkeypatch):
     v.rs[v.T_cap + v.T - 1] = float("nan")
     with pytest.raises(hqmq.HqmqError, match="bounded wait"):
         cache.check()
+
+
+def test_a_copied_cache_goes_on_by_itself():
+    """copy.deepcopy of a cache between two steps (one prompt, several continuations): both go on with planes of their own."""
+    q = hqmq.with_outlier_extraction(hqmq.HQMQ(2, 2, 96, 4, device="cuda"), 3.0)
+    cache = PackedKVCache(q, max_tokens=512, sliding_window={1: 64})
+    x = lambda T, seed: make_kv("spiky", (2, 2, T, 128), seed=seed, dtype=torch.bfloat16).cuda()
+    Q = [(torch.randn(2, 8, 1, 128, device="cuda") / 11).bfloat16() for _ in range(2)]
+
+    def go_on(c, seed):
+        out = []
+        for step in range(3):
+            for layer in range(2):
+                c.update(x(1, seed + step), x(1, seed + 50 + step), layer)
+                out.append(c.attend(Q[layer], layer))
+        return out
+    for layer in range(2):
+        cache.update(x(300, 150 + layer), x(300, 160 + layer), layer)
+        cache.attend(Q[layer], layer)
+    first = copy.deepcopy(cache)
+    go_on(cache, 200)
+    second = copy.deepcopy(first)
+    a, b = go_on(first, 300), go_on(second, 300)
+    assert all(torch.equal(u, v) for u, v in zip(a, b))
+    assert cache.get_seq_length(1) == 303 == second.get_seq_length(1)
+    want = go_on(copy.deepcopy(second), 400)
+    del first, cache
+    assert all(torch.equal(u, v) for u, v in zip(go_on(second, 400), want))
