@@ -364,8 +364,9 @@ int hqmq_attn_decode(const hqmq_attn_args* args, void* workspace, size_t workspa
  * no cudaMalloc / cudaFree and no allocating library routine; Q, O and the cache planes are still the
  * caller's.
  *
- *   - A problem whose partials do not fit (hqmq_attn_workspace_bytes(args) > HQMQ_ATTN_STATIC_SCRATCH_BYTES)
- *     is rejected with HQMQ_ERR_STATIC_SCRATCH before anything is launched; use hqmq_attn_decode then.
+ *   - A problem whose partials do not fit (hqmq_attn_workspace_bytes(args) > HQMQ_ATTN_STATIC_SCRATCH_BYTES below
+ *     HQMQ_ATTN_PROMPT_QUERIES query positions) is rejected with HQMQ_ERR_STATIC_SCRATCH before anything is launched; use
+ *     hqmq_attn_decode then.  A prompt whose decoded cache does not fit takes the path of fewer positions.
  *   - The first call on a device looks up the buffer's device address (cudaGetSymbolAddress) with that
  *     device current, and caches it; make that first call during set-up, before any stream capture begins.
  *     Call it with the device current that owns `stream`.
