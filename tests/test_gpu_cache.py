@@ -345,19 +345,19 @@ def test_threads_of_one_stream_attend_over_one_cache(monkeypatch):
 
     def second():
         got["warm"] = hqmq.fused_attention_packed(Qs[1], Kp, Vp, tk, tv)
-        go.wait()
+        go.wait(20)
         got["out"] = hqmq.fused_attention_packed(Qs[1], Kp, Vp, tk, tv)
         gone.set()
     L = _lib.lib()
     real, thread, me = L.hqmq_attn_decode, threading.Thread(target=second), threading.get_ident()
     thread.start()
-    while "warm" not in got:
+    while "warm" not in got and thread.is_alive():
         pass
 
     def attn_decode(*args):
         if threading.get_ident() == me:
             go.set()
-            gone.wait()
+            gone.wait(20)
         return real(*args)
     monkeypatch.setattr(L, "hqmq_attn_decode", attn_decode)
     out = torch.full_like(Qs[0], 7)
