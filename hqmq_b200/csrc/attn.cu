@@ -119,7 +119,7 @@ __global__ void combine_kernel(const float* __restrict__ parts, int n_parts, int
     }
     if (failed) acc = NAN;
     if (merged) merged[row * (d + 2) + x] = acc;
-    else store_float(out, b * os_b + hq * os_h + tq * os_t + x, l_star > 0.f || failed ? acc / l_star : 0.f, out_dtype);
+    else store_float(out, b * os_b + hq * os_h + tq * os_t + x, l_star != 0.f || failed ? acc / l_star : 0.f, out_dtype);
   }
   if (merged && threadIdx.x == 0) { merged[row * (d + 2) + d] = m_star; merged[row * (d + 2) + d + 1] = l_star; }
 }

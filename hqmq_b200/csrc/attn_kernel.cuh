@@ -1028,7 +1028,7 @@ __device__ __forceinline__ void attn_decode_body(const AttnParams& p) {
           if (x == 0) { p.merged[row * PD + 4 * N] = m_star; p.merged[row * PD + 4 * N + 1] = l_star; }
         } else {
           store_float(p.O, (int64_t)b * p.os_b + (int64_t)(h * p.G + g) * p.os_h + (int64_t)tq * p.os_t + x,
-                      l_star > 0.f || l_star != l_star ? v / l_star : 0.f, p.o_dtype);
+                      l_star != 0.f ? v / l_star : 0.f, p.o_dtype);
         }
       };
       const bool failed = __syncthreads_or(gave_up ? 1 : 0) != 0;

@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
         const int b = bh / p.Hkv, h = bh - b * p.Hkv;
         const float l = l2.x + l2.y, vmul = p.vmul[bh];
         const bool whole = q.head && q.tail;
-        const float mul = whole ? (l > 0.f ? vmul / l : 0.f) : vmul;
+        const float mul = whole ? (l != 0.f ? vmul / l : 0.f) : vmul;
         // a partial is stored column by column ([d + 2][256 rows]), so that the lanes of a store are neighbours
         float* part = p.part + ((int64_t)blockIdx.x * 2 + (q.head ? 1 : 0)) * (256 * (D + 2)) + s * 128 + row;
         const uint32_t stage = sO + warp * (32 * kPfOutRow);
@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const PrefillParams 
     for (int e = 0; e < E; ++e) acc[e] = fmaf(col[e * 256], w, acc[e]);
   }
   const bool failed = *p.status == p.epoch;                 // the attention kernel gave up on a wait
-  const float inv = failed ? NAN : l > 0.f ? 1.f / l : 0.f;
+  const float inv = failed ? NAN : l != 0.f ? 1.f / l : 0.f;
 #pragma unroll
   for (int e = 0; e < E; ++e) tile[lane][warp * E + e] = acc[e] * inv;
   __syncthreads();

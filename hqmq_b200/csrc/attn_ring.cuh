@@ -856,7 +856,7 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
           if (x == 0) { p.merged[row * (D + 2) + D] = m_star; p.merged[row * (D + 2) + D + 1] = l_star; }
         } else {
           store_float(p.O, (int64_t)b * p.os_b + (int64_t)(h * p.G + g) * p.os_h + (int64_t)tq * p.os_t + x,
-                      l_star > 0.f ? v / l_star : 0.f, p.o_dtype);
+                      l_star != 0.f ? v / l_star : 0.f, p.o_dtype);
         }
       };
       if (n_ctas == 1) {

@@ -645,7 +645,8 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
       }
       const int64_t row = ((int64_t)b * p.Hq + h * p.G + g) * p.Tq + tq;
       float* dst = SMALL ? s_part + g * PD : p.partials + (row * p.P + part) * PD;
-      dst[x] = SMALL && cta_failed ? NAN : acc;
+      if (SMALL && cta_failed) acc = l_star = NAN;
+      dst[x] = acc;
       if (x == 0) { dst[4 * N] = m_star; dst[4 * N + 1] = l_star; }
     }
     if constexpr (SMALL) {
@@ -669,7 +670,7 @@ __device__ __forceinline__ void attn_decode_tma_body(const AttnParams& p, uint32
           if (x == 0) { p.merged[row * PD + 4 * N] = m_star; p.merged[row * PD + 4 * N + 1] = l_star; }
         } else {
           store_float(p.O, (int64_t)b * p.os_b + (int64_t)(h * p.G + g) * p.os_h + (int64_t)tq * p.os_t + x,
-                      l_star > 0.f || !(acc == acc) ? acc / l_star : 0.f, p.o_dtype);
+                      l_star != 0.f ? acc / l_star : 0.f, p.o_dtype);
         }
       }
       cluster_sync();      // nobody leaves while its partial is being read

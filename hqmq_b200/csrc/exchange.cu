@@ -133,7 +133,7 @@ step_kernel(hqmq_exchange x, const float* __restrict__ local, uint32_t epoch, ui
       if (w != 0.f) acc += __ldcg(blocks + (int64_t)r * x.block_floats + (int64_t)row * (d + 2) + c) * w;
     }
     if (s_miss) acc = NAN;
-    store_float(out, (int64_t)row * d + c, l_star > 0.f || s_miss ? acc / l_star : 0.f, out_dtype);
+    store_float(out, (int64_t)row * d + c, l_star != 0.f || s_miss ? acc / l_star : 0.f, out_dtype);
   }
 }
 

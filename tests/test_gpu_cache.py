@@ -416,3 +416,18 @@ def test_a_copied_cache_goes_on_by_itself():
     want = go_on(copy.deepcopy(second), 400)
     del first, cache
     assert all(torch.equal(u, v) for u, v in zip(go_on(second, 400), want))
+
+
+@pytest.mark.parametrize("S,br,T,Tq,splits", [(96, 4, 300, 1, None), (96, 4, 2000, 1, 3), (192, 6, 20000, 1, None), (96, 4, 70000, 1, None),
+                                              (48, 4, 500, 1, None), (96, 4, 500, 20, None), (24, 3, 9000, 200, None)])
+@pytest.mark.parametrize("kv", [0, 1])
+def test_a_scale_that_is_no_number_shows(S, br, T, Tq, splits, kv):
+    """The token of a call that gave up makes the rows that see it NaN, in every kernel, and no row of another head or sequence."""
+    q = hqmq.HQMQ(1, 4, S, br, device="cuda")
+    pair = [q.encode(make_kv("randn", (2, 4, T, 128), seed=170 + i, dtype=torch.bfloat16).cuda(), 0, i, median_mult=3.0) for i in (0, 1)]
+    pair[kv].rs.view(-1)[(1 * 4 + 2) * pair[kv].T_cap + T // 2] = float("nan")
+    Q = (torch.randn(2, 8, Tq, 128, device="cuda") / 11).bfloat16()
+    O = hqmq.fused_attention_packed(Q, *pair, q.tables(0, 0, "cuda")["table16"], q.tables(0, 1, "cuda")["table16"],
+                                    causal="bottom_right" if Tq > 1 else False, kv_splits=splits)
+    bad = O.isnan()
+    assert bad[1, 4:6].all() and not bad[0].any() and not bad[1, :4].any() and not bad[1, 6:].any()
