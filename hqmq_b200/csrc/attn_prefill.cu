@@ -4,8 +4,9 @@
 // token, 2048 times the decoding for a 2048-token prompt chunk.  Here the cache is decoded ONCE per call into operand
 // tiles, and the attention runs on the tensor cores over those:
 //
-//   expand   (prefill_expand_kernel) per (b, KV head) and 128-token tile: K as a K-major and V^T as a K-major fp16 operand
-//            image in the 128-byte swizzle that tcgen05.mma reads, so that a tile is one contiguous bulk copy later.
+//   expand   (prefill_expand_kernel) per (b, KV head) and 128-token tile: K and V as fp16 operand images in the 128-byte
+//            swizzle that tcgen05.mma reads (tokens down, 64 elements of d across: K-major for Q K^T, MN-major for P V), so
+//            that a tile is one contiguous bulk copy later.
 //            A value is codeword * (rq * rs / qmax * 2^(10-e)), e the exponent of the largest scale of the (b, head), outliers
 //            are x * 2^(10-e): everything lies below 2^10 and keeps its 11 bits down to 2^-24 of the largest token.
 //   attend   (prefill_attn_kernel) persistent, one CTA per SM.  A unit is (b, KV head, up to 2 x 128 rows), a row one
@@ -139,8 +140,16 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
   return (uint64_t)((addr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
          ((uint64_t)2 << 61);
 }
-// kind::f16, fp16 operands (both K-major), fp32 accumulators
-__host__ __device__ constexpr uint32_t f16_idesc(int M, int N) { return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24); }
+// MN-major operand in the same swizzle: k rows of 128 bytes (64 elements across), groups of eight rows 1024 bytes apart, the
+// next 64 elements across in a plane of 128 rows of their own.
+__device__ __forceinline__ uint64_t sw128_mn_desc(uint32_t addr) {
+  return (uint64_t)((addr & 0x3ffffu) >> 4) | ((uint64_t)(16384 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
+         ((uint64_t)2 << 61);
+}
+// kind::f16, fp16 operands (A K-major; B K-major, or MN-major), fp32 accumulators
+__host__ __device__ constexpr uint32_t f16_idesc(int M, int N, bool b_mn = false) {
+  return (1u << 4) | (b_mn ? 1u << 16 : 0u) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
 
 // Two fp32 operations per instruction.
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -243,7 +252,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
     PfPiece q;
     it.init(p, (int)blockIdx.x);
     auto wait_w = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, wait(bar, parity)) != 0; };   // one answer per warp
-    constexpr uint32_t id_qk = f16_idesc(128, 128), id_pv = f16_idesc(128, D);
+    constexpr uint32_t id_qk = f16_idesc(128, 128), id_pv = f16_idesc(128, D, true);
     // S of the tile in stage st; O += P V of half hb of its keys
     auto qk = [&](uint32_t st) {
       const uint64_t a0 = sw128_desc(sQ + s * TB), b0 = sw128_desc(sK + st * TB);
@@ -256,10 +265,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
       tc_commit(kempty + 8 * st);
     };
     auto pv = [&](uint32_t st, int hb, bool acc) {
-      const uint64_t b0 = sw128_desc(sV + st * TB + hb * (D * 128));
+      const uint64_t b0 = sw128_mn_desc(sV + st * TB + hb * (64 * 128));
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        tc_mma_ts(256 + D * s, 128 * s + 32 * hb + 8 * k, b0 + ((k * 32) >> 4), id_pv, acc || k > 0 ? 1u : 0u);
+        tc_mma_ts(256 + D * s, 128 * s + 32 * hb + 8 * k, b0 + ((k * 16 * 128) >> 4), id_pv, acc || k > 0 ? 1u : 0u);
     };
     uint32_t g = 0, u = 0;     // tiles, units
     bool ok = true;
@@ -569,21 +578,23 @@ __device__ __forceinline__ void pf_scale_of(float big, float& mul, float& inv) {
 }
 
 // grid (tile chunks, (b, head) of the group, 2): blockIdx.z = 0 K, 1 V.  Eight warps; a warp takes the 16 tokens of one
-// outlier block of the tile with a lane per chunk.  K goes straight to its image (the lanes of a token fill whole 128-byte
-// rows); V is unpacked to shared memory first and decoded with a lane per token, so that the transposed image is written 64
-// bytes at a time.  Flagged chunks decode to zero (radius code 0) and are overwritten afterwards from a list of the block's
+// outlier block of a tile with a lane per chunk, and writes them straight to the image (the lanes of a token fill whole
+// 128-byte rows).  Flagged chunks decode to zero (radius code 0) and are overwritten afterwards from a list of the block's
 // entries, a lane per entry: the payload is then read in order, 32 entries at a time.  (Looked up chunk by chunk inside the
 // decode loop they tripled its instructions: 46 us for 8192 tokens of 8 heads, K with 6 % flagged.)
+// Bound: latency of a CTA's dependent loads (table, scales, rows, then payload): the issue slots are a quarter busy, DRAM
+// less.  So the table comes by bulk copy, the scale scan and the first tile's rows are in flight with it, and a tile's rows are
+// fetched while the payload of the one before is written.  8192 tokens of 8 heads, s96, K with 6 % flagged: 17.4 us (35 with V
+// turned into a K-major image through shared memory, three barriers a tile and 68 KB a CTA); the tuple, 2048 tokens: 11.4 (24).
 template <int N, int LAYOUT>
-__global__ void __launch_bounds__(256, 3) prefill_expand_kernel(const ExpandParams e) {
+__global__ void __launch_bounds__(256, 4) prefill_expand_kernel(const ExpandParams e) {
   constexpr int D = 4 * N;
   constexpr uint32_t TB = (uint32_t)pf_tile_bytes(D);
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  uint4* img = reinterpret_cast<uint4*>(smem_raw);                                       // V only: the tile's image
-  uint32_t* fields = reinterpret_cast<uint32_t*>(smem_raw + (blockIdx.z ? TB : 0));         // V only: [128][N + 1]
-  uint2* tbl = reinterpret_cast<uint2*>(smem_raw + (blockIdx.z ? TB + 128 * (N + 1) * 4 : 0));
-  __shared__ float s_big[8], s_fac[kPfTok];
+  uint2* tbl = reinterpret_cast<uint2*>(smem_raw);
+  __shared__ float s_big[8];
   __shared__ uint16_t s_list[8][16 * N];       // (token of the block) * 32 + chunk of the block's payload entries
+  __shared__ __align__(8) uint64_t s_bar;
   grid_dep_launch();
   const bool is_v = blockIdx.z != 0;
   const hqmq_packed& pk = is_v ? e.V : e.K;
@@ -591,51 +602,38 @@ __global__ void __launch_bounds__(256, 3) prefill_expand_kernel(const ExpandPara
   const int bh = e.bh0 + blockIdx.y, b = bh / e.Hkv, h = bh - b * e.Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  // ---- the head's table, the largest scale of the keys in range ------------------------------------------------------
-  if (LAYOUT == 0) {
-    const uint2* src = reinterpret_cast<const uint2*>(is_v ? e.tblV : e.tblK) + (int64_t)h * e.table_rows;
+  // ---- the head's table on its way: entries of four fp16 values by bulk copy where their address allows -----------------------
+  const void* jt = is_v ? e.jV : e.jK;
+  const uint2* src = (LAYOUT == 0 ? reinterpret_cast<const uint2*>(is_v ? e.tblV : e.tblK) : reinterpret_cast<const uint2*>(jt)) + (int64_t)h * e.table_rows;
+  const uint32_t bar = smem_u32(&s_bar), tbytes = (uint32_t)e.table_rows * 8u;
+  const bool bulk = (LAYOUT == 0 || e.j_dtype == HQMQ_F16) && ((reinterpret_cast<uintptr_t>(src) | tbytes) & 15u) == 0;
+  if (bulk) {
+    if (threadIdx.x == 0) {
+      mbar_init(bar, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      mbar_expect_tx(bar, tbytes);
+      bulk_g2s(smem_u32(tbl), src, tbytes, bar);
+    }
+  } else if (LAYOUT == 0) {
     for (int i = threadIdx.x; i < e.table_rows; i += 256) tbl[i] = src[i];
+  } else if (e.j_dtype != HQMQ_F32 && (reinterpret_cast<uintptr_t>(src) & 7u) == 0) {
+    for (int i = threadIdx.x; i < e.table_rows; i += 256) {
+      const uint2 w = src[i];
+      const float2 a = pair16_to_float2(w.x, e.j_dtype), d = pair16_to_float2(w.y, e.j_dtype);
+      tbl[i] = make_uint2(pack_half2(a.x, a.y), pack_half2(d.x, d.y));
+    }
   } else {
-    const void* j = is_v ? e.jV : e.jK;
     for (int i = threadIdx.x; i < e.table_rows; i += 256) {
       const int64_t o = ((int64_t)h * e.table_rows + i) * 4;
-      tbl[i] = make_uint2(pack_half2(load_float(j, o, e.j_dtype), load_float(j, o + 1, e.j_dtype)),
-                          pack_half2(load_float(j, o + 2, e.j_dtype), load_float(j, o + 3, e.j_dtype)));
+      tbl[i] = make_uint2(pack_half2(load_float(jt, o, e.j_dtype), load_float(jt, o + 1, e.j_dtype)),
+                          pack_half2(load_float(jt, o + 2, e.j_dtype), load_float(jt, o + 3, e.j_dtype)));
     }
   }
-  const int t_first = e.kt0 * kPfTok, t_end = min(e.Tkv, (e.kt0 + e.nt) * kPfTok);
-  auto scale_of = [&](int t) {
-    return LAYOUT == 0 ? load_scale(pk, (int64_t)bh * pk.T_cap + t)
-                       : load_float(rf.rs, b * rf.rs_stride[0] + h * rf.rs_stride[1] + t, rf.rs_dtype);
-  };
-  float big = 0.f;
-  if (LAYOUT == 0 && pk.scale_dtype != HQMQ_F32) {
-    // eight 16-bit scales per load (they are positive: their bits order like their values)
-    const uint16_t* rs = reinterpret_cast<const uint16_t*>(pk.rs) + (int64_t)bh * pk.T_cap;
-    uint32_t mx = 0u;
-    for (int t = t_first + threadIdx.x * 8; t + 8 <= t_end; t += 256 * 8) {
-      const uint4 v = *reinterpret_cast<const uint4*>(rs + t);
-      mx = __vmaxu2(mx, __vmaxu2(__vmaxu2(v.x, v.y), __vmaxu2(v.z, v.w)));
-    }
-    big = fmaxf(bits16_to_float(mx & 0xffff, pk.scale_dtype), bits16_to_float(mx >> 16, pk.scale_dtype));
-    const int t = (t_end & ~7) + (int)threadIdx.x;
-    if (t < t_end) big = fmaxf(big, scale_of(t));
-  } else {
-    for (int t = t_first + threadIdx.x; t < t_end; t += 256) big = fmaxf(big, fabsf(scale_of(t)));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
-  if (lane == 0) s_big[warp] = big;
-  __syncthreads();
-#pragma unroll
-  for (int w = 0; w < 8; ++w) big = fmaxf(big, s_big[w]);
-  float mul, inv;
-  pf_scale_of(big, mul, inv);
-  if (blockIdx.x == 0 && threadIdx.x == 0) (is_v ? e.vmul : e.kmul)[bh] = is_v ? inv : inv * e.qscale;
 
   // what this lane needs of the planes, as bases and 32-bit steps (a lane keeps its chunk for the whole kernel)
   const bool outl = LAYOUT == 0 && pk.flags != nullptr;
   constexpr int TPW = 32 / N;                 // tokens a warp takes at a time
+  constexpr int NF = 16 / TPW;                // fields of a lane
   const int half = N == 32 ? 0 : lane >> 4, c = N == 32 ? lane : lane & 15;
   const uint32_t* rows = nullptr;
   int row_words = 0, w1 = 0, sh = 0;
@@ -652,127 +650,133 @@ __global__ void __launch_bounds__(256, 3) prefill_expand_kernel(const ExpandPara
   const int out_dtype = pk.out_dtype;
   const uint32_t* flags = outl ? pk.flags + (int64_t)bh * pk.T_cap : nullptr;
   const uint32_t* offs = outl ? pk.out_off + (int64_t)bh * (pk.T_cap / HQMQ_OUT_BLOCK + 1) : nullptr;
+  auto scale_of = [&](int t) {
+    return LAYOUT == 0 ? load_scale(pk, (int64_t)bh * pk.T_cap + t)
+                       : load_float(rf.rs, b * rf.rs_stride[0] + h * rf.rs_stride[1] + t, rf.rs_dtype);
+  };
+  // the rows of a tile's 16 tokens of this warp: fields (index | radius code << 16), lanes 0..15 the scale and flag word of a token
+  uint32_t f[NF], myflag, run;
+  float rs;
+  auto fetch = [&](int tile) {
+    const int tb = (e.kt0 + tile) * kPfTok + warp * 16;
+    rs = 0.f; myflag = 0u; run = 0u;
+    if (lane < 16 && tb + lane < e.Tkv) {
+      rs = scale_of(tb + lane);
+      if (outl) myflag = flags[tb + lane];
+    }
+    if (outl && tb < e.Tkv) run = offs[tb / HQMQ_OUT_BLOCK];
+#pragma unroll
+    for (int k = 0; k < NF; ++k) {
+      const int t = tb + k * TPW + half;
+      f[k] = 0u;
+      if (t < e.Tkv) {
+        if constexpr (LAYOUT == 0) {
+          const uint32_t* r = rows + t * row_words;
+          const uint32_t raw = __funnelshift_r(r[0], r[w1], sh) & fmask;
+          f[k] = (raw & imask) | ((raw >> e.ib) << 16);
+        } else {
+          const int64_t io = b * rf.idx_stride[0] + h * rf.idx_stride[1] + t * rf.idx_stride[2] + c;
+          const int64_t ro = b * rf.rq_stride[0] + h * rf.rq_stride[1] + t * rf.rq_stride[2] + c;
+          if (rf.idx_dtype == HQMQ_I32 && rf.rq_dtype == HQMQ_I32) {
+            const int i = reinterpret_cast<const int32_t*>(rf.idx)[io], r = reinterpret_cast<const int32_t*>(rf.rq)[ro];
+            f[k] = (uint32_t)min(max(i, 0), e.table_rows - 1) | ((uint32_t)min(max(r, 0), 1023) << 16);
+          } else {
+            long long i = load_int(rf.idx, io, rf.idx_dtype), r = load_int(rf.rq, ro, rf.rq_dtype);
+            i = i < 0 ? 0 : (i >= e.table_rows ? e.table_rows - 1 : i);
+            r = r < 0 ? 0 : (r > 1023 ? 1023 : r);
+            f[k] = (uint32_t)i | ((uint32_t)r << 16);
+          }
+        }
+      }
+    }
+  };
+  const int tile_hi = min(e.nt, (int)(blockIdx.x + 1) * e.per);
+  fetch(blockIdx.x * e.per);
+
+  // ---- the largest scale of the keys in range -----------------------------------------------------------------------------
+  const int t_first = e.kt0 * kPfTok, t_end = min(e.Tkv, (e.kt0 + e.nt) * kPfTok);
+  float big = 0.f;
+  if (LAYOUT == 0 && pk.scale_dtype != HQMQ_F32) {
+    // eight 16-bit scales per load (they are positive: their bits order like their values)
+    const uint16_t* rsp = reinterpret_cast<const uint16_t*>(pk.rs) + (int64_t)bh * pk.T_cap;
+    uint32_t mx = 0u;
+    for (int t = t_first + threadIdx.x * 8; t + 8 <= t_end; t += 256 * 8) {
+      const uint4 v = *reinterpret_cast<const uint4*>(rsp + t);
+      mx = __vmaxu2(mx, __vmaxu2(__vmaxu2(v.x, v.y), __vmaxu2(v.z, v.w)));
+    }
+    big = fmaxf(bits16_to_float(mx & 0xffff, pk.scale_dtype), bits16_to_float(mx >> 16, pk.scale_dtype));
+    const int t = (t_end & ~7) + (int)threadIdx.x;
+    if (t < t_end) big = fmaxf(big, scale_of(t));
+  } else {
+    for (int t = t_first + threadIdx.x; t < t_end; t += 256) big = fmaxf(big, fabsf(scale_of(t)));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+  if (lane == 0) s_big[warp] = big;
+  __syncthreads();                             // (the barrier word of the table's copy is initialised, too)
+#pragma unroll
+  for (int w = 0; w < 8; ++w) big = fmaxf(big, s_big[w]);
+  float mul, inv;
+  pf_scale_of(big, mul, inv);
+  if (blockIdx.x == 0 && threadIdx.x == 0) (is_v ? e.vmul : e.kmul)[bh] = is_v ? inv : inv * e.qscale;
+  if (bulk) {
+    // (every thread waits: a CTA must not exit with a copy into it in flight.  Bounded; a table that never came reads as it is,
+    //  and the attention kernel's status word is raised.)
+    uint32_t spins = 0;
+    while (!mbar_try_wait(bar, 0)) {
+      if (++spins > kWaitLimit) { if (threadIdx.x == 0) *e.status = e.epoch; break; }
+    }
+  }
+
   // four fp16 values of a chunk from its codeword and radius code
-  auto value_of = [&](uint32_t f, float fac) {
-    const uint2 cw = tbl[f & 0xffffu];
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&cw.x)), c = __half22float2(*reinterpret_cast<const __half2*>(&cw.y));
-    fac *= (float)(f >> 16);
-    return make_uint2(pack_half2(a.x * fac, a.y * fac), pack_half2(c.x * fac, c.y * fac));
+  auto value_of = [&](uint32_t fv, float fac) {
+    const uint2 cw = tbl[fv & 0xffffu];
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&cw.x)), d = __half22float2(*reinterpret_cast<const __half2*>(&cw.y));
+    fac *= (float)(fv >> 16);
+    return make_uint2(pack_half2(a.x * fac, a.y * fac), pack_half2(d.x * fac, d.y * fac));
   };
   // ... of a flagged chunk from its payload entry (an entry the encoder dropped reads as 0)
   auto payload_of = [&](uint32_t slot) {
     if (slot >= cap) return make_uint2(0u, 0u);
     return *reinterpret_cast<const uint2*>(vals + (int64_t)slot * 8);
   };
-  auto payload_half = [&](uint2 v) {           // (converted when they are used)
-    const float2 a = pair16_to_float2(v.x, out_dtype), d = pair16_to_float2(v.y, out_dtype);
-    return make_uint2(pack_half2(a.x * mul, a.y * mul), pack_half2(d.x * mul, d.y * mul));
-  };
-  // V^T image: the four dims of chunk cc of token tl
-  auto put_v = [&](int tl, int cc, uint2 v) {
-    unsigned char* im = reinterpret_cast<unsigned char*>(img) + (tl >> 6) * (D * 128) + (tl & 7) * 2 + cc * 512;
-    const int sw = ((tl & 63) >> 3) ^ ((cc & 1) * 4);
-    *reinterpret_cast<uint16_t*>(im + (sw << 4)) = (uint16_t)v.x;
-    *reinterpret_cast<uint16_t*>(im + 128 + ((sw ^ 1) << 4)) = (uint16_t)(v.x >> 16);
-    *reinterpret_cast<uint16_t*>(im + 256 + ((sw ^ 2) << 4)) = (uint16_t)v.y;
-    *reinterpret_cast<uint16_t*>(im + 384 + ((sw ^ 3) << 4)) = (uint16_t)(v.y >> 16);
-  };
-  const int tile_hi = min(e.nt, (int)(blockIdx.x + 1) * e.per);
   for (int tile = blockIdx.x * e.per; tile < tile_hi; ++tile) {
-    const int t0 = (e.kt0 + tile) * kPfTok;
     unsigned char* dst = (is_v ? e.vimg : e.kimg) + ((int64_t)blockIdx.y * e.nt + tile) * TB;
-    uint32_t n_ent = 0u, run = 0u;
+    const float myfac = rs * e.vscale * mul;
+    // the block's payload entries in order; the first 32 are fetched now
+    uint32_t n_ent = 0u;
+    const uint32_t run0 = run;
     uint2 ent = make_uint2(0u, 0u);
-    {
-      const int tb = t0 + warp * 16;
-      // all fields of the warp's tokens first (independent loads), with the scales and flag words of the block
-      constexpr int NF = 16 / TPW;
-      uint32_t f[NF];
+    if (outl) {
+      uint32_t incl = __popc(myflag);
 #pragma unroll
-      for (int k = 0; k < NF; ++k) {
-        const int t = tb + k * TPW + half;
-        f[k] = 0u;
-        if (t < e.Tkv) {
-          if constexpr (LAYOUT == 0) {
-            const uint32_t* r = rows + t * row_words;
-            const uint32_t raw = __funnelshift_r(r[0], r[w1], sh) & fmask;
-            f[k] = (raw & imask) | ((raw >> e.ib) << 16);
-          } else {
-            const int64_t io = b * rf.idx_stride[0] + h * rf.idx_stride[1] + t * rf.idx_stride[2] + c;
-            const int64_t ro = b * rf.rq_stride[0] + h * rf.rq_stride[1] + t * rf.rq_stride[2] + c;
-            if (rf.idx_dtype == HQMQ_I32 && rf.rq_dtype == HQMQ_I32) {
-              const int i = reinterpret_cast<const int32_t*>(rf.idx)[io], r = reinterpret_cast<const int32_t*>(rf.rq)[ro];
-              f[k] = (uint32_t)min(max(i, 0), e.table_rows - 1) | ((uint32_t)min(max(r, 0), 1023) << 16);
-            } else {
-              long long i = load_int(rf.idx, io, rf.idx_dtype), r = load_int(rf.rq, ro, rf.rq_dtype);
-              i = i < 0 ? 0 : (i >= e.table_rows ? e.table_rows - 1 : i);
-              r = r < 0 ? 0 : (r > 1023 ? 1023 : r);
-              f[k] = (uint32_t)i | ((uint32_t)r << 16);
-            }
-          }
-        }
-      }
-      float myfac = 0.f;                     // lanes 0..15: the factor of the block's tokens
-      uint32_t myflag = 0u;
-      if (lane < 16 && tb + lane < e.Tkv) {
-        myfac = scale_of(tb + lane) * e.vscale * mul;
-        if (outl) myflag = flags[tb + lane];
-      }
-      if (is_v && lane < 16) s_fac[warp * 16 + lane] = myfac;
-      // the block's payload entries in order; the first 32 are fetched now
-      const uint32_t mine = __popc(myflag), incl = outl ? [&] { uint32_t v = mine;
-#pragma unroll
-        for (int o = 1; o < 16; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += y; }
-        return v; }() : 0u;
+      for (int o = 1; o < 16; o <<= 1) { const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
       n_ent = __shfl_sync(0xffffffffu, incl, 15);
       if (n_ent) {
-        run = offs[tb / HQMQ_OUT_BLOCK];
-        uint32_t pos = incl - mine;
+        if (lane < n_ent) ent = payload_of(run0 + lane);
+        uint32_t pos = incl - __popc(myflag);
         for (uint32_t w = myflag; w; w &= w - 1u) s_list[warp][pos++] = (uint16_t)(lane * 32 + __ffs(w) - 1);
-        __syncwarp();
-        if (lane < n_ent) ent = payload_of(run + lane);
-      }
-      unsigned char* kd = dst + (c >> 4) * 16384 + (c & 1) * 8;
-#pragma unroll
-      for (int k = 0; k < NF; ++k) {
-        const int tl = warp * 16 + k * TPW + half;
-        if (is_v) {
-          fields[tl * (N + 1) + c] = f[k];
-        } else {
-          const float fac = __shfl_sync(0xffffffffu, myfac, k * TPW + half);
-          *reinterpret_cast<uint2*>(kd + tl * 128 + ((((c & 15) >> 1) ^ (tl & 7)) << 4)) = value_of(f[k], fac);
-        }
       }
     }
-    auto put_entries = [&](auto put) {         // put(token of the tile, chunk, values)
+    unsigned char* kd = dst + (c >> 4) * 16384 + (c & 1) * 8;
+#pragma unroll
+    for (int k = 0; k < NF; ++k) {
+      const int tl = warp * 16 + k * TPW + half;
+      const float fac = __shfl_sync(0xffffffffu, myfac, k * TPW + half);
+      *reinterpret_cast<uint2*>(kd + tl * 128 + ((((c & 15) >> 1) ^ (tl & 7)) << 4)) = value_of(f[k], fac);
+    }
+    if (tile + 1 < tile_hi) fetch(tile + 1);
+    if (n_ent) {
+      __syncwarp();                            // (the list, and the zeros of the flagged chunks, were stored by other lanes)
       for (uint32_t i = lane; i < n_ent; i += 32) {
-        if (i != lane) ent = payload_of(run + i);
+        if (i != lane) ent = payload_of(run0 + i);
         const uint32_t at = s_list[warp][i];
-        put(warp * 16 + (int)(at >> 5), (int)(at & 31u), payload_half(ent));
+        const int tl = warp * 16 + (int)(at >> 5), cc = (int)(at & 31u);
+        const float2 a = pair16_to_float2(ent.x, out_dtype), d = pair16_to_float2(ent.y, out_dtype);
+        *reinterpret_cast<uint2*>(dst + (cc >> 4) * 16384 + tl * 128 + ((((cc & 15) >> 1) ^ (tl & 7)) << 4) + (cc & 1) * 8) =
+            make_uint2(pack_half2(a.x * mul, a.y * mul), pack_half2(d.x * mul, d.y * mul));
       }
-      __syncwarp();
-    };
-    if (!is_v) {
-      __syncwarp();                            // (the zeros of the flagged chunks were stored by other lanes)
-      put_entries([&](int tl, int cc, uint2 v) {
-        *reinterpret_cast<uint2*>(dst + (cc >> 4) * 16384 + tl * 128 + ((((cc & 15) >> 1) ^ (tl & 7)) << 4) + (cc & 1) * 8) = v;
-      });
-    } else {
-      __syncthreads();
-      const int tl = (warp & 3) * 32 + lane;
-      const float fac = s_fac[tl];
-#pragma unroll 8
-      for (int k = 0; k < N / 2; ++k) {
-        const int cc = (warp >> 2) * (N / 2) + k;
-        put_v(tl, cc, value_of(fields[tl * (N + 1) + cc], fac));
-      }
-      if (outl) {
-        __syncthreads();
-        put_entries(put_v);
-      }
-      __syncthreads();
-      for (int i = threadIdx.x; i < (int)(TB / 16); i += 256) reinterpret_cast<uint4*>(dst)[i] = img[i];
-      // (a warp ahead writes the next tile's `fields`, `s_fac` and list meanwhile; `img` only behind the next barrier)
+      __syncwarp();                            // (the next tile's list takes this one's place)
     }
   }
 }
@@ -868,6 +872,7 @@ int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspa
   e.Hkv = a->H_kv; e.Tkv = a->T_kv; e.kt0 = p.kt0; e.nt = p.nt;
   e.qscale = qscale; e.vscale = 1.0f / (float)a->r_qmax;
   e.kmul = mul; e.vmul = mul + bh_all;
+  e.status = p.status; e.epoch = epoch;
   if (a->layout == 0) {
     e.K = a->K; e.V = a->V; e.tblK = a->table_K; e.tblV = a->table_V;
     e.ib = idx_bits_for(a->K.S); e.table_rows = 24 * a->K.S;
@@ -880,7 +885,7 @@ int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspa
   p.kimg = e.kimg; p.vimg = e.vimg;
   p.part = reinterpret_cast<float*>(ws + pl.off_part);
   const int N = d / 4;
-  const size_t esmem = pf_tile_bytes(d) + (size_t)128 * (N + 1) * 4 + (size_t)e.table_rows * 8;
+  const size_t esmem = (size_t)e.table_rows * 8;
   const void* ek = N == 32 ? (a->layout == 0 ? (const void*)&prefill_expand_kernel<32, 0> : (const void*)&prefill_expand_kernel<32, 1>)
                            : (a->layout == 0 ? (const void*)&prefill_expand_kernel<16, 0> : (const void*)&prefill_expand_kernel<16, 1>);
   const void* ak = d == 128 ? (const void*)&prefill_attn_kernel<128> : (const void*)&prefill_attn_kernel<64>;

@@ -45,6 +45,7 @@ struct ExpandParams {
   float qscale, vscale;                           // softmax scale * log2(e), 1 / qmax
   unsigned char* kimg; unsigned char* vimg;
   float* kmul; float* vmul;
+  uint32_t* status; uint32_t epoch;
 };
 
 struct PrefillPlan {

@@ -136,3 +136,35 @@ def test_prompt_calls_leave_no_workspace_behind():
         for out in O:
             hqmq.fused_attention_packed(Q, Kp, Vp, tk, tv, causal=False, out=out)
         assert torch.cuda.memory_allocated() - before < 1 << 20 and torch.equal(*O)
+
+
+@pytest.mark.parametrize("form", ["native", torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shift", [0, 4])
+def test_tables_of_every_alignment(form, shift):
+    """Codeword tables 16 bytes aligned are copied in one piece, others (4 elements further on) entry by entry; T ends inside a tile
+    and inside the tiles of one CTA."""
+    Hq, Hkv, d, T, Tq = 8, 2, 128, 1100, 40
+    q = hqmq.HQMQ(1, Hkv, 24, 3, device="cuda")
+
+    def moved(t):
+        room = torch.empty(t.numel() + 8, dtype=t.dtype, device="cuda")
+        out = room[shift:shift + t.numel()].view(t.shape).copy_(t)
+        assert (out.data_ptr() % 16 != 0) == (shift * t.element_size() % 16 != 0)
+        return out
+
+    Q = (torch.randn(1, Hq, Tq, d, generator=torch.Generator().manual_seed(87)) / math.sqrt(d)).half().cuda()
+    O = torch.empty(Q.shape, dtype=torch.float32, device="cuda")
+    packed = [q.encode(make_kv("randn", (1, Hkv, T, d), seed=88 + kv, dtype=torch.bfloat16).cuda(), 0, kv) for kv in (0, 1)]
+    if form == "native":
+        dense = [q.decode(pk, 0, kv) for kv, pk in enumerate(packed)]
+        tabs = [moved(q.tables(0, kv, "cuda")["table16"]) for kv in (0, 1)]
+        hqmq.fused_attention_packed(Q, *packed, *tabs, causal="bottom_right", out=O)
+        causal = "bottom_right"
+    else:
+        args, dense, causal = [], [], False
+        for kv, pk in enumerate(packed):
+            idx, rq, rs, _ = pk.to_reference()
+            args += [idx, rq, rs.to(form), moved(q.tables(0, kv, "cuda")["joint"].to(form))]
+            dense.append(kernels.decode_dequant(idx, rq, args[-2].float(), args[-1].float(), 7))
+        hqmq.fused_attention(Q, *args, 7, causal=False, out=O)
+    _check(O, _dense_attention(Q, *dense, causal, None))
