@@ -19,7 +19,12 @@
 //            The tiles of all units form one flat sequence cut into equal pieces, one per CTA, whatever the mask leaves of
 //            each unit; a unit that is cut leaves partials, merged by prefill_merge_kernel.
 //
-// Bound: per 256 rows x 128 keys, 2048 tensor clocks and as many of the exponential unit; the rest has to hide behind them.
+// Bound: per 256 rows x 128 keys, 2048 tensor clocks and as many of the exponential unit; 3110 clocks a tile with the two streams'
+// softmax out of step.  Measured and left: part of the exponentials as a polynomial on the FMA pipe (3240 to 4000), P handed over
+// after 96 keys instead of 64 (3100), two threads to a row (246 us against 236 for 2048 queries over 8192 keys).  A prompt of a few
+// tiles pays for what a unit costs once: queries 3000 to 6000 clocks, output 4000, a first pass through cold code 1000.  Loads and
+// stores in one small copy each, masks 32 columns at a time and the streams out of step from the start took the attention of
+// 2048 causal tuple queries from 58 to 47 us, of 4 x 500 with heads of 64 from 45 to 33.
 #include "attn_prefill.cuh"
 #include "attn_ring.cuh"
 
@@ -34,6 +39,8 @@ constexpr int kPfSoftmaxRegs = 208, kPfOtherRegs = 80;
 static_assert(256 * kPfSoftmaxRegs + 128 * kPfOtherRegs <= kPfThreads * 168, "register split beyond the launch's share");
 constexpr float kPfSlack = 8.f;             // log2 units a row's maximum may rise before its accumulator is rescaled
 constexpr uint32_t kPfTmemCols = 512;
+constexpr int kPfStaggerPolls = 64;
+constexpr int kPfFirst = 64;                     // keys of a tile whose P is handed over first (32: 3800 clocks a tile; 64 and 96: 3110)
 
 __host__ __device__ constexpr int pf_stages(int d) { return d == 128 ? 2 : 4; }
 __host__ __device__ constexpr size_t pf_tile_bytes(int d) { return (size_t)d * 256; }
@@ -133,6 +140,10 @@ __device__ __forceinline__ void tc_st32(uint32_t addr, const uint32_t* r) {
       "%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
       ::"r"(addr), PF_I8(r, 0), PF_I8(r, 8), PF_I8(r, 16), PF_I8(r, 24) : "memory");
 }
+__device__ __forceinline__ void tc_st16(uint32_t addr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(addr), PF_I8(r, 0), PF_I8(r, 8) : "memory");
+}
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // K-major operand in the 128-byte swizzle: rows of 128 bytes, groups of eight rows 1024 bytes apart.
@@ -158,6 +169,11 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
       : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
   return d;
 }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+  return d;
+}
 __device__ __forceinline__ float2 add2(float2 a, float2 b) {
   float2 d;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
@@ -174,9 +190,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
   unsigned char* base = smem_raw + (s_base - smem_u32(smem_raw));
   const uint32_t sQ = s_base, sK = sQ + 2 * TB, sV = sK + NS * TB, sO = sV + NS * TB, bars = sO + 8 * 32 * kPfOutRow;
   const uint32_t kfull = bars, kempty = kfull + 8 * NS, vfull = kempty + 8 * NS, vempty = vfull + 8 * NS;
-  // per stream: queries written, S of a tile computed, either half of its P written, the unit's last P V done
+  // per stream: queries written, S of a tile computed, either part of its P written, the unit's last P V done
   const uint32_t qfull = vempty + 8 * NS, sfull = qfull + 16, pfull = sfull + 16, odone = pfull + 32;
   volatile uint32_t* abort_word = reinterpret_cast<volatile uint32_t*>(base + (odone + 16 - s_base));
+  volatile uint32_t* progress = abort_word + 2;      // units that stream 0 has half of its first P of (the word between is tcgen05.alloc's)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) {
@@ -187,6 +204,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
       mbar_init(pfull + 16 * s, 4); mbar_init(pfull + 16 * s + 8, 4);
     }
     *abort_word = 0u;
+    *progress = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 8) {
@@ -226,6 +244,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
           if (g >= NS && !wait(kempty + 8 * st, ph ^ 1u)) { ok = false; break; }
           mbar_expect_tx(kfull + 8 * st, TB);
           bulk_g2s(sK + st * TB, kp + (int64_t)i * TB, TB, kfull + 8 * st);
+          // (all CTAs start at once, and the first S wants a tile of K and the queries: what is needed later waits for those)
+          if (g == 0) { wait(qfull, 0u); if (p.streams > 1) wait(qfull + 8, 0u); }
           if (g >= NS && !wait(vempty + 8 * st, ph ^ 1u)) {
             ok = false;
             uint32_t spins = 0;      // the K copy just issued must have landed before the CTA leaves
@@ -253,7 +273,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
     it.init(p, (int)blockIdx.x);
     auto wait_w = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, wait(bar, parity)) != 0; };   // one answer per warp
     constexpr uint32_t id_qk = f16_idesc(128, 128), id_pv = f16_idesc(128, D, true);
-    // S of the tile in stage st; O += P V of half hb of its keys
+    // S of the tile in stage st; O += P V of a part of its keys
     auto qk = [&](uint32_t st) {
       const uint64_t a0 = sw128_desc(sQ + s * TB), b0 = sw128_desc(sK + st * TB);
 #pragma unroll
@@ -264,17 +284,25 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
       tc_commit(sfull + 8 * s);
       tc_commit(kempty + 8 * st);
     };
-    auto pv = [&](uint32_t st, int hb, bool acc) {
-      const uint64_t b0 = sw128_mn_desc(sV + st * TB + hb * (64 * 128));
+    auto pv = [&](uint32_t st, int part, bool acc) {
+      const uint64_t b0 = sw128_mn_desc(sV + st * TB);
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        tc_mma_ts(256 + D * s, 128 * s + 32 * hb + 8 * k, b0 + ((k * 16 * 128) >> 4), id_pv, acc || k > 0 ? 1u : 0u);
+      for (int k = 0; k < 8; ++k)
+        if ((16 * k < kPfFirst) == (part == 0))
+          tc_mma_ts(256 + D * s, 128 * s + 8 * k, b0 + ((k * 16 * 128) >> 4), id_pv, acc || k > 0 ? 1u : 0u);
     };
     uint32_t g = 0, u = 0;     // tiles, units
     bool ok = true;
     while (ok && it.next(p, q)) {
       ok = wait_w(kfull + 8 * (g % NS), (g / NS) & 1u) && wait_w(qfull + 8 * s, u & 1u);
       if (!ok) break;
+      // The second stream starts a unit half a tile behind the first, so that their softmax warps, which share the exponential
+      // units, take turns from the first tile on.  In step they took 4600 clocks a tile; out of step, where they drift to after
+      // five to fifteen tiles by themselves, 3070.  (A bound of a few thousand clocks, not a condition: nothing depends on it.)
+      if (s == 1 && q.n > 1) {
+        for (int spins = 0; (int)(*progress - (u + 1u)) < 0 && spins < kPfStaggerPolls; ++spins) {}
+      }
+      __syncwarp();
       tc_fence_after();
       if (elect_one()) qk(g % NS);
       for (int i = 0; i < q.n && ok; ++i, ++g) {
@@ -282,6 +310,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
         const uint32_t st = g % NS, ph = (g / NS) & 1u, st1 = (g + 1) % NS, ph1 = ((g + 1) / NS) & 1u;
         ok = wait_w(vfull + 8 * st, ph) && (last || wait_w(kfull + 8 * st1, ph1)) && wait_w(pfull + 16 * s, g & 1u);
         if (!ok) break;
+        if (s == 0 && i == 0) *progress = u + 1u;
         tc_fence_after();
         if (elect_one()) pv(st, 0, i > 0);
         ok = wait_w(pfull + 16 * s + 8, g & 1u);
@@ -310,42 +339,56 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
     const int pl = row / p.G, gh = row - pl * p.G;
     const uint32_t lane_sel = (uint32_t)(warp & 3) << 21;               // TMEM lane 32 * (warp & 3), bits 31:16 of an address
     const uint32_t tS = tmem + 128 * s + lane_sel, tO = tmem + 256 + D * s + lane_sel;
-    // The queries of a unit: a warp loads its 32 rows together, D / 8 lanes of 16 bytes to a row.
+    // The queries of a unit: a warp loads its 32 rows together, D / 8 lanes of 16 bytes to a row, eight loads in flight.  (Loads
+    // and stores of every form, unrolled and in two places, were cold code of several thousand instructions at every unit.)
     constexpr int QL = D / 8, QR = 32 / QL;      // lanes per row, rows per warp-wide load
+    const int c_q = lane % QL;
+    const uint32_t g_inv = 65536u / (uint32_t)p.G + 1u;                   // rw / G = rw * g_inv >> 16 for rw < 128
     auto load_q = [&](const PfPiece& w) {
-      const int bh = p.bh0 + w.bh, b = bh / p.Hkv, h = bh - b * p.Hkv, c = lane % QL;
-      const int64_t qb = (int64_t)b * p.qs_b + (int64_t)(h * p.G) * p.qs_h + 8 * c;
+      const int bh = p.bh0 + w.bh, b = bh / p.Hkv, h = bh - b * p.Hkv;
+      const int64_t qb = (int64_t)b * p.qs_b + (int64_t)(h * p.G) * p.qs_h + 8 * c_q;
       const int tq0 = (w.m * p.streams + s) * p.P;
-      int pw = ((warp & 3) * 32 + lane / QL) / p.G, gw = (warp & 3) * 32 + lane / QL - pw * p.G;
+      auto put = [&](int rw, uint4 v) {
+        const uint32_t dst = sQ + s * TB + rw * 128 + (c_q >> 3) * 16384 + (((c_q & 7) ^ (rw & 7)) << 4);
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+      };
+      const int rw0 = (warp & 3) * 32 + lane / QL;
+      if (p.q_vec) {
+        // (offsets in the unit are 32-bit counts of 16 bytes: with 64-bit strides the addresses of eight loads took 1600 clocks)
+        const uint4* qp = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.Q) + qb + (int64_t)tq0 * p.qs_t);
+        const int st_h = (int)(p.qs_h >> 3), st_t = (int)(p.qs_t >> 3), n_pos = min(p.P, p.Tq - tq0);
+#pragma unroll 1
+        for (int k0 = 0; k0 < QL; k0 += 8) {
+          uint4 v[8];
 #pragma unroll
-      for (int k0 = 0; k0 < QL; k0 += QL) {       // all of them in flight
-        uint4 v[QL];
-#pragma unroll
-        for (int k = 0; k < QL; ++k) {
-          const bool live = pw < p.P && tq0 + pw < p.Tq;
-          const int64_t o = qb + (int64_t)gw * p.qs_h + (int64_t)(tq0 + pw) * p.qs_t;
-          v[k] = make_uint4(0u, 0u, 0u, 0u);
-          if (p.q_vec) {
-            if (live) v[k] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.Q) + o);
-          } else if (live) {
-            float f[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = load_float(p.Q, o + e, p.q_dtype);
-            v[k] = make_uint4(pack_half2(f[0], f[1]), pack_half2(f[2], f[3]), pack_half2(f[4], f[5]), pack_half2(f[6], f[7]));
+          for (int k = 0; k < 8; ++k) {
+            const int rw = rw0 + (k0 + k) * QR, pw = (int)((uint32_t)rw * g_inv >> 16), gw = rw - pw * p.G;
+            v[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (pw < n_pos) v[k] = __ldg(qp + (gw * st_h + pw * st_t));
           }
-          gw += QR;
-          while (gw >= p.G) { gw -= p.G; ++pw; }
-        }
+          const bool bf = p.q_dtype == HQMQ_BF16;
 #pragma unroll
-        for (int k = 0; k < QL; ++k) {
-          if (p.q_vec && p.q_dtype == HQMQ_BF16) {
+          for (int k = 0; k < 8; ++k) {
             uint32_t* w4 = reinterpret_cast<uint32_t*>(&v[k]);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) w4[e] = pack_half2(__uint_as_float(w4[e] << 16), __uint_as_float(w4[e] & 0xffff0000u));
+            for (int e = 0; e < 4; ++e) {
+              const uint32_t hv = pack_half2(__uint_as_float(w4[e] << 16), __uint_as_float(w4[e] & 0xffff0000u));
+              w4[e] = bf ? hv : w4[e];
+            }
+            put(rw0 + (k0 + k) * QR, v[k]);
           }
-          const int rw = (warp & 3) * 32 + (k0 + k) * QR + lane / QL;
-          const uint32_t dst = sQ + s * TB + rw * 128 + (c >> 3) * 16384 + (((c & 7) ^ (rw & 7)) << 4);
-          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(v[k].x), "r"(v[k].y), "r"(v[k].z), "r"(v[k].w) : "memory");
+        }
+      } else {
+#pragma unroll 1
+        for (int k = 0; k < QL; ++k) {
+          const int rw = rw0 + k * QR, pw = (int)((uint32_t)rw * g_inv >> 16), gw = rw - pw * p.G;
+          const int64_t o = qb + (int64_t)gw * p.qs_h + (int64_t)(tq0 + pw) * p.qs_t;
+          float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+          if (pw < p.P && tq0 + pw < p.Tq) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = load_float(p.Q, o + e, p.q_dtype);
+          }
+          put(rw, make_uint4(pack_half2(f[0], f[1]), pack_half2(f[2], f[3]), pack_half2(f[4], f[5]), pack_half2(f[6], f[7])));
         }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // the MMA reads it through the async proxy
@@ -353,26 +396,114 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
       if (lane == 0) mbar_arrive(qfull + 8 * s);
     };
     PfIter it;
-    PfPiece q;
+    PfPiece q, nq;
     it.init(p, (int)blockIdx.x);
     uint32_t g = 0, u = 0;
-    bool have = it.next(p, q), ok = true;
-    if (have) load_q(q);
-    while (ok && have) {
-      PfPiece nq;
-      const bool more = it.next(p, nq);
-      const int bh = p.bh0 + q.bh;
-      const int tq = (q.m * p.streams + s) * p.P + pl;
-      const bool live = pl < p.P && tq < p.Tq;
-      // this row's keys; a row without a query is computed unmasked (its queries are zero) and not written
-      int beg = 0, end = 0x7fffffff;
+    bool more = it.next(p, nq), ok = true;
+    int tq = 0;
+    bool live = false, w_live = false;
+    float m_run = -INFINITY, vmul = 0.f;
+    float2 l2 = make_float2(0.f, 0.f);
+    for (bool first = true;; first = false) {
+      // the last Q K^T of the unit is complete (or there is no unit yet): the next unit's queries may take their place
+      if (more) load_q(nq);
+      if (!first) {
+        ok = wait(odone + 8 * s, u & 1u);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        if (w_live) {
+          const int bh = p.bh0 + q.bh, b = bh / p.Hkv, h = bh - b * p.Hkv;
+          const float l = l2.x + l2.y;
+          const bool whole = q.head && q.tail;
+          const float mul = whole ? (l != 0.f ? vmul / l : 0.f) : vmul;
+          // a partial is stored four columns at a time ([d / 4][256 rows][4], then m and l of the rows), so that a lane stores 16 bytes
+          // and its neighbours the next
+          float* part0 = p.part + ((int64_t)blockIdx.x * 2 + (q.head ? 1 : 0)) * (256 * (D + 2)) + s * 128 + row;
+          float* part = part0 + 3 * (s * 128 + row);
+          const uint32_t stage = sO + warp * (32 * kPfOutRow);
+          uint16_t* orow[4];                       // the rows this lane writes 16 bytes of (null: not a query)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int rw = (warp & 3) * 32 + 8 * k + (lane >> 2), pw = (int)((uint32_t)rw * g_inv >> 16), gw = rw - pw * p.G;
+            const int tw = (q.m * p.streams + s) * p.P + pw;
+            orow[k] = pw < p.P && tw < p.Tq ? reinterpret_cast<uint16_t*>(p.O) + (int64_t)b * p.os_b + (int64_t)(h * p.G + gw) * p.os_h +
+                                                  (int64_t)tw * p.os_t + (lane & 3) * 8 : nullptr;
+          }
+          const bool bf = p.o_dtype == HQMQ_BF16;
+          const float2 mul2v = make_float2(mul, mul);
+#pragma unroll 1
+          for (int c = 0; c < D; c += 32) {        // (one small body: this code runs once or twice a call, from a cold instruction cache)
+            uint32_t o[32];
+            tc_ld32(o, tO + c);
+            tc_wait_ld();
+            float2 x[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) x[e] = mul2(make_float2(__uint_as_float(o[2 * e]), __uint_as_float(o[2 * e + 1])), mul2v);
+            if (!whole) {
+#pragma unroll
+              for (int e = 0; e < 16; e += 2)
+                *reinterpret_cast<float4*>(part + (c + 2 * e) * 256) = make_float4(x[e].x, x[e].y, x[e + 1].x, x[e + 1].y);
+            } else if (p.o_vec) {
+              // through shared memory: four lanes of 16 bytes to a row's 32 columns
+              uint32_t w[16];
+              if (bf) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) { const __nv_bfloat162 t = __float22bfloat162_rn(x[e]); w[e] = *reinterpret_cast<const uint32_t*>(&t); }
+              } else {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) { const __half2 t = __float22half2_rn(x[e]); w[e] = *reinterpret_cast<const uint32_t*>(&t); }
+              }
+              __syncwarp();
+#pragma unroll
+              for (int e = 0; e < 16; e += 4)
+                asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(stage + lane * kPfOutRow + 4 * e), "r"(w[e]), "r"(w[e + 1]), "r"(w[e + 2]), "r"(w[e + 3]) : "memory");
+              __syncwarp();
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                uint4 v;
+                asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                             : "r"(stage + (8 * k + (lane >> 2)) * kPfOutRow + (lane & 3) * 16) : "memory");
+                if (orow[k]) *reinterpret_cast<uint4*>(orow[k] + c) = v;
+              }
+            } else {
+              // any strides, any type: parked in shared memory (fp32) and stored an element at a time
+              const int64_t oo = (int64_t)b * p.os_b + (int64_t)(h * p.G + gh) * p.os_h + (int64_t)tq * p.os_t + c;
+              float* mine = reinterpret_cast<float*>(base + (stage - s_base)) + lane;      // [16][32 lanes]: half of the columns at a time
+#pragma unroll
+              for (int e0 = 0; e0 < 32; e0 += 16) {
+#pragma unroll
+                for (int e = 0; e < 16; e += 2) { mine[e * 32] = x[(e0 + e) / 2].x; mine[(e + 1) * 32] = x[(e0 + e) / 2].y; }
+#pragma unroll 1
+                for (int e = 0; e < 16; ++e)
+                  if (live) store_float(p.O, oo + e0 + e, mine[e * 32], p.o_dtype);
+              }
+            }
+          }
+          if (!whole) { part0[D * 256] = m_run; part0[(D + 1) * 256] = l; }
+          __syncwarp();
+          tc_fence_before();
+        }
+        ++u;
+      }
+      if (!more) break;
+      q = nq;
+      more = it.next(p, nq);
+      tq = (q.m * p.streams + s) * p.P + pl;
+      live = pl < p.P && tq < p.Tq;
+      w_live = __any_sync(0xffffffffu, live);
+      // this row's keys; the least and the most that a row of the warp sees.  (A row without a query is not written; its queries
+      // are zero, and it takes whatever mask leaves the warp's loops alone.)
+      int beg = 0, end = 0;
       if (live) key_range(p.Tkv, p.Tq, p.causal, p.window, tq, beg, end);
-      const int w_beg = __reduce_max_sync(0xffffffffu, beg), w_end = __reduce_min_sync(0xffffffffu, end);
-      const bool w_live = __any_sync(0xffffffffu, live);
-      const float kmul = p.kmul[bh];
-      float m_run = -INFINITY;
-      float2 l2 = make_float2(0.f, 0.f);
+      const int beg_lo = __reduce_min_sync(0xffffffffu, live ? beg : 0x7fffffff), beg_hi = __reduce_max_sync(0xffffffffu, live ? beg : 0);
+      const int end_lo = __reduce_min_sync(0xffffffffu, live ? end : 0x7fffffff), end_hi = __reduce_max_sync(0xffffffffu, live ? end : 0);
+      if (!live) { beg = beg_lo; end = end_hi; }
+      const float kmul = p.kmul[p.bh0 + q.bh];
+      vmul = p.vmul[p.bh0 + q.bh];
       const float2 kmul2 = make_float2(kmul, kmul);
+      m_run = -INFINITY;
+      l2 = make_float2(0.f, 0.f);
       for (int i = 0; i < q.n; ++i, ++g) {
         ok = wait(sfull + 8 * s, g & 1u);
         ok = __all_sync(0xffffffffu, ok);
@@ -384,11 +515,21 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
           for (int c = 0; c < 4; ++c) tc_ld32(r + 32 * c, tS + 32 * c);
           tc_wait_ld();
           const int t0 = (q.tile0 + i) * kPfTok;
-          if (t0 < w_beg || t0 + kPfTok > w_end) {
-            const int lo = beg - t0, hi = end - t0;
+          // Masks, 32 columns at a time and only where a row of the warp needs one: a warp's rows are a few neighbouring positions.
+          // (Compared column by column against both ends a masked tile took 4200 clocks, an unmasked one 1850.)
+          if (t0 < beg_hi || t0 + kPfTok > end_lo) {
 #pragma unroll
-            for (int c = 0; c < 128; ++c)
-              if (c < lo || c >= hi) r[c] = 0xff800000u;
+            for (int gc = 0; gc < 4; ++gc) {
+              const int tg = t0 + 32 * gc;
+              if (tg < beg_hi || tg + 32 > end_lo) {
+                const int hi = end - tg, lo = beg - tg;
+                uint32_t see = hi >= 32 ? 0xffffffffu : hi <= 0 ? 0u : (1u << hi) - 1u;
+                if (lo > 0) see &= lo >= 32 ? 0u : 0xffffffffu << lo;
+#pragma unroll
+                for (int e = 0; e < 32; ++e)
+                  if (!(see & (1u << e))) r[32 * gc + e] = 0xff800000u;
+              }
+            }
           }
           float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -417,25 +558,47 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
           }
           const float nb = m_run == -INFINITY ? 0.f : -m_run;
           const float2 nb2 = make_float2(nb, nb);
-          // P goes to the tensor cores in halves of 64 keys: the first half's P V runs under the second half's exponentials
+          // P goes to the tensor cores in two parts: the first part's P V runs under the other's exponentials
+          auto pairs_of = [&](int grp, uint32_t* pk) {          // 32 keys
 #pragma unroll
-          for (int hb = 0; hb < 2; ++hb) {
-            uint32_t pk[32];
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-              float2 x = fma2(make_float2(__uint_as_float(r[64 * hb + 2 * e]), __uint_as_float(r[64 * hb + 2 * e + 1])), kmul2, nb2);
+            for (int e = 0; e < 16; ++e) {
+              float2 x = fma2(make_float2(__uint_as_float(r[32 * grp + 2 * e]), __uint_as_float(r[32 * grp + 2 * e + 1])), kmul2, nb2);
               x.x = fast_exp2(x.x); x.y = fast_exp2(x.y);
               const __half2 h = __float22half2_rn(x);
               // (the weights that are summed are the rounded ones the tensor cores see: the rounding cancels)
               l2 = add2(l2, __half22float2(h));
               pk[e] = *reinterpret_cast<const uint32_t*>(&h);
             }
-            tc_st32(tS + 32 * hb, pk);
+          };
+          auto hand_over = [&](int part) {
             tc_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(pfull + 16 * s + 8 * hb);
+            if (lane == 0) mbar_arrive(pfull + 16 * s + 8 * part);
+          };
+          if (t0 + 96 < end_hi && t0 + 32 > beg_lo) {
+#pragma unroll
+            for (int grp = 0; grp < 4; ++grp) {
+              uint32_t pk[16];
+              pairs_of(grp, pk);
+              tc_st16(tS + 16 * grp, pk);
+              if (32 * (grp + 1) == kPfFirst) hand_over(0);
+            }
+          } else {                               // 32 keys that no row of the warp sees have weights of zero
+#pragma unroll
+            for (int grp = 0; grp < 4; ++grp) {
+              uint32_t pk[16];
+              if (t0 + 32 * grp < end_hi && t0 + 32 * grp + 32 > beg_lo) {
+                pairs_of(grp, pk);
+              } else {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) pk[e] = 0u;
+              }
+              tc_st16(tS + 16 * grp, pk);
+              if (32 * (grp + 1) == kPfFirst) hand_over(0);
+            }
           }
+          hand_over(1);
         } else {
           tc_fence_before();
           __syncwarp();
@@ -443,68 +606,6 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
         }
       }
       if (!ok) break;
-      // the last Q K^T of the unit is complete: the next unit's queries may take the place of this one's
-      if (more) load_q(nq);
-      ok = wait(odone + 8 * s, u & 1u);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
-      if (w_live) {
-        const int b = bh / p.Hkv, h = bh - b * p.Hkv;
-        const float l = l2.x + l2.y, vmul = p.vmul[bh];
-        const bool whole = q.head && q.tail;
-        const float mul = whole ? (l != 0.f ? vmul / l : 0.f) : vmul;
-        // a partial is stored column by column ([d + 2][256 rows]), so that the lanes of a store are neighbours
-        float* part = p.part + ((int64_t)blockIdx.x * 2 + (q.head ? 1 : 0)) * (256 * (D + 2)) + s * 128 + row;
-        const uint32_t stage = sO + warp * (32 * kPfOutRow);
-        uint16_t* orow[4];                       // the rows this lane writes 16 bytes of (null: not a query)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int rw = (warp & 3) * 32 + 8 * k + (lane >> 2), pw = rw / p.G, gw = rw - pw * p.G;
-          const int tw = (q.m * p.streams + s) * p.P + pw;
-          orow[k] = pw < p.P && tw < p.Tq ? reinterpret_cast<uint16_t*>(p.O) + (int64_t)b * p.os_b + (int64_t)(h * p.G + gw) * p.os_h +
-                                                (int64_t)tw * p.os_t + (lane & 3) * 8 : nullptr;
-        }
-#pragma unroll 1
-        for (int c = 0; c < D; c += 32) {
-          uint32_t o[32];
-          __syncwarp();
-          tc_ld32(o, tO + c);
-          tc_wait_ld();
-          if (!whole) {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) part[(c + e) * 256] = __uint_as_float(o[e]) * mul;
-          } else if (p.o_vec) {
-            // through shared memory: four lanes of 16 bytes to a row's 32 columns
-#pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-              uint32_t w[4];
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const float f0 = __uint_as_float(o[e + 2 * k]) * mul, f1 = __uint_as_float(o[e + 2 * k + 1]) * mul;
-                w[k] = (uint32_t)float_to_bits16(f0, p.o_dtype) | ((uint32_t)float_to_bits16(f1, p.o_dtype) << 16);
-              }
-              asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(stage + lane * kPfOutRow + 2 * e), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
-            }
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              uint4 v;
-              asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                           : "r"(stage + (8 * k + (lane >> 2)) * kPfOutRow + (lane & 3) * 16) : "memory");
-              if (orow[k]) *reinterpret_cast<uint4*>(orow[k] + c) = v;
-            }
-          } else if (live) {
-            const int64_t oo = (int64_t)b * p.os_b + (int64_t)(h * p.G + gh) * p.os_h + (int64_t)tq * p.os_t + c;
-#pragma unroll
-            for (int e = 0; e < 32; ++e) store_float(p.O, oo + e, __uint_as_float(o[e]) * mul, p.o_dtype);
-          }
-        }
-        if (!whole) { part[D * 256] = m_run; part[(D + 1) * 256] = l; }
-        __syncwarp();
-        tc_fence_before();
-      }
-      q = nq; have = more; ++u;
     }
   }
   }
@@ -546,9 +647,13 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const PrefillParams 
     const float* pp = slot(k);
     const float w = fast_exp2(pp[D * 256] - mu);
     l = fmaf(pp[(D + 1) * 256], w, l);
-    const float* col = pp + warp * E * 256;
+    const float4* col = reinterpret_cast<const float4*>(pp - row) + warp * (E / 4) * 256 + row;
 #pragma unroll
-    for (int e = 0; e < E; ++e) acc[e] = fmaf(col[e * 256], w, acc[e]);
+    for (int e = 0; e < E; e += 4) {
+      const float4 v = col[e / 4 * 256];
+      acc[e] = fmaf(v.x, w, acc[e]); acc[e + 1] = fmaf(v.y, w, acc[e + 1]);
+      acc[e + 2] = fmaf(v.z, w, acc[e + 2]); acc[e + 3] = fmaf(v.w, w, acc[e + 3]);
+    }
   }
   const bool failed = *p.status == p.epoch;                 // the attention kernel gave up on a wait
   const float inv = failed ? NAN : l != 0.f ? 1.f / l : 0.f;
@@ -863,7 +968,9 @@ int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspa
   auto vec = [](const void* ptr, const int64_t* s, int dt) {
     return dt != HQMQ_F32 && ((uintptr_t)ptr & 15) == 0 && s[0] % 8 == 0 && s[1] % 8 == 0 && s[2] % 8 == 0;
   };
-  p.q_vec = vec(a->Q, a->q_stride, a->q_dtype); p.o_vec = vec(a->O, a->o_stride, a->o_dtype);
+  // (offsets inside a unit, up to 128 positions or heads away, are 32-bit counts of 16 bytes)
+  auto near = [](int64_t st) { return st > -((int64_t)1 << 26) && st < ((int64_t)1 << 26); };
+  p.q_vec = vec(a->Q, a->q_stride, a->q_dtype) && near(a->q_stride[1]) && near(a->q_stride[2]); p.o_vec = vec(a->O, a->o_stride, a->o_dtype);
   p.status = reinterpret_cast<uint32_t*>(ws); p.epoch = epoch;
   float* mul = reinterpret_cast<float*>(ws + pl.off_mul);
   p.kmul = mul; p.vmul = mul + bh_all;

@@ -31,7 +31,7 @@ struct PrefillParams {
   int units_all;                                  // units of the group
   const unsigned char* kimg; const unsigned char* vimg;
   const float* kmul; const float* vmul;           // [B * H_kv] what a score / an output is multiplied by
-  float* part;                                    // [CTA][2][d + 2][256 rows]
+  float* part;                                    // [CTA][2][256 rows x (d + 2)]: [d / 4][256][4], m [256], l [256]
   uint32_t* status; uint32_t epoch;
   int start_m[kPfMaxCtas], start_off[kPfMaxCtas];  // first unit of every CTA's piece, the unit's tiles before it
 };

@@ -168,3 +168,24 @@ def test_tables_of_every_alignment(form, shift):
             dense.append(kernels.decode_dequant(idx, rq, args[-2].float(), args[-1].float(), 7))
         hqmq.fused_attention(Q, *args, 7, causal=False, out=O)
     _check(O, _dense_attention(Q, *dense, causal, None))
+
+
+@pytest.mark.parametrize("d,Tq,window", [(128, 70, None), (64, 33, 50)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_queries_and_outputs_of_any_stride(d, Tq, window, dtype):
+    """Rows that are 16 bytes aligned are read and written 16 bytes at a time, others an element at a time: same bits.  Seven heads
+    to a group (rows of a block without a query), positions that end inside a stream, masks inside 32-key groups at both ends."""
+    Hq, Hkv, T = 14, 2, 333
+    q = hqmq.HQMQ(1, Hkv, 96, 4, device="cuda")
+    packed = [q.encode(make_kv("spiky", (2, Hkv, T, d), seed=91 + kv, dtype=torch.bfloat16).cuda(), 0, kv, median_mult=3.0) for kv in (0, 1)]
+    tabs = [q.tables(0, kv, "cuda")["table16"] for kv in (0, 1)]
+    Q = (torch.randn(2, Hq, Tq, d, generator=torch.Generator().manual_seed(93)) / math.sqrt(d)).to(dtype).cuda()
+    want = torch.empty_like(Q)
+    hqmq.fused_attention_packed(Q, *packed, *tabs, causal="bottom_right", window=window, out=want)
+    odd = torch.zeros(2, Hq, Tq, d + 4, dtype=dtype, device="cuda")
+    Qo, O = odd[..., 4:].copy_(Q), torch.zeros(2, Hq, Tq, d + 4, dtype=dtype, device="cuda")
+    hqmq.fused_attention_packed(Qo, *packed, *tabs, causal="bottom_right", window=window, out=O[..., :d])
+    assert torch.equal(O[..., :d], want) and not O[..., d:].any()
+    O32 = torch.empty(Q.shape, dtype=torch.float32, device="cuda")
+    hqmq.fused_attention_packed(Qo, *packed, *tabs, causal="bottom_right", window=window, out=O32)
+    _check(O32, _dense_attention(Q, q.decode(packed[0], 0, 0), q.decode(packed[1], 0, 1), "bottom_right", window))
