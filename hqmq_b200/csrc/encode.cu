@@ -835,6 +835,17 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
   }
 }
 
+// Clear the radius code of chunk c in a packed row (atomics: other threads may own neighbouring chunks).
+__device__ __forceinline__ void clear_radius(uint32_t* rowp, int c, int ib, int rbits) {
+  const int cb = ib + rbits;
+  const int lo = c * cb + ib, hi = (c + 1) * cb;   // bit range of the radius code
+  const int w0 = lo >> 5, w1 = (hi - 1) >> 5;
+  const uint32_t m0 = ~0u << (lo & 31);
+  const uint32_t m1 = (hi & 31) ? ~(~0u << (hi & 31)) : ~0u;
+  if (w0 == w1) atomicAnd(&rowp[w0], ~(m0 & m1));
+  else { atomicAnd(&rowp[w0], ~m0); atomicAnd(&rowp[w1], ~m1); }
+}
+
 #include "encode_fused.cuh"
 
 // ---- Med3x: radix select of the two middle order statistics ------------------------------
@@ -1177,17 +1188,6 @@ list_select_kernel(uint32_t* __restrict__ bp_all, const uint32_t* __restrict__ h
     st[7] = __float_as_uint(med);
     if (med_out) med_out[h] = med;
   }
-}
-
-// Clear the radius code of chunk c in a packed row (atomics: other threads may own neighbouring chunks).
-__device__ __forceinline__ void clear_radius(uint32_t* rowp, int c, int ib, int rbits) {
-  const int cb = ib + rbits;
-  const int lo = c * cb + ib, hi = (c + 1) * cb;   // bit range of the radius code
-  const int w0 = lo >> 5, w1 = (hi - 1) >> 5;
-  const uint32_t m0 = ~0u << (lo & 31);
-  const uint32_t m1 = (hi & 31) ? ~(~0u << (hi & 31)) : ~0u;
-  if (w0 == w1) atomicAnd(&rowp[w0], ~(m0 & m1));
-  else { atomicAnd(&rowp[w0], ~m0); atomicAnd(&rowp[w1], ~m1); }
 }
 
 // Flag a chunk found to be an outlier after the provisional pass.
@@ -1850,8 +1850,22 @@ const Mul24& mul24_native() {
   static const Mul24 m = make_mul24_native();
   return m;
 }
+// The same products as reference primaries (the order of the joint table), behind the native ones in a table's memory.
+struct Mul24Both { Mul24 native, ref; };
+const Mul24Both& mul24_both() {
+  static const Mul24Both both = [] {
+    Mul24Both b;
+    b.native = mul24_native();
+    uint8_t native_to_ref[256] = {0};
+    for (int p = 0; p < 24; ++p) native_to_ref[index_maps().ref_to_native[p]] = (uint8_t)p;
+    for (int g = 0; g < 24; ++g)
+      for (int p = 0; p < 24; ++p) b.ref.v[g][p] = native_to_ref[b.native.v[g][p]];
+    return b;
+  }();
+  return both;
+}
 
-inline size_t lut_bytes(int H) { return kLutOffHeads + (size_t)H * kLutHeadBytes + 576; }   // (+ the index table for small calls)
+inline size_t lut_bytes(int H) { return kLutOffHeads + (size_t)H * kLutHeadBytes + sizeof(Mul24Both); }   // (+ the index tables)
 inline size_t lut_ws_bytes(int H) { return (size_t)H * kLutCellCap * 4 + (size_t)H * kLutCellCap * kLutMaxList * 2; }
 // shared memory a main-pass kernel can give to a table next to its other arrays (fp32 joint table, histograms, rows)
 inline size_t lut_smem_budget(int S) { return (size_t)226 * 1024 - (size_t)24 * S * 16 - (size_t)S * 16 - 3 * kHistBins * 4 - 4096; }
@@ -1987,8 +2001,8 @@ extern "C" int hqmq_encode_lut_build(const float* joint, int H, int S, void* lut
   unsigned char* L = reinterpret_cast<unsigned char*>(lut);
   uint32_t* cnt = reinterpret_cast<uint32_t*>(workspace);
   uint16_t* tmp = reinterpret_cast<uint16_t*>(cnt + (size_t)H * kLutCellCap);
-  // the index table of the fold units, for the kernels that read the table in place
-  HQMQ_CHECK_CUDA(cudaMemcpyAsync(L + kLutOffHeads + (size_t)H * kLutHeadBytes, &mul24_native(), 576, cudaMemcpyHostToDevice, st));
+  // the index tables of the fold units
+  HQMQ_CHECK_CUDA(cudaMemcpyAsync(L + kLutOffHeads + (size_t)H * kLutHeadBytes, &mul24_both(), sizeof(Mul24Both), cudaMemcpyHostToDevice, st));
   // the finest grid whose tables fit the encoder's shared memory next to this codebook
   for (int n = kLutNMax; n >= 16; n -= 4) {
     lut_rows_kernel<<<1, 1024, 0, st>>>(n, reinterpret_cast<uint32_t*>(L), reinterpret_cast<uint32_t*>(L + kLutOffRows));
@@ -2174,6 +2188,13 @@ static void fill_fused(const hqmq_encode_args* a, int tensors, uint32_t* status,
   if (cph > (W + kEnc32Warps - 1) / kEnc32Warps) cph = (W + kEnc32Warps - 1) / kEnc32Warps;
   f.per = (int)((W + cph - 1) / cph);
   f.cph = (int)((W + f.per - 1) / f.per);
+  const uint32_t T2 = (uint32_t)(W / d.B);
+  f.t2_mul = 0u; f.t2_sh = 0;
+  if (T2 > 1) {
+    int s = 1;
+    while (((uint64_t)1 << s) < T2) ++s;
+    f.t2_mul = (uint32_t)(((uint64_t)1 << (31 + s)) / T2 + 1); f.t2_sh = s - 1;
+  }
 }
 // `tensors` of one geometry, element type and codebook size, each with its own threshold or all without.
 static int launch_fused(const FusedPair& f, int tensors, int x_dtype, size_t lut_foot, cudaStream_t st) {
@@ -2193,8 +2214,7 @@ static int launch_fused(const FusedPair& f, int tensors, int x_dtype, size_t lut
   HQMQ_CHECK_CUDA(attn::raise_smem_limit(k, smem));
   Maps24 maps;
   memcpy(maps.ref_to_native, index_maps().ref_to_native, 24);
-  const Mul24& nmul = mul24_native();
-  void* args[] = {(void*)&f, &maps, (void*)&nmul};
+  void* args[] = {(void*)&f, &maps};
   const dim3 grid(f.t[0].cph * g.H, tensors);
   // (the CTAs of a head wait for one another only for a threshold of the call's own)
   const bool waits = f.t[0].C > 0.f && !f.t[0].med_in && f.t[0].cph > 1;

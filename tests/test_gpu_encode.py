@@ -566,3 +566,12 @@ def test_tables_are_built_once_per_device():
     t = q.tables(0, 0, "cuda")
     q.quantize_K(torch.randn(1, 2, 3, 32, device="cuda"), 0)
     assert q.tables(0, 0, "cuda:0") is t and q.tables(0, 0, torch.device("cuda")) is t and len(q._tables) == 1
+
+
+@pytest.mark.parametrize("shape,S,br", [((90, 2, 1, 128), 96, 4), ((201, 1, 1, 64), 96, 4), ((60, 3, 3, 128), 24, 3), ((41, 2, 33, 128), 192, 6),
+                                        ((1, 60, 1111, 128), 24, 3), ((2, 50, 1001, 64), 96, 4)])
+def test_one_launch_encoder_places(shape, S, br):
+    """Sequences shorter than a round of warps (one token, three, one more than a round), and heads of few CTAs whose warps hold
+    more tokens than they encode ahead of the threshold."""
+    test_one_launch_encoder(shape, S, br, 3.0, False)
+    test_one_launch_encoder(shape, S, br, 3.0, True)
