@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
   // The tables have arrived (all threads; bounded).  A CTA without tables goes on for the others' sake: it counts and meets them,
   // and gives its tokens up at the end.
   auto tables = [&] {
+    __syncthreads();                           // (the barrier that is waited for has been initialised)
     uint32_t ok = 0u, tries = 0u;
     while (!ok && ++tries < (1u << 24))
       asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar) : "memory");
