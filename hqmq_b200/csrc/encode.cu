@@ -41,7 +41,7 @@ constexpr int kUndCap = 4096;     // undecided chunks listed per head at least; 
 // the nearest one for some direction in the (slightly grown) cell: all k not beaten over the whole cell by the
 // winner at the cell's centre, minus those beaten over the whole cell by another listed one -- the comparison of
 // two codewords is linear in w, so its extreme over the box is at a corner.  A cell with ONE possible winner stores
-// it in its own word (no similarity is evaluated at all); the others point at a list, padded to groups of four,
+// it in its own word (no similarity is evaluated at all); the others point at a list, padded to a multiple of four,
 // which is evaluated with the same fp32 dot product an exhaustive scan of the joint table would use.  At n = 48
 // and S = 96 a list holds 1.9 codewords on average (8 at most) and 98 % of the lists are one group.
 constexpr int kLutNMax = 48;
@@ -51,15 +51,20 @@ constexpr int kLutCandCap = 65528;          // candidate entries per head (list 
 constexpr int kLutMaxList = 16;             // longest list a cell may have; longer -> exhaustive search there
 constexpr float kLutBoxEps = 1e-5f;         // the boxes are grown by this much (cell assignment rounding)
 constexpr float kLutMargin = 1e-5f;         // a codeword is dropped only if it loses by more than this
-// device layout of a table (bytes): global header {n, n_cells, ...} | rows[kLutRows] uint32 = base (20 bits) |
-// first stored cz (6) | stored cells of the row (6) | per head: {total candidates, valid, -, -} uint32, then
+// device layout of a table (bytes): global header {n, n_cells, ...} | rows[kLutRows] uint32 = first cell (16 bits) |
+// first stored cz (8; kLutNoCells: none) | stored cells of the row - 1 (8) | per head: {total candidates, valid, -, -} uint32, then
 // cells[kLutCellCap] uint16 (0xFFFF: exhaustive; bit 15: the single winner in bits 0..14; else list offset / 4),
-// cands[kLutCandCap] uint16 (bit 15 of a group's first entry marks the list's last group)
+// cands[kLutCandCap] uint16 (lists of a multiple of four entries; bit 15 of a list's first entry: there are at most four codewords,
+// else bit 15 marks the last one) | Mul24Both
+constexpr uint32_t kLutNoCells = 255u;
 constexpr size_t kLutOffRows = 32;
 constexpr size_t kLutOffHeads = kLutOffRows + (size_t)kLutRows * 4;
 constexpr size_t kLutHeadBytes = 16 + (size_t)kLutCellCap * 2 + (size_t)kLutCandCap * 2;
 
-struct Mul24 { uint8_t v[24][24]; };       // reference index of (unit g) * (primary p)
+// (fold unit g, primary p of the folded winner) -> what the codeword of g * p and secondary 0 is called: its native index, or its
+// index in the joint table
+struct Mul24 { uint16_t v[24][24]; };
+struct Mul24Both { Mul24 native, ref; };
 
 struct Maps24 { uint8_t ref_to_native[24]; };
 
@@ -71,8 +76,7 @@ struct EncGeom {
   // d_head 64 through the kernels written for 32 chunks per token: with the tokens contiguous in memory, an even
   // token count and an even first row, two consecutive tokens form one "token" of 32 chunks (T_new, xs_t and the
   // packed rows are then those of the pairs); what is per token -- the maximum radius, the scale, the flag word, the
-  // row number -- is taken per half-warp.
-  int pair16;
+  // row number -- is taken per half-warp (PAIR).
 };
 
 // Workspace layout (uint32 words)
@@ -140,11 +144,20 @@ __device__ __forceinline__ int search_exhaustive(const float4* __restrict__ qs, 
 // A table as a kernel sees it (global or shared memory).
 struct LutView {
   const uint32_t* rows; const uint16_t* cells; const uint16_t* cands;
-  const uint8_t* nm;     // [24][24]: (fold unit g, primary p of the folded winner) -> primary of g * p, in the form the caller wants
-  int n; float hn;       // cells per axis, n / 2
+  const uint16_t* nm;    // [24][24], one of Mul24Both
+  int n, step;           // cells per axis; what the next secondary adds to a codeword's index: 8 (native) or 1 (joint table)
+  uint32_t k_row;        // 0x4B000000 * (n + 1): the exponents of two cell coordinates in n * cx + cy
+  float hn, off;         // n / 2 less four parts per million, n / 2 + 2^23
+  uint32_t s_mul;        // k / S = umulhi(2 k, s_mul) for k < 32768
 };
+__device__ __forceinline__ void lut_set(LutView& L, int n, int S, bool ref) {
+  L.n = n; L.step = ref ? 1 : 8;
+  L.k_row = 0x4B000000u * (uint32_t)(n + 1);
+  // (the shrunk scale keeps |w| <= 1 inside the grid without a clamp; it moves a direction by 4e-6 of a box grown by 1e-5)
+  L.hn = 0.5f * (float)n * (1.f - 4e-6f); L.off = 0.5f * (float)n + 8388608.f;
+  L.s_mul = (0x80000000u + (uint32_t)S - 1u) / (uint32_t)S;
+}
 
-__device__ __forceinline__ float xor_sign(float x, uint32_t sign_bits) { return __uint_as_float(__float_as_uint(x) ^ sign_bits); }
 __device__ __forceinline__ float rcp_approx(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -172,81 +185,101 @@ __device__ __forceinline__ float quantile_lerp(float a, float b, float w) {
   return w < 0.5f ? __fmaf_rn(w, diff, a) : __fmaf_rn(-diff, __fsub_rn(1.f, w), b);
 }
 
-// Nearest codeword of the direction u through the table: writes nm[g][p'] and the secondary index, returns
-// false when the chunk has to take the exhaustive search (zero direction, a cell without a list).
-__device__ __forceinline__ bool search_fold24(const float4* __restrict__ joint, const LutView& L, int S, float inv_S,
-                                              float u0, float u1, float u2, float u3, int& prim, int& sidx) {
+// Nearest codeword of the direction u through the table: writes its index (native or joint, by the view) and returns true, or
+// false when the chunk has to take the exhaustive search (zero direction, one that is no number, a cell without a list).
+// Every issue slot here is paid once per 32 chunks and bounds the encoders.  So there is one way through: what has to take the other
+// search is found on the way (every look-up stays inside its table whatever the direction), not branched for.
+__device__ __forceinline__ bool search_fold24(const float4* __restrict__ joint, const LutView& L, int S,
+                                              float u0, float u1, float u2, float u3, uint32_t& code) {
   const float a0 = fabsf(u0), a1 = fabsf(u1), a2 = fabsf(u2), a3 = fabsf(u3);
-  int ax = 0; float am = a0;
-  if (a1 > am) { am = a1; ax = 1; }
-  if (a2 > am) { am = a2; ax = 2; }
-  if (a3 > am) { am = a3; ax = 3; }
-  if (!(am > 0.f)) return false;
   const float hs = ((a0 + a1) + a2) + a3;          // twice the similarity of the nearest half-integer unit
+  bool found = hs > 0.f && hs < 4.f;                // (a direction has |u_0| + .. + |u_3| <= 2)
+  const float m01 = fmaxf(a0, a1), m23 = fmaxf(a2, a3), am = fmaxf(m01, m23);
   // Both folds are taken and one is selected: the lanes of a warp need either and all four axes, and as branches they were a
   // quarter of the kernel's instructions (28 BRA, 30 BSSY / BSYNC of 411 per token).
-  // g = (s0, s1, s2, s3) / 2 with s_i = sign(u_i); 2 conj(g) u in terms of the |u_i|
+  // g = (s0, s1, s2, s3) / 2 with s_i = sign(u_i); 2 conj(g) u in terms of s_i u_j (products with +-1 are exact, so every difference
+  // is rounded once, on the FMA pipe)
   const uint32_t b0 = __float_as_uint(u0), b1 = __float_as_uint(u1), b2 = __float_as_uint(u2), b3 = __float_as_uint(u3);
+  auto sign_of = [](uint32_t b) { return __uint_as_float((b & 0x80000000u) | 0x3f800000u); };
+  const float s0 = sign_of(b0), s1 = sign_of(b1), s2 = sign_of(b2), s3 = sign_of(b3);
   const bool half = hs > 2.f * am;
-  const float h1 = xor_sign(a1 - a0, (b0 ^ b1) & 0x80000000u) + xor_sign(a2 - a3, (b2 ^ b3) & 0x80000000u);
-  const float h2 = xor_sign(a2 - a0, (b0 ^ b2) & 0x80000000u) + xor_sign(a3 - a1, (b1 ^ b3) & 0x80000000u);
-  const float h3 = xor_sign(a3 - a0, (b0 ^ b3) & 0x80000000u) + xor_sign(a1 - a2, (b1 ^ b2) & 0x80000000u);
-  // g = the axis of the largest |u_i| with its sign: conj(g) u swaps neighbours (ax & 1), pairs (ax & 2), and signs
-  const bool o = ax & 1, w = ax & 2;
+  const float h1 = __fadd_rn(__fmaf_rn(s0, u1, -(s1 * u0)), __fmaf_rn(s3, u2, -(s2 * u3)));
+  const float h2 = __fadd_rn(__fmaf_rn(s0, u2, -(s2 * u0)), __fmaf_rn(s1, u3, -(s3 * u1)));
+  const float h3 = __fadd_rn(__fmaf_rn(s0, u3, -(s3 * u0)), __fmaf_rn(s2, u1, -(s1 * u2)));
+  // g = the axis of the largest |u_i| (the first of equals) with its sign: conj(g) u swaps neighbours (o), pairs (w), and signs
+  const bool w = m23 > m01, o = w ? a3 > a2 : a1 > a0;
   const uint32_t q0 = o ? b1 : b0, q1 = o ? b0 : b1, q2 = o ? b3 : b2, q3 = o ? b2 : b3;
   const uint32_t e0 = w ? q2 : q0, e1 = w ? q3 : q1, e2 = w ? q0 : q2, e3 = w ? q1 : q3;
-  const uint32_t neg = e0 & 0x80000000u, f3 = (uint32_t)ax << 31, f2 = ((uint32_t)ax << 30) & 0x80000000u;
+  const uint32_t neg = e0 & 0x80000000u, f3 = o ? 0x80000000u : 0u, f2 = w ? 0x80000000u : 0u;
   const float v0 = half ? hs : am;
-  const float v1 = half ? h1 : __uint_as_float(e1 ^ neg ^ f2 ^ f3);
+  const float v1 = half ? h1 : __uint_as_float(e1 ^ neg ^ (f2 ^ f3));
   const float v2 = half ? h2 : __uint_as_float(e2 ^ neg ^ f2);
   const float v3 = half ? h3 : __uint_as_float(e3 ^ neg ^ f3);
-  const int gp = half ? 8 + (int)(((b0 >> 31) << 3) | ((b1 >> 31) << 2) | ((b2 >> 31) << 1) | (b3 >> 31)) : 2 * ax + (int)(neg >> 31);
+  const uint32_t signs = __funnelshift_l(b3, __funnelshift_l(b2, __funnelshift_l(b1, b0 >> 31, 1), 1), 1);
+  const uint32_t gp = half ? 8u + signs : (w ? 4u : 0u) + (o ? 2u : 0u) + (neg >> 31);
+  // cell coordinates as the low bits of floats of 2^23 and more, rounded down; what is in no cell (it would have to be no direction)
+  // is clamped once, for memory's sake
   const float inv = rcp_approx(v0) * L.hn;
-  const int cx = min(L.n - 1, max(0, (int)fmaf(v1, inv, L.hn)));
-  const int cy = min(L.n - 1, max(0, (int)fmaf(v2, inv, L.hn)));
-  const int cz = (int)fmaf(v3, inv, L.hn);
-  const uint32_t row = L.rows[cx * L.n + cy];
-  const int zcnt = (int)(row >> 26);
-  if (zcnt == 0) return false;
-  const int zc = min(zcnt - 1, max(0, cz - (int)((row >> 20) & 63u)));
-  const uint32_t cw = L.cells[(row & 0xfffffu) + zc];
-  if (cw == 0xffffu) return false;
-  int bk;
-  if (cw & 0x8000u) {
-    bk = (int)(cw & 0x7fffu);
-  } else {
+  const uint32_t cx = __float_as_uint(__fmaf_rd(v1, inv, L.off)), cy = __float_as_uint(__fmaf_rd(v2, inv, L.off)),
+                 cz = __float_as_uint(__fmaf_rd(v3, inv, L.off));
+  const uint32_t row = L.rows[min(cx * (uint32_t)L.n + (cy - L.k_row), (uint32_t)(L.n * L.n - 1))];
+  const uint32_t zc = min(cz - 0x4B000000u - ((row >> 16) & 255u), row >> 24);
+  const uint32_t cw = L.cells[(row & 0xffffu) + zc];
+  found &= cw != 0xffffu;
+  uint32_t bk = found ? cw & 0x7fffu : 0u;          // the single winner, if that is what the cell names
+  if (cw < 0x8000u) {
     float best = -3.f;
     bk = 0;
+    // Four at once, and the rest one by one: the warp goes on for its longest list, 5 or 6 codewords where a lane has more than 4
+    // (a second group of four cost 45 instructions for what 12 or 24 do; s96: two thirds of the warps).
     const uint16_t* e = L.cands + cw * 4u;
-    for (;;) {
-      const uint2 kk = *reinterpret_cast<const uint2*>(e);
-      const int k0 = kk.x & 0x7fff, k1 = kk.x >> 16, k2 = kk.y & 0xffff, k3 = kk.y >> 16;
-      const float4 c0 = joint[k0], c1 = joint[k1], c2 = joint[k2], c3 = joint[k3];
-      const float s0 = fmaf(v3, c0.w, fmaf(v2, c0.z, fmaf(v1, c0.y, v0 * c0.x)));
-      const float s1 = fmaf(v3, c1.w, fmaf(v2, c1.z, fmaf(v1, c1.y, v0 * c1.x)));
-      const float s2 = fmaf(v3, c2.w, fmaf(v2, c2.z, fmaf(v1, c2.y, v0 * c2.x)));
-      const float s3 = fmaf(v3, c3.w, fmaf(v2, c3.z, fmaf(v1, c3.y, v0 * c3.x)));
-      if (s0 > best) { best = s0; bk = k0; }
-      if (s1 > best) { best = s1; bk = k1; }
-      if (s2 > best) { best = s2; bk = k2; }
-      if (s3 > best) { best = s3; bk = k3; }
-      if (kk.x & 0x8000u) break;
-      e += 4;
+    const uint2 kk = *reinterpret_cast<const uint2*>(e);
+    const uint32_t k0 = kk.x & 0x7fff, k1 = kk.x >> 16, k2 = kk.y & 0xffff, k3 = kk.y >> 16;
+    const float4 c0 = joint[k0], c1 = joint[k1], c2 = joint[k2], c3 = joint[k3];
+    const float t0 = fmaf(v3, c0.w, fmaf(v2, c0.z, fmaf(v1, c0.y, v0 * c0.x)));
+    const float t1 = fmaf(v3, c1.w, fmaf(v2, c1.z, fmaf(v1, c1.y, v0 * c1.x)));
+    const float t2 = fmaf(v3, c2.w, fmaf(v2, c2.z, fmaf(v1, c2.y, v0 * c2.x)));
+    const float t3 = fmaf(v3, c3.w, fmaf(v2, c3.z, fmaf(v1, c3.y, v0 * c3.x)));
+    if (t0 > best) { best = t0; bk = k0; }
+    if (t1 > best) { best = t1; bk = k1; }
+    if (t2 > best) { best = t2; bk = k2; }
+    if (t3 > best) { best = t3; bk = k3; }
+    for (uint32_t last = kk.x; !(last & 0x8000u);) {
+      last = e[4];
+      ++e;
+      const uint32_t k = last & 0x7fffu;
+      const float4 c = joint[k];
+      const float t = fmaf(v3, c.w, fmaf(v2, c.z, fmaf(v1, c.y, v0 * c.x)));
+      if (t > best) { best = t; bk = k; }
     }
   }
-  const int pf = (int)(((float)bk + 0.5f) * inv_S);
-  sidx = bk - pf * S;
-  prim = L.nm[gp * 24 + pf];
-  return true;
+  const uint32_t pf = __umulhi(2u * bk, L.s_mul);
+  code = L.nm[gp * 24u + pf] + (bk - pf * (uint32_t)S) * (uint32_t)L.step;
+  return found;
+}
+// The same index of the codeword that the exhaustive search names (ref: the one in the joint table).
+template <bool REF>
+__device__ __forceinline__ uint32_t code_of(int p, int sidx, int S, const Maps24& maps) {
+  if (REF) return (uint32_t)(p * S + sidx);
+  const int au = maps.ref_to_native[p];
+  return (uint32_t)((((au >> 3) * S + sidx) << 3) | (au & 7));
+}
+// x / b for a small whole b, rounded to nearest: y = 1 / b rounded, a first quotient and one step with its exact remainder
+// (P. Markstein, IBM J. Res. Dev. 34, 1990: correctly rounded where y is and nothing under- or overflows; checked against the
+// division for every fraction and b = 1, 3, .., 255).  An infinite x takes the division.
+template <int B>
+__device__ __forceinline__ float div_whole(float x) {
+  constexpr float y = 1.0f / (float)B;
+  const float q = x * y;
+  return x < 1e38f ? __fmaf_rn(__fmaf_rn(-q, (float)B, x), y, q) : __fdiv_rn(x, (float)B);
 }
 
 // Bytes of shared memory a kernel needs for a table of n cells per axis, n_cells stored cells and n_cand candidates.
 __host__ __device__ inline size_t lut_smem_bytes(int n, int n_cells, int n_cand) {
-  return (size_t)n * n * 4 + (((size_t)n_cells * 2 + 15) & ~(size_t)15) + (((size_t)n_cand * 2 + 15) & ~(size_t)15) + 576;
+  return (size_t)n * n * 4 + (((size_t)n_cells * 2 + 15) & ~(size_t)15) + (((size_t)n_cand * 2 + 15) & ~(size_t)15) + sizeof(Mul24);
 }
 // Copy head h's table into shared memory at `dst` (all threads of the CTA; the caller synchronises) and return the view.
-__device__ __forceinline__ LutView lut_to_smem(const unsigned char* __restrict__ lut, int h, unsigned char* dst,
-                                               const Mul24& nm) {
+__device__ __forceinline__ LutView lut_to_smem(const unsigned char* __restrict__ lut, int h, int H, int S, unsigned char* dst) {
   const uint32_t* gh = reinterpret_cast<const uint32_t*>(lut);
   const int n = (int)gh[0], n_cells = (int)gh[1];
   const unsigned char* head = lut + kLutOffHeads + (size_t)h * kLutHeadBytes;
@@ -254,27 +287,30 @@ __device__ __forceinline__ LutView lut_to_smem(const unsigned char* __restrict__
   uint32_t* rows = reinterpret_cast<uint32_t*>(dst);
   uint16_t* cells = reinterpret_cast<uint16_t*>(dst + (size_t)n * n * 4);
   uint16_t* cands = reinterpret_cast<uint16_t*>(dst + (size_t)n * n * 4 + (((size_t)n_cells * 2 + 15) & ~(size_t)15));
-  uint8_t* snm = reinterpret_cast<uint8_t*>(cands) + (((size_t)total * 2 + 15) & ~(size_t)15);
+  uint16_t* snm = cands + (((size_t)total + 7) & ~(size_t)7);
   const uint32_t* grows = reinterpret_cast<const uint32_t*>(lut + kLutOffRows);
   for (int i = threadIdx.x; i < n * n; i += blockDim.x) rows[i] = grows[i];
   const uint32_t* gc = reinterpret_cast<const uint32_t*>(head + 16);
   for (int i = threadIdx.x; i < (n_cells + 1) / 2; i += blockDim.x) reinterpret_cast<uint32_t*>(cells)[i] = gc[i];
   const uint32_t* gd = reinterpret_cast<const uint32_t*>(head + 16 + (size_t)kLutCellCap * 2);
   for (uint32_t i = threadIdx.x; i < (total + 1) / 2; i += blockDim.x) reinterpret_cast<uint32_t*>(cands)[i] = gd[i];
-  for (int i = threadIdx.x; i < 576; i += blockDim.x) snm[i] = nm.v[i / 24][i % 24];
+  const uint16_t* gn = reinterpret_cast<const uint16_t*>(lut + kLutOffHeads + (size_t)H * kLutHeadBytes);
+  for (int i = threadIdx.x; i < 576; i += blockDim.x) snm[i] = gn[i];
   LutView L;
-  L.rows = rows; L.cells = cells; L.cands = cands; L.nm = snm; L.n = n; L.hn = 0.5f * (float)n;
+  L.rows = rows; L.cells = cells; L.cands = cands; L.nm = snm;
+  lut_set(L, n, S, false);
   return L;
 }
 // The same table read in place from global memory (small calls).
-__device__ __forceinline__ LutView lut_global(const unsigned char* __restrict__ lut, int h, const uint8_t* nm) {
+__device__ __forceinline__ LutView lut_global(const unsigned char* __restrict__ lut, int h, int H, int S, bool ref) {
   const uint32_t* gh = reinterpret_cast<const uint32_t*>(lut);
   const unsigned char* head = lut + kLutOffHeads + (size_t)h * kLutHeadBytes;
   LutView L;
   L.rows = reinterpret_cast<const uint32_t*>(lut + kLutOffRows);
   L.cells = reinterpret_cast<const uint16_t*>(head + 16);
   L.cands = reinterpret_cast<const uint16_t*>(head + 16 + (size_t)kLutCellCap * 2);
-  L.nm = nm; L.n = (int)gh[0]; L.hn = 0.5f * (float)L.n;
+  L.nm = reinterpret_cast<const uint16_t*>(lut + kLutOffHeads + (size_t)H * kLutHeadBytes) + (ref ? 576 : 0);
+  lut_set(L, (int)gh[0], S, ref);
   return L;
 }
 __device__ __forceinline__ bool lut_head_valid(const unsigned char* __restrict__ lut, int h) {
@@ -285,7 +321,7 @@ template <bool LUT>
 __global__ void __launch_bounds__(kEncThreads)
 encode_main_kernel(EncGeom g, const void* __restrict__ x, const float* __restrict__ qs_all, hqmq_packed dst,
                    int t_start, uint32_t* __restrict__ hist, Maps24 maps, const float* __restrict__ joint_all,
-                   const unsigned char* __restrict__ lut, Mul24 nmul) {
+                   const unsigned char* __restrict__ lut) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float4* qs = reinterpret_cast<float4*>(smem_raw);
   uint32_t* rows = reinterpret_cast<uint32_t*>(qs + g.S);            // [warps][tpw][kMaxRowWords]
@@ -303,10 +339,9 @@ encode_main_kernel(EncGeom g, const void* __restrict__ x, const float* __restric
     use_lut = lut_head_valid(lut, h);
     if (use_lut) {
       for (int i = threadIdx.x; i < 24 * g.S; i += blockDim.x) sjoint[i] = reinterpret_cast<const float4*>(joint_all)[(int64_t)h * 24 * g.S + i];
-      L = lut_to_smem(lut, h, reinterpret_cast<unsigned char*>(sjoint + 24 * g.S), nmul);
+      L = lut_to_smem(lut, h, g.H, g.S, reinterpret_cast<unsigned char*>(sjoint + 24 * g.S));
     }
   }
-  const float inv_S = 1.0f / (float)g.S;
   __syncthreads();
 
   const int sub = lane / g.npl, c = lane % g.npl;
@@ -348,10 +383,12 @@ encode_main_kernel(EncGeom g, const void* __restrict__ x, const float* __restric
       // normalised copy (keeps the values in range) instead of the reference's exact x / radius
       const float inv_r = __frcp_rn(radius);
       const float u0 = v[0] * inv_r, u1 = v[1] * inv_r, u2 = v[2] * inv_r, u3 = v[3] * inv_r;
-      int s, au;
-      if (!(LUT && use_lut && search_fold24(sjoint, L, g.S, inv_S, u0, u1, u2, u3, au, s)))
-        au = maps.ref_to_native[search_exhaustive(qs, g.S, u0, u1, u2, u3, s)];
-      const uint32_t ni = (uint32_t)((((au >> 3) * g.S + s) << 3) | (au & 7));
+      uint32_t ni;
+      if (!(LUT && use_lut && search_fold24(sjoint, L, g.S, u0, u1, u2, u3, ni))) {
+        int s;
+        const int p = search_exhaustive(qs, g.S, u0, u1, u2, u3, s);
+        ni = code_of<false>(p, s, g.S, maps);
+      }
       const uint32_t f = ni | ((uint32_t)rqf << g.ib);
       const int bit = c * cb, w = bit >> 5, sh = bit & 31;
       atomicOr(&myrow[w], f << sh);
@@ -397,7 +434,7 @@ template <bool DENSE>
 __device__ __forceinline__ void
 encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __restrict__ qs_all, const hqmq_packed& dst,
                   int t_start, const Maps24& maps, const float* __restrict__ joint_all, const unsigned char* __restrict__ lut,
-                  const uint8_t* __restrict__ nmul_dev, float C, float* __restrict__ med_out, float quantile,
+                  float C, float* __restrict__ med_out, float quantile,
                   void* __restrict__ out = nullptr, uint32_t* __restrict__ n_flagged = nullptr) {
   __shared__ uint32_t keys[kSmallMax];                    // norm bits of every chunk of the head
   __shared__ uint32_t tokmax[kSmallTok];                  // bits of the largest radius of a token
@@ -407,7 +444,6 @@ encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __r
   const int n = g.n, per_b = g.T_new * n;                 // chunks of one batch entry
   const int N = g.B * per_b, n_tok = g.B * g.T_new;
   const int S = g.S;
-  const float inv_S = 1.0f / (float)S;
   const bool med = C > 0.f;
   const float qmaxf = (float)g.qmax;
   for (int i = threadIdx.x; i < n_tok; i += blockDim.x) { tokmax[i] = 0u; tokflags[i] = 0u; }
@@ -415,13 +451,13 @@ encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __r
 
   const bool use_lut = lut && lut_head_valid(lut, h);
   LutView L = {};
-  if (use_lut) L = lut_global(lut, h, nmul_dev);
+  if (use_lut) L = lut_global(lut, h, g.H, S, DENSE);
   const float4* joint = reinterpret_cast<const float4*>(joint_all) + (int64_t)h * 24 * S;
   const float4* qs = reinterpret_cast<const float4*>(qs_all) + (int64_t)h * S;
 
   // ---- phase A: norms, token maxima, nearest codewords ------------------------------------------------------
   float nrm[2], radius[2];
-  uint32_t ni[2];
+  uint32_t ni[2];          // native indices (DENSE: indices in the joint table)
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     const int i = threadIdx.x + k * NT;
@@ -436,10 +472,11 @@ encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __r
       atomicMax(&tokmax[b * g.T_new + t], __float_as_uint(radius[k]));   // positive floats order like their bits
       const float inv_r = __frcp_rn(radius[k]);
       const float u0 = v[0] * inv_r, u1 = v[1] * inv_r, u2 = v[2] * inv_r, u3 = v[3] * inv_r;
-      int sidx, au;
-      if (!(use_lut && search_fold24(joint, L, S, inv_S, u0, u1, u2, u3, au, sidx)))
-        au = maps.ref_to_native[search_exhaustive(qs, S, u0, u1, u2, u3, sidx)];
-      ni[k] = (uint32_t)((((au >> 3) * S + sidx) << 3) | (au & 7));
+      if (!(use_lut && search_fold24(joint, L, S, u0, u1, u2, u3, ni[k]))) {
+        int sidx;
+        const int p = search_exhaustive(qs, S, u0, u1, u2, u3, sidx);
+        ni[k] = code_of<DENSE>(p, sidx, S, maps);
+      }
     }
   }
   __syncthreads();
@@ -549,11 +586,8 @@ encode_small_body(const EncGeom& g, const void* __restrict__ x, const float* __r
           ++fl;
           load_chunk(x, b * g.xs_b + h * g.xs_h + t * g.xs_t + 4 * c, g.x_dtype, v);
         } else {
-          int p = 0;
-          const int au = (int)((ni[k] >> 3) / (uint32_t)S) << 3 | (int)(ni[k] & 7u);
-          for (int q = 0; q < 24; ++q) if (maps.ref_to_native[q] == au) p = q;
           const float rad = __fmul_rn(rqf, scale);
-          const float4 cw = joint[p * S + (int)((ni[k] >> 3) % (uint32_t)S)];
+          const float4 cw = joint[ni[k]];
           v[0] = __fmul_rn(cw.x, rad); v[1] = __fmul_rn(cw.y, rad); v[2] = __fmul_rn(cw.z, rad); v[3] = __fmul_rn(cw.w, rad);
         }
         if (g.x_dtype == HQMQ_F32) {
@@ -639,7 +673,6 @@ struct SmallArgs {
   int t_start;
   const float* joint;
   const unsigned char* lut;
-  const uint8_t* nmul;
   float C;
   float* med_out;
   float quantile;
@@ -656,11 +689,11 @@ struct SmallPair { SmallArgs t[2]; Maps24 maps; };
 
 __global__ void __launch_bounds__(kSmallThreads) encode_small_kernel(SmallArgs a, Maps24 maps) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.status = 0u;
-  encode_small_body<false>(a.g, a.x, a.qs, a.dst, a.t_start, maps, a.joint, a.lut, a.nmul, a.C, a.med_out, a.quantile);
+  encode_small_body<false>(a.g, a.x, a.qs, a.dst, a.t_start, maps, a.joint, a.lut, a.C, a.med_out, a.quantile);
 }
 
 __global__ void __launch_bounds__(kSmallThreads) fake_quant_small_kernel(SmallArgs a, Maps24 maps) {
-  encode_small_body<true>(a.g, a.x, a.qs, a.dst, a.t_start, maps, a.joint, a.lut, a.nmul, a.C, a.med_out, a.quantile, a.out, a.n_flagged);
+  encode_small_body<true>(a.g, a.x, a.qs, a.dst, a.t_start, maps, a.joint, a.lut, a.C, a.med_out, a.quantile, a.out, a.n_flagged);
 }
 
 // ---- main pass for the common geometry ------------------------------------------------------------------
@@ -687,10 +720,10 @@ struct BracketArgs {
 };
 constexpr int kBpWords = 16;
 
-template <int DT, int IB, int RB>
+template <int DT, int IB, int RB, bool PAIR>
 __global__ void __launch_bounds__(kEnc32Threads, 1)
 encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __restrict__ qs_all, hqmq_packed dst,
-                     int t_start, Maps24 maps, const float* __restrict__ joint_all, const unsigned char* __restrict__ lut, Mul24 nmul,
+                     int t_start, Maps24 maps, const float* __restrict__ joint_all, const unsigned char* __restrict__ lut,
                      int64_t per, BracketArgs br) {
   __shared__ uint32_t s_below, s_rcount;
   constexpr int CB = IB + RB;
@@ -704,7 +737,6 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = g.S;
-  const float inv_S = 1.0f / (float)S;
   uint32_t* myrow = rows + warp * kMaxRowWords;
   // The tokens of all heads form one sequence, head by head, cut into equal pieces, one per CTA and SM: the tables are
   // loaded once or twice per CTA, and all SMs finish together.  (Cut per (batch, head), 384 CTAs of 16 x 8 heads x 8192
@@ -718,7 +750,7 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
   for (int i = threadIdx.x; i < S; i += blockDim.x) qs[i] = reinterpret_cast<const float4*>(qs_all)[(int64_t)h * S + i];
   for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) shist[i] = 0;
   for (int i = threadIdx.x; i < 24 * S; i += blockDim.x) sjoint[i] = reinterpret_cast<const float4*>(joint_all)[(int64_t)h * 24 * S + i];
-  const LutView L = lut_to_smem(lut, h, reinterpret_cast<unsigned char*>(sjoint + 24 * S), nmul);
+  const LutView L = lut_to_smem(lut, h, g.H, S, reinterpret_cast<unsigned char*>(sjoint + 24 * S));
   const int region = blockIdx.x + h;              // (the next piece has the next CTA or the next head, or both)
   const uint32_t r_lo = br.bp[h * kBpWords + 0], r_hi = br.bp[h * kBpWords + 1], s1 = br.bp[h * kBpWords + 5];
   const float thr_lo = __uint_as_float(br.bp[h * kBpWords + 2]), thr_hi = __uint_as_float(br.bp[h * kBpWords + 3]);
@@ -727,7 +759,7 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
   __syncthreads();
 
   // this warp's token w = b * T_new + t of the head, its chunks in x and its row, advanced by kEnc32Warps tokens
-  const int rpt = g.pair16 ? 2 : 1;
+  const int rpt = PAIR ? 2 : 1;
   int w = w0 + warp;
   int b = w / g.T_new, t = w - b * g.T_new;
   const uint16_t* xp = x + b * g.xs_b + h * g.xs_h + (int64_t)t * g.xs_t + 4 * lane;
@@ -748,9 +780,9 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
     const float nrm = chunk_norm(v);
     const float radius = fmaxf(nrm, 1e-8f);
     // (radii are positive: their bits order like the values)
-    const float rmax = __uint_as_float(g.pair16 ? __reduce_max_sync(lane & 16 ? 0xffff0000u : 0xffffu, __float_as_uint(radius))
-                                          : __reduce_max_sync(0xffffffffu, __float_as_uint(radius)));
-    const float scale = __fdiv_rn(rmax, qmaxf);
+    const float rmax = __uint_as_float(PAIR ? __reduce_max_sync(lane & 16 ? 0xffff0000u : 0xffffu, __float_as_uint(radius))
+                                        : __reduce_max_sync(0xffffffffu, __float_as_uint(radius)));
+    const float scale = div_whole<(1 << RB) - 1>(rmax);
     // radius code: the quotient is first taken with an approximate reciprocal; only a lane whose quotient
     // lies close to a rounding boundary repeats it with the IEEE division the contract names
     float quo = radius * rcp_approx(scale);
@@ -763,17 +795,10 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
       const bool certain = nrm > thr_hi;
       if (certain) rqf = 0.f;                       // a flagged chunk's values live in the side buffer
       flag_word = __ballot_sync(0xffffffffu, certain);
-      if (!certain && nrm > thr_lo) {               // rare: settled against the exact threshold afterwards
-        const uint32_t pos = atomicAdd(&br.band[h * kBandWords + 2], 1u);
-        if (pos < (uint32_t)br.und_cap)
-          br.und[(int64_t)h * br.und_cap + pos] =
-              g.pair16 ? (uint32_t)(((int64_t)b * (2 * g.T_new) + 2 * t + (lane >> 4)) * 32 + (lane & 15))
-                       : (uint32_t)(((int64_t)b * g.T_new + t) * 32 + lane);
-      }
       n_below += __popc(__ballot_sync(0xffffffffu, key < r_lo));       // (every lane keeps the warp's count)
-      const bool in_range = key >= r_lo && key <= r_hi;
-      const uint32_t m = __ballot_sync(0xffffffffu, in_range);
-      if (m) {
+      const bool in_range = key >= r_lo && key <= r_hi, undecided = !certain && nrm > thr_lo;
+      if (__any_sync(0xffffffffu, in_range || undecided)) {
+        const uint32_t m = __ballot_sync(0xffffffffu, in_range);
         uint32_t base = 0u;
         if (lane == 0) base = atomicAdd(&s_rcount, (uint32_t)__popc(m));
         base = __shfl_sync(0xffffffffu, base, 0);
@@ -782,6 +807,14 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
           if (pos < (uint32_t)br.rcap) br.rlist[(int64_t)region * br.rcap + pos] = key;
           atomicAdd(&shist[((key - r_lo) >> s1) & (kHistBins - 1)], 1u);
         }
+        if (undecided) {                            // rare: settled against the exact threshold afterwards
+          const uint32_t pos = atomicAdd(&br.band[h * kBandWords + 2], 1u);
+          if (pos < (uint32_t)br.und_cap)
+            br.und[(int64_t)h * br.und_cap + pos] =
+                PAIR ? (uint32_t)(((int64_t)b * (2 * g.T_new) + 2 * t + (lane >> 4)) * 32 + (lane & 15))
+                     : (uint32_t)(((int64_t)b * g.T_new + t) * 32 + lane);
+        }
+        __syncwarp();
       }
     }
 
@@ -790,14 +823,13 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
     // values in range)
     const float inv_r = rcp_approx(radius);
     const float u0 = v[0] * inv_r, u1 = v[1] * inv_r, u2 = v[2] * inv_r, u3 = v[3] * inv_r;
-    int au, sidx;
-    if (!search_fold24(sjoint, L, S, inv_S, u0, u1, u2, u3, au, sidx)) {
+    uint32_t ni;
+    if (!search_fold24(sjoint, L, S, u0, u1, u2, u3, ni)) {
       // zero direction (every similarity is 0, the first index wins) or a cell without a list
-      int p = 0; sidx = 0;
+      int p = 0, sidx = 0;
       if (fmaxf(fmaxf(fabsf(u0), fabsf(u1)), fmaxf(fabsf(u2), fabsf(u3))) > 0.f) p = search_exhaustive(qs, S, u0, u1, u2, u3, sidx);
-      au = maps.ref_to_native[p];
+      ni = code_of<false>(p, sidx, S, maps);
     }
-    const uint32_t ni = (uint32_t)((((au >> 3) * S + sidx) << 3) | (au & 7));
     const uint32_t f = ni | ((uint32_t)rqf << IB);
 
     // ---- packed row, scale, flag word ---------------------------------------------------------------------
@@ -815,10 +847,10 @@ encode_main32_kernel(EncGeom g, const uint16_t* __restrict__ x, const float* __r
       if (lane < RW) out[lane] = myrow[lane];
       __syncwarp();
     }
-    if (lane == 0 || (g.pair16 && lane == 16)) {
+    if (lane == 0 || (PAIR && lane == 16)) {
       const int half = lane >> 4;
       store_scale(dst, row_now + half, rmax);
-      if (dst.flags) dst.flags[row_now + half] = g.pair16 ? (half ? flag_word >> 16 : flag_word & 0xffffu) : flag_word;
+      if (dst.flags) dst.flags[row_now + half] = PAIR ? (half ? flag_word >> 16 : flag_word & 0xffffu) : flag_word;
     }
   }
   if (lane == 0 && n_below) atomicAdd(&s_below, n_below);
@@ -982,7 +1014,7 @@ struct Fast32 {
   const uint16_t* x;
   int64_t xs_b, xs_h, xs_t;
   int H, T_new;
-  int pair;      // 1: every "token" here is two consecutive tokens of 16 chunks (d_head 64), see EncGeom::pair16
+  int pair;      // 1: every "token" here is two consecutive tokens of 16 chunks (d_head 64), see EncGeom
 };
 
 template <int DT>
@@ -1629,7 +1661,7 @@ __global__ void __launch_bounds__(kScanSmallBlocks * 32) side_small_kernel(const
 // another CTA has started.
 __global__ void __launch_bounds__(kSmallThreads) append_pair_kernel(SmallPair p) {
   const SmallArgs& a = p.t[blockIdx.y];
-  encode_small_body<false>(a.g, a.x, a.qs, a.dst, a.t_start, p.maps, a.joint, a.lut, a.nmul, a.C, a.med_out, a.quantile);
+  encode_small_body<false>(a.g, a.x, a.qs, a.dst, a.t_start, p.maps, a.joint, a.lut, a.C, a.med_out, a.quantile);
   if (!a.scan) return;
   __syncthreads();          // the head's flag words and scales are in global memory for the other warps of the CTA
   const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1669,7 +1701,7 @@ __global__ void __launch_bounds__(1024) lut_rows_kernel(int n, uint32_t* __restr
   if (threadIdx.x == 0) {
     uint32_t run = 0;
     for (int col = 0; col < n * n; ++col) {
-      rows[col] = run | (s_min[col] << 20) | (s_cnt[col] << 26);
+      rows[col] = s_cnt[col] ? run | (s_min[col] << 16) | ((s_cnt[col] - 1u) << 24) : kLutNoCells << 16;
       run += s_cnt[col];
     }
     ghdr[0] = (uint32_t)n; ghdr[1] = run; ghdr[2] = ghdr[3] = 0u;
@@ -1690,7 +1722,7 @@ lut_cells_kernel(const float* __restrict__ joint_all, int S, int n, const uint32
   const int col = blockIdx.x, h = blockIdx.y, K = 24 * S;
   const float4* joint = reinterpret_cast<const float4*>(joint_all) + (int64_t)h * K;
   const uint32_t row = rows[col];
-  const int zcnt = (int)(row >> 26), zmin = (int)((row >> 20) & 63u), base = (int)(row & 0xfffffu);
+  const int zmin = (int)((row >> 16) & 255u), zcnt = (uint32_t)zmin == kLutNoCells ? 0 : (int)(row >> 24) + 1, base = (int)(row & 0xffffu);
   const int cx = col / n, cy = col - cx * n;
   const float step = 2.0f / (float)n;
   const float w1 = (cx + 0.5f) * step - 1.f, w2 = (cy + 0.5f) * step - 1.f;
@@ -1767,7 +1799,7 @@ lut_cells_kernel(const float* __restrict__ joint_all, int S, int n, const uint32
 }
 
 // Per head: cell words and the padded candidate lists.  A list of one needs no entry; longer ones are padded to a
-// multiple of four with their last codeword, and the first entry of a list's last group carries bit 15.
+// multiple of four with their last codeword.  Bit 15: on the first entry of a list of up to four, on the last codeword of a longer one.
 __global__ void __launch_bounds__(1024)
 lut_pack_kernel(const uint16_t* __restrict__ tmp, const uint32_t* __restrict__ cnt, unsigned char* __restrict__ lut, int S) {
   __shared__ uint32_t s_sum[1024];
@@ -1810,7 +1842,7 @@ lut_pack_kernel(const uint16_t* __restrict__ tmp, const uint32_t* __restrict__ c
       cells[c] = (uint16_t)(run >> 2);
       for (uint32_t i = 0; i < pm; ++i) {
         uint16_t v = src[i < m ? i : m - 1];
-        if (i == pm - 4) v |= 0x8000u;
+        if (i == (m <= 4 ? 0u : m - 1)) v |= 0x8000u;
         cands[run + i] = v;
       }
       run += pm;
@@ -1818,14 +1850,15 @@ lut_pack_kernel(const uint16_t* __restrict__ tmp, const uint32_t* __restrict__ c
   }
 }
 
-// (unit g) * (primary p) for all 24 units, as the native primary code (a << 3) | u of the product
-Mul24 make_mul24_native() {
+// (unit g) * (primary p) for all 24 units: the reference primary of the product
+struct RefMul24 { uint8_t v[24][24]; };
+RefMul24 make_mul24() {
   auto prim = [](int p, double v[4]) {
     for (int i = 0; i < 4; ++i) v[i] = 0;
     if (p < 8) v[p >> 1] = (p & 1) ? -1.0 : 1.0;
     else for (int i = 0; i < 4; ++i) v[i] = (((p - 8) >> (3 - i)) & 1) ? -0.5 : 0.5;
   };
-  Mul24 m;
+  RefMul24 m;
   for (int g = 0; g < 24; ++g)
     for (int p = 0; p < 24; ++p) {
       double a[4], b[4], c[4];
@@ -1842,27 +1875,21 @@ Mul24 make_mul24_native() {
         for (int i = 0; i < 4; ++i) dd += (e[i] - c[i]) * (e[i] - c[i]);
         if (dd < 1e-12) ref = q;
       }
-      m.v[g][p] = index_maps().ref_to_native[ref];
+      m.v[g][p] = (uint8_t)ref;
     }
   return m;
 }
-const Mul24& mul24_native() {
-  static const Mul24 m = make_mul24_native();
-  return m;
-}
-// The same products as reference primaries (the order of the joint table), behind the native ones in a table's memory.
-struct Mul24Both { Mul24 native, ref; };
-const Mul24Both& mul24_both() {
-  static const Mul24Both both = [] {
-    Mul24Both b;
-    b.native = mul24_native();
-    uint8_t native_to_ref[256] = {0};
-    for (int p = 0; p < 24; ++p) native_to_ref[index_maps().ref_to_native[p]] = (uint8_t)p;
-    for (int g = 0; g < 24; ++g)
-      for (int p = 0; p < 24; ++p) b.ref.v[g][p] = native_to_ref[b.native.v[g][p]];
-    return b;
-  }();
-  return both;
+// What a codebook of S secondaries calls the products (see Mul24).
+Mul24Both mul24_both(int S) {
+  static const RefMul24 m = make_mul24();
+  Mul24Both b;
+  for (int g = 0; g < 24; ++g)
+    for (int p = 0; p < 24; ++p) {
+      const int ref = m.v[g][p], au = index_maps().ref_to_native[ref];
+      b.native.v[g][p] = (uint16_t)((((au >> 3) * S) << 3) | (au & 7));
+      b.ref.v[g][p] = (uint16_t)(ref * S);
+    }
+  return b;
 }
 
 inline size_t lut_bytes(int H) { return kLutOffHeads + (size_t)H * kLutHeadBytes + sizeof(Mul24Both); }   // (+ the index tables)
@@ -1879,7 +1906,7 @@ static MainGrid main_grid(int T_new, int B, int H) {
   m.ctas = (int)((total + m.per - 1) / m.per);
   return m;
 }
-// d_head 64 as pairs of tokens (see EncGeom::pair16): the call's geometry must allow it, and a token's row must be whole
+// d_head 64 as pairs of tokens (see EncGeom): the call's geometry must allow it, and a token's row must be whole
 // words without padding (16-bit fields; rows of 13- and 19-bit fields are padded, so two of them are not one longer row).
 static bool pair16_of(const hqmq_encode_args& a) {
   return a.dst.n_chunks == 16 && (16 * (idx_bits_for(a.dst.S) + a.dst.radius_bits)) % 32 == 0 && is_half_dtype(a.x_dtype) && a.x_stride[2] == 64 && a.T_new >= 2 && a.T_new % 2 == 0 &&
@@ -2002,7 +2029,9 @@ extern "C" int hqmq_encode_lut_build(const float* joint, int H, int S, void* lut
   uint32_t* cnt = reinterpret_cast<uint32_t*>(workspace);
   uint16_t* tmp = reinterpret_cast<uint16_t*>(cnt + (size_t)H * kLutCellCap);
   // the index tables of the fold units
-  HQMQ_CHECK_CUDA(cudaMemcpyAsync(L + kLutOffHeads + (size_t)H * kLutHeadBytes, &mul24_both(), sizeof(Mul24Both), cudaMemcpyHostToDevice, st));
+  // (pageable memory: the copy has left it when the call returns)
+  const Mul24Both products = mul24_both(S);
+  HQMQ_CHECK_CUDA(cudaMemcpyAsync(L + kLutOffHeads + (size_t)H * kLutHeadBytes, &products, sizeof(products), cudaMemcpyHostToDevice, st));
   // the finest grid whose tables fit the encoder's shared memory next to this codebook
   for (int n = kLutNMax; n >= 16; n -= 4) {
     lut_rows_kernel<<<1, 1024, 0, st>>>(n, reinterpret_cast<uint32_t*>(L), reinterpret_cast<uint32_t*>(L + kLutOffRows));
@@ -2105,7 +2134,6 @@ static EncGeom geom_of(const hqmq_encode_args* a) {
   g.S = d.S; g.ib = idx_bits_for(d.S); g.rbits = d.radius_bits; g.qmax = (1 << d.radius_bits) - 1;
   g.x_dtype = a->x_dtype;
   g.xs_b = a->x_stride[0]; g.xs_h = a->x_stride[1]; g.xs_t = a->x_stride[2];
-  g.pair16 = 0;
   return g;
 }
 
@@ -2126,7 +2154,6 @@ static int fill_small(const hqmq_encode_args* a, const WsPlan& wp, uint32_t* ws,
   sa.g = geom_of(a);
   sa.x = a->x; sa.qs = a->qs; sa.dst = d; sa.t_start = a->t_start; sa.joint = a->joint;
   sa.lut = lut_ok ? lut_b : nullptr;
-  sa.nmul = lut_ok ? lut_b + kLutOffHeads + (size_t)d.H * kLutHeadBytes : nullptr;
   sa.C = a->median_mult; sa.med_out = a->med_out; sa.quantile = a->quantile;
   sa.status = ws + wp.status;
   sa.blk0 = wp.blk0; sa.nblk = wp.nblk;
@@ -2412,7 +2439,6 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
   }
   HQMQ_CHECK_CUDA(cudaMemsetAsync(ws, 0, wp.zero_bytes, st));
   const uint64_t N = (uint64_t)d.B * a->T_new * d.n_chunks;
-  const Mul24& nmul = mul24_native();
   const bool h16 = a->x_dtype == HQMQ_F16;
   if (bracket) {
     // A sample of the tokens predicts the threshold statistic, the main pass needs x only once; should the prediction fail,
@@ -2420,7 +2446,7 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
     const bool pair16 = pair16_of(*a);
     const int T32 = pair16 ? a->T_new / 2 : a->T_new;
     EncGeom g32 = g;
-    if (pair16) { g32.n = 32; g32.npl = 32; g32.tpw = 1; g32.T_new = T32; g32.xs_t = 2 * g.xs_t; g32.pair16 = 1; }
+    if (pair16) { g32.n = 32; g32.npl = 32; g32.tpw = 1; g32.T_new = T32; g32.xs_t = 2 * g.xs_t; }
     const uint16_t* x16 = reinterpret_cast<const uint16_t*>(a->x);
     const unsigned char* lut_arg = reinterpret_cast<const unsigned char*>(a->lut);
     const Fast32 f32{x16, g.xs_b, g.xs_h, g32.xs_t, d.H, T32, pair16 ? 1 : 0};
@@ -2438,9 +2464,9 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
       else sample32_kernel<HQMQ_BF16><<<dim3(gs, d.B * d.H), 256, 0, st>>>(f32, sa, level);
     }
     const void* k = nullptr;
-#define HQMQ_PICK(IB_, RB_) \
-    if (g.ib == IB_ && g.rbits == RB_) k = h16 ? (const void*)&encode_main32_kernel<HQMQ_F16, IB_, RB_> : (const void*)&encode_main32_kernel<HQMQ_BF16, IB_, RB_>;
-    HQMQ_PICK(10, 3) HQMQ_PICK(12, 4) HQMQ_PICK(13, 6)
+#define HQMQ_PICK(IB_, RB_, PAIR_) \
+    if (g.ib == IB_ && g.rbits == RB_ && pair16 == PAIR_) k = h16 ? (const void*)&encode_main32_kernel<HQMQ_F16, IB_, RB_, PAIR_> : (const void*)&encode_main32_kernel<HQMQ_BF16, IB_, RB_, PAIR_>;
+    HQMQ_PICK(10, 3, false) HQMQ_PICK(12, 4, false) HQMQ_PICK(13, 6, false) HQMQ_PICK(12, 4, true)
 #undef HQMQ_PICK
     const size_t smem = (size_t)g.S * 16 + (size_t)kEnc32Warps * kMaxRowWords * 4 + kHistBins * 4 + (size_t)24 * g.S * 16 + lut_foot_of(a) + 16;
     HQMQ_CHECK_CUDA(attn::raise_smem_limit(k, smem));
@@ -2449,7 +2475,7 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
     int t_start = a->t_start;
     BracketArgs br{bp, bp, ws + wp.band, ws + wp.und, ws + wp.rcnt, ws + wp.rlist, ws + wp.histA, wp.rcap, wp.und_cap};
     void* kargs[] = {(void*)&g32, (void*)&x16, (void*)&a->qs, (void*)&d, (void*)&t_start, (void*)&maps, (void*)&a->joint, (void*)&lut_arg,
-                     (void*)&nmul, (void*)&per, (void*)&br};
+                     (void*)&per, (void*)&br};
     HQMQ_CHECK_CUDA(cudaLaunchKernel(k, dim3(mg.ctas), dim3(kEnc32Threads), kargs, smem, st));
     const int64_t W32 = (int64_t)d.B * T32;
     const int shares = (int)((W32 + mg.per - 2) / mg.per) + 1;             // most CTAs that share a head
@@ -2483,11 +2509,11 @@ extern "C" int hqmq_encode(const hqmq_encode_args* a, void* workspace, size_t wo
     if (smem_lut > 48 * 1024)
       HQMQ_CHECK_CUDA(cudaFuncSetAttribute(encode_main_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_lut));
     encode_main_kernel<true><<<grid, kEncThreads, smem_lut, st>>>(g, a->x, a->qs, d, a->t_start, hist_arg, maps, a->joint,
-                                                                  reinterpret_cast<const unsigned char*>(a->lut), nmul);
+                                                                  reinterpret_cast<const unsigned char*>(a->lut));
   } else {
     if (smem_base > 48 * 1024)
       HQMQ_CHECK_CUDA(cudaFuncSetAttribute(encode_main_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_base));
-    encode_main_kernel<false><<<grid, kEncThreads, smem_base, st>>>(g, a->x, a->qs, d, a->t_start, hist_arg, maps, a->joint, nullptr, nmul);
+    encode_main_kernel<false><<<grid, kEncThreads, smem_base, st>>>(g, a->x, a->qs, d, a->t_start, hist_arg, maps, a->joint, nullptr);
   }
   HQMQ_LAUNCH_CHECK();
   SidePair sp;

@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(2 * kAppendMax) append_one_kernel(const Append
   LutView L = {};
   if (!grpA) {
     use_lut = a.lut && lut_head_valid(a.lut, h);
-    if (use_lut) L = lut_global(a.lut, h, a.nmul);
+    if (use_lut) L = lut_global(a.lut, h, g.H, S, false);
   }
   if (p.clear) {
     if (h == 0 && threadIdx.x == 0) *a.status = 0u;
@@ -154,12 +154,13 @@ __global__ void __launch_bounds__(2 * kAppendMax) append_one_kernel(const Append
     if (live) {
       const float4* joint = reinterpret_cast<const float4*>(a.joint) + (int64_t)h * 24 * S;
       const float4* qs = reinterpret_cast<const float4*>(a.qs) + (int64_t)h * S;
-      const float inv_r = __frcp_rn(radius), inv_S = 1.0f / (float)S;
+      const float inv_r = __frcp_rn(radius);
       const float u0 = v[0] * inv_r, u1 = v[1] * inv_r, u2 = v[2] * inv_r, u3 = v[3] * inv_r;
-      int sidx, au;
-      if (!(use_lut && search_fold24(joint, L, S, inv_S, u0, u1, u2, u3, au, sidx)))
-        au = p.maps.ref_to_native[search_exhaustive(qs, S, u0, u1, u2, u3, sidx)];
-      ni = (uint32_t)((((au >> 3) * S + sidx) << 3) | (au & 7));
+      if (!(use_lut && search_fold24(joint, L, S, u0, u1, u2, u3, ni))) {
+        int sidx;
+        const int q = search_exhaustive(qs, S, u0, u1, u2, u3, sidx);
+        ni = code_of<false>(q, sidx, S, p.maps);
+      }
     }
     bar_group(2, 2 * NP);
     if (live) {

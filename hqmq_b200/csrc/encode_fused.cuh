@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
   unsigned char* slut = reinterpret_cast<unsigned char*>(sjoint + 24 * S);
 
   // ---- this CTA's tokens: warp token w = (b, i), i a token or (16 chunks) a pair of tokens -----------------------------
-  const bool pair = g.n == 16;
+  const bool pair = (IB == 0 || IB + RB == 16) && g.n == 16;      // (pairs have fields of 16 bits)
   const int T2 = pair ? (g.T_new + 1) >> 1 : g.T_new, W = g.B * T2;
   const int w0 = part * a.per, w1 = min(W, w0 + a.per);
   const int sub = pair ? lane >> 4 : 0, c = pair ? lane & 15 : lane;
@@ -125,20 +125,21 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(slut), bj = (uint32_t)(24 * S * 16), bq = (uint32_t)S * 16u;
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bj + bq + b_rows + b_cells + b_cands + 576u) : "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bj + bq + b_rows + b_cells + b_cands + (uint32_t)sizeof(Mul24)) : "memory");
     fused_bulk((uint32_t)__cvta_generic_to_shared(sjoint), a.joint + (int64_t)h * 24 * S * 4, bj, bar);
     fused_bulk((uint32_t)__cvta_generic_to_shared(qs), a.qs + (int64_t)h * S * 4, bq, bar);
     fused_bulk(d, a.lut + kLutOffRows, b_rows, bar);
     fused_bulk(d + b_rows, head + 16, b_cells, bar);
     if (b_cands) fused_bulk(d + b_rows + b_cells, head + 16 + (size_t)kLutCellCap * 2, b_cands, bar);
-    // (DENSE decodes with the reference-order joint table: the product table then names reference primaries)
-    fused_bulk(d + b_rows + b_cells + b_cands, a.lut + kLutOffHeads + (size_t)g.H * kLutHeadBytes + (DENSE ? 576 : 0), 576u, bar);
+    // (DENSE decodes with the joint table: its indices, then)
+    fused_bulk(d + b_rows + b_cells + b_cands, a.lut + kLutOffHeads + (size_t)g.H * kLutHeadBytes + (DENSE ? sizeof(Mul24) : 0), (uint32_t)sizeof(Mul24), bar);
     s_flagged = s_gave_up = 0u;
   }
   LutView L;
   L.rows = reinterpret_cast<const uint32_t*>(slut); L.cells = reinterpret_cast<const uint16_t*>(slut + b_rows);
   L.cands = reinterpret_cast<const uint16_t*>(slut + b_rows + b_cells);
-  L.nm = slut + b_rows + b_cells + b_cands; L.n = n; L.hn = 0.5f * (float)n;
+  L.nm = reinterpret_cast<const uint16_t*>(slut + b_rows + b_cells + b_cands);
+  lut_set(L, n, S, DENSE);
 
   // The tables have arrived (all threads; bounded).  A CTA without tables goes on for the others' sake: it counts and meets them,
   // and gives its tokens up at the end.
@@ -151,7 +152,6 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
   };
 
   // ---- one token: radius codes, nearest codewords, row or dense values ---------------------------------------------------------
-  const float inv_S = 1.0f / (float)S;
   uint32_t* myrow = rows + warp * kMaxRowWords;
   uint32_t n_fl = 0u;
   float thr = INFINITY;
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
     // (radii are positive: their bits order like the values)
     const float rmax = __uint_as_float(pair ? __reduce_max_sync(lane & 16 ? 0xffff0000u : 0xffffu, __float_as_uint(radius))
                                           : __reduce_max_sync(0xffffffffu, __float_as_uint(radius)));
-    const float scale = __fdiv_rn(rmax, qmaxf);
+    const float scale = IB ? div_whole<(1 << (IB ? RB : 1)) - 1>(rmax) : __fdiv_rn(rmax, qmaxf);
     // (radius code: see encode_main32_kernel)
     const float quo = radius * rcp_approx(scale);
     float rqf = rintf(quo);
@@ -173,24 +173,23 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
     const uint32_t flag_word = __ballot_sync(0xffffffffu, flagged);
     n_fl += __popc(flag_word);
     const float inv_r = a.rcp_rn ? __frcp_rn(radius) : rcp_approx(radius);
-    int au, sidx;
+    uint32_t ni;                                   // native index (DENSE: index in the joint table)
     const float u0 = v[0] * inv_r, u1 = v[1] * inv_r, u2 = v[2] * inv_r, u3 = v[3] * inv_r;
-    if (!search_fold24(sjoint, L, S, inv_S, u0, u1, u2, u3, au, sidx)) {
-      int p = 0; sidx = 0;
+    if (!search_fold24(sjoint, L, S, u0, u1, u2, u3, ni)) {
+      int p = 0, sidx = 0;
       if (fmaxf(fmaxf(fabsf(u0), fabsf(u1)), fmaxf(fabsf(u2), fabsf(u3))) > 0.f) p = search_exhaustive(qs, S, u0, u1, u2, u3, sidx);
-      au = DENSE ? p : maps.ref_to_native[p];
+      ni = code_of<DENSE>(p, sidx, S, maps);
     }
     if constexpr (DENSE) {
       uint2 o = raw;
       if (!flagged) {
         const float rad = __fmul_rn(rqf, scale);
-        const float4 cw = sjoint[au * S + sidx];
+        const float4 cw = sjoint[ni];
         o.x = float_to_bits16(__fmul_rn(cw.x, rad), DT) | ((uint32_t)float_to_bits16(__fmul_rn(cw.y, rad), DT) << 16);
         o.y = float_to_bits16(__fmul_rn(cw.z, rad), DT) | ((uint32_t)float_to_bits16(__fmul_rn(cw.w, rad), DT) << 16);
       }
       if (live) *reinterpret_cast<uint2*>(a.out + (row * g.n + c) * 4) = o;
     } else {
-      const uint32_t ni = (uint32_t)((((au >> 3) * S + sidx) << 3) | (au & 7));
       const uint32_t f = ni | ((flagged ? 0u : (uint32_t)rqf) << ib);
       if (CB == 16) {
         const uint32_t other = __shfl_xor_sync(0xffffffffu, f, 1);
