@@ -13,7 +13,7 @@ namespace attn {
 const void* fast_kernel(int n_chunks, int ib, int rb, bool outl, bool small);
 size_t fast_warp_bytes(int n_chunks, int ib, int rb, bool outl);
 bool ring_kernel(int n_chunks, int ib, int rb, bool outl, int scale_dtype, RingKernelInfo& k);
-size_t ring_smem_total(int table_rows, int repk_log2, int repv_log2, int d, bool outl, int stages, int merge_slots,
+size_t ring_smem_total(int table_rows, int rows_v, int repk_log2, int repv_log2, int d, bool outl, int stages, int merge_slots,
                        size_t stage_bytes, int warps);
 // Pieces of a unit beyond which the ring kernel with the wide merge runs (see attn_ring_body).  Wide / narrow merge, us: 18 pieces
 // (8 units) 92.2 / 97.8, 9 (16 units) 88.0 / 88.3, s192 78.8 / 80.6, 6 (24) 84.1 / 85.4, s192 100.7 / 103.1, 4 (32) 95.1 / 94.2,
@@ -332,23 +332,28 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
   // third stage bought nothing where it cost a table replica).
   RingKernelInfo rk;
   bool ring = false;
+  // (a table of V's decoded values has no replicas: what replicas fit go to K)
+  const bool full_v = ring_full_v(pl.ib, a->K.radius_bits);
+  const int ring_rows_v = full_v ? kFullRows : pl.table_rows, most_reps = full_v ? 4 : 8;
+  auto rep_k = [&](int rsum) { return full_v ? rsum : (rsum + 1) / 2; };
+  auto rep_v = [&](int rsum) { return full_v ? 0 : rsum / 2; };
   const int64_t tiles_all = (int64_t)a->B * a->T_q * a->H_kv * ((keys + kTile - 1) / kTile);
   if (fast && keys >= kRingMinKeys && tiles_all >= kRingMinTiles && ring_kernel(n, pl.ib, a->K.radius_bits, outl, a->K.scale_dtype, rk)) {
     auto fits = [&](int rsum, int ns, int ms) {
-      return ring_smem_total(pl.table_rows, (rsum + 1) / 2, rsum / 2, a->d, outl, ns, ms, rk.stage_bytes, rk.warps) <= kSmemLimit;
+      return ring_smem_total(pl.table_rows, ring_rows_v, rep_k(rsum), rep_v(rsum), a->d, outl, ns, ms, rk.stage_bytes, rk.warps) <= kSmemLimit;
     };
     if (fits(0, 2, 1)) {
       int rsum = 0;
-      while (rsum < 8 && fits(rsum + 1, 2, 1)) ++rsum;
+      while (rsum < most_reps && fits(rsum + 1, 2, 1)) ++rsum;
       ring = true;
-      pl.rep_log2 = (rsum + 1) / 2; pl.repv_log2 = rsum / 2; pl.ring_stages = 2; pl.merge_slots = 1;
+      pl.rep_log2 = rep_k(rsum); pl.repv_log2 = rep_v(rsum); pl.ring_stages = 2; pl.merge_slots = 1;
       while (pl.ring_stages < 4 && fits(rsum, pl.ring_stages + 1, 1)) ++pl.ring_stages;
       // The d_head-64 kernels (19 consumer warps, bigger stages, a tile that is done sooner) run out of staged tiles
       // with two stages: there the last replica of V goes to a third stage instead (measured on a B64 x 16384-token
       // layer: 463 -> 437 us; at d_head 128 a third stage bought nothing where it cost a replica).
       if (rk.warps > 15 && pl.ring_stages < 3 && rsum > 0 && fits(rsum - 1, 3, 1)) {
         --rsum;
-        pl.rep_log2 = (rsum + 1) / 2; pl.repv_log2 = rsum / 2; pl.ring_stages = 3;
+        pl.rep_log2 = rep_k(rsum); pl.repv_log2 = rep_v(rsum); pl.ring_stages = 3;
       }
       for (int ms : {5, 3})
         if (fits(rsum, pl.ring_stages, ms)) { pl.merge_slots = ms; break; }
@@ -395,7 +400,7 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
     pl.kernel = rk.fn[0];
     pl.nw = rk.warps;
     pl.threads = (rk.warps + 1) * 32;
-    pl.smem = ring_smem_total(pl.table_rows, pl.rep_log2, pl.repv_log2, a->d, outl, pl.ring_stages, pl.merge_slots, rk.stage_bytes, rk.warps);
+    pl.smem = ring_smem_total(pl.table_rows, ring_rows_v, pl.rep_log2, pl.repv_log2, a->d, outl, pl.ring_stages, pl.merge_slots, rk.stage_bytes, rk.warps);
   } else {
   const int nheads = G > 8 ? 16 : 8;
   size_t extra = outl ? (size_t)nheads * a->d * 4 + (size_t)pl.nw * (2 * kStage * 8 + 16 * nheads * 4) : 0;

@@ -76,6 +76,11 @@ struct AttnParams {
 // A ring kernel (attn_ring.cu) and the bytes of one of its stages.
 struct RingKernelInfo { const void* fn[2]; size_t stage_bytes; int warps; };   // fn[1]: units cut into many pieces; warps: consumers (one more warp produces)
 
+// Whether the ring kernels of a field layout keep a table of V's decoded values (see attn_ring.cuh), and the rows that ring_smem must
+// count for it (it halves them).
+__host__ __device__ constexpr bool ring_full_v(int ib, int rb) { return ib + rb <= 13; }
+constexpr int kFullRows = 2 << 13;
+
 // Key range [beg, end) of query position tq.  causal 1: the reference's top-left aligned mask (query i sees keys
 // 0..i); causal 2: bottom-right aligned (the Tq queries are the LAST Tq positions of the Tkv keys: query i sees keys
 // 0..Tkv - Tq + i, a prompt chunk attending over a cache that already holds it).
@@ -273,6 +278,15 @@ struct FastLoader {
         rr = r2;
       }
     }
+  }
+  // Field F -> eight times the field: the byte offset in a table of decoded values, one of 8 bytes per index and radius code.
+  template <int F>
+  static __device__ __forceinline__ uint32_t cut_field8(const uint32_t* w) {
+    constexpr int bit = F * CB, a = bit >> 5, s = bit & 31;
+    constexpr uint32_t mask = ((1u << CB) - 1u) << 3;
+    if constexpr (s + CB > 32) return __funnelshift_r(w[a], w[a + 1], s - 3) & mask;
+    else if constexpr (s >= 3) return (w[a] >> (s - 3)) & mask;
+    else return (w[a] << (3 - s)) & mask;
   }
   template <int NT, int KS> __device__ __forceinline__ void kfield(const Raw& raw, uint32_t& idx, __half2& rr) const {
     cut<KS>(raw.kw[NT], idx, rr);

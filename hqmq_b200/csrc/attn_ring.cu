@@ -42,9 +42,9 @@ bool ring_kernel(int n_chunks, int ib, int rb, bool outl, int scale_dtype, RingK
   return false;
 }
 
-size_t ring_smem_total(int table_rows, int repk_log2, int repv_log2, int d, bool outl, int stages, int merge_slots,
+size_t ring_smem_total(int table_rows, int rows_v, int repk_log2, int repv_log2, int d, bool outl, int stages, int merge_slots,
                        size_t stage_bytes, int warps) {
-  return ring_smem(table_rows, repk_log2, repv_log2, d, outl, stages, merge_slots, stage_bytes, warps).total;
+  return ring_smem(table_rows, rows_v, repk_log2, repv_log2, d, outl, stages, merge_slots, stage_bytes, warps).total;
 }
 
 }  // namespace attn

@@ -12,6 +12,11 @@
 // into the radius) and replicated 2^r times, interleaved entry by entry: random 8-byte gathers cost 5.0 / 4.6 /
 // 3.8 / 2.8 shared-memory cycles per warp at 1 / 4 / 8 / 16 replicas (measured), so K and V each get as many
 // replicas as shared memory allows.
+// Fields of 13 bits (s24_r3) have a table of DECODED values for V, codeword times radius code for all 8192 fields, 64 KB without
+// replicas: a chunk of V is then a shift, a mask and the look-up (3 instructions instead of 15 for index, radius, sign and two
+// multiplies), at 6 wavefronts a gather instead of 3.  That kernel is bound by instructions (1075 a tile) with the shared-memory
+// pipe at a third; with both tensors decoded it is bound by the pipe (272 wavefronts, 744 instructions a tile).  One sequence of
+// 131072 tokens, 8 heads, spikes: neither 109.3 us, K 109.5, both 110, V 106.3.
 // Outliers: a tile of K that owns fragment records adds them with one shared-memory load and one MMA per
 // record; every other flagged chunk (K tiles without records, all of V) is corrected in fp32 on the CUDA cores,
 // one warp-wide step per flagged chunk, from the staged payload slice: its decoded value is 0 (radius code 0),
@@ -60,12 +65,12 @@ struct RingLayout {
 struct RingSmem {
   size_t tblK, tblV, q, bars, merge, ring, total;
 };
-__host__ __device__ inline RingSmem ring_smem(int table_rows, int repk_log2, int repv_log2, int d, bool outl, int stages,
+__host__ __device__ inline RingSmem ring_smem(int table_rows, int rows_v, int repk_log2, int repv_log2, int d, bool outl, int stages,
                                                int merge_slots, size_t stage_bytes, int warps) {
   RingSmem s;
   size_t o = 0;
   s.tblK = o; o += (size_t)(table_rows >> 1) * (8u << repk_log2);
-  s.tblV = o; o += (size_t)(table_rows >> 1) * (8u << repv_log2);
+  s.tblV = o; o += (size_t)(rows_v >> 1) * (8u << repv_log2);
   s.q = o; o += outl ? (size_t)8 * (d + kQPad) * 2 : 0;
   o = (o + 15) & ~(size_t)15;
   s.bars = o; o += 64;                                   // full[4], empty[4]
@@ -175,12 +180,13 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
   constexpr int NKS = G_::NKS, NVG = G_::NVG, NOT = 2 * G_::NVG;
   constexpr int ROW = RL::ROW;
   constexpr int D = 4 * N;
+  constexpr bool FULLV = ring_full_v(IB, RB);
   constexpr int kRingWarps = RL::W, kRingTiles = RL::W, kRingRec = RL::kRec, kRingConsumerThreads = RL::W * 32;
   auto consumer_bar = [] { consumer_bar_n<kRingConsumerThreads>(); };
   auto consumer_bar_or = [](bool pred) { return consumer_bar_or_n<kRingConsumerThreads>(pred); };
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int NS = p.ring_stages;
-  const RingSmem sl = ring_smem(p.table_rows, p.rep_log2, p.repv_log2, p.d, OUTL, NS, p.merge_slots, RL::BYTES, kRingWarps);
+  const RingSmem sl = ring_smem(p.table_rows, FULLV ? kFullRows : p.table_rows, p.rep_log2, p.repv_log2, p.d, OUTL, NS, p.merge_slots, RL::BYTES, kRingWarps);
   unsigned char* tblK = smem_raw + sl.tblK;
   unsigned char* tblV = smem_raw + sl.tblV;
   __half* qh16 = reinterpret_cast<__half*>(smem_raw + sl.q);
@@ -367,28 +373,39 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
     // ---- tables of the KV head (sign-folded, replicated) and the unit's queries --------------------------------
     // (every consumer is past the previous unit's merge barrier here, so nobody still reads the old contents)
     if (h != cur_h) {
-      const int repsK = 1 << p.rep_log2, repsV = 1 << p.repv_log2;
       const uint2* srcK = reinterpret_cast<const uint2*>(p.tblK) + (int64_t)h * p.table_rows;
       const uint2* srcV = reinterpret_cast<const uint2*>(p.tblV) + (int64_t)h * p.table_rows;
       // A warp loads 32 consecutive entries (one per lane) and writes their replicas -- entry after entry, `reps` copies
       // each, which is one contiguous stretch -- with lane-contiguous stores, the values passed by shuffles.  (One lane
       // storing all replicas of its own entry put every store of a warp into two banks: 4 us per table load.)
+      auto replicate = [&](unsigned char* tbl, uint2 e, int i0, int rep_log2) {
+        uint2* d = reinterpret_cast<uint2*>(tbl) + ((size_t)i0 << rep_log2);
+        for (int k = 0; k < 1 << rep_log2; ++k) {
+          const int s = k * 32 + lane, from = s >> rep_log2;
+          const uint2 v = make_uint2(__shfl_sync(0xffffffffu, e.x, from), __shfl_sync(0xffffffffu, e.y, from));
+          if (i0 + from < rows_f) d[s] = v;
+        }
+      };
+      // V, decoded: the entry times every radius code (fields beyond the codebook, which no encoder writes, decode to zero)
+      if constexpr (FULLV) {
+        for (int i = threadIdx.x; i < (1 << IB); i += kRingConsumerThreads) {
+          const uint2 e = i < p.table_rows ? srcV[i] : make_uint2(0u, 0u);
+#pragma unroll
+          for (int rq = 0; rq < (1 << RB); ++rq) {
+            const __half2 rr = __float2half2_rn((float)rq);
+            reinterpret_cast<uint2*>(tblV)[(rq << IB) + i] = make_uint2(hmul2_u32(e.x, rr), hmul2_u32(e.y, rr));
+          }
+        }
+      }
       for (int i0 = warp * 32; i0 < rows_f; i0 += kRingConsumerThreads) {
         const int i = i0 + lane;
         uint2 ek = make_uint2(0u, 0u), ev = make_uint2(0u, 0u);
-        if (i < rows_f) { ek = srcK[2 * i]; ev = srcV[2 * i]; }
-        uint2* dk = reinterpret_cast<uint2*>(tblK) + ((size_t)i0 << p.rep_log2);
-        uint2* dv = reinterpret_cast<uint2*>(tblV) + ((size_t)i0 << p.repv_log2);
-        for (int k = 0; k < repsK; ++k) {
-          const int s = k * 32 + lane, from = s >> p.rep_log2;
-          const uint2 v = make_uint2(__shfl_sync(0xffffffffu, ek.x, from), __shfl_sync(0xffffffffu, ek.y, from));
-          if (i0 + from < rows_f) dk[s] = v;
+        if (i < rows_f) {
+          ek = srcK[2 * i];
+          if constexpr (!FULLV) ev = srcV[2 * i];
         }
-        for (int k = 0; k < repsV; ++k) {
-          const int s = k * 32 + lane, from = s >> p.repv_log2;
-          const uint2 v = make_uint2(__shfl_sync(0xffffffffu, ev.x, from), __shfl_sync(0xffffffffu, ev.y, from));
-          if (i0 + from < rows_f) dv[s] = v;
-        }
+        replicate(tblK, ek, i0, p.rep_log2);
+        if constexpr (!FULLV) replicate(tblV, ev, i0, p.repv_log2);
       }
       cur_h = h;
     }
@@ -635,11 +652,17 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
           uint32_t lo[4], hi[4];
           static_for<0, 4>([&](auto i_) {
             constexpr int i = decltype(i_)::value;
-            uint32_t idx; __half2 rr;
-            FL::template cut<g>(cur.vw[i], idx, rr);
-            const uint2 cw = *reinterpret_cast<const uint2*>(tblV + (idx * strideV + laneoffV));
-            lo[i] = hmul2_u32(cw.x, rr);
-            hi[i] = hmul2_u32(cw.y, rr);
+            if constexpr (FULLV) {
+              const uint2 cw = *reinterpret_cast<const uint2*>(tblV + FL::template cut_field8<g>(cur.vw[i]));
+              lo[i] = cw.x;
+              hi[i] = cw.y;
+            } else {
+              uint32_t idx; __half2 rr;
+              FL::template cut<g>(cur.vw[i], idx, rr);
+              const uint2 cw = *reinterpret_cast<const uint2*>(tblV + (idx * strideV + laneoffV));
+              lo[i] = hmul2_u32(cw.x, rr);
+              hi[i] = hmul2_u32(cw.y, rr);
+            }
           });
           const uint32_t a0 = __byte_perm(lo[0], lo[1], 0x5410), a1 = __byte_perm(lo[0], lo[1], 0x7632);
           const uint32_t a2 = __byte_perm(lo[2], lo[3], 0x5410), a3 = __byte_perm(lo[2], lo[3], 0x7632);
@@ -725,7 +748,60 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
                 }
               }
             }
-            if (!by_column) {
+            if constexpr (N == 32) {
+              // The four lanes of a row r own its NVG chunk columns; the eight rows take their flagged chunks side by side, each by
+              // token (the order every element is summed in) and column.  (One flagged chunk after another, all lanes together, took
+              // 650 clocks each, a third of a tile with two or three spikes.)
+              static_assert(NVG <= 4, "sixteen tokens of a row's columns are 64 bits");
+              const uint32_t ex = excl_scan16(__popc(fw), lane);           // lanes 0..15: entries of the tile's earlier tokens
+              uint64_t left;
+              {
+                const uint4 f4 = *reinterpret_cast<const uint4*>(sb + RL::kFlV + (warp * kTile + 4 * j) * 4);
+                constexpr uint32_t cols = (1u << NVG) - 1u;
+                const int sh = r * NVG;
+                uint32_t v = ((f4.x >> sh) & cols) | (((f4.y >> sh) & cols) << 4) | (((f4.z >> sh) & cols) << 8) | (((f4.w >> sh) & cols) << 12);
+                v <<= (j & 1) * 16;
+                v |= __shfl_xor_sync(0xffffffffu, v, 1);
+                const uint32_t o_ = __shfl_xor_sync(0xffffffffu, v, 2);
+                left = j < 2 ? (uint64_t)v | ((uint64_t)o_ << 32) : (uint64_t)o_ | ((uint64_t)v << 32);
+                if constexpr (EDGE) { if (t0 + kTile > t_end) left &= (1ull << (4 * (t_end - t0))) - 1ull; }
+              }
+              while (__any_sync(0xffffffffu, left != 0ull)) {
+                const bool act = left != 0ull;
+                const int at = act ? __ffsll((long long)left) - 1 : 0, t = at >> 2, g = at & 3, c = r * NVG + g;
+                left &= left - 1ull;
+                const uint32_t fwt = __shfl_sync(0xffffffffu, fw, t);
+                const uint32_t e = th0.z + __shfl_sync(0xffffffffu, ex, t) + __popc(fwt & ((1u << c) - 1u));
+                // P of token t for heads 2j, 2j+1 lives in the lane with r = t & 7 and the same j
+                const int src = ((t & 7) << 2) | j;
+                const float pa0 = __shfl_sync(0xffffffffu, pe[0], src), pa1 = __shfl_sync(0xffffffffu, pe[1], src);
+                const float pb0 = __shfl_sync(0xffffffffu, pe[2], src), pb1 = __shfl_sync(0xffffffffu, pe[3], src);
+                const float p0 = t & 8 ? pb0 : pa0, p1 = t & 8 ? pb1 : pa1;
+                float x0 = 0.f, x1 = 0.f, x2 = 0.f, x3 = 0.f;
+                if (act && e < (uint32_t)p.V.out_cap) {
+                  if (p.V.out_dtype == HQMQ_F32) {
+                    const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.V.out_vals) + (bh * p.V.out_cap + e) * 4);
+                    x0 = v.x; x1 = v.y; x2 = v.z; x3 = v.w;
+                  } else {
+                    const uint32_t rel = e - sh0.z;
+                    uint2 v;
+                    if (rel < sh0.w) v = reinterpret_cast<const uint2*>(sb + RL::kPayV)[rel];
+                    else v = __ldg(reinterpret_cast<const uint2*>(p.V.out_vals) + bh * p.V.out_cap + e);
+                    const float2 a = pair16_to_float2(v.x, p.V.out_dtype), bb = pair16_to_float2(v.y, p.V.out_dtype);
+                    x0 = a.x; x1 = a.y; x2 = bb.x; x3 = bb.y;
+                  }
+                }
+                static_for<0, NVG>([&](auto gg_) {
+                  constexpr int gg = decltype(gg_)::value;
+                  if (act && g == gg) {
+                    o[2 * gg][0] = fmaf(p0, x0, o[2 * gg][0]); o[2 * gg][1] = fmaf(p1, x0, o[2 * gg][1]);
+                    o[2 * gg][2] = fmaf(p0, x1, o[2 * gg][2]); o[2 * gg][3] = fmaf(p1, x1, o[2 * gg][3]);
+                    o[2 * gg + 1][0] = fmaf(p0, x2, o[2 * gg + 1][0]); o[2 * gg + 1][1] = fmaf(p1, x2, o[2 * gg + 1][1]);
+                    o[2 * gg + 1][2] = fmaf(p0, x3, o[2 * gg + 1][2]); o[2 * gg + 1][3] = fmaf(p1, x3, o[2 * gg + 1][3]);
+                  }
+                });
+              }
+            } else if (!by_column) {
             uint32_t tm = __ballot_sync(0xffffffffu, fw != 0u);
             uint32_t e = th0.z;
             while (tm) {

@@ -234,3 +234,32 @@ def test_all_zero_value_rows_keep_their_softmax_weight(T, B):
     for q in (hqmq.HQMQ(1, Hkv, S, br, device="cuda"), hqmq.with_outlier_extraction(hqmq.HQMQ(1, Hkv, S, br, device="cuda"), 3.0)):
         Kp, Vp = _attend_and_check(q, _queries(B, Hq, d, 3101, dtype=torch.float16), K, V, S, br, "zero V rows", splits=(None, 3))
         assert (Vp.to_reference()[2][:, :, ::3] == 0).all()
+
+
+@pytest.mark.parametrize("S,br", [(24, 3), (42, 3), (96, 4)])
+@pytest.mark.parametrize("T", [16000, 15993])
+def test_ring_decode_spikes_everywhere(S, br, T):
+    """Long key ranges with flagged chunks anywhere in both tensors: several in one row of four lanes, none, and in the last, partial
+    tile; codebooks that fill the 10-bit indices of a 13-bit field in part."""
+    B, Hq, Hkv, d = 2, 32, 8, 128
+    q = hqmq.HQMQ(1, Hkv, S, br, device="cuda")
+    gen = torch.Generator().manual_seed(5)
+    K, V = (torch.randn(B, Hkv, T, d, generator=gen).cuda() for _ in range(2))
+    for x in (K, V):
+        spike = torch.rand(B, Hkv, T, 32, generator=gen).cuda() < 0.01
+        spike[:, :, 5:T:61, 4:12] = True                # eight chunks of a token: two rows of lanes, all four columns of each
+        spike[:, :, T - 3:, ::5] = True
+        x.view(B, Hkv, T, 32, 4)[spike] *= 20.0
+    Kp, Vp = (q.encode(x.bfloat16(), 0, kv, median_mult=3.0) for kv, x in enumerate((K, V)))
+    tk, tv = q.tables(0, 0, "cuda"), q.tables(0, 1, "cuda")
+    Q = (torch.randn(B, Hq, 1, d, generator=gen) / math.sqrt(d)).cuda()
+    out = torch.empty(B, Hq, 1, d, device="cuda")
+    hqmq.fused_attention_packed(Q.half(), Kp, Vp, tk["table16"], tv["table16"], out=out)
+    Kd, Vd = q.decode(Kp, 0, 0).repeat_interleave(Hq // Hkv, 1), q.decode(Vp, 0, 1).repeat_interleave(Hq // Hkv, 1)
+    Qf = Q.half().float()
+    p = torch.softmax((Qf @ Kd.transpose(-1, -2)) / math.sqrt(d), -1)
+    want, size = p @ Vd, p @ Vd.abs()
+    # Products of a score have an fp16 operand (2^-11, and 2^-11 more where it is a product itself): a score moves by 2^-10 of the sum
+    # of their sizes, every weight by that share of itself, numerator and normaliser alike; P is one fp16 rounding in both.
+    share = 2.0 ** -10 * (1.0 + (Qf.abs() @ Kd.abs().transpose(-1, -2)).amax(-1, keepdim=True) / math.sqrt(d))
+    assert ((out - want).abs() <= 1e-4 + 2.0 * share * size).all() and rel_l2(out, want) < MAX_ABS
