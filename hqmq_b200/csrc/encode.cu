@@ -1337,7 +1337,7 @@ __device__ __forceinline__ int ofrag_records_for(uint32_t any_c) {
 // and every block after it in this call, gets none: the running total is monotone, so that is every block
 // whose inclusive total exceeds the capacity).  `payload` = 0 on a call without Med3x (nothing flagged).
 constexpr int kScanWarps = 8;
-constexpr int kScanIters = 16;     // blocks per lane: up to 8 * 32 * 16 = 4096 blocks (64 k tokens) in one sweep
+constexpr int kScanIters = 16;     // blocks per lane at most: 8 * 32 * 16 = 4096 blocks (64 k tokens) in one sweep
 __device__ __forceinline__ void
 scan_body(const hqmq_packed& dst, int t_start, int T_new, int blk0, int nblk, int payload, uint32_t* __restrict__ status) {
   __shared__ uint32_t w_tot[kScanWarps], w_ftot[kScanWarps], s_last_ok[kScanWarps];
@@ -1350,19 +1350,20 @@ scan_body(const hqmq_packed& dst, int t_start, int T_new, int blk0, int nblk, in
   uint32_t run = payload ? dst.out_count[bh] : 0u;
   uint32_t frun = foff ? foff[blk0] : 0u;
   const int t_end = t_start + T_new;
-  const int sweep = kScanWarps * 32 * kScanIters;
+  // (no more blocks to a lane than it takes: with sixteen whatever the call, 8192 tokens were the work of one warp, 16.5 us)
+  const int iters = min(kScanIters, (nblk + kScanWarps * 32 - 1) / (kScanWarps * 32)), sweep = kScanWarps * 32 * iters;
   bool full = false;       // a block of an earlier sweep did not fit the record capacity
   for (int s0 = 0; s0 < nblk; s0 += sweep) {
-    // warp w owns the contiguous blocks [s0 + w*32*kScanIters, ...): lane-major inside an iteration
+    // warp w owns the contiguous blocks [s0 + w * 32 * iters, ...): lane-major inside an iteration
     uint32_t c[kScanIters], fc[kScanIters];
     uint32_t wsum = 0, wfsum = 0;
 #pragma unroll
     for (int it = 0; it < kScanIters; ++it) {
-      const int i = s0 + (warp * kScanIters + it) * 32 + lane, ba = blk0 + i;
+      const int i = s0 + (warp * iters + it) * 32 + lane, ba = blk0 + i;
       uint32_t cc = 0, any_c = 0;
       // (an iteration whose 32 blocks all lie past the call -- every one but the first in a one-token append --
       //  is skipped here and in the scan below: it would add zeros)
-      if (i - lane >= nblk) { c[it] = fc[it] = 0u; continue; }
+      if (it >= iters || i - lane >= nblk) { c[it] = fc[it] = 0u; continue; }
       if (i < nblk) {
         const int tb = ba * HQMQ_OUT_BLOCK;
 #pragma unroll
@@ -1395,8 +1396,8 @@ scan_body(const hqmq_packed& dst, int t_start, int T_new, int blk0, int nblk, in
     uint32_t my_last_ok = frun;      // largest inclusive record total within the capacity seen by this warp
 #pragma unroll
     for (int it = 0; it < kScanIters; ++it) {
-      const int i = s0 + (warp * kScanIters + it) * 32 + lane, ba = blk0 + i;
-      if (i - lane >= nblk) continue;
+      const int i = s0 + (warp * iters + it) * 32 + lane, ba = blk0 + i;
+      if (it >= iters || i - lane >= nblk) continue;
       uint32_t incl = c[it], fincl = fc[it];
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -1425,8 +1426,8 @@ scan_body(const hqmq_packed& dst, int t_start, int T_new, int blk0, int nblk, in
       for (int w = 0; w < kScanWarps; ++w) last_ok = max(last_ok, s_last_ok[w]);
 #pragma unroll
       for (int it = 0; it < kScanIters; ++it) {
-        const int i = s0 + (warp * kScanIters + it) * 32 + lane;
-        if (i < nblk) foff[blk0 + i + 1] = fc[it] != 0xffffffffu ? fc[it] : last_ok;
+        const int i = s0 + (warp * iters + it) * 32 + lane;
+        if (it < iters && i < nblk) foff[blk0 + i + 1] = fc[it] != 0xffffffffu ? fc[it] : last_ok;
       }
       full = full || frun + fall > last_ok;   // some block of this sweep was over the capacity
       frun = last_ok;

@@ -182,3 +182,28 @@ def test_records_under_token_by_token_appends():
     O = _attend(Q, Kp, Vp, tk, tv)
     err, r2 = (O - ref).abs().max().item(), rel_l2(O, ref)
     assert err < MAX_ABS * max(1.0, float(ref.abs().max())) and r2 < REL_L2, f"{err:.2e} {r2:.2e}"
+
+
+@pytest.mark.parametrize("T", [4095, 4096, 4113, 8190, 65552])
+@pytest.mark.parametrize("rate", [0.002, 0.02])
+def test_offset_scan_at_its_splits(T, rate):
+    """Payload and record offsets of calls at the edges of what one iteration of the scan's warps, and one sweep, take; records
+    within their capacity and past it (a block whose running total passes it gets none, and so does every later one)."""
+    x = torch.randn(1, 2, T, 128, generator=torch.Generator().manual_seed(T), dtype=torch.float32).cuda()
+    x.view(1, 2, T, 32, 4)[torch.rand(1, 2, T, 32, generator=torch.Generator().manual_seed(1)).cuda() < rate] *= 30.0
+    q = hqmq.HQMQ(1, 2, 24, 3, device="cuda")
+    pk = q.encode(x.bfloat16(), 0, 0, median_mult=3.0, ofrag=True)
+    nb = (T + 15) // 16
+    flags = pk.flags[:2 * pk.T_cap].view(2, -1)[:, :nb * 16].view(2, nb, 16)
+    bits = (flags.unsqueeze(-1) >> torch.arange(32, device="cuda", dtype=torch.int32)) & 1
+    want = bits.sum((2, 3)).cumsum(1)
+    off = pk.out_off.view(2, -1)
+    assert torch.equal(off[:, 1:nb + 1].long(), want) and not off[:, 0].any() and torch.equal(pk.out_count.view(-1).long(), want[:, -1])
+    records = (bits.any(2).sum(-1) + 3) // 4
+    records[records > 2] = 0                                    # (HQMQ_OFRAG_MAX_PER_TILE)
+    if T % 16:
+        records[:, -1] = 0
+    total = records.cumsum(1)
+    kept = torch.where(total <= pk.ofrag_cap, total, torch.zeros_like(total)).cummax(1).values
+    assert torch.equal(pk.ofrag_off.view(2, -1)[:, 1:nb + 1].long(), kept)
+    assert rate < 0.01 or bool((total > pk.ofrag_cap).any())
