@@ -332,9 +332,11 @@ static int make_plan_impl(const hqmq_attn_args* a, Plan& pl, bool query_device, 
   // third stage bought nothing where it cost a table replica).
   RingKernelInfo rk;
   bool ring = false;
-  // (a table of V's decoded values has no replicas: what replicas fit go to K)
+  // (a table of V's decoded values has no replicas: what replicas fit go to K.  With outliers, eight of K leave room for a third
+  // stage and five merge slots, sixteen for one slot: 105.1 against 109.1 us for one sequence of 131072 tokens, 45.4 / 51.4 for 4 x
+  // 20000 on 4 heads, 168.6 / 194.9 for 64 x 3000; without, the stages are smaller and sixteen are better, 67.8 against 71.8.)
   const bool full_v = ring_full_v(pl.ib, a->K.radius_bits);
-  const int ring_rows_v = full_v ? kFullRows : pl.table_rows, most_reps = full_v ? 4 : 8;
+  const int ring_rows_v = full_v ? kFullRows : pl.table_rows, most_reps = full_v ? (outl ? 3 : 4) : 8;
   auto rep_k = [&](int rsum) { return full_v ? rsum : (rsum + 1) / 2; };
   auto rep_v = [&](int rsum) { return full_v ? 0 : rsum / 2; };
   const int64_t tiles_all = (int64_t)a->B * a->T_q * a->H_kv * ((keys + kTile - 1) / kTile);

@@ -7,14 +7,14 @@ namespace attn {
 
 constexpr int kPfTok = 128;                       // tokens per operand tile
 constexpr int kPfMaxCtas = 148;                   // one CTA per SM
-// Query positions from which a call decodes the cache once instead of once per position.  This path / the decode kernels, us:
-//   16 positions  8 heads of 128, G 4, s96 with outliers, 1 sequence: 300 tokens 21 / 16, 1000 29 / 25, 4000 46 / 45, 16000
-//                 136 / 144, 64000 347 / 469; 16 sequences: 300 35 / 169, 4000 297 / 556, 16000 1122 / 2006
-//                 4 heads, G 7, s192, 4 sequences: 1000 31 / 67, 16000 191 / 345;  8 heads of 64, G 8, 4 sequences: 1000 27 / 61
-//   8 positions   1 sequence: 1000 29 / 18, 16000 136 / 87; 16 sequences: 1000 85 / 159, 4000 296 / 288, 16000 1118 / 1014
-//   24 positions  1 sequence: 300 20 / 35, 4000 46 / 75, 64000 348 / 704
-// (The decode kernels stay shorter while every position and head can have a cluster of its own, 148 in all, up to about 2000
-// tokens: 2 heads, 48 positions, 1000 tokens 33 / 24.  The line does not look at that.)
+// Query positions from which a call decodes the cache once instead of once per position.  This path at 16 positions / the decode
+// kernels at 15, us:
+//   8 heads of 128, G 4, s96 with outliers, 1 sequence: 300 tokens 22.5 / 14.6, 1000 25.6 / 22.8, 4000 33 / 45, 16000 81 / 137, 64000
+//   198 / 434; 16 sequences: 300 25 / 155, 4000 168 / 518, 16000 621 / 1884
+//   4 heads, G 7, s192, 4 sequences: 1000 27 / 63, 16000 109 / 329;  8 heads of 64, G 8, 4 sequences: 1000 23 / 78
+// (At 24 positions it costs what it costs at 16.  The decode kernels stay shorter while every position and head can have a cluster
+// of its own, 148 in all, up to about 2000 tokens, and at 8 positions of one short sequence: 1000 tokens 18.  The line does not look
+// at that, nor at 8 to 15 positions of many sequences, where this path would be the shorter: 16000 tokens of 16, 8 positions, 1014.)
 constexpr int kPrefillMinQueries = HQMQ_ATTN_PROMPT_QUERIES;
 constexpr int kPrefillMaxTable = 8192;            // codewords per head that fit the expand kernel's shared memory
 constexpr size_t kPrefillImageBytes = (size_t)512 << 20;   // operand images held at a time; larger caches go by groups of (b, head)

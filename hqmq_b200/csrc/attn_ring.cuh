@@ -16,7 +16,7 @@
 // replicas: a chunk of V is then a shift, a mask and the look-up (3 instructions instead of 15 for index, radius, sign and two
 // multiplies), at 6 wavefronts a gather instead of 3.  That kernel is bound by instructions (1075 a tile) with the shared-memory
 // pipe at a third; with both tensors decoded it is bound by the pipe (272 wavefronts, 744 instructions a tile).  One sequence of
-// 131072 tokens, 8 heads, spikes: neither 109.3 us, K 109.5, both 110, V 106.3.
+// 131072 tokens, 8 heads, spikes: neither 109.3 us, K 109.5, both 110, V 106.3 (105.1 with a third stage).
 // Outliers: a tile of K that owns fragment records adds them with one shared-memory load and one MMA per
 // record; every other flagged chunk (K tiles without records, all of V) is corrected in fp32 on the CUDA cores,
 // one warp-wide step per flagged chunk, from the staged payload slice: its decoded value is 0 (radius code 0),

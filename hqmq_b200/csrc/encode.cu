@@ -1917,10 +1917,10 @@ static bool pair16_of(const hqmq_encode_args& a) {
 // the sampled norms per head (a 1/32 sample of B * T_new tokens, 32 norms each), so the bracket's half-width is
 // 3 / sqrt(norms) (about six standard errors of a median), at least 0.2 % and at most 1.2 %; calls too small for that,
 // and quantiles out in the tails (few norms nearby: a much larger error), take the one-launch encoder.
-// 65536 tokens are where 1.2 % still holds six standard errors.  One read / one launch, us a tensor, s96, 8 heads of 128 with 6 %
-// flagged: 65536 tokens a head 359 / 480, 98304 487 / 705, 131072 612 / 933 (s24, none flagged: 65536 331 / 457; four heads, s192:
-// 337 / 362; heads of 64: 131072 362 / 477).  Below the line the one read would still be the shorter at 8 heads (32768: 217 / 247,
-// 49152: 295 / 362; four heads 220 / 219; 16384: 134 / 135), but its bracket would hold four standard errors, three at 16384.
+// 65536 tokens are where 1.2 % still holds six standard errors.  One read / one launch, us a tensor, s96, 8 heads of 128 with some
+// flagged: 65536 tokens a head 328 / 392, 98304 436 / 570, 131072 535 / 749 (s24, none flagged: 65536 304 / 351; four heads, s192:
+// 331 / 353; heads of 64: 131072 326 / 432).  Below the line the one read is the shorter by little (32768: 201 / 208, 49152: 272 / 306;
+// four heads 230 / 223; 16384: 139 / 125), and its bracket would hold four standard errors, three at 16384.
 constexpr int64_t kBracketMinTokens = 65536;     // B * T_new per head (of 32 chunks each)
 static bool bracket_wanted(const hqmq_encode_args& a) {
   const bool pair = pair16_of(a);

@@ -185,7 +185,7 @@ def test_records_under_token_by_token_appends():
 
 
 @pytest.mark.parametrize("T", [4095, 4096, 4113, 8190, 65552])
-@pytest.mark.parametrize("rate", [0.002, 0.02])
+@pytest.mark.parametrize("rate", [0.002, 0.012])
 def test_offset_scan_at_its_splits(T, rate):
     """Payload and record offsets of calls at the edges of what one iteration of the scan's warps, and one sweep, take; records
     within their capacity and past it (a block whose running total passes it gets none, and so does every later one)."""
