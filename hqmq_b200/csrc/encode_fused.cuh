@@ -9,7 +9,7 @@
 // and radius codes are final as they are written; the waits for the others are filled with the first tokens.  Bound: the issue
 // slots of the search, then what happens once: 57 k clocks of a 4096-token call of 8 heads (fake-quant, s24) are 27 k of search, 7 k
 // until the norms are there, three levels of about 1500 for the histogram, 1800 for its sum, 1400 to see the others' and 1700 to
-// scan.  K and V: 75.0 -> 69.8 us.
+// scan.  K and V: 75.0 -> 69.8 us, 63.8 with the shorter search.
 struct FusedArgs {
   // (what a CTA needs first lies together: a line of the parameters that is not in the constant cache costs some 500 clocks)
   EncGeom g;                  // the call's own geometry: n = 32 chunks per token, or 16 (two tokens per warp)
