@@ -220,6 +220,15 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
   constexpr uint32_t tmem = 0u;               // an allocation of all columns starts at column 0
   // (a wait that runs out raises the abort word: every role then stops at its next wait.  No suspend hint: these waits are
   //  links of the per-tile chain, and a hinted wait was seen to wake late.)
+  // A wait by parity takes a barrier that is two phases on for one that has not moved, so whoever waits has to have a part in the
+  // next phase.  Tile g, unit u of the CTA:
+  //   kfull, vfull    (MMA issuers)  the stage is filled again only after the commits of both streams for tile g
+  //   kempty, vempty  (loader)       freed again only after the tile that the loader is about to put there
+  //   qfull           (MMA issuer)   the next queries need S of the unit's last tile, which it issues after this wait
+  //   qfull           (loader)       the first unit's, before K of its second tile
+  //   sfull           (softmax)      the next S needs P of this one, or the next unit's queries, of all four warps
+  //   pfull           (MMA issuer)   the next P needs the S that it issues after both parts of this one
+  //   odone           (softmax)      the next unit's needs all four warps' P of that unit
   auto wait = [&](uint32_t bar, uint32_t parity) {
     for (uint32_t spins = 0; !mbar_try_wait(bar, parity);) {
       if (++spins > kWaitLimit || ((spins & 255u) == 0u && *abort_word)) { *abort_word = 1u; return false; }
@@ -244,8 +253,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
           if (g >= NS && !wait(kempty + 8 * st, ph ^ 1u)) { ok = false; break; }
           mbar_expect_tx(kfull + 8 * st, TB);
           bulk_g2s(sK + st * TB, kp + (int64_t)i * TB, TB, kfull + 8 * st);
-          // (all CTAs start at once, and the first S wants a tile of K and the queries: what is needed later waits for those)
-          if (g == 0) { wait(qfull, 0u); if (p.streams > 1) wait(qfull + 8, 0u); }
+          // (all CTAs start at once, and the first S wants a tile of K and the queries: what is needed later waits for those.  Only
+          //  where the piece has a second tile: its K is issued behind this wait, so no stream gets to its next queries before.  Of a
+          //  piece of one tile a stream does without V, its barrier is then two phases on, and this wait would never end.)
+          if (g == 0 && q.n > 1) { wait(qfull, 0u); if (p.streams > 1) wait(qfull + 8, 0u); }
           if (g >= NS && !wait(vempty + 8 * st, ph ^ 1u)) {
             ok = false;
             uint32_t spins = 0;      // the K copy just issued must have landed before the CTA leaves

@@ -189,3 +189,23 @@ def test_queries_and_outputs_of_any_stride(d, Tq, window, dtype):
     O32 = torch.empty(Q.shape, dtype=torch.float32, device="cuda")
     hqmq.fused_attention_packed(Qo, *packed, *tabs, causal="bottom_right", window=window, out=O32)
     _check(O32, _dense_attention(Q, q.decode(packed[0], 0, 0), q.decode(packed[1], 0, 1), "bottom_right", window))
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,d,T", [(32, 32, 8, 128, 80), (64, 64, 8, 64, 80), (40, 32, 8, 128, 96), (24, 14, 2, 128, 128)])
+@pytest.mark.parametrize("causal", ["bottom_right", False])
+def test_many_prompts_of_one_tile(B, Hq, Hkv, d, T, causal):
+    """A batch of prompts with all keys in one tile: several units to a CTA, and in the last row block of each a second stream that
+    holds no query (or few), which is through with a unit before the first stream has loaded its queries.  Queries 16 bytes at a time,
+    in fp32 and at odd addresses (an element at a time, the slowest load)."""
+    q = hqmq.HQMQ(1, Hkv, 96, 4, device="cuda")
+    packed = [q.encode(make_kv("spiky", (B, Hkv, T, d), seed=94 + kv, dtype=torch.bfloat16).cuda(), 0, kv, median_mult=3.0) for kv in (0, 1)]
+    tabs = [q.tables(0, kv, "cuda")["table16"] for kv in (0, 1)]
+    Q = (torch.randn(B, Hq, T, d, generator=torch.Generator().manual_seed(96)) / math.sqrt(d)).half().cuda()
+    O = torch.full(Q.shape, float("nan"), device="cuda")
+    hqmq.fused_attention_packed(Q, *packed, *tabs, causal=causal, out=O)
+    _check(O, _dense_attention(Q, q.decode(packed[0], 0, 0), q.decode(packed[1], 0, 1), causal, None))
+    odd = torch.zeros(B, Hq, T, d + 4, dtype=Q.dtype, device="cuda")[..., 4:].copy_(Q)
+    for queries in (Q.float(), odd):
+        same = torch.full_like(O, float("nan"))
+        hqmq.fused_attention_packed(queries, *packed, *tabs, causal=causal, out=same)
+        assert torch.equal(same, O)
