@@ -411,6 +411,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
     it.init(p, (int)blockIdx.x);
     uint32_t g = 0, u = 0;
     bool more = it.next(p, nq), ok = true;
+    // (the expansion, complete by now, went on without a table somewhere: no row of the call is a result.  Units that are cut get
+    //  their NaN from the merge.)
+    const bool lost = __ldcg(p.status) == p.epoch;
     int tq = 0;
     bool live = false, w_live = false;
     float m_run = -INFINITY, vmul = 0.f;
@@ -511,7 +514,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
       const int end_lo = __reduce_min_sync(0xffffffffu, live ? end : 0x7fffffff), end_hi = __reduce_max_sync(0xffffffffu, live ? end : 0);
       if (!live) { beg = beg_lo; end = end_hi; }
       const float kmul = p.kmul[p.bh0 + q.bh];
-      vmul = p.vmul[p.bh0 + q.bh];
+      vmul = lost ? NAN : p.vmul[p.bh0 + q.bh];
       const float2 kmul2 = make_float2(kmul, kmul);
       m_run = -INFINITY;
       l2 = make_float2(0.f, 0.f);
@@ -617,6 +620,18 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
         }
       }
       if (!ok) break;
+    }
+    // A wait ran out: the rows of this unit and of the CTA's others become NaN (of a unit that is cut, the merge's do).
+    for (bool left = !ok; left;) {
+      const int bh = p.bh0 + q.bh, b = bh / p.Hkv, h = bh - b * p.Hkv, tn = (q.m * p.streams + s) * p.P + pl;
+      if (q.head && q.tail && pl < p.P && tn < p.Tq) {
+        const int64_t oo = (int64_t)b * p.os_b + (int64_t)(h * p.G + gh) * p.os_h + (int64_t)tn * p.os_t;
+#pragma unroll 1
+        for (int x = 0; x < D; ++x) store_float(p.O, oo + x, NAN, p.o_dtype);
+      }
+      left = more;
+      q = nq;
+      if (left) more = it.next(p, nq);
     }
   }
   }
@@ -836,11 +851,11 @@ __global__ void __launch_bounds__(256, 4) prefill_expand_kernel(const ExpandPara
   pf_scale_of(big, mul, inv);
   if (blockIdx.x == 0 && threadIdx.x == 0) (is_v ? e.vmul : e.kmul)[bh] = is_v ? inv : inv * e.qscale;
   if (bulk) {
-    // (every thread waits: a CTA must not exit with a copy into it in flight.  Bounded; a table that never came reads as it is,
-    //  and the attention kernel's status word is raised.)
+    // (every thread waits: a CTA must not exit with a copy into it in flight.  Bounded: whoever goes on without the table raises the
+    //  status word, and the rows of the whole call become NaN, see prefill_attn_kernel.)
     uint32_t spins = 0;
     while (!mbar_try_wait(bar, 0)) {
-      if (++spins > kWaitLimit) { if (threadIdx.x == 0) *e.status = e.epoch; break; }
+      if (++spins > kWaitLimit) { *e.status = e.epoch; break; }
     }
   }
 

@@ -270,7 +270,8 @@ int hqmq_med3x_select(int H, int level, uint64_t n_total, float median_mult, voi
  *                                   calls with a threshold of their own)
  *   workspace of hqmq_attn_decode:  non-zero = some call on this workspace gave up on a bounded wait
  *                                   for a staged copy; the output rows of that call are not valid (NaN where
- *                                   a merge still ran, untouched elsewhere)
+ *                                   a merge still ran, and from HQMQ_ATTN_PROMPT_QUERIES query positions on in
+ *                                   every row concerned; untouched elsewhere)
  * No counterpart in the reference (its kernels have no device-side status).
  */
 int hqmq_read_status(const void* workspace, uint32_t* status, void* stream);

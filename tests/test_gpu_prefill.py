@@ -1,6 +1,9 @@
 """Attention of many query positions (tensor-core path) against a plain fp32 evaluation of the same operation on the
 dense reconstruction: edges of the 128-token tiles and of the row blocks, ragged groups, every mask, units cut between CTAs."""
 import math
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -209,3 +212,33 @@ def test_many_prompts_of_one_tile(B, Hq, Hkv, d, T, causal):
         same = torch.full_like(O, float("nan"))
         hqmq.fused_attention_packed(queries, *packed, *tabs, causal=causal, out=same)
         assert torch.equal(same, O)
+
+
+_LOST_CALL = '''
+import torch
+import hqmq_b200 as hqmq
+from hqmq_b200 import _lib
+L, calls, lost = _lib.lib(), 0, 0
+real = L.hqmq_attn_decode
+def attn_decode(a, ws, nbytes, st):
+    # the calls of a process are numbered from 0x5eed0001
+    global calls
+    calls += 1
+    held = torch.zeros((nbytes + 3) // 4, dtype=torch.int32, device="cuda")
+    held[0] = 0x5eed0000 + calls - 1 + lost
+    return real(a, held.data_ptr(), nbytes, st)
+L.hqmq_attn_decode = attn_decode
+for B, Hq, T, Tq in ((2, 4, 80, 80), (20, 32, 300, 40), (1, 8, 3000, 64)):
+    q = hqmq.HQMQ(1, 2, 96, 4, device="cuda")
+    packed = [q.encode(torch.randn(B, 2, T, 128, device="cuda").bfloat16(), 0, kv) for kv in (0, 1)]
+    tabs = [q.tables(0, kv, "cuda")["table16"] for kv in (0, 1)]
+    for lost in (1, 0):
+        O = hqmq.fused_attention_packed(torch.randn(B, Hq, Tq, 128, device="cuda").half(), *packed, *tabs, causal="bottom_right")
+        assert (O.isnan() if lost else O.isfinite()).all(), (B, T, lost)
+'''
+
+
+def test_call_whose_expansion_gave_up_is_all_nan():
+    """The status word of a call, raised ahead of the attention kernel as the expansion does when it goes on without a codeword
+    table: every row is NaN, of units that one CTA does whole and of those that are merged.  The word of another call does nothing."""
+    subprocess.run([sys.executable, "-c", _LOST_CALL], check=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
