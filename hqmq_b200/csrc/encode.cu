@@ -2197,6 +2197,15 @@ static bool bracket_call(const hqmq_encode_args* a) {
   return bracket_wanted(*a) && common_layout(a) && fused_call(a) && ((uintptr_t)a->x & 15) == 0 && a->x_stride[0] % 8 == 0 && a->x_stride[1] % 8 == 0 &&
          a->x_stride[2] % 8 == 0;
 }
+// Whether the dense tensor of a call (16-bit values) shares memory with what the call reads of x.
+static bool overlaps_x(const hqmq_encode_args* a, const void* out) {
+  const hqmq_packed& d = a->dst;
+  const int64_t last[3] = {d.B - 1, d.H - 1, (int64_t)a->T_new - 1};
+  int64_t lo = 0, hi = 4 * (int64_t)d.n_chunks;
+  for (int i = 0; i < 3; ++i) (a->x_stride[i] < 0 ? lo : hi) += last[i] * a->x_stride[i];
+  const uintptr_t x = (uintptr_t)a->x, o = (uintptr_t)out;
+  return o < x + 2 * hi && x + 2 * lo < o + 2 * ((int64_t)d.B * d.H * a->T_new * d.n_chunks * 4);
+}
 static void fill_fused(const hqmq_encode_args* a, int tensors, uint32_t* status, uint32_t* hist, uint32_t* bars, void* out, uint32_t* n_flagged,
                        FusedArgs& f) {
   const hqmq_packed& d = a->dst;
@@ -2209,6 +2218,7 @@ static void fill_fused(const hqmq_encode_args* a, int tensors, uint32_t* status,
   // (the near-ties of the generic kernels, which divide with the rounded reciprocal, are kept where those used to run: other
   //  field widths, 64-wide tokens outside the paired geometry)
   f.rcp_rn = !common_layout(a) || (d.n_chunks == 16 && !(pair16_of(*a) && ((uintptr_t)a->x & 15) == 0 && a->x_stride[0] % 8 == 0 && a->x_stride[1] % 8 == 0));
+  f.early = out && overlaps_x(a, out) ? 0 : kFusedEarly;
   // one CTA per SM in all, no fewer than a round of its warps each
   const int64_t W = (int64_t)d.B * (d.n_chunks == 16 ? (a->T_new + 1) / 2 : a->T_new);
   int64_t cph = sm_count() / (tensors * d.H);

@@ -10,6 +10,7 @@
 // slots of the search, then what happens once: 57 k clocks of a 4096-token call of 8 heads (fake-quant, s24) are 27 k of search, 7 k
 // until the norms are there, three levels of about 1500 for the histogram, 1800 for its sum, 1400 to see the others' and 1700 to
 // scan.  K and V: 75.0 -> 69.8 us, 63.8 with the shorter search.
+constexpr int kFusedEarly = 3;                // rounds of tokens encoded between the levels, see below
 struct FusedArgs {
   // (what a CTA needs first lies together: a line of the parameters that is not in the constant cache costs some 500 clocks)
   EncGeom g;                  // the call's own geometry: n = 32 chunks per token, or 16 (two tokens per warp)
@@ -31,6 +32,7 @@ struct FusedArgs {
   hqmq_packed dst;            // packed rows (DENSE = false)
   int t_start;
   int rcp_rn;                 // directions are normalised with the rounded reciprocal (as the generic passes do)
+  int early;                  // rounds of tokens that may be written ahead of the threshold: kFusedEarly, 0 where out overlaps x
 };
 struct FusedPair { FusedArgs t[2]; };            // blockIdx.y: the tensor (K and V of a layer in one launch, or one tensor)
 constexpr uint32_t kFusedPolls = 1u << 20;       // about a second
@@ -99,7 +101,6 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
   // them again: 4.6 us of load latency and norm arithmetic a level).  Eight tokens a warp are 4096 tokens of 8 heads; what is beyond
   // is read again, which the call's time does not show.  They are on their way before anything else.
   constexpr int kKeep = 8;
-  constexpr int kEarly = 3;                    // rounds of tokens encoded between the levels, see below
   uint32_t keys[kKeep];                        // bits of the norms; 0xffffffff, which no prefix equals: no token
   const bool select = a.C > 0.f && !a.med_in;
   uint2 first[kKeep];
@@ -231,12 +232,13 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
   // Between a level's arrival and its wait a warp encodes a token as if nothing were flagged (a round of tokens takes 3600 to 4000
   // clocks, the wait would take about 2000); once the threshold is known the flagged chunks of those are put right, 650 clocks a
   // token, and the other tokens are encoded with it.  (All eight kept tokens ahead of the threshold: the last step alone 4400.)
+  // Putting right reads x again: a dense tensor that is written over its own x has no token encoded ahead.
   bool usable = true;
   if (select) {
     const QRank qr = quantile_rank((uint64_t)g.B * g.T_new * g.n, a.quantile);
 #pragma unroll
     for (int u = 0; u < kKeep; ++u) keys[u] |= __float_as_uint(norm_of(first[u]));
-    const int early = min(kEarly, (w1 - w0 + kEnc32Warps - 1) / kEnc32Warps);      // rounds of the warps
+    const int early = min(a.early, (w1 - w0 + kEnc32Warps - 1) / kEnc32Warps);      // rounds of the warps
     uint32_t p0 = 0u, p1 = 0u, k0 = (uint32_t)qr.lo, k1 = (uint32_t)qr.hi;      // prefixes and ranks of the two statistics
 #pragma unroll 1
     for (int level = 0; level < 3; ++level) {
@@ -325,15 +327,15 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
     thr = __fmul_rn(med, a.C);
     if (part == 0 && threadIdx.x == 0 && a.med_out) a.med_out[h] = med;
     // the flagged chunks of the tokens encoded ahead
-    if (usable && !s_gave_up) {
+    if (usable && !s_gave_up && early) {
       // (what is read first, for all of them, then what is written: one by one the eight took 4000 clocks)
-      uint2 was[DENSE ? kEarly : 1];
-      uint16_t code[DENSE ? 1 : kEarly];
+      uint2 was[DENSE ? kFusedEarly : 1];
+      uint16_t code[DENSE ? 1 : kFusedEarly];
       Place at = place_of(min(w0 + warp, W - 1));
       const Place at0 = at;
       if constexpr (!DENSE) __syncwarp();        // (the rows were stored by other lanes)
 #pragma unroll
-      for (int u = 0; u < kEarly; ++u) {
+      for (int u = 0; u < kFusedEarly; ++u) {
         if (keys[u] != 0xffffffffu && __uint_as_float(keys[u]) > thr) {
           if constexpr (DENSE) was[u] = *reinterpret_cast<const uint2*>(at.x);
           else if (CB == 16) code[u] = reinterpret_cast<const uint16_t*>(a.dst.codes + at.row * a.dst.row_bytes)[c];
@@ -342,7 +344,7 @@ __global__ void __launch_bounds__(kEnc32Threads, 1) encode_fused_kernel(const Fu
       }
       at = at0;
 #pragma unroll
-      for (int u = 0; u < kEarly; ++u) {
+      for (int u = 0; u < kFusedEarly; ++u) {
         const bool flagged = keys[u] != 0xffffffffu && __uint_as_float(keys[u]) > thr;
         const uint32_t word = __ballot_sync(0xffffffffu, flagged);
         n_fl += __popc(word);

@@ -216,7 +216,8 @@ int hqmq_encode(const hqmq_encode_args* args, void* workspace, size_t workspace_
  * The dense fake-quantised tensor straight from x: what hqmq_encode followed by hqmq_dequant(layout 0, scale_first,
  * merge_outliers) gives on an fp32 scale plane, bit for bit, without the planes in between.  Of args->dst only the geometry
  * (B, H, n_chunks, S, radius_bits) is read; t_start must be 0.  out: (B, H, T_new, 4 n_chunks) contiguous, element type of
- * x, 16-byte aligned.  n_flagged (may be NULL): device uint32 that the call's flagged chunks are added to.
+ * x, 16-byte aligned; it may be x itself where x is contiguous, and shares no memory with x otherwise.  n_flagged (may be NULL):
+ * device uint32 that the call's flagged chunks are added to.
  * HQMQ_ERR_UNSUPPORTED for the calls that only the two-step route takes (workspace size 0): more than a small call in fp32,
  * without a look-up table, or in a geometry other than 32 chunks per token (16 with 16-bit fields).
  */

@@ -7,6 +7,7 @@ import pytest
 import torch
 
 import hqmq_b200 as hqmq
+from hqmq_b200 import _lib
 from oracle import hqmq_oracle as orc
 from tests.util import classify_idx, load_npz, make_kv
 
@@ -575,3 +576,16 @@ def test_one_launch_encoder_places(shape, S, br):
     more tokens than they encode ahead of the threshold."""
     test_one_launch_encoder(shape, S, br, 3.0, False)
     test_one_launch_encoder(shape, S, br, 3.0, True)
+
+
+@pytest.mark.parametrize("shape,S,br", [((1, 2, 97, 128), 24, 3), ((1, 8, 4096, 128), 24, 3), ((3, 3, 1001, 128), 192, 6), ((2, 8, 777, 64), 96, 4),
+                                        ((16, 2, 1, 128), 96, 4)])
+@pytest.mark.parametrize("C", [None, 3.0])
+def test_fake_quant_over_its_own_input(shape, S, br, C):
+    """The dense tensor may take the place of x: a flagged chunk keeps its values there too."""
+    q = hqmq.HQMQ(1, shape[1], S, br, device="cuda")
+    x = make_kv("hot" if shape[3] == 128 else "spiky", shape, seed=7, dtype=torch.bfloat16).cuda()
+    want = q._qdq(x, 0, 0, median_mult=C)
+    a, ref, ws, ws_ptr, nbytes = q._fake_quant_args(x, 0, 0, C, None)
+    assert _lib.lib().hqmq_fake_quant(ref, x.data_ptr(), None, ws_ptr, nbytes, _lib.stream_ptr()) == 0
+    assert torch.equal(x, want)
