@@ -46,13 +46,13 @@ constexpr int kUndCap = 4096;     // undecided chunks listed per head at least; 
 // and S = 96 a list holds 1.9 codewords on average (8 at most) and 98 % of the lists are one group.
 constexpr int kLutNMax = 48;
 constexpr int kLutRows = kLutNMax * kLutNMax;
-constexpr int kLutCellCap = 24576;          // stored cells (23.4 k at n = 48)
+constexpr int kLutCellCap = 24576;          // stored cells (23.4 k at n = 48), and the one that rows without cells point at
 constexpr int kLutCandCap = 65528;          // candidate entries per head (list offsets / 4 are 15-bit cell words; every head's part a multiple of 16 bytes)
 constexpr int kLutMaxList = 16;             // longest list a cell may have; longer -> exhaustive search there
 constexpr float kLutBoxEps = 1e-5f;         // the boxes are grown by this much (cell assignment rounding)
 constexpr float kLutMargin = 1e-5f;         // a codeword is dropped only if it loses by more than this
 // device layout of a table (bytes): global header {n, n_cells, ...} | rows[kLutRows] uint32 = first cell (16 bits) |
-// first stored cz (8; kLutNoCells: none) | stored cells of the row - 1 (8) | per head: {total candidates, valid, -, -} uint32, then
+// first stored cz (8; kLutNoCells: none, and the first cell is the last of all, 0xFFFF) | stored cells of the row - 1 (8) | per head: {total candidates, valid, -, -} uint32, then
 // cells[kLutCellCap] uint16 (0xFFFF: exhaustive; bit 15: the single winner in bits 0..14; else list offset / 4),
 // cands[kLutCandCap] uint16 (lists of a multiple of four entries; bit 15 of a list's first entry: there are at most four codewords,
 // else bit 15 marks the last one) | Mul24Both
@@ -217,8 +217,10 @@ __device__ __forceinline__ bool search_fold24(const float4* __restrict__ joint, 
   const float v3 = half ? h3 : __uint_as_float(e3 ^ neg ^ f3);
   const uint32_t signs = __funnelshift_l(b3, __funnelshift_l(b2, __funnelshift_l(b1, b0 >> 31, 1), 1), 1);
   const uint32_t gp = half ? 8u + signs : (w ? 4u : 0u) + (o ? 2u : 0u) + (neg >> 31);
-  // cell coordinates as the low bits of floats of 2^23 and more, rounded down; what is in no cell (it would have to be no direction)
-  // is clamped once, for memory's sake
+  // Cell coordinates as the low bits of floats of 2^23 and more, rounded down; clamped once, for memory's sake.  A row without cells
+  // has one that sends the chunk to the other search.  A cz outside its row's cells would be taken for the last of them, and none
+  // is: a folded direction lies in the octahedron but for its roundings (the sums, the approximate reciprocal and the product, less
+  // than 1e-6 of a coordinate) and the shrunk scale's 4e-6, and the cells are those whose boxes, grown by 1e-5, meet it.
   const float inv = rcp_approx(v0) * L.hn;
   const uint32_t cx = __float_as_uint(__fmaf_rd(v1, inv, L.off)), cy = __float_as_uint(__fmaf_rd(v2, inv, L.off)),
                  cz = __float_as_uint(__fmaf_rd(v3, inv, L.off));
@@ -1700,12 +1702,13 @@ __global__ void __launch_bounds__(1024) lut_rows_kernel(int n, uint32_t* __restr
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t run = 0;
+    uint32_t run = 0, all = 0;
+    for (int col = 0; col < n * n; ++col) all += s_cnt[col];
     for (int col = 0; col < n * n; ++col) {
-      rows[col] = s_cnt[col] ? run | (s_min[col] << 16) | ((s_cnt[col] - 1u) << 24) : kLutNoCells << 16;
+      rows[col] = s_cnt[col] ? run | (s_min[col] << 16) | ((s_cnt[col] - 1u) << 24) : all | (kLutNoCells << 16);
       run += s_cnt[col];
     }
-    ghdr[0] = (uint32_t)n; ghdr[1] = run; ghdr[2] = ghdr[3] = 0u;
+    ghdr[0] = (uint32_t)n; ghdr[1] = all + 1u; ghdr[2] = ghdr[3] = 0u;
   }
 }
 
@@ -1812,9 +1815,10 @@ lut_pack_kernel(const uint16_t* __restrict__ tmp, const uint32_t* __restrict__ c
   uint16_t* cands = reinterpret_cast<uint16_t*>(head + 16 + (size_t)kLutCellCap * 2);
   const int per = (n_cells + 1023) / 1024;
   const int c0 = threadIdx.x * per, c1 = min(n_cells, c0 + per);
+  auto length = [&](int c) { return c == n_cells - 1 ? 0u : cnt[(int64_t)h * kLutCellCap + c]; };      // (the last: of rows without cells)
   uint32_t tot = 0;
   for (int c = c0; c < c1; ++c) {
-    const uint32_t m = cnt[(int64_t)h * kLutCellCap + c];
+    const uint32_t m = length(c);
     tot += m > 1 ? (m + 3u) & ~3u : 0u;
   }
   s_sum[threadIdx.x] = tot;
@@ -1834,7 +1838,7 @@ lut_pack_kernel(const uint16_t* __restrict__ tmp, const uint32_t* __restrict__ c
   if (!valid) return;
   uint32_t run = s_sum[threadIdx.x] - tot;
   for (int c = c0; c < c1; ++c) {
-    const uint32_t m = cnt[(int64_t)h * kLutCellCap + c];
+    const uint32_t m = length(c);
     const uint16_t* src = tmp + ((int64_t)h * kLutCellCap + c) * kLutMaxList;
     if (m == 0) cells[c] = 0xffffu;
     else if (m == 1) cells[c] = (uint16_t)(0x8000u | src[0]);

@@ -589,3 +589,41 @@ def test_fake_quant_over_its_own_input(shape, S, br, C):
     a, ref, ws, ws_ptr, nbytes = q._fake_quant_args(x, 0, 0, C, None)
     assert _lib.lib().hqmq_fake_quant(ref, x.data_ptr(), None, ws_ptr, nbytes, _lib.stream_ptr()) == 0
     assert torch.equal(x, want)
+
+
+@pytest.mark.parametrize("S", [24, 96, 192, 256, 300])
+def test_table_rows_without_cells_and_directions_on_every_edge(S):
+    """Rows of the look-up table that hold no cell name one that takes the exhaustive search.  Directions on the faces, edges and corners
+    of the octahedron that the table covers, in every image of it, and a rounding to either side: the codeword is one of the nearest."""
+    q = hqmq.HQMQ(1, 1, S, 4, device="cuda")
+    tb = q.tables(0, 0, "cuda")
+    raw = tb["lut"].cpu().numpy()
+    n, n_cells = (int(v) for v in raw[:8].view(np.uint32))
+    rows = raw[32:32 + 4 * n * n].view(np.uint32)
+    cells = raw[32 + 4 * 48 * 48 + 16:][:2 * n_cells].view(np.uint16)
+    none = (rows >> 16 & 255) == 255
+    assert none.any() and (cells[rows[none] & 0xffff] == 0xffff).all()
+    held = (rows[~none] >> 24) + 1
+    assert held.sum() == n_cells - 1 and ((rows[~none] & 0xffff) + held <= n_cells - 1).all()
+
+    g = torch.Generator().manual_seed(5)
+    w = torch.rand(60, 3, generator=g, dtype=torch.float64)
+    w[:20, 2] = 0.0                                               # edges
+    w[20:23] = torch.eye(3, dtype=torch.float64)                  # corners
+    w[23] = torch.tensor([0.5, 0.5, 0.0], dtype=torch.float64)
+    w[24] = 1 / 3
+    w /= w.sum(1, keepdim=True)                                   # faces, the others
+    signs = torch.tensor([[1 - 2 * (i >> k & 1) for k in range(3)] for i in range(8)], dtype=torch.float64)
+    v = torch.cat([torch.ones(480, 1, dtype=torch.float64), (w[:, None] * signs).reshape(480, 3)], 1)
+    units = orc.joint_codebook(torch.tensor([[[1.0, 0.0, 0.0, 0.0]]]))[0].double()            # the 24 units themselves
+    x = orc.quat_mul(units[:, None], v[None]).reshape(-1, 4).repeat(3, 1).float()
+    x *= 1 + torch.randint(-1, 2, x.shape, generator=g) * 2.0 ** -23
+    x *= torch.exp(torch.randn(len(x), 1, generator=g))
+    x = x.reshape(1, 1, -1, 128)
+    joint = tb["joint"][0].double()
+    for dtype in (torch.float32, torch.float16, torch.bfloat16):
+        xd = x.to(dtype).cuda()
+        idx = q.encode(xd, 0, 0).to_reference()[0].long().flatten()
+        u = xd.double().reshape(-1, 4)
+        sims = u / u.norm(dim=1, keepdim=True) @ joint.T
+        assert (sims.max(1).values - sims.gather(1, idx[:, None])[:, 0]).max() < NEAR_TIE
