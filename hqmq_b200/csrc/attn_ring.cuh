@@ -14,14 +14,15 @@
 // replicas as shared memory allows.
 // Fields of 13 bits (s24_r3) have a table of DECODED values for V, codeword times radius code for all 8192 fields, 64 KB without
 // replicas: a chunk of V is then a shift, a mask and the look-up (3 instructions instead of 15 for index, radius, sign and two
-// multiplies), at 6 wavefronts a gather instead of 3.  That kernel is bound by instructions (1075 a tile) with the shared-memory
-// pipe at a third; with both tensors decoded it is bound by the pipe (272 wavefronts, 744 instructions a tile).  One sequence of
-// 131072 tokens, 8 heads, spikes: neither 109.3 us, K 109.5, both 110, V 106.3 (105.1 with a third stage).
+// multiplies), at 6 wavefronts a gather instead of 3.  With neither tensor decoded instructions bind (1075 a tile, the shared-memory
+// pipe at a third); with both, 744 instructions and 272 wavefronts a tile, neither pipe is full and the chain of a tile binds.  One
+// sequence of 131072 tokens, 8 heads, spikes: neither 109.3 us, K 109.5, both 110, V 106.3 (105.1 with a third stage).
 // Outliers: a tile of K that owns fragment records adds them with one shared-memory load and one MMA per
-// record; every other flagged chunk (K tiles without records, all of V) is corrected in fp32 on the CUDA cores,
-// one warp-wide step per flagged chunk, from the staged payload slice: its decoded value is 0 (radius code 0),
-// so the correction is purely additive.  V tiles of d_head 64 whose flagged chunks fill a few chunk columns (an
-// outlier channel) add them column by column with two MMAs each instead.
+// record; every other flagged chunk (K tiles without records, all of V) is corrected in fp32 on the CUDA cores
+// from the staged payload slice: its decoded value is 0 (radius code 0), so the correction is purely additive.  K takes
+// a warp-wide step per flagged chunk; V at d_head 128 a step per flagged chunk of the fullest row of lanes where rows share
+// the steps, else one per chunk; V tiles of d_head 64 whose flagged chunks fill a few chunk columns (an outlier channel) add
+// them column by column with two MMAs each, the others take a step per chunk.
 // The arithmetic of the tile (fragment layouts, online softmax) is the one described in attn_kernel.cuh.
 #pragma once
 #include "attn_tma.cuh"
@@ -683,8 +684,8 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
             // lanes that own the column's rows of V^T collect their tokens' values by shuffles, and two MMAs with the
             // tile's P add the column to the output.  About 45 warp instructions per column, whatever it holds; the
             // per-chunk fp32 step below costs about 25 per flagged chunk and stays the path of scattered outliers.
-            // (compiled for d_head 64 only, like its predecessor, a patch of the decoded fragments inside the V loop:
-            //  in the d_head 128 kernels any addition to the tile costs registers that the common path needs)
+            // (compiled for d_head 64 only, like its predecessor, a patch of the decoded fragments inside the V loop: the
+            //  d_head 128 kernels use all of their 128 registers, and each walk more in their tile costs 1 to 2 %)
             bool by_column = false;
             if constexpr (N == 16) {
               const uint32_t cnt = th0.w - th0.z;
@@ -748,10 +749,16 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
                 }
               }
             }
+            bool side_by_side = N == 32;
             if constexpr (N == 32) {
               // The four lanes of a row r own its NVG chunk columns; the eight rows take their flagged chunks side by side, each by
               // token (the order every element is summed in) and column.  (One flagged chunk after another, all lanes together, took
-              // 650 clocks each, a third of a tile with two or three spikes.)
+              // 650 clocks each, a third of a tile with two or three spikes.)  A step of this walk is the dearer one, so it pays where
+              // rows share the steps: the steps are the fullest row's chunks.  An outlier channel fills one row, and two channels may share
+              // one.  8 x 32768 tokens, V as named, always side by side / by this rule / always one after another, us: one channel, s96
+              // 517 / 425 / 432, s24 521 / 438 / 457, s192 549 / 463 / 466; four channels 675 / 642 / 669; two channels of one row (s96)
+              // 906 / 649 / 660; spikes 169 / 171 / 186.  (Under eight chunks it is not worth finding out.  The other walk's presence costs
+              // 1 to 2 % of a call of spikes; it is not compiled for fp32 side buffers here.)
               static_assert(NVG <= 4, "sixteen tokens of a row's columns are 64 bits");
               const uint32_t ex = excl_scan16(__popc(fw), lane);           // lanes 0..15: entries of the tile's earlier tokens
               uint64_t left;
@@ -766,7 +773,9 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
                 left = j < 2 ? (uint64_t)v | ((uint64_t)o_ << 32) : (uint64_t)o_ | ((uint64_t)v << 32);
                 if constexpr (EDGE) { if (t0 + kTile > t_end) left &= (1ull << (4 * (t_end - t0))) - 1ull; }
               }
-              while (__any_sync(0xffffffffu, left != 0ull)) {
+              const uint32_t cnt = th0.w - th0.z;
+              side_by_side = p.V.out_dtype == HQMQ_F32 || cnt < 8u || 2u * __reduce_max_sync(0xffffffffu, (uint32_t)__popcll(left)) <= cnt;
+              if (side_by_side) while (__any_sync(0xffffffffu, left != 0ull)) {
                 const bool act = left != 0ull;
                 const int at = act ? __ffsll((long long)left) - 1 : 0, t = at >> 2, g = at & 3, c = r * NVG + g;
                 left &= left - 1ull;
@@ -801,7 +810,8 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
                   }
                 });
               }
-            } else if (!by_column) {
+            }
+            if (!by_column && !side_by_side) {
             uint32_t tm = __ballot_sync(0xffffffffu, fw != 0u);
             uint32_t e = th0.z;
             while (tm) {
@@ -817,7 +827,7 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
                 w &= w - 1;
                 float x0 = 0.f, x1 = 0.f, x2 = 0.f, x3 = 0.f;
                 if (e < (uint32_t)p.V.out_cap) {
-                  if (p.V.out_dtype == HQMQ_F32) {
+                  if (N == 16 && p.V.out_dtype == HQMQ_F32) {
                     const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.V.out_vals) + (bh * p.V.out_cap + e) * 4);
                     x0 = v.x; x1 = v.y; x2 = v.z; x3 = v.w;
                   } else {
@@ -842,7 +852,7 @@ __device__ __forceinline__ void attn_ring_body(const AttnParams& p) {
                 ++e;
               }
             }
-            }   // !by_column
+            }   // !by_column && !side_by_side
           }
         }
         };   // tile_body

@@ -263,3 +263,29 @@ def test_ring_decode_spikes_everywhere(S, br, T):
     # of their sizes, every weight by that share of itself, numerator and normaliser alike; P is one fp16 rounding in both.
     share = 2.0 ** -10 * (1.0 + (Qf.abs() @ Kd.abs().transpose(-1, -2)).amax(-1, keepdim=True) / math.sqrt(d))
     assert ((out - want).abs() <= 1e-4 + 2.0 * share * size).all() and rel_l2(out, want) < MAX_ABS
+
+
+@pytest.mark.parametrize("S,br", [(24, 3), (96, 4), (192, 6)])
+@pytest.mark.parametrize("channels", [(9,), (16, 20), (1, 33, 66, 127)])
+@pytest.mark.parametrize("rate", [0.3, 0.45, 0.6, 1.0])
+def test_ring_decode_value_channels_at_head_dim_128(S, br, channels, rate):
+    """Values whose flagged chunks lie in one chunk column, in two columns of one row of lanes, or in rows of their own, as often as
+    puts tiles on either side of what decides how they are added; against the fp32 evaluation."""
+    B, Hq, Hkv, d, T = 2, 32, 8, 128, 15993
+    q = hqmq.HQMQ(1, Hkv, S, br, device="cuda")
+    gen = torch.Generator().manual_seed(6)
+    K, V = (torch.randn(B, Hkv, T, d, generator=gen).cuda() for _ in range(2))
+    for c in channels:
+        at = (torch.rand(B, Hkv, T, generator=gen) < rate).cuda()
+        V[..., 4 * (c // 4)][at] = 40.0 * V[..., 4 * (c // 4)][at].sign()
+    Kp, Vp = (q.encode(x.bfloat16(), 0, kv, median_mult=3.0) for kv, x in enumerate((K, V)))
+    tk, tv = q.tables(0, 0, "cuda"), q.tables(0, 1, "cuda")
+    Q = (torch.randn(B, Hq, 1, d, generator=gen) / math.sqrt(d)).cuda().half()
+    out = torch.empty(B, Hq, 1, d, device="cuda")
+    hqmq.fused_attention_packed(Q, Kp, Vp, tk["table16"], tv["table16"], out=out)
+    Kd, Vd = q.decode(Kp, 0, 0).repeat_interleave(Hq // Hkv, 1), q.decode(Vp, 0, 1).repeat_interleave(Hq // Hkv, 1)
+    p = torch.softmax((Q.float() @ Kd.transpose(-1, -2)) / math.sqrt(d), -1)
+    want, size = p @ Vd, p @ Vd.abs()
+    # (the bound of the test above)
+    share = 2.0 ** -10 * (1.0 + (Q.float().abs() @ Kd.abs().transpose(-1, -2)).amax(-1, keepdim=True) / math.sqrt(d))
+    assert ((out - want).abs() <= 1e-4 + 2.0 * share * size).all()
