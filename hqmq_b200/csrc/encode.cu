@@ -42,8 +42,9 @@ constexpr int kUndCap = 4096;     // undecided chunks listed per head at least; 
 // winner at the cell's centre, minus those beaten over the whole cell by another listed one -- the comparison of
 // two codewords is linear in w, so its extreme over the box is at a corner.  A cell with ONE possible winner stores
 // it in its own word (no similarity is evaluated at all); the others point at a list, padded to a multiple of four,
-// which is evaluated with the same fp32 dot product an exhaustive scan of the joint table would use.  At n = 48
-// and S = 96 a list holds 1.9 codewords on average (8 at most) and 98 % of the lists are one group.
+// which is evaluated with the same fp32 dot product an exhaustive scan of the joint table would use.  At S = 96
+// (n = 44) 39 % of the cells have one winner; a list holds 2.7 codewords on average (11 at most) and 5 % are longer than four.  S = 24
+// (n = 48): 60 %, 2.3, 1 %; S = 192 (n = 36): 20 %, 3.2, 15 %.
 constexpr int kLutNMax = 48;
 constexpr int kLutRows = kLutNMax * kLutNMax;
 constexpr int kLutCellCap = 24576;          // stored cells (23.4 k at n = 48), and the one that rows without cells point at
@@ -1923,8 +1924,8 @@ static bool pair16_of(const hqmq_encode_args& a) {
 // and quantiles out in the tails (few norms nearby: a much larger error), take the one-launch encoder.
 // 65536 tokens are where 1.2 % still holds six standard errors.  One read / one launch, us a tensor, s96, 8 heads of 128 with some
 // flagged: 65536 tokens a head 328 / 392, 98304 436 / 570, 131072 535 / 749 (s24, none flagged: 65536 304 / 351; four heads, s192:
-// 331 / 353; heads of 64: 131072 326 / 432).  Below the line the one read is the shorter by little (32768: 201 / 208, 49152: 272 / 306;
-// four heads 230 / 223; 16384: 139 / 125), and its bracket would hold four standard errors, three at 16384.
+// 331 / 353; heads of 64: 131072 326 / 432).  Below the line the one read is the shorter by little for 8 heads (32768: 201 / 208, 49152:
+// 272 / 306) and the longer for four (230 / 223) and at 16384 (139 / 125); its bracket would hold four standard errors, three at 16384.
 constexpr int64_t kBracketMinTokens = 65536;     // B * T_new per head (of 32 chunks each)
 static bool bracket_wanted(const hqmq_encode_args& a) {
   const bool pair = pair16_of(a);
