@@ -253,8 +253,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attn_kernel(const Prefi
           if (g >= NS && !wait(kempty + 8 * st, ph ^ 1u)) { ok = false; break; }
           mbar_expect_tx(kfull + 8 * st, TB);
           bulk_g2s(sK + st * TB, kp + (int64_t)i * TB, TB, kfull + 8 * st);
-          // (all CTAs start at once, and the first S wants a tile of K and the queries: what is needed later waits for those, which is
-          //  worth 0.1 to 0.6 % of a call, 2.6 of a causal prompt of 500, and costs 4 x 500 with heads of 64 0.3.  Only
+          // (all CTAs start at once, and the first S wants a tile of K and the queries: what is needed later waits for those.  Only
           //  where the piece has a second tile: its K is issued behind this wait, so no stream gets to its next queries before.  Of a
           //  piece of one tile a stream does without V, its barrier is then two phases on, and this wait would never end.)
           if (g == 0 && q.n > 1) { wait(qfull, 0u); if (p.streams > 1) wait(qfull + 8, 0u); }
@@ -1049,12 +1048,9 @@ int prefill_launch(const hqmq_attn_args* a, const PrefillPlan& pl, void* workspa
         p.start_m[c] = m; p.start_off[c] = (int)(pos - at);
       }
     }
-    // Tiles per expand CTA: four CTAs per SM in all, as many as are resident at a time, so that a CTA's table and scale scan serve
-    // several tiles of a long cache.  Four / six / eight / twelve per SM, us a call: 16 queries over 65536 keys of 8 heads 176 / 199 /
-    // 181 / 187, 4 x 64 over 16384 192 / 203 / 193 / 193, 16 x 32 over 2000 89 / 92 / 86 / 90, 64 over 8192 47.4 / 47.4 / 49.3 / 49.3,
-    // 2048 over 8192 within noise.
-    constexpr int64_t kCtas = 4 * kPfMaxCtas;
-    const int64_t per = ((int64_t)p.nt * n_bh * 2 + kCtas - 1) / kCtas;
+    // tiles per expand CTA: about six CTAs per SM in all (three at a time), so that a CTA's table and scale scan serve
+    // several tiles of a long cache
+    const int64_t per = ((int64_t)p.nt * n_bh * 2 + 6 * kPfMaxCtas - 1) / (6 * kPfMaxCtas);
     e.per = per < 1 ? 1 : per > p.nt ? p.nt : (int)per;
     void* ea[] = {&e};
     HQMQ_CHECK_CUDA(cudaLaunchKernel(ek, dim3((p.nt + e.per - 1) / e.per, n_bh, 2), dim3(256), ea, esmem, st));
